@@ -108,6 +108,7 @@ Params make_params(const gd_config& c) {
     P.hgm1 = 0.5 * (c.gamma - 1.0);
     P.g_gm1 = c.gamma / (c.gamma - 1.0);
     P.ambient_p = 1.0 / c.gamma;
+    P.gas = gd::fx::gas_of(c.gamma);
     // rad passed to the flux: dy on x-faces in the Euler kernels (kernel.cu:1811, 3562),
     // dx on x-faces in the MHD kernels (kernel.cu:2560)
     if (c.physics == GD_EULER) {
@@ -564,6 +565,7 @@ gd_status gd_probe_faces(int physics, int method, double gamma, int axis, long l
     P.inv_gm1 = 1.0 / (gamma - 1.0);
     P.hgm1 = 0.5 * (gamma - 1.0);
     P.g_gm1 = gamma / (gamma - 1.0);
+    P.gas = gd::fx::gas_of(gamma);
     const cudaStream_t st = (cudaStream_t)stream;
     GD_CUDA(physics == GD_EULER ? gd::launch_euler_face_probe(P, n, axis, L, R, flux, speed, st)
                                 : gd::launch_mhd_face_probe(P, n, axis, L, R, flux, speed, st));

@@ -44,6 +44,9 @@ namespace {
 
 constexpr int NT = 256;
 constexpr int NF = 4;
+// CTAs per SM that the shared memory of a tile shape leaves room for
+template <int TX, int TY>
+constexpr int kCtas = TX * TY > 256 ? 2 : 4;
 
 template <class T>
 struct FluxE {
@@ -212,6 +215,177 @@ __device__ __forceinline__ void store_cell(const DualOut& out, long long k, int 
     out.d.f[f][k] = x.d;
 }
 
+// The arrays of a tile in shared memory.
+template <class T, int ORDER, int TX, int TY>
+struct TileMem {
+    using S = Shape<ORDER, TX, TY>;
+    T *prim;  // [NF][SY][SX]
+    T *slx;   // [NF][TY][TX+2]   cells x in [-1, TX]
+    T *sly;   // [NF][TY+2][TX]   cells y in [-1, TY]
+    T *fx;    // [NF][TY][TX+1]   face between x-1 and x
+    T *fy;    // [NF][TY+1][TX]   face between y-1 and y
+    __device__ explicit TileMem(T* smem)
+        : prim(smem), slx(prim + S::kPrim), sly(slx + S::kSlx), fx(sly + S::kSly),
+          fy(fx + S::kFx) {}
+};
+
+// One face of a tile: faces 0 .. NFX-1 have an x normal, the rest a y normal.
+template <class T, int ORDER, int TX, int TY>
+struct Face {
+    using S = Shape<ORDER, TX, TY>;
+    static constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
+    bool isx, used;
+    int lx, ly;
+    // used: inside the grid, and next to a cell that the step updates
+    __device__ Face(const Params& P, int tx0, int ty0, int i) {
+        isx = i < NFX;
+        if (isx) {
+            ly = i / (TX + 1);
+            lx = i - ly * (TX + 1);
+            used = tx0 + lx <= P.N && ty0 + ly < P.M;
+        } else {
+            const int j = i - NFX;
+            ly = j / TX;
+            lx = j - ly * TX;
+            used = tx0 + lx < P.N && ty0 + ly <= P.M;
+        }
+        if (used && P.frozen)
+            used = cell_active(P, tx0 + (isx ? lx - 1 : lx), ty0 + (isx ? ly : ly - 1)) ||
+                   cell_active(P, tx0 + lx, ty0 + ly);
+    }
+    // the states on its low (a) and high (b) side, {rho, p, normal, tangential velocity}
+    __device__ __forceinline__ void states(const TileMem<T, ORDER, TX, TY>& t, T* qa, T* qb) const {
+        constexpr int H = S::H, SX = S::SX, SY = S::SY;
+        const T* pb = t.prim + (ly + H) * SX + (lx + H);
+        const T* pa = pb - (isx ? 1 : SX);
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            // field of the local frame's component f
+            const int g = f < 2 ? f : (isx ? f : 5 - f);
+            const T ca = pa[g * SY * SX], cb = pb[g * SY * SX];
+            if (ORDER == 2) {
+                T da, db;
+                if (isx) {
+                    da = t.slx[(g * TY + ly) * (TX + 2) + lx];
+                    db = t.slx[(g * TY + ly) * (TX + 2) + lx + 1];
+                } else {
+                    da = t.sly[(g * (TY + 2) + ly) * TX + lx];
+                    db = t.sly[(g * (TY + 2) + ly + 1) * TX + lx];
+                }
+                T a = fma(0.5, da, ca), b = fma(-0.5, db, cb);
+                if (f < 2) {  // rho, p fall back to the cell value (kernel.cu:3436-3470)
+                    a = le_zero(a) ? ca : a;
+                    b = le_zero(b) ? cb : b;
+                }
+                qa[f] = a;
+                qb[f] = b;
+            } else {
+                qa[f] = ca;
+                qb[f] = cb;
+            }
+        }
+    }
+    __device__ __forceinline__ void store(const TileMem<T, ORDER, TX, TY>& t, T m, T e, T mn,
+                                          T mt) const {
+        if (isx) {
+            T* fo = t.fx + ly * (TX + 1) + lx;
+            fo[0 * TY * (TX + 1)] = m;
+            fo[1 * TY * (TX + 1)] = e;
+            fo[2 * TY * (TX + 1)] = mn;  // x momentum
+            fo[3 * TY * (TX + 1)] = mt;  // y momentum
+        } else {
+            T* fo = t.fy + ly * TX + lx;
+            fo[0 * (TY + 1) * TX] = m;
+            fo[1 * (TY + 1) * TX] = e;
+            fo[2 * (TY + 1) * TX] = mt;  // x momentum
+            fo[3 * (TY + 1) * TX] = mn;  // y momentum
+        }
+    }
+};
+
+// The flux of one face with the solver of the step's method in floating point.
+template <class T, int ORDER, int TX, int TY>
+__device__ __forceinline__ T face_flux(const Params& P, const TileMem<T, ORDER, TX, TY>& t,
+                                       const Face<T, ORDER, TX, TY>& f) {
+    T qa[NF], qb[NF], UU;
+    f.states(t, qa, qb);
+    const FluxE<T> F =
+        P.method == GD_METHOD_HLL
+            ? hll_local(qa[0], qa[1], qa[2], qa[3], qb[0], qb[1], qb[2], qb[3], P, UU)
+            : hllc_local(qa[0], qa[1], qa[2], qa[3], qb[0], qb[1], qb[2], qb[3], P, UU);
+    f.store(t, F.m, F.e, F.mn, F.mt);
+    return UU;
+}
+
+struct Speeds {
+    double x, y;
+    __device__ __forceinline__ void take(bool isx, double UU) {
+        if (isx) x = max_nonneg(x, UU);
+        else y = max_nonneg(y, UU);
+    }
+};
+
+// Every face of a tile in floating point: the HLL method, and the tangent.
+template <class T, int ORDER, int TX, int TY>
+__device__ __noinline__ void faces_float(const Params& P, T* smem, int tx0, int ty0, Speeds& u) {
+    using F = Face<T, ORDER, TX, TY>;
+    const TileMem<T, ORDER, TX, TY> t(smem);
+    Speeds v{0.0, 0.0};
+    for (int i = threadIdx.x; i < F::NFX + F::NFY; i += NT) {
+        const F f(P, tx0, ty0, i);
+        if (f.used) v.take(f.isx, value_of(face_flux(P, t, f)));
+    }
+    u = v;
+}
+
+// The faces of a thread that the integer solver left (bit k: the k-th), in floating point.
+// Out of line, and after the loop over the faces: a call or a second solver inside it would
+// take registers from every face for what a few need.
+template <int ORDER, int TX, int TY>
+__device__ __noinline__ void faces_left(const Params& P, double* smem, int tx0, int ty0,
+                                        unsigned int left, unsigned int left_speed, Speeds& u) {
+    using F = Face<double, ORDER, TX, TY>;
+    const TileMem<double, ORDER, TX, TY> t(smem);
+    while (left) {
+        const int k = __ffs((int)left) - 1;
+        left &= left - 1;
+        const F f(P, tx0, ty0, threadIdx.x + k * NT);
+        const double UU = face_flux(P, t, f);
+        if (left_speed >> k & 1) u.take(f.isx, UU);
+    }
+}
+
+// Every face of a tile with the HLLC flux in 64-bit integers (gd_fixed.cuh): no FP64 instruction
+// but the two multiply-adds per reconstructed value.  dt_only: the wave speeds alone.
+template <int ORDER, int TX, int TY>
+__device__ __noinline__ void faces_hllc(const Params& P, double* smem, int tx0, int ty0,
+                                        int dt_only, Speeds& u) {
+    using F = Face<double, ORDER, TX, TY>;
+    const TileMem<double, ORDER, TX, TY> t(smem);
+    Speeds v{0.0, 0.0};
+    unsigned int left = 0, left_speed = 0, bit = 1;
+    for (int i = threadIdx.x; i < F::NFX + F::NFY; i += NT, bit <<= 1) {
+        const F f(P, tx0, ty0, i);
+        if (!f.used) continue;
+        double qa[NF], qb[NF], UU;
+        f.states(t, qa, qb);
+        const fx::Fan fan =
+            fx::fan_of(qa[0], qa[1], qa[2], qa[3], qb[0], qb[1], qb[2], qb[3], P.gas, UU);
+        if (!fan.ok) {
+            left |= bit;
+            left_speed |= bit;
+            continue;
+        }
+        v.take(f.isx, UU);
+        if (dt_only) continue;
+        double m, mn, mt, e;
+        if (fx::hllc(fan, qa[3], qb[3], P.gas, m, mn, mt, e)) f.store(t, m, e, mn, mt);
+        else left |= bit;
+    }
+    if (left) faces_left<ORDER, TX, TY>(P, smem, tx0, ty0, left, left_speed, v);
+    u = v;
+}
+
 struct TileResult {
     double umax_x, umax_y;
     bool any_active;
@@ -231,11 +405,8 @@ __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT
                                         TileResult& res, double* aux) {
     using S = Shape<ORDER, TX, TY>;
     constexpr int H = S::H, SX = S::SX, SY = S::SY;
-    T* prim = smem;                 // [NF][SY][SX]
-    T* slx = prim + S::kPrim;       // [NF][TY][TX+2]   cells x in [-1, TX]
-    T* sly = slx + S::kSlx;         // [NF][TY+2][TX]   cells y in [-1, TY]
-    T* fx = sly + S::kSly;          // [NF][TY][TX+1]   face between x-1 and x
-    T* fy = fx + S::kFx;            // [NF][TY+1][TX]   face between y-1 and y
+    const TileMem<T, ORDER, TX, TY> mem(smem);
+    T *prim = mem.prim, *slx = mem.slx, *sly = mem.sly, *fx = mem.fx, *fy = mem.fy;
 
     const int tid = threadIdx.x;
     const int N = P.N, M = P.M;
@@ -302,75 +473,14 @@ __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT
     }
 
     // ---- F: faces ---------------------------------------------------------------------------
-    double umax_x = 0.0, umax_y = 0.0;
-    constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
-    for (int i = tid; i < NFX + NFY; i += NT) {
-        const bool isx = i < NFX;
-        int lx, ly;
-        if (isx) {
-            ly = i / (TX + 1);
-            lx = i - ly * (TX + 1);
-            if (tx0 + lx > N || ty0 + ly >= M) continue;
-        } else {
-            const int j = i - NFX;
-            ly = j / TX;
-            lx = j - ly * TX;
-            if (tx0 + lx >= N || ty0 + ly > M) continue;
-        }
-        // cells on either side: A (low) and B (high)
-        const int ax = isx ? lx - 1 : lx, ay = isx ? ly : ly - 1;
-        if (P.frozen && !cell_active(P, tx0 + ax, ty0 + ay) &&
-            !cell_active(P, tx0 + lx, ty0 + ly))
-            continue;  // no updated cell uses this face
-        const T* pa = prim + (ay + H) * SX + (ax + H);
-        const T* pb = pa + (isx ? 1 : SX);
-        T qa[NF], qb[NF];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            const T ca = pa[f * SY * SX], cb = pb[f * SY * SX];
-            if (ORDER == 2) {
-                T da, db;
-                if (isx) {
-                    da = slx[(f * TY + ly) * (TX + 2) + lx];
-                    db = slx[(f * TY + ly) * (TX + 2) + lx + 1];
-                } else {
-                    da = sly[(f * (TY + 2) + ly) * TX + lx];
-                    db = sly[(f * (TY + 2) + ly + 1) * TX + lx];
-                }
-                T a = fma(0.5, da, ca), b = fma(-0.5, db, cb);
-                if (f < 2) {  // rho, p fall back to the cell value (kernel.cu:3436-3470)
-                    a = le_zero(a) ? ca : a;
-                    b = le_zero(b) ? cb : b;
-                }
-                qa[f] = a;
-                qb[f] = b;
-            } else {
-                qa[f] = ca;
-                qb[f] = cb;
-            }
-        }
-        T UU;
-        const FluxE<T> F =
-            P.method == GD_METHOD_HLL
-                ? hll_local(qa[0], qa[1], isx ? qa[2] : qa[3], isx ? qa[3] : qa[2], qb[0], qb[1],
-                            isx ? qb[2] : qb[3], isx ? qb[3] : qb[2], P, UU)
-                : hllc_local(qa[0], qa[1], isx ? qa[2] : qa[3], isx ? qa[3] : qa[2], qb[0], qb[1],
-                             isx ? qb[2] : qb[3], isx ? qb[3] : qb[2], P, UU);
-        if (isx) {
-            T* fo = fx + ly * (TX + 1) + lx;
-            fo[0 * TY * (TX + 1)] = F.m;
-            fo[1 * TY * (TX + 1)] = F.e;
-            fo[2 * TY * (TX + 1)] = F.mn;  // x momentum
-            fo[3 * TY * (TX + 1)] = F.mt;  // y momentum
-            umax_x = max_nonneg(umax_x, value_of(UU));
-        } else {
-            T* fo = fy + ly * TX + lx;
-            fo[0 * (TY + 1) * TX] = F.m;
-            fo[1 * (TY + 1) * TX] = F.e;
-            fo[2 * (TY + 1) * TX] = F.mt;  // x momentum
-            fo[3 * (TY + 1) * TX] = F.mn;  // y momentum
-            umax_y = max_nonneg(umax_y, value_of(UU));
-        }
+    Speeds fastest;
+    if constexpr (std::is_same<T, double>::value) {
+        if (P.method == GD_METHOD_HLL)
+            faces_float<T, ORDER, TX, TY>(P, smem, tx0, ty0, fastest);
+        else
+            faces_hllc<ORDER, TX, TY>(P, smem, tx0, ty0, dt_only, fastest);
+    } else {
+        faces_float<T, ORDER, TX, TY>(P, smem, tx0, ty0, fastest);
     }
     __syncthreads();
 
@@ -426,8 +536,8 @@ __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT
         store_cell2(out, k, 0, r2, p2);
         store_cell2(out, k, 2, u2, v2);
     }
-    res.umax_x = umax_x;
-    res.umax_y = umax_y;
+    res.umax_x = fastest.x;
+    res.umax_y = fastest.y;
     res.any_active = any_active;
     res.nfl_r = nfl_r;
     res.nfl_p = nfl_p;
@@ -443,7 +553,7 @@ __device__ __forceinline__ void add_counters(Scalars* ctr, const TileResult& r) 
 }
 
 template <int ORDER, int TX, int TY>
-__global__ void __launch_bounds__(NT) euler_fast_kernel(Params P, CPlanes in, Planes out,
+__global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_fast_kernel(Params P, CPlanes in, Planes out,
                                                         const double* __restrict__ T_do_ptr,
                                                         unsigned long long* T_bits, Scalars* rot,
                                                         Scalars* ctr, int dt_only,
@@ -481,7 +591,7 @@ __global__ void __launch_bounds__(NT) euler_tangent_kernel(Params P, CPlanes in,
 // `sc_override` (may be null) replaces every grid's scalars (the autotuner times steps
 // without touching the real dt and time).
 template <int ORDER, int TX, int TY>
-__global__ void __launch_bounds__(NT) euler_batch_kernel(const BatchGrid* __restrict__ grids,
+__global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_batch_kernel(const BatchGrid* __restrict__ grids,
                                                          const int2* __restrict__ items,
                                                          int nitems, int cur, int dt_only,
                                                          Scalars* sc_override) {
@@ -684,13 +794,18 @@ __global__ void euler_face_probe_kernel(Params P, long long n, int axis,
     const double* a = L + 4 * i;
     const double* b = R + 4 * i;
     const bool isx = axis == 0;
+    const double uL = isx ? a[2] : a[3], vL = isx ? a[3] : a[2];
+    const double uR = isx ? b[2] : b[3], vR = isx ? b[3] : b[2];
     double UU;
-    const FluxE<double> F =
-        P.method == GD_METHOD_HLL
-            ? hll_local(a[0], a[1], isx ? a[2] : a[3], isx ? a[3] : a[2], b[0], b[1],
-                        isx ? b[2] : b[3], isx ? b[3] : b[2], P, UU)
-            : hllc_local(a[0], a[1], isx ? a[2] : a[3], isx ? a[3] : a[2], b[0], b[1],
-                         isx ? b[2] : b[3], isx ? b[3] : b[2], P, UU);
+    FluxE<double> F;
+    bool done = false;
+    if (P.method != GD_METHOD_HLL) {
+        const fx::Fan fan = fx::fan_of(a[0], a[1], uL, vL, b[0], b[1], uR, vR, P.gas, UU);
+        done = fan.ok && fx::hllc(fan, vL, vR, P.gas, F.m, F.mn, F.mt, F.e);
+    }
+    if (!done)
+        F = P.method == GD_METHOD_HLL ? hll_local(a[0], a[1], uL, vL, b[0], b[1], uR, vR, P, UU)
+                                      : hllc_local(a[0], a[1], uL, vL, b[0], b[1], uR, vR, P, UU);
     double* o = flux + 4 * i;
     o[0] = F.m;
     o[1] = F.e;

@@ -1,0 +1,301 @@
+// gd_fixed.cuh -- scaled 64-bit integer arithmetic for the step's face solvers.
+//
+// GB300's FP64 unit takes 64 cycles of an SM sub-partition per warp instruction, the integer
+// pipes two for an add or a shift and four for a 32x32->64 multiply-add (measured: 1.88 DFMA,
+// 59 64-bit adds, 25 wide multiply-adds per clock and SM; all three run side by side).  A face
+// flux is a short chain of products and sums of quantities of a few known sizes, so it can be
+// formed in integers: each quantity is a signed 64-bit integer times a power of two chosen per
+// face from the exponents of its inputs (one for all velocities, one per density, ...).  A
+// sum is then one 64-bit add, a product mulk() below, and nothing is rounded to 53 bits before
+// the result is.  Units keep 57 bits or more below the face's velocity, momentum and energy
+// scales, against the 53 of a binary64 rounding.
+//
+// Host-compilable, so that the same arithmetic is checked on the CPU against 113-bit floats.
+#pragma once
+
+#include <cmath>
+#include <cstdint>
+
+#include "gd_swfp.cuh"
+
+namespace gd {
+namespace fx {
+
+using i64 = long long;
+using u64 = unsigned long long;
+
+GD_HD int32_t hi32(i64 x) { return (int32_t)(x >> 32); }
+GD_HD uint32_t lo32(i64 x) { return (uint32_t)x; }
+
+// x y / 2^(64 - KX - KY), |x| < 2^(63 - KX), |y| < 2^(63 - KY), to 3 units below.  Three wide
+// multiply-adds: the product of the low words and their lowest bits are left out.
+template <int KX, int KY>
+GD_HD i64 mulk(i64 x, i64 y) {
+    x = (i64)((u64)x << KX);
+    y = (i64)((u64)y << KY);
+    const int32_t xh = hi32(x), yh = hi32(y);
+    const int32_t xl = (int32_t)(lo32(x) >> 1), yl = (int32_t)(lo32(y) >> 1);
+    return (i64)xh * yh + (((i64)xh * yl + ((i64)yh * xl + 0x7fffffffLL)) >> 31);
+}
+// x y / 2^32 for a 32-bit y
+GD_HD i64 mul32(i64 x, uint32_t y) {
+    return (i64)((u64)((i64)hi32(x) * (i64)(int32_t)y) + (((u64)lo32(x) * y) >> 32));
+}
+
+GD_HD int clz32(uint32_t x) {  // 32 for 0
+#if defined(__CUDA_ARCH__)
+    return __clz((int)x);
+#else
+    return x ? __builtin_clz(x) : 32;
+#endif
+}
+GD_HD int clz64(u64 x) {  // 64 for 0
+#if defined(__CUDA_ARCH__)
+    return __clzll((i64)x);
+#else
+    return x ? __builtin_clzll(x) : 64;
+#endif
+}
+GD_HD int imax(int a, int b) { return a > b ? a : b; }
+GD_HD int imin(int a, int b) { return a < b ? a : b; }
+// arithmetic shift right by any n >= 0
+GD_HD i64 sra(i64 x, int n) { return x >> (n < 63 ? n : 63); }
+
+GD_HD float rsqrt_seed(float x) {
+#if defined(__CUDA_ARCH__)
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#else
+    return 1.0f / std::sqrt(x);
+#endif
+}
+GD_HD float rcp_seed(float x) {
+#if defined(__CUDA_ARCH__)
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+#else
+    return 1.0f / x;
+#endif
+}
+
+// A positive normal double as m 2^(e - 62), m in [2^62, 2^63); e is its unbiased exponent.
+struct Pos {
+    i64 m;
+    int e;
+};
+// sign and exponent field of x
+GD_HD uint32_t sexp(double x) {
+    uint32_t hi, lo;
+    swfp::halves(x, hi, lo);
+    return hi >> 20;
+}
+GD_HD Pos pos_of(double x) {
+    uint32_t hi, lo;
+    swfp::halves(x, hi, lo);
+    Pos p;
+    p.e = (int)(hi >> 20) - 1023;
+    const uint32_t h = (hi & 0xfffffu) | 0x100000u;
+    p.m = (i64)(((u64)((h << 10) | (lo >> 22)) << 32) | (lo << 10));
+    return p;
+}
+// x in units of 2^(E - 61), |x| < 2^(E - 1); what lies below the unit is dropped
+GD_HD i64 in_units(double x, int E) {
+    uint32_t hi, lo;
+    swfp::halves(x, hi, lo);
+    const int e = (int)((hi >> 20) & 0x7ffu) - 1023;
+    const uint32_t h = (hi & 0xfffffu) | 0x100000u;
+    const u64 s = ((u64)((h << 9) | (lo >> 23)) << 32) | (lo << 9);
+    const i64 v = (i64)(s >> imin(E - e, 63));
+    return (int32_t)hi < 0 ? -v : v;
+}
+// x as a signed m 2^(e - 62), m = 0 for zero and subnormal x
+GD_HD Pos signed_of(double x) {
+    uint32_t hi, lo;
+    swfp::halves(x, hi, lo);
+    Pos p;
+    p.e = (int)((hi >> 20) & 0x7ffu) - 1023;
+    const uint32_t h = (hi & 0xfffffu) | 0x100000u;
+    i64 v = (i64)(((u64)((h << 10) | (lo >> 22)) << 32) | (lo << 10));
+    if (p.e == -1023) v = 0;
+    p.m = (int32_t)hi < 0 ? -v : v;
+    return p;
+}
+// x 2^ue rounded to the nearest double (ties away from zero); results are normal or 0
+GD_HD double pack(i64 x, int ue) {
+    const uint32_t neg = (uint32_t)(hi32(x) >> 31);
+    u64 a = (u64)(x < 0 ? -x : x);
+    const int lz = clz64(a);
+    a = lz < 64 ? a << lz : 0;
+    const u64 m = (a >> 11) + ((a >> 10) & 1);
+    const u64 b = m + ((u64)(uint32_t)(ue - lz + 63 + 1022) << 52);
+    return a == 0 ? 0.0 : swfp::from_halves((uint32_t)(b >> 32) | (neg & 0x80000000u), (uint32_t)b);
+}
+
+// 1 / x for x > 0 with a nonzero high word: r 2^(lz - 124), lz the leading zeros of x, r in
+// (2^60, 2^61).  The FP32 reciprocal y of the leading 24 bits, then y (1 + e + e^2) with
+// e = 1 - x y (Newton's iteration with the quadratic term kept) in units of 2^-62.
+GD_HD i64 rcp(i64 x, int& lz) {
+    lz = clz32((uint32_t)hi32(x));
+    const u64 n = (u64)x << lz;
+    const float f = swfp::f32_from_bits(0x3f800000u | ((uint32_t)(n >> 40) & 0x7fffffu));
+    // y in [1/2, 1] as an integer of unit 2^-31 (the pattern's step at 1 keeps this linear)
+    const uint32_t y = ((swfp::bits_of_f32(rcp_seed(f)) - 0x3e800000u) << 7) - 1u;
+    const u64 xy = (u64)(uint32_t)(n >> 32) * y + (((u64)(uint32_t)n * y) >> 32);
+    const i64 e = (i64)(0x4000000000000000ULL - xy);
+    const int32_t es = (int32_t)(e >> 20);
+    const i64 g = e + (((i64)es * es) >> 22);
+    return ((i64)((u64)y << 30) - 1) + mul32(g, y);
+}
+
+// sqrt(a / r) of a = am 2^(ea - 60), am in [2^60, 2^62), and r = rm 2^(er - 62): w 2^(k - 60),
+// w in [2^58, 2^61).  The FP32 seed y of 1/sqrt(a r), w = a y, e = 1 - w (r y), and
+// w (1 + e/2 + 3 e^2 / 8), the series of 1/sqrt(1 - e).
+GD_HD i64 sqrt_over(i64 am, int ea, Pos r, int& k) {
+    const int d = ea - r.e + 2;
+    k = d >> 1;
+    const i64 a = am << (d & 1);
+    const float f = (float)hi32(a) * (float)hi32(r.m);
+    // 2^60 y, between 2^29 and 2^31
+    const uint32_t y = (uint32_t)(rsqrt_seed(f) * 1152921229728940032.0f);
+    const i64 w = mul32(a, y), t = mul32(r.m, y);
+    const i64 e = (1LL << 59) - mulk<2, 1>(w, t);
+    const int32_t es = (int32_t)(e >> 16);
+    const i64 g = (e << 2) + (((i64)es * (3 * es)) >> 27);
+    return w + (mulk<0, 0>(w, g << 21) >> 19);
+}
+
+// The constants a face solver needs of gamma, as m 2^(e - 62).
+struct Gas {
+    i64 g, gg;    // gamma, gamma / (gamma - 1)
+    int ge, gge;
+    int room;     // extra bits that gamma / (gamma - 1) p takes beside rho c^2; -1: no integer path
+};
+inline Gas gas_of(double gamma) {
+    Gas G;
+    const Pos a = pos_of(gamma), b = pos_of(gamma / (gamma - 1.0));
+    G.g = a.m;
+    G.ge = a.e;
+    G.gg = b.m;
+    G.gge = b.e;
+    G.room = b.e > 2 ? b.e - 2 : 0;
+    if (a.e > 16 || b.e > 16) G.room = -1;  // gamma beyond 2^16, or within 2^-16 of 1
+    return G;
+}
+
+// The wave speeds of the face between (rL, pL, uL, vL) and (rR, pR, uR, vR), its frame local:
+// all velocities in units of 2^(E - 61).  |u|, c < 2^(E - 1), so |S| < 2^61 and
+// |S - u| < 1.5 2^61 in these units.
+struct Fan {
+    Pos RL, RR, PL, PR;
+    i64 uL, uR, SL, SR;
+    int E, kmin;  // kmin: 2^kmin is about the smaller sound speed
+    bool ok;
+};
+// ok is false where a scale would leave a quantity fewer bits than binary64 does, or an input is
+// not a normal positive density or pressure or a finite velocity.  Accepted: densities and
+// pressures in 2^[-128, 128], densities within 2^8 of each other, velocities below 2^128, sound
+// speeds within a factor of about 4 of each other, normal velocities to about 64 of them.
+// UU: the larger wave speed.
+GD_HD Fan fan_of(double rL, double pL, double uL, double vL, double rR, double pR, double uR,
+                 double vR, const Gas& G, double& UU) {
+    const uint32_t low = 1023 - 128, span = 256, top = 1023 + 128;
+    const int xuL = (int)(sexp(uL) & 0x7ffu), xuR = (int)(sexp(uR) & 0x7ffu);
+    Fan f;
+    f.RL = pos_of(rL);
+    f.RR = pos_of(rR);
+    f.PL = pos_of(pL);
+    f.PR = pos_of(pR);
+    int kL, kR;
+    const i64 wL = sqrt_over(mulk<0, 0>(f.PL.m, G.g), f.PL.e + G.ge, f.RL, kL);
+    const i64 wR = sqrt_over(mulk<0, 0>(f.PR.m, G.g), f.PR.e + G.ge, f.RR, kR);
+    const int kmax = imax(kL, kR);
+    f.kmin = imin(kL, kR);
+    f.E = imax(kmax, imax(xuL, xuR) - 1023) + 2;
+    const int dr = f.RL.e - f.RR.e;
+    f.ok = G.room >= 0 && sexp(rL) - low <= span && sexp(rR) - low <= span && sexp(pL) - low <= span &&
+           sexp(pR) - low <= span && (uint32_t)xuL <= top && (uint32_t)xuR <= top &&
+           (sexp(vL) & 0x7ffu) <= top && (sexp(vR) & 0x7ffu) <= top && kmax - f.kmin <= 2 &&
+           f.E - kmax <= 8 && (uint32_t)(dr + 8) <= 16u;
+    if (!f.ok) return f;
+    const i64 cL = wL >> (f.E - 1 - kL), cR = wR >> (f.E - 1 - kR);
+    f.uL = in_units(uL, f.E);
+    f.uR = in_units(uR, f.E);
+    const i64 aL = f.uL - cL, aR = f.uR - cR, bL = f.uL + cL, bR = f.uR + cR;
+    f.SL = aL < aR ? aL : aR;
+    f.SR = bL > bR ? bL : bR;
+    UU = pack(-f.SL > f.SR ? -f.SL : f.SR, f.E - 61);
+    return f;
+}
+
+// HLLC flux (mass, normal and tangential momentum, energy) of that face: the formulas of
+// hllc_local.  Returns false, with nothing formed, where the face lies inside the fan and a
+// velocity is more than about 4 sound speeds; the caller then takes hllc_local.  SL < S_M < SR
+// (the Davis speeds, with positive pressures), and inside the fan S_M and S have opposite signs,
+// so |S_M / (S - S_M)| <= 1: no product below overflows.
+GD_HD bool hllc(const Fan& f, double vL, double vR, const Gas& G, double& Fm, double& Fn,
+                double& Ft, double& Fe) {
+    const int E = f.E, ER = imax(f.RL.e, f.RR.e);
+    const i64 suL = f.SL - f.uL, suR = f.SR - f.uR;
+    // r (S - u), each side in units of its own density's, 2^(e + E - 59), and in the larger's
+    const i64 oL = mulk<0, 0>(f.RL.m, suL), oR = mulk<0, 0>(f.RR.m, suR);
+    const i64 mL = oL >> (ER - f.RL.e), mR = oR >> (ER - f.RR.e);
+    const i64 D = mR - mL;
+    // units 2^(ER + 2E - 60)
+    const int sp = ER + 2 * E + 2;
+    const i64 N = mulk<1, 3>(mR, f.uR) - mulk<1, 3>(mL, f.uL) +
+                  ((f.PL.m >> imin(sp - f.PL.e, 63)) - (f.PR.m >> imin(sp - f.PR.e, 63)));
+    int lz;
+    const i64 iD = rcp(D, lz);
+    i64 SM = mulk<0, 2>(N << (lz - 2), iD);
+
+    const bool takeL = f.SL > 0 || N >= 0;
+    const bool star = takeL ? f.SL <= 0 : f.SR >= 0;
+    const Pos R{takeL ? f.RL.m : f.RR.m, takeL ? f.RL.e : f.RR.e};
+    const Pos Pk{takeL ? f.PL.m : f.PR.m, takeL ? f.PL.e : f.PR.e};
+    const i64 un = takeL ? f.uL : f.uR, S = takeL ? f.SL : f.SR;
+    const i64 o = takeL ? oL : oR;
+    const Pos T = signed_of(takeL ? vL : vR);
+
+    i64 qs = un;  // outside the fan the physical flux: S_M -> u, q (S - u) -> u
+    if (star) {
+        if (E - f.kmin > 3) return false;
+        const i64 su = takeL ? suL : suR;
+        const i64 ad = takeL ? SM - S : S - SM;
+        if (hi32(ad) <= 0) return false;
+        int lz2;
+        const i64 iA = rcp(ad, lz2);
+        const i64 q = mulk<0, 2>(SM << (lz2 - 2), iA);  // |S_M / (S - S_M)| 2^60, signed as S_M
+        qs = mulk<2, 1>(takeL ? -q : q, su) << 1;
+    } else {
+        SM = un;
+    }
+    const i64 SMu = SM - un;
+    const int32_t qh = hi32(qs);
+    const int z = clz32((uint32_t)(qh ^ (qh >> 31))) - 1;
+    const i64 qn = qs << z;
+    const i64 M = mulk<0, 0>(R.m, qn);
+    const int em = R.e + E - 59 - z;
+    Fm = pack(M, em);
+    // momentum: p + r q su S_M + r su (S_M - u); exactly p where the rest is 0
+    const i64 t = (mulk<1, 2>(M, SM) >> z) + mulk<2, 1>(o, SMu);
+    const int et = R.e + 2 * E - 59;
+    const i64 pt = (Pk.m >> imin(et - Pk.e + 62, 63)) + t;
+    Fn = pack(t == 0 ? Pk.m : pt, t == 0 ? Pk.e - 62 : et);
+    const i64 MT = mulk<0, 0>(M, T.m);
+    Ft = pack(MT, em + T.e + 2);
+    // energy: q su (p gamma / (gamma - 1) + r (u^2 / 2 + S (S_M - u))) + (mass flux) v^2 / 2
+    const i64 H = mulk<1, 1>(un, un) + mulk<2, 1>(S, SMu);
+    const i64 B = sra(mulk<0, 0>(Pk.m, G.gg), R.e + 2 * E - Pk.e - G.gge + G.room) +
+                  (mulk<0, 1>(R.m, H) >> G.room);
+    const i64 e1 = mulk<0, 0>(qn, B);
+    const i64 e2 = mulk<2, 0>(MT, T.m);
+    const int dx = 2 * (E - T.e) + 1 + G.room;
+    const int x1 = R.e + 3 * E - 57 - z + G.room;
+    Fe = pack(sra(e1, imax(-dx, 0)) + sra(e2, imax(dx, 0)), dx > 0 ? x1 : x1 - dx);
+    return true;
+}
+
+}  // namespace fx
+}  // namespace gd

@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/gd2d.h"
+#include "gd_fixed.cuh"
 #include "gd_swfp.cuh"
 
 namespace gd {
@@ -47,6 +48,7 @@ struct Params {
     double ambient_p;   // 1/gamma
     double krad_x;      // krit * rad used for faces with an x normal
     double krad_y;      // krit * rad used for faces with a y normal
+    fx::Gas gas;        // gamma's constants for the integer face solvers
 };
 
 // A state: SoA planes, f[k] + m*N + n; or, where s is set, the reference's AoS layout
