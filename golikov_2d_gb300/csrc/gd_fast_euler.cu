@@ -172,7 +172,10 @@ struct Shape {
     static constexpr int kSly = ORDER == 2 ? NF * (TY + 2) * TX : 0;
     static constexpr int kFx = NF * TY * (TX + 1);
     static constexpr int kFy = NF * (TY + 1) * TX;
-    static constexpr size_t bytes = sizeof(double) * (kPrim + kSlx + kSly + kFx + kFy);
+    static constexpr int kFloat = kPrim + kSlx + kSly + kFx + kFy;
+    static constexpr int kInt = kPrim + NF * TY * TX + kFx + kFy;  // TileMemInt
+    static constexpr int doubles = kFloat > kInt ? kFloat : kInt;
+    static constexpr size_t bytes = sizeof(double) * doubles;
 };
 
 // Value and tangent planes (the tangent step of the adjoint checks).
@@ -228,11 +231,22 @@ struct TileMem {
         : prim(smem), slx(prim + S::kPrim), sly(slx + S::kSlx), fx(sly + S::kSly),
           fy(fx + S::kFx) {}
 };
+// The same of a tile held in integers: no slopes, and the cells' own values beside them.
+template <int ORDER, int TX, int TY>
+struct TileMemInt {
+    using S = Shape<ORDER, TX, TY>;
+    fx::i64* q;    // [NF][SY][SX]
+    double* cell;  // [NF][TY][TX]
+    double *fx, *fy;
+    __device__ explicit TileMemInt(double* smem)
+        : q(reinterpret_cast<fx::i64*>(smem)), cell(smem + S::kPrim), fx(cell + NF * TY * TX),
+          fy(fx + S::kFx) {}
+    static_assert(S::kPrim + NF * TY * TX + S::kFx + S::kFy <= S::doubles, "fits the tile's room");
+};
 
 // One face of a tile: faces 0 .. NFX-1 have an x normal, the rest a y normal.
-template <class T, int ORDER, int TX, int TY>
+template <int TX, int TY>
 struct Face {
-    using S = Shape<ORDER, TX, TY>;
     static constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
     bool isx, used;
     int lx, ly;
@@ -253,48 +267,16 @@ struct Face {
             used = cell_active(P, tx0 + (isx ? lx - 1 : lx), ty0 + (isx ? ly : ly - 1)) ||
                    cell_active(P, tx0 + lx, ty0 + ly);
     }
-    // the states on its low (a) and high (b) side, {rho, p, normal, tangential velocity}
-    __device__ __forceinline__ void states(const TileMem<T, ORDER, TX, TY>& t, T* qa, T* qb) const {
-        constexpr int H = S::H, SX = S::SX, SY = S::SY;
-        const T* pb = t.prim + (ly + H) * SX + (lx + H);
-        const T* pa = pb - (isx ? 1 : SX);
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            // field of the local frame's component f
-            const int g = f < 2 ? f : (isx ? f : 5 - f);
-            const T ca = pa[g * SY * SX], cb = pb[g * SY * SX];
-            if (ORDER == 2) {
-                T da, db;
-                if (isx) {
-                    da = t.slx[(g * TY + ly) * (TX + 2) + lx];
-                    db = t.slx[(g * TY + ly) * (TX + 2) + lx + 1];
-                } else {
-                    da = t.sly[(g * (TY + 2) + ly) * TX + lx];
-                    db = t.sly[(g * (TY + 2) + ly + 1) * TX + lx];
-                }
-                T a = fma(0.5, da, ca), b = fma(-0.5, db, cb);
-                if (f < 2) {  // rho, p fall back to the cell value (kernel.cu:3436-3470)
-                    a = le_zero(a) ? ca : a;
-                    b = le_zero(b) ? cb : b;
-                }
-                qa[f] = a;
-                qb[f] = b;
-            } else {
-                qa[f] = ca;
-                qb[f] = cb;
-            }
-        }
-    }
-    __device__ __forceinline__ void store(const TileMem<T, ORDER, TX, TY>& t, T m, T e, T mn,
-                                          T mt) const {
+    template <class T>
+    __device__ __forceinline__ void store(T* fx, T* fy, T m, T e, T mn, T mt) const {
         if (isx) {
-            T* fo = t.fx + ly * (TX + 1) + lx;
+            T* fo = fx + ly * (TX + 1) + lx;
             fo[0 * TY * (TX + 1)] = m;
             fo[1 * TY * (TX + 1)] = e;
             fo[2 * TY * (TX + 1)] = mn;  // x momentum
             fo[3 * TY * (TX + 1)] = mt;  // y momentum
         } else {
-            T* fo = t.fy + ly * TX + lx;
+            T* fo = fy + ly * TX + lx;
             fo[0 * (TY + 1) * TX] = m;
             fo[1 * (TY + 1) * TX] = e;
             fo[2 * (TY + 1) * TX] = mt;  // x momentum
@@ -303,17 +285,54 @@ struct Face {
     }
 };
 
-// The flux of one face with the solver of the step's method in floating point.
+// The flux in floating point between the states qa (low side) and qb, {rho, p, normal,
+// tangential velocity}, with the solver of the step's method.
+template <class T>
+__device__ __forceinline__ FluxE<T> flux_of(const Params& P, const T* qa, const T* qb, T& UU) {
+    return P.method == GD_METHOD_HLL
+               ? hll_local(qa[0], qa[1], qa[2], qa[3], qb[0], qb[1], qb[2], qb[3], P, UU)
+               : hllc_local(qa[0], qa[1], qa[2], qa[3], qb[0], qb[1], qb[2], qb[3], P, UU);
+}
+// The states on either side of a face, c + d/2 and c - d/2; rho and p fall back to the cell
+// value (kernel.cu:3436-3470).
+template <class T>
+__device__ __forceinline__ void side_states(int f, T ca, T da, T cb, T db, T& a, T& b) {
+    a = fma(0.5, da, ca);
+    b = fma(-0.5, db, cb);
+    if (f < 2) {
+        a = le_zero(a) ? ca : a;
+        b = le_zero(b) ? cb : b;
+    }
+}
+
 template <class T, int ORDER, int TX, int TY>
 __device__ __forceinline__ T face_flux(const Params& P, const TileMem<T, ORDER, TX, TY>& t,
-                                       const Face<T, ORDER, TX, TY>& f) {
+                                       const Face<TX, TY>& w) {
+    using S = Shape<ORDER, TX, TY>;
+    constexpr int H = S::H, SX = S::SX, SY = S::SY;
+    const int lx = w.lx, ly = w.ly;
+    const T* pb = t.prim + (ly + H) * SX + (lx + H);
+    const T* pa = pb - (w.isx ? 1 : SX);
     T qa[NF], qb[NF], UU;
-    f.states(t, qa, qb);
-    const FluxE<T> F =
-        P.method == GD_METHOD_HLL
-            ? hll_local(qa[0], qa[1], qa[2], qa[3], qb[0], qb[1], qb[2], qb[3], P, UU)
-            : hllc_local(qa[0], qa[1], qa[2], qa[3], qb[0], qb[1], qb[2], qb[3], P, UU);
-    f.store(t, F.m, F.e, F.mn, F.mt);
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        const int g = f < 2 ? f : (w.isx ? f : 5 - f);  // field of the local frame's component f
+        qa[f] = pa[g * SY * SX];
+        qb[f] = pb[g * SY * SX];
+        if (ORDER == 2) {
+            T da, db;
+            if (w.isx) {
+                da = t.slx[(g * TY + ly) * (TX + 2) + lx];
+                db = t.slx[(g * TY + ly) * (TX + 2) + lx + 1];
+            } else {
+                da = t.sly[(g * (TY + 2) + ly) * TX + lx];
+                db = t.sly[(g * (TY + 2) + ly + 1) * TX + lx];
+            }
+            side_states(f, qa[f], da, qb[f], db, qa[f], qb[f]);
+        }
+    }
+    const FluxE<T> F = flux_of(P, qa, qb, UU);
+    w.store(t.fx, t.fy, F.m, F.e, F.mn, F.mt);
     return UU;
 }
 
@@ -325,72 +344,75 @@ struct Speeds {
     }
 };
 
-// Every face of a tile in floating point: the HLL method, and the tangent.
-template <class T, int ORDER, int TX, int TY>
-__device__ __noinline__ void faces_float(const Params& P, T* smem, int tx0, int ty0, Speeds& u) {
-    using F = Face<T, ORDER, TX, TY>;
-    const TileMem<T, ORDER, TX, TY> t(smem);
-    Speeds v{0.0, 0.0};
-    for (int i = threadIdx.x; i < F::NFX + F::NFY; i += NT) {
-        const F f(P, tx0, ty0, i);
-        if (f.used) v.take(f.isx, value_of(face_flux(P, t, f)));
-    }
-    u = v;
-}
-
-// The faces of a thread that the integer solver left (bit k: the k-th), in floating point.
-// Out of line, and after the loop over the faces: a call or a second solver inside it would
-// take registers from every face for what a few need.
-template <int ORDER, int TX, int TY>
-__device__ __noinline__ void faces_left(const Params& P, double* smem, int tx0, int ty0,
-                                        unsigned int left, unsigned int left_speed, Speeds& u) {
-    using F = Face<double, ORDER, TX, TY>;
-    const TileMem<double, ORDER, TX, TY> t(smem);
-    while (left) {
-        const int k = __ffs((int)left) - 1;
-        left &= left - 1;
-        const F f(P, tx0, ty0, threadIdx.x + k * NT);
-        const double UU = face_flux(P, t, f);
-        if (left_speed >> k & 1) u.take(f.isx, UU);
-    }
-}
-
-// Every face of a tile with the HLLC flux in 64-bit integers (gd_fixed.cuh): no FP64 instruction
-// but the two multiply-adds per reconstructed value.  dt_only: the wave speeds alone.
-template <int ORDER, int TX, int TY>
-__device__ __noinline__ void faces_hllc(const Params& P, double* smem, int tx0, int ty0,
-                                        int dt_only, Speeds& u) {
-    using F = Face<double, ORDER, TX, TY>;
-    const TileMem<double, ORDER, TX, TY> t(smem);
-    Speeds v{0.0, 0.0};
-    unsigned int left = 0, left_speed = 0, bit = 1;
-    for (int i = threadIdx.x; i < F::NFX + F::NFY; i += NT, bit <<= 1) {
-        const F f(P, tx0, ty0, i);
-        if (!f.used) continue;
-        double qa[NF], qb[NF], UU;
-        f.states(t, qa, qb);
-        const fx::Fan fan =
-            fx::fan_of(qa[0], qa[1], qa[2], qa[3], qb[0], qb[1], qb[2], qb[3], P.gas, UU);
-        if (!fan.ok) {
-            left |= bit;
-            left_speed |= bit;
-            continue;
-        }
-        v.take(f.isx, UU);
-        if (dt_only) continue;
-        double m, mn, mt, e;
-        if (fx::hllc(fan, qa[3], qb[3], P.gas, m, mn, mt, e)) f.store(t, m, e, mn, mt);
-        else left |= bit;
-    }
-    if (left) faces_left<ORDER, TX, TY>(P, smem, tx0, ty0, left, left_speed, v);
-    u = v;
-}
-
 struct TileResult {
     double umax_x, umax_y;
     bool any_active;
     unsigned int nfl_r, nfl_p, nbad;
 };
+
+// ---- U: conservative update of the tile's cells ---------------------------------------------
+// cell: the tile's own values, rows RS and fields FS apart.
+template <class T, int ORDER, int TX, int TY, int RS, int FS, class OUT>
+__device__ __forceinline__ void update_cells(const Params& P, const OUT& out, int tx0, int ty0,
+                                             double T_do, int dt_only, const T* cell, const T* fx,
+                                             const T* fy, TileResult& res, double* aux) {
+    const int N = P.N, M = P.M;
+    const double kx = T_do * P.inv_dx, ky = T_do * P.inv_dy;
+    bool any_active = false;
+    unsigned int nfl_r = 0, nfl_p = 0, nbad = 0;
+    for (int i = threadIdx.x; i < TX * TY; i += NT) {
+        const int ly = i / TX, lx = i - ly * TX;
+        const int gx = tx0 + lx, gy = ty0 + ly;
+        if (gx >= N || gy >= M) continue;
+        const T* c = cell + ly * RS + lx;
+        const T r = c[0], p = c[FS], u = c[2 * FS], v = c[3 * FS];
+        const long long k = (long long)gy * N + gx;
+        if (P.frozen && !cell_active(P, gx, gy)) {  // the faces' own test
+            if (!dt_only) {
+                store_cell2(out, k, 0, r, p);
+                store_cell2(out, k, 2, u, v);
+            }
+            continue;
+        }
+        any_active = true;
+        if (dt_only) continue;
+        const T* fxc = fx + ly * (TX + 1) + lx;
+        const T* fyc = fy + ly * TX + lx;
+        T d[NF];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const T* a = fxc + f * TY * (TX + 1);
+            const T* b = fyc + f * (TY + 1) * TX;
+            d[f] = fma(kx, a[1] - a[0], mulx(ky, b[TX] - b[0]));
+        }
+        if constexpr (std::is_same<T, double>::value) {
+            if (aux != nullptr) {  // the recording of the adjoint: the flux differences used
+                const long long KK = (long long)N * M;
+#pragma unroll
+                for (int f = 0; f < NF; ++f) aux[f * KK + k] = d[f];
+            }
+        }
+        T r2 = r - d[0];
+        if (le_zero(r2)) { r2 = cst<T>(0.0001); ++nfl_r; }
+        const T inv = rcp_2op(r2);
+        const T mx2 = fma(r, u, -d[2]), my2 = fma(r, v, -d[3]);
+        const T u2 = mulx(mx2, inv);
+        const T v2 = mulx(my2, inv);
+        // p' = (gamma - 1) (E - d_E - K'/2) with E = p / (gamma - 1) + K / 2, K = rho |v|^2,
+        // K' = rho' |v'|^2 = m' . v' (kernel.cu:1861-1870)
+        const T K1 = r * fma(u, u, mulx(v, v));
+        const T K2 = fma(mx2, u2, mulx(my2, v2));
+        T p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, d[1], p));
+        if (le_zero(p2)) { p2 = cst<T>(0.000001); ++nfl_p; }
+        if (!finite_bits(r2) || !finite_bits(p2) || !finite_bits(u2) || !finite_bits(v2)) ++nbad;
+        store_cell2(out, k, 0, r2, p2);
+        store_cell2(out, k, 2, u2, v2);
+    }
+    res.any_active = any_active;
+    res.nfl_r = nfl_r;
+    res.nfl_p = nfl_p;
+    res.nbad = nbad;
+}
 
 // One TX x TY tile whose lower-left cell is (tx0, ty0).  Reads `in`, writes `out`, returns
 // the per-thread wave-speed maxima and counters.  Every thread of the block must call it.
@@ -473,75 +495,186 @@ __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT
     }
 
     // ---- F: faces ---------------------------------------------------------------------------
-    Speeds fastest;
-    if constexpr (std::is_same<T, double>::value) {
-        if (P.method == GD_METHOD_HLL)
-            faces_float<T, ORDER, TX, TY>(P, smem, tx0, ty0, fastest);
-        else
-            faces_hllc<ORDER, TX, TY>(P, smem, tx0, ty0, dt_only, fastest);
-    } else {
-        faces_float<T, ORDER, TX, TY>(P, smem, tx0, ty0, fastest);
+    Speeds fastest{0.0, 0.0};
+    for (int i = tid; i < Face<TX, TY>::NFX + Face<TX, TY>::NFY; i += NT) {
+        const Face<TX, TY> f(P, tx0, ty0, i);
+        if (f.used) fastest.take(f.isx, value_of(face_flux<T, ORDER, TX, TY>(P, mem, f)));
     }
     __syncthreads();
 
-    // ---- U: update --------------------------------------------------------------------------
-    const double kx = T_do * P.inv_dx, ky = T_do * P.inv_dy;
-    bool any_active = false;
-    unsigned int nfl_r = 0, nfl_p = 0, nbad = 0;
-    for (int i = tid; i < TX * TY; i += NT) {
-        const int ly = i / TX, lx = i - ly * TX;
-        const int gx = tx0 + lx, gy = ty0 + ly;
-        if (gx >= N || gy >= M) continue;
-        const T* c = prim + (ly + H) * SX + (lx + H);
-        const T r = c[0], p = c[SY * SX], u = c[2 * SY * SX], v = c[3 * SY * SX];
-        const long long k = (long long)gy * N + gx;
-        if (P.frozen && !cell_active(P, gx, gy)) {  // the faces' own test
-            if (!dt_only) {
-                store_cell2(out, k, 0, r, p);
-                store_cell2(out, k, 2, u, v);
-            }
-            continue;
-        }
-        any_active = true;
-        if (dt_only) continue;
-        const T* fxc = fx + ly * (TX + 1) + lx;
-        const T* fyc = fy + ly * TX + lx;
-        T d[NF];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            const T* a = fxc + f * TY * (TX + 1);
-            const T* b = fyc + f * (TY + 1) * TX;
-            d[f] = fma(kx, a[1] - a[0], mulx(ky, b[TX] - b[0]));
-        }
-        if constexpr (std::is_same<T, double>::value) {
-            if (aux != nullptr) {  // the recording of the adjoint: the flux differences used
-                const long long KK = (long long)N * M;
-#pragma unroll
-                for (int f = 0; f < NF; ++f) aux[f * KK + k] = d[f];
-            }
-        }
-        T r2 = r - d[0];
-        if (le_zero(r2)) { r2 = cst<T>(0.0001); ++nfl_r; }
-        const T inv = rcp_2op(r2);
-        const T mx2 = fma(r, u, -d[2]), my2 = fma(r, v, -d[3]);
-        const T u2 = mulx(mx2, inv);
-        const T v2 = mulx(my2, inv);
-        // p' = (gamma - 1) (E - d_E - K'/2) with E = p / (gamma - 1) + K / 2, K = rho |v|^2,
-        // K' = rho' |v'|^2 = m' . v' (kernel.cu:1861-1870)
-        const T K1 = r * fma(u, u, mulx(v, v));
-        const T K2 = fma(mx2, u2, mulx(my2, v2));
-        T p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, d[1], p));
-        if (le_zero(p2)) { p2 = cst<T>(0.000001); ++nfl_p; }
-        if (!finite_bits(r2) || !finite_bits(p2) || !finite_bits(u2) || !finite_bits(v2)) ++nbad;
-        store_cell2(out, k, 0, r2, p2);
-        store_cell2(out, k, 2, u2, v2);
-    }
+    update_cells<T, ORDER, TX, TY, SX, SY * SX>(P, out, tx0, ty0, T_do, dt_only,
+                                                prim + H * SX + H, fx, fy, res, aux);
     res.umax_x = fastest.x;
     res.umax_y = fastest.y;
-    res.any_active = any_active;
-    res.nfl_r = nfl_r;
-    res.nfl_p = nfl_p;
-    res.nbad = nbad;
+}
+
+// ---- The same tile with its face work in 64-bit integers --------------------------------------
+//
+// The cells of the tile and its halo are held as integers in units of one power of two for the
+// densities, one for the pressures and one for the velocities (fx::Tops), taken from the tile's
+// own largest values.  Slopes, minmod and face states are then plain 64-bit adds and selects, and
+// the HLLC flux is fx::hllc: the FP64 pipe is left with the conversion of the fluxes and the
+// update (about 40 instructions a cell instead of 103).
+
+// The faces of a thread that the integer solver left (bit k: the k-th), in floating point.  Out of
+// line, and after the loop over the faces: a second solver inside it would take registers from
+// every face for what a few need.  speed: the faces whose wave speed is missing too.
+template <int ORDER, int TX, int TY>
+__device__ __noinline__ void faces_left(const Params& P, double* smem, const fx::Tops& X, int tx0,
+                                        int ty0, unsigned int left, unsigned int speed,
+                                        Speeds& u) {
+    using S = Shape<ORDER, TX, TY>;
+    const TileMemInt<ORDER, TX, TY> t(smem);
+    while (left) {
+        const int k = __ffs((int)left) - 1;
+        left &= left - 1;
+        const Face<TX, TY> w(P, tx0, ty0, threadIdx.x + k * NT);
+        const int st = w.isx ? 1 : S::SX;
+        double qa[NF], qb[NF], UU;
+        for (int f = 0; f < NF; ++f) {
+            const int g = f < 2 ? f : (w.isx ? f : 5 - f);
+            const int ue = (f == 0 ? X.r : (f == 1 ? X.p : X.v)) - 60;
+            const fx::i64* q = t.q + (g * S::SY + w.ly + S::H) * S::SX + w.lx + S::H;
+            const double ca = fx::to_double(q[-st], ue), cb = fx::to_double(q[0], ue);
+            qa[f] = ca;
+            qb[f] = cb;
+            if (ORDER == 2) {
+                const double d = cb - ca;
+                side_states(f, ca, minmod(ca - fx::to_double(q[-2 * st], ue), d), cb,
+                            minmod(d, fx::to_double(q[st], ue) - cb), qa[f], qb[f]);
+            }
+        }
+        const FluxE<double> F = flux_of(P, qa, qb, UU);
+        w.store(t.fx, t.fy, F.m, F.e, F.mn, F.mt);
+        if (speed & (1u << k)) u.take(w.isx, UU);
+    }
+}
+
+// Every face of a tile held in integers.  dt_only: the wave speeds alone.
+template <int ORDER, int TX, int TY>
+__device__ __forceinline__ void faces_hllc(const Params& P, double* smem, const fx::Tops& X,
+                                           int tx0, int ty0, int dt_only, Speeds& u) {
+    using S = Shape<ORDER, TX, TY>;
+    using fx::i64;
+    constexpr int FS = S::SY * S::SX;
+    const TileMemInt<ORDER, TX, TY> t(smem);
+    unsigned int left = 0, speed = 0, bit = 1;
+    for (int i = threadIdx.x; i < Face<TX, TY>::NFX + Face<TX, TY>::NFY; i += NT, bit <<= 1) {
+        const Face<TX, TY> w(P, tx0, ty0, i);
+        if (!w.used) continue;
+        const int st = w.isx ? 1 : S::SX;
+        const i64* q = t.q + (w.ly + S::H) * S::SX + w.lx + S::H;
+        i64 a[NF], b[NF];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const i64* p = q + (f < 2 ? f * FS : (w.isx ? f : 5 - f) * FS);
+            const i64 ca = p[-st], cb = p[0];
+            a[f] = 2 * ca;
+            b[f] = 2 * cb;
+            if (ORDER == 2) {  // between the cell and the middle to its neighbour: rho, p > 0
+                const i64 d = cb - ca;
+                a[f] += fx::minmod(ca - p[-2 * st], d);
+                b[f] -= fx::minmod(d, p[st] - cb);
+            }
+        }
+        const fx::States s{a[0], b[0], a[1], b[1], a[2], b[2], a[3], b[3]};
+        double UU;
+        const fx::Fan fan = fx::fan_of(s, X, P.gas, UU);
+        if (!fan.ok) {
+            left |= bit;
+            speed |= bit;
+            continue;
+        }
+        u.take(w.isx, UU);
+        if (dt_only) continue;
+        double m, mn, mt, e;
+        if (fx::hllc(fan, s, X, P.gas, m, mn, mt, e)) w.store(t.fx, t.fy, m, e, mn, mt);
+        else left |= bit;
+    }
+    if (left) faces_left<ORDER, TX, TY>(P, smem, X, tx0, ty0, left, speed, u);
+}
+
+// Returns false, with nothing written, where the tile's cells cannot be held in common units.
+// Every thread of the block must call it, and all get the same answer.
+template <int ORDER, int TX, int TY>
+__device__ __noinline__ bool euler_tile_int(const Params& P, const CPlanes& in, const Planes& out,
+                                            int tx0, int ty0, double T_do, int dt_only,
+                                            double* smem, TileResult& res, double* aux) {
+    using S = Shape<ORDER, TX, TY>;
+    constexpr int H = S::H, SX = S::SX, SY = S::SY, NC = (SY * SX + NT - 1) / NT;
+    const TileMemInt<ORDER, TX, TY> t(smem);
+    // keys of the tile's exponents: the largest and (negated) the smallest of rho and p, and the
+    // largest of the velocities
+    __shared__ unsigned int keys[5][NT / 32];
+    const int tid = threadIdx.x, N = P.N, M = P.M;
+
+    double v[NC][NF];
+    unsigned int key[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int i = tid + c * NT;
+        const int ly = i / SX, lx = i - ly * SX;
+        const bool xh = lx < H || lx >= TX + H, yh = ly < H || ly >= TY + H;
+        const int gx = tx0 + lx - H, gy = ty0 + ly - H;
+        const bool some = i < SY * SX && !(xh && yh) && gx >= -2 && gx < N + 2 && gy >= -2 &&
+                          gy < M + 2 && !((gx < 0 || gx >= N) && (gy < 0 || gy >= M));
+#pragma unroll
+        for (int f = 0; f < NF; ++f) v[c][f] = 0.0;  // never used
+        if (some) {
+            load_cell(P, in, gx, gy, v[c]);
+            const unsigned int r = fx::signed_exp_field(v[c][0]), p = fx::signed_exp_field(v[c][1]);
+            key[0] = max(key[0], r);
+            key[1] = max(key[1], 0xfffu - r);
+            key[2] = max(key[2], p);
+            key[3] = max(key[3], 0xfffu - p);
+            key[4] = max(key[4], max(fx::exp_field(v[c][2]), fx::exp_field(v[c][3])));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        const unsigned int m = __reduce_max_sync(0xffffffffu, key[k]);
+        if ((tid & 31) == 0) keys[k][tid >> 5] = m;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 5; ++k)
+        key[k] = __reduce_max_sync(0xffffffffu, keys[k][tid & (NT / 32 - 1)]);
+    fx::Tops X;
+    if (!fx::tops_of(0xfffu - key[1], key[0], 0xfffu - key[3], key[2], key[4], P.gas, X))
+        return false;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int i = tid + c * NT;
+        if (i >= SY * SX) break;
+        const int ly = i / SX, lx = i - ly * SX;
+        const bool own = lx >= H && lx < TX + H && ly >= H && ly < TY + H;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            t.q[f * SY * SX + i] = fx::to_units(v[c][f], f == 0 ? X.r : (f == 1 ? X.p : X.v));
+            if (own) t.cell[(f * TY + ly - H) * TX + lx - H] = v[c][f];
+        }
+    }
+    __syncthreads();
+    Speeds fastest{0.0, 0.0};
+    faces_hllc<ORDER, TX, TY>(P, smem, X, tx0, ty0, dt_only, fastest);
+    __syncthreads();
+    update_cells<double, ORDER, TX, TY, TX, TX * TY>(P, out, tx0, ty0, T_do, dt_only, t.cell, t.fx,
+                                                     t.fy, res, aux);
+    res.umax_x = fastest.x;
+    res.umax_y = fastest.y;
+    return true;
+}
+
+// A tile of the step: in integers where the method is HLLC and the tile's range allows it.
+template <int ORDER, int TX, int TY>
+__device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, const Planes& out,
+                                          int tx0, int ty0, double T_do, int dt_only,
+                                          double* smem, TileResult& res, double* aux) {
+    if (P.method != GD_METHOD_HLL && euler_tile_int<ORDER, TX, TY>(P, in, out, tx0, ty0, T_do,
+                                                                   dt_only, smem, res, aux))
+        return;
+    __syncthreads();
+    euler_tile<double, ORDER, TX, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, res, aux);
 }
 
 __device__ __forceinline__ void add_counters(Scalars* ctr, const TileResult& r) {
@@ -560,9 +693,8 @@ __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_fast_kernel(Params P,
                                                         double* aux) {
     extern __shared__ double smem[];
     TileResult r;
-    euler_tile<double, ORDER, TX, TY>(P, in, out, blockIdx.x * TX,
-                                      (blockIdx.y + P.tile_row0) * TY, *T_do_ptr, dt_only, smem,
-                                      r, aux);
+    step_tile<ORDER, TX, TY>(P, in, out, blockIdx.x * TX, (blockIdx.y + P.tile_row0) * TY,
+                             *T_do_ptr, dt_only, smem, r, aux);
     add_counters(ctr, r);
     block_dt_and_rotate<NT>(P, r.umax_x, r.umax_y, r.any_active, T_bits, rot, P.tile_nblocks);
 }
@@ -618,8 +750,7 @@ __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_batch_kernel(const Ba
         const int tx0 = (tile % g.tiles_x) * TX, ty0 = (tile / g.tiles_x) * TY;
         const double T_do = g.sc->T_do;
         TileResult r;
-        euler_tile<double, ORDER, TX, TY>(g.P, in, out, tx0, ty0, T_do, dt_only, smem, r,
-                                          nullptr);
+        step_tile<ORDER, TX, TY>(g.P, in, out, tx0, ty0, T_do, dt_only, smem, r, nullptr);
         add_counters(dt_only ? nullptr : g.sc, r);
         block_dt_and_rotate<NT>(g.P, r.umax_x, r.umax_y, r.any_active, &g.sc->T_bits,
                                 dt_only ? nullptr : g.sc, (unsigned int)g.ntiles);
@@ -794,18 +925,14 @@ __global__ void euler_face_probe_kernel(Params P, long long n, int axis,
     const double* a = L + 4 * i;
     const double* b = R + 4 * i;
     const bool isx = axis == 0;
-    const double uL = isx ? a[2] : a[3], vL = isx ? a[3] : a[2];
-    const double uR = isx ? b[2] : b[3], vR = isx ? b[3] : b[2];
-    double UU;
+    const double qa[NF] = {a[0], a[1], isx ? a[2] : a[3], isx ? a[3] : a[2]};
+    const double qb[NF] = {b[0], b[1], isx ? b[2] : b[3], isx ? b[3] : b[2]};
+    double UU, f[NF];
     FluxE<double> F;
-    bool done = false;
-    if (P.method != GD_METHOD_HLL) {
-        const fx::Fan fan = fx::fan_of(a[0], a[1], uL, vL, b[0], b[1], uR, vR, P.gas, UU);
-        done = fan.ok && fx::hllc(fan, vL, vR, P.gas, F.m, F.mn, F.mt, F.e);
-    }
-    if (!done)
-        F = P.method == GD_METHOD_HLL ? hll_local(a[0], a[1], uL, vL, b[0], b[1], uR, vR, P, UU)
-                                      : hllc_local(a[0], a[1], uL, vL, b[0], b[1], uR, vR, P, UU);
+    if (P.method != GD_METHOD_HLL && fx::hllc_face(qa, qb, P.gas, f, UU))
+        F = FluxE<double>{f[0], f[1], f[2], f[3]};
+    else
+        F = flux_of(P, qa, qb, UU);
     double* o = flux + 4 * i;
     o[0] = F.m;
     o[1] = F.e;

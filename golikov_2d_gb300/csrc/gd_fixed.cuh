@@ -85,12 +85,6 @@ struct Pos {
     i64 m;
     int e;
 };
-// sign and exponent field of x
-GD_HD uint32_t sexp(double x) {
-    uint32_t hi, lo;
-    swfp::halves(x, hi, lo);
-    return hi >> 20;
-}
 GD_HD Pos pos_of(double x) {
     uint32_t hi, lo;
     swfp::halves(x, hi, lo);
@@ -100,37 +94,11 @@ GD_HD Pos pos_of(double x) {
     p.m = (i64)(((u64)((h << 10) | (lo >> 22)) << 32) | (lo << 10));
     return p;
 }
-// x in units of 2^(E - 61), |x| < 2^(E - 1); what lies below the unit is dropped
-GD_HD i64 in_units(double x, int E) {
-    uint32_t hi, lo;
-    swfp::halves(x, hi, lo);
-    const int e = (int)((hi >> 20) & 0x7ffu) - 1023;
-    const uint32_t h = (hi & 0xfffffu) | 0x100000u;
-    const u64 s = ((u64)((h << 9) | (lo >> 23)) << 32) | (lo << 9);
-    const i64 v = (i64)(s >> imin(E - e, 63));
-    return (int32_t)hi < 0 ? -v : v;
-}
-// x as a signed m 2^(e - 62), m = 0 for zero and subnormal x
-GD_HD Pos signed_of(double x) {
-    uint32_t hi, lo;
-    swfp::halves(x, hi, lo);
-    Pos p;
-    p.e = (int)((hi >> 20) & 0x7ffu) - 1023;
-    const uint32_t h = (hi & 0xfffffu) | 0x100000u;
-    i64 v = (i64)(((u64)((h << 10) | (lo >> 22)) << 32) | (lo << 10));
-    if (p.e == -1023) v = 0;
-    p.m = (int32_t)hi < 0 ? -v : v;
-    return p;
-}
-// x 2^ue rounded to the nearest double (ties away from zero); results are normal or 0
-GD_HD double pack(i64 x, int ue) {
-    const uint32_t neg = (uint32_t)(hi32(x) >> 31);
-    u64 a = (u64)(x < 0 ? -x : x);
-    const int lz = clz64(a);
-    a = lz < 64 ? a << lz : 0;
-    const u64 m = (a >> 11) + ((a >> 10) & 1);
-    const u64 b = m + ((u64)(uint32_t)(ue - lz + 63 + 1022) << 52);
-    return a == 0 ? 0.0 : swfp::from_halves((uint32_t)(b >> 32) | (neg & 0x80000000u), (uint32_t)b);
+// a signed state in units of 2^(top - 61) as m 2^(e - 62), m as large as fits unless tiny
+GD_HD Pos signed_of(i64 a, int top) {
+    const int32_t h = hi32(a);
+    const int z = clz32((uint32_t)(h ^ (h >> 31))) - 1;
+    return Pos{a << z, top + 1 - z};
 }
 
 // 1 / x for x > 0 with a nonzero high word: r 2^(lz - 124), lz the leading zeros of x, r in
@@ -184,48 +152,85 @@ inline Gas gas_of(double gamma) {
     return G;
 }
 
-// The wave speeds of the face between (rL, pL, uL, vL) and (rR, pR, uR, vR), its frame local:
-// all velocities in units of 2^(E - 61).  |u|, c < 2^(E - 1), so |S| < 2^61 and
-// |S - u| < 1.5 2^61 in these units.
+// The top exponents of a set of cells: densities, pressures and velocities are held in units of
+// 2^(r - 60), 2^(p - 60) and 2^(v - 60), below 2^61 each.  Densities and pressures within 2^8 of
+// each other (kSpan) are held exactly; a velocity is cut below 2^-60 of the largest.
+struct Tops {
+    int r, p, v;
+};
+constexpr int kSpan = 8;        // exponents that the densities, and the pressures, may span
+constexpr int kRange = 128;     // exponents of densities, pressures (both signs) and velocities
+// x in units of 2^(top - 60), |x| < 2^(top + 1)
+GD_HD i64 to_units(double x, int top) {
+    uint32_t hi, lo;
+    swfp::halves(x, hi, lo);
+    const int e = (int)((hi >> 20) & 0x7ffu) - 1023;
+    const uint32_t h = (hi & 0xfffffu) | 0x100000u;
+    const i64 v = (i64)((((u64)((h << 8) | (lo >> 24)) << 32) | (lo << 8)) >> imin(top - e, 63));
+    return (int32_t)hi < 0 ? -v : v;
+}
+// x 2^ue as a double
+GD_HD double to_double(i64 x, int ue) {
+#if defined(__CUDA_ARCH__)
+    uint32_t hi, lo;
+    swfp::halves(__ll2double_rn(x), hi, lo);
+    return swfp::from_halves(x == 0 ? 0u : hi + ((uint32_t)ue << 20), lo);
+#else
+    return std::ldexp((double)x, ue);
+#endif
+}
+// 0 unless a and b have the same sign, else the one of smaller magnitude
+GD_HD i64 minmod(i64 a, i64 b) {
+    const bool lt = a < b, neg = hi32(a) < 0;
+    const i64 m = lt != neg ? a : b;
+    return (hi32(a) ^ hi32(b)) < 0 ? 0 : m;
+}
+
+// The two sides of a face in its local frame, in units of half those of Tops (below 2^62).
+struct States {
+    i64 rL, rR, pL, pR, uL, uR, vL, vR;
+};
+// a positive state in units of 2^(top - 61), its high word not 0
+GD_HD Pos pos_of(i64 a, int top) {
+    const int lz = clz32((uint32_t)hi32(a));
+    return Pos{a << (lz - 1), top - lz + 2};
+}
+
+// The wave speeds of a face, all velocities in units of 2^(E - 61).  |u|, c < 2^(E - 1), so
+// |S| < 2^61 and |S - u| < 1.5 2^61 in these units.
 struct Fan {
     Pos RL, RR, PL, PR;
     i64 uL, uR, SL, SR;
     int E, kmin;  // kmin: 2^kmin is about the smaller sound speed
     bool ok;
 };
-// ok is false where a scale would leave a quantity fewer bits than binary64 does, or an input is
-// not a normal positive density or pressure or a finite velocity.  Accepted: densities and
-// pressures in 2^[-128, 128], densities within 2^8 of each other, velocities below 2^128, sound
-// speeds within a factor of about 4 of each other, normal velocities to about 64 of them.
-// UU: the larger wave speed.
-GD_HD Fan fan_of(double rL, double pL, double uL, double vL, double rR, double pR, double uR,
-                 double vR, const Gas& G, double& UU) {
-    const uint32_t low = 1023 - 128, span = 256, top = 1023 + 128;
-    const int xuL = (int)(sexp(uL) & 0x7ffu), xuR = (int)(sexp(uR) & 0x7ffu);
+// ok is false where a scale would leave a quantity fewer bits than binary64 does: accepted are
+// sound speeds within a factor of about 4 of each other, and normal velocities to about 64 of
+// them.  UU: the larger wave speed.
+GD_HD Fan fan_of(const States& q, const Tops& X, const Gas& G, double& UU) {
     Fan f;
-    f.RL = pos_of(rL);
-    f.RR = pos_of(rR);
-    f.PL = pos_of(pL);
-    f.PR = pos_of(pR);
+    f.RL = pos_of(q.rL, X.r);
+    f.RR = pos_of(q.rR, X.r);
+    f.PL = pos_of(q.pL, X.p);
+    f.PR = pos_of(q.pR, X.p);
     int kL, kR;
     const i64 wL = sqrt_over(mulk<0, 0>(f.PL.m, G.g), f.PL.e + G.ge, f.RL, kL);
     const i64 wR = sqrt_over(mulk<0, 0>(f.PR.m, G.g), f.PR.e + G.ge, f.RR, kR);
     const int kmax = imax(kL, kR);
     f.kmin = imin(kL, kR);
-    f.E = imax(kmax, imax(xuL, xuR) - 1023) + 2;
-    const int dr = f.RL.e - f.RR.e;
-    f.ok = G.room >= 0 && sexp(rL) - low <= span && sexp(rR) - low <= span && sexp(pL) - low <= span &&
-           sexp(pR) - low <= span && (uint32_t)xuL <= top && (uint32_t)xuR <= top &&
-           (sexp(vL) & 0x7ffu) <= top && (sexp(vR) & 0x7ffu) <= top && kmax - f.kmin <= 2 &&
-           f.E - kmax <= 8 && (uint32_t)(dr + 8) <= 16u;
+    const int32_t hL = hi32(q.uL), hR = hi32(q.uR);
+    const int lz = clz32((uint32_t)((hL ^ (hL >> 31)) | (hR ^ (hR >> 31))));
+    f.E = imax(kmax + 2, X.v + imax(4 - lz, 0));
+    f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 8;
     if (!f.ok) return f;
     const i64 cL = wL >> (f.E - 1 - kL), cR = wR >> (f.E - 1 - kR);
-    f.uL = in_units(uL, f.E);
-    f.uR = in_units(uR, f.E);
+    const int sh = imin(f.E - X.v, 63);
+    f.uL = q.uL >> sh;
+    f.uR = q.uR >> sh;
     const i64 aL = f.uL - cL, aR = f.uR - cR, bL = f.uL + cL, bR = f.uR + cR;
     f.SL = aL < aR ? aL : aR;
     f.SR = bL > bR ? bL : bR;
-    UU = pack(-f.SL > f.SR ? -f.SL : f.SR, f.E - 61);
+    UU = to_double(-f.SL > f.SR ? -f.SL : f.SR, f.E - 61);
     return f;
 }
 
@@ -234,8 +239,8 @@ GD_HD Fan fan_of(double rL, double pL, double uL, double vL, double rR, double p
 // velocity is more than about 4 sound speeds; the caller then takes hllc_local.  SL < S_M < SR
 // (the Davis speeds, with positive pressures), and inside the fan S_M and S have opposite signs,
 // so |S_M / (S - S_M)| <= 1: no product below overflows.
-GD_HD bool hllc(const Fan& f, double vL, double vR, const Gas& G, double& Fm, double& Fn,
-                double& Ft, double& Fe) {
+GD_HD bool hllc(const Fan& f, const States& s, const Tops& X, const Gas& G, double& Fm,
+                double& Fn, double& Ft, double& Fe) {
     const int E = f.E, ER = imax(f.RL.e, f.RR.e);
     const i64 suL = f.SL - f.uL, suR = f.SR - f.uR;
     // r (S - u), each side in units of its own density's, 2^(e + E - 59), and in the larger's
@@ -256,7 +261,7 @@ GD_HD bool hllc(const Fan& f, double vL, double vR, const Gas& G, double& Fm, do
     const Pos Pk{takeL ? f.PL.m : f.PR.m, takeL ? f.PL.e : f.PR.e};
     const i64 un = takeL ? f.uL : f.uR, S = takeL ? f.SL : f.SR;
     const i64 o = takeL ? oL : oR;
-    const Pos T = signed_of(takeL ? vL : vR);
+    const Pos T = signed_of(takeL ? s.vL : s.vR, X.v);
 
     i64 qs = un;  // outside the fan the physical flux: S_M -> u, q (S - u) -> u
     if (star) {
@@ -277,14 +282,14 @@ GD_HD bool hllc(const Fan& f, double vL, double vR, const Gas& G, double& Fm, do
     const i64 qn = qs << z;
     const i64 M = mulk<0, 0>(R.m, qn);
     const int em = R.e + E - 59 - z;
-    Fm = pack(M, em);
+    Fm = to_double(M, em);
     // momentum: p + r q su S_M + r su (S_M - u); exactly p where the rest is 0
     const i64 t = (mulk<1, 2>(M, SM) >> z) + mulk<2, 1>(o, SMu);
     const int et = R.e + 2 * E - 59;
     const i64 pt = (Pk.m >> imin(et - Pk.e + 62, 63)) + t;
-    Fn = pack(t == 0 ? Pk.m : pt, t == 0 ? Pk.e - 62 : et);
+    Fn = to_double(t == 0 ? Pk.m : pt, t == 0 ? Pk.e - 62 : et);
     const i64 MT = mulk<0, 0>(M, T.m);
-    Ft = pack(MT, em + T.e + 2);
+    Ft = to_double(MT, em + T.e + 2);
     // energy: q su (p gamma / (gamma - 1) + r (u^2 / 2 + S (S_M - u))) + (mass flux) v^2 / 2
     const i64 H = mulk<1, 1>(un, un) + mulk<2, 1>(S, SMu);
     const i64 B = sra(mulk<0, 0>(Pk.m, G.gg), R.e + 2 * E - Pk.e - G.gge + G.room) +
@@ -293,8 +298,48 @@ GD_HD bool hllc(const Fan& f, double vL, double vR, const Gas& G, double& Fm, do
     const i64 e2 = mulk<2, 0>(MT, T.m);
     const int dx = 2 * (E - T.e) + 1 + G.room;
     const int x1 = R.e + 3 * E - 57 - z + G.room;
-    Fe = pack(sra(e1, imax(-dx, 0)) + sra(e2, imax(dx, 0)), dx > 0 ? x1 : x1 - dx);
+    Fe = to_double(sra(e1, imax(-dx, 0)) + sra(e2, imax(dx, 0)), dx > 0 ? x1 : x1 - dx);
     return true;
+}
+
+// Exponent field of x (0x7ff for infinities and NaN), and with its sign bit above it.
+GD_HD uint32_t exp_field(double x) {
+    uint32_t hi, lo;
+    swfp::halves(x, hi, lo);
+    return (hi >> 20) & 0x7ffu;
+}
+GD_HD uint32_t signed_exp_field(double x) {
+    uint32_t hi, lo;
+    swfp::halves(x, hi, lo);
+    return hi >> 20;
+}
+// Whether cells whose densities have exponent fields (sign bit included) in [r0, r1], pressures
+// in [p0, p1] and velocities up to v1 can be held in the units of Tops.
+GD_HD bool tops_of(uint32_t r0, uint32_t r1, uint32_t p0, uint32_t p1, uint32_t v1, const Gas& G,
+                   Tops& X) {
+    const uint32_t low = 1023 - kRange, high = 1023 + kRange;
+    X.r = (int)r1 - 1023;
+    X.p = (int)p1 - 1023;
+    X.v = imax((int)v1 - 1023, -900);  // zeros and subnormals come out as 0
+    return G.room >= 0 && r0 >= low && r1 <= high && r1 - r0 <= kSpan && p0 >= low &&
+           p1 <= high && p1 - p0 <= kSpan && v1 <= high;
+}
+// The flux and the larger wave speed of one face given by its two states; false where the
+// integer solver does not take it.
+GD_HD bool hllc_face(const double* L, const double* R, const Gas& G, double* F, double& UU) {
+    const uint32_t rL = signed_exp_field(L[0]), rR = signed_exp_field(R[0]);
+    const uint32_t pL = signed_exp_field(L[1]), pR = signed_exp_field(R[1]);
+    const uint32_t v0 = imax(exp_field(L[2]), exp_field(L[3]));
+    const uint32_t v1 = imax(exp_field(R[2]), exp_field(R[3]));
+    Tops X;
+    if (!tops_of(rL < rR ? rL : rR, rL < rR ? rR : rL, pL < pR ? pL : pR, pL < pR ? pR : pL,
+                 v0 < v1 ? v1 : v0, G, X))
+        return false;
+    const States s{2 * to_units(L[0], X.r), 2 * to_units(R[0], X.r), 2 * to_units(L[1], X.p),
+                   2 * to_units(R[1], X.p), 2 * to_units(L[2], X.v), 2 * to_units(R[2], X.v),
+                   2 * to_units(L[3], X.v), 2 * to_units(R[3], X.v)};
+    const Fan f = fan_of(s, X, G, UU);
+    return f.ok && hllc(f, s, X, G, F[0], F[1], F[2], F[3]);
 }
 
 }  // namespace fx
