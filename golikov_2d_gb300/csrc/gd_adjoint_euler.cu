@@ -43,13 +43,12 @@ __global__ void __launch_bounds__(NT) eadj_update_kernel(Params P, CPlanes U, co
         double r2 = r - d[0];
         const bool rfl = le_zero(r2);
         if (rfl) r2 = 0.0001;
-        const double inv = rcp_2op(r2);
+        const double inv = rcp_fast(r2);
         const double mx2 = fma(r, u, -d[2]), my2 = fma(r, v, -d[3]);
         const double u2 = imul(mx2, inv), v2 = imul(my2, inv);
         const double w = fma(u, u, imul(v, v));
-        const double K1 = r * w;
         const double K2 = fma(mx2, u2, imul(my2, v2));
-        const double p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, d[1], p));
+        const double p2 = fma(P.hgm1, fma(r, w, -K2), fma(-P.gm1, d[1], p));
         const bool pfl = le_zero(p2);
         // reverse; a floored value is a constant
         double r2b = lam_out.f[0][k], u2b = lam_out.f[2][k], v2b = lam_out.f[3][k];
@@ -57,7 +56,7 @@ __global__ void __launch_bounds__(NT) eadj_update_kernel(Params P, CPlanes U, co
         double db[NF] = {0, 0, 0, 0};
         double rb = 0.0, pb = 0.0, ub = 0.0, vb = 0.0, mx2b = 0.0, my2b = 0.0;
         if (!pfl) {
-            // p2 = p - gm1 d1 + hgm1 (K1 - K2), K1 = r (u^2 + v^2), K2 = mx2 u2 + my2 v2
+            // p2 = p - gm1 d1 + hgm1 (r (u^2 + v^2) - K2), K2 = mx2 u2 + my2 v2
             pb = p2b;
             db[1] = -p2b * P.gm1;
             const double Kb = p2b * P.hgm1;

@@ -350,6 +350,12 @@ struct TileResult {
     unsigned int nfl_r, nfl_p, nbad;
 };
 
+// a b rounded by itself: every operation of the update is written out, so that the kernels that
+// inline it round alike whatever the compiler would contract in each.
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ Dual mul_rn(Dual a, Dual b) { return a * b; }
+__device__ __forceinline__ Dual mul_rn(double a, Dual b) { return a * b; }
+
 // ---- U: conservative update of the tile's cells ---------------------------------------------
 // cell: the tile's own values, rows RS and fields FS apart.
 template <class T, int ORDER, int TX, int TY, int RS, int FS, class OUT>
@@ -383,7 +389,7 @@ __device__ __forceinline__ void update_cells(const Params& P, const OUT& out, in
         for (int f = 0; f < NF; ++f) {
             const T* a = fxc + f * TY * (TX + 1);
             const T* b = fyc + f * (TY + 1) * TX;
-            d[f] = fma(kx, a[1] - a[0], mulx(ky, b[TX] - b[0]));
+            d[f] = fma(kx, a[1] - a[0], mul_rn(ky, b[TX] - b[0]));
         }
         if constexpr (std::is_same<T, double>::value) {
             if (aux != nullptr) {  // the recording of the adjoint: the flux differences used
@@ -394,15 +400,15 @@ __device__ __forceinline__ void update_cells(const Params& P, const OUT& out, in
         }
         T r2 = r - d[0];
         if (le_zero(r2)) { r2 = cst<T>(0.0001); ++nfl_r; }
-        const T inv = rcp_2op(r2);
+        const T inv = rcp_fast(r2);
         const T mx2 = fma(r, u, -d[2]), my2 = fma(r, v, -d[3]);
-        const T u2 = mulx(mx2, inv);
-        const T v2 = mulx(my2, inv);
+        const T u2 = mul_rn(mx2, inv);
+        const T v2 = mul_rn(my2, inv);
         // p' = (gamma - 1) (E - d_E - K'/2) with E = p / (gamma - 1) + K / 2, K = rho |v|^2,
         // K' = rho' |v'|^2 = m' . v' (kernel.cu:1861-1870)
-        const T K1 = r * fma(u, u, mulx(v, v));
-        const T K2 = fma(mx2, u2, mulx(my2, v2));
-        T p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, d[1], p));
+        const T K2 = fma(mx2, u2, mul_rn(my2, v2));
+        const T dK = fma(r, fma(u, u, mul_rn(v, v)), -K2);
+        T p2 = fma(P.hgm1, dK, fma(-P.gm1, d[1], p));
         if (le_zero(p2)) { p2 = cst<T>(0.000001); ++nfl_p; }
         if (!finite_bits(r2) || !finite_bits(p2) || !finite_bits(u2) || !finite_bits(v2)) ++nbad;
         store_cell2(out, k, 0, r2, p2);
@@ -597,7 +603,7 @@ __device__ __forceinline__ void faces_hllc(const Params& P, double* smem, const 
 // Returns false, with nothing written, where the tile's cells cannot be held in common units.
 // Every thread of the block must call it, and all get the same answer.
 template <int ORDER, int TX, int TY>
-__device__ __noinline__ bool euler_tile_int(const Params& P, const CPlanes& in, const Planes& out,
+__device__ __forceinline__ bool euler_tile_int(const Params& P, const CPlanes& in, const Planes& out,
                                             int tx0, int ty0, double T_do, int dt_only,
                                             double* smem, TileResult& res, double* aux) {
     using S = Shape<ORDER, TX, TY>;
@@ -686,7 +692,9 @@ __device__ __forceinline__ void add_counters(Scalars* ctr, const TileResult& r) 
 }
 
 template <int ORDER, int TX, int TY>
-__global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_fast_kernel(Params P, CPlanes in, Planes out,
+__global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_fast_kernel(const __grid_constant__ Params P,
+                                                        const __grid_constant__ CPlanes in,
+                                                        const __grid_constant__ Planes out,
                                                         const double* __restrict__ T_do_ptr,
                                                         unsigned long long* T_bits, Scalars* rot,
                                                         Scalars* ctr, int dt_only,
