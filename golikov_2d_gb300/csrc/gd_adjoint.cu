@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(NT) adj_update_kernel(Params P, CPlanes U, con
         // forward (same operations as the tile update)
         const double ub = fma(u, bx, imul(v, by));
         const double bb = fma(bz, bz, fma(by, by, imul(bx, bx)));
-        const double E = fma(p, P.inv_gm1, half_exact(fma(r, fma(u, u, imul(v, v)), bb)));
+        const double K1 = fma(r, fma(u, u, imul(v, v)), bb);
         double r2 = r - d[0];
         const bool rfl = le_zero(r2);
         if (rfl) r2 = r;
@@ -59,11 +59,12 @@ __global__ void __launch_bounds__(NT) adj_update_kernel(Params P, CPlanes U, con
         const double bx2 = bx - fma(u, divb, d[4]);
         const double by2 = by - fma(v, divb, d[5]);
         const double bz2 = bz - d[6];
-        const double E2 = E - fma(ub, divb, d[1]);
+        const double dE = fma(ub, divb, d[1]);
         const double inv = rcp_fast(r2);
         const double u2 = imul(mx2, inv), v2 = imul(my2, inv);
-        const double p2 = (E2 - 0.5 * fma(r2, fma(u2, u2, imul(v2, v2)),
-                                          fma(bz2, bz2, fma(by2, by2, imul(bx2, bx2))))) * P.gm1;
+        const double K2 = fma(r2, fma(u2, u2, imul(v2, v2)),
+                              fma(bz2, bz2, fma(by2, by2, imul(bx2, bx2))));
+        const double p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, dE, p));
         const bool pfl = le_zero(p2);
         // reverse
         double r2b = lam_out.f[0][k], p2b = lam_out.f[1][k];
@@ -1023,7 +1024,7 @@ __device__ __forceinline__ unsigned int floor_code(const Params& P, const CPlane
     const double divb = aux[(size_t)7 * K + k];
     const double ub = fma(u, bx, v * by);
     const double bb = fma(bz, bz, fma(by, by, bx * bx));
-    const double E = fma(p, P.inv_gm1, 0.5 * fma(r, fma(u, u, v * v), bb));
+    const double K1 = fma(r, fma(u, u, v * v), bb);
     double r2 = r - d[0];
     const bool rfl = le_zero(r2);
     if (rfl) r2 = r;
@@ -1032,11 +1033,11 @@ __device__ __forceinline__ unsigned int floor_code(const Params& P, const CPlane
     const double bx2 = bx - fma(u, divb, d[4]);
     const double by2 = by - fma(v, divb, d[5]);
     const double bz2 = bz - d[6];
-    const double E2 = E - fma(ub, divb, d[1]);
+    const double dE = fma(ub, divb, d[1]);
     const double inv = rcp_fast(r2);
     const double u2 = mx2 * inv, v2 = my2 * inv;
-    const double p2 = (E2 - 0.5 * fma(r2, fma(u2, u2, v2 * v2),
-                                      fma(bz2, bz2, fma(by2, by2, bx2 * bx2)))) * P.gm1;
+    const double K2 = fma(r2, fma(u2, u2, v2 * v2), fma(bz2, bz2, fma(by2, by2, bx2 * bx2)));
+    const double p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, dE, p));
     return (rfl ? 1u : 0u) | (le_zero(p2) ? 2u : 0u);
 }
 

@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "gd_dual.cuh"
+#include "gd_fixed_mhd.cuh"
 #include "gd_internal.cuh"
 #include "gd_kernels.h"
 #include "gd_mhd_flux.cuh"
@@ -104,18 +105,28 @@ __device__ __forceinline__ void copy_cell(const DualCPlanes& in, const DualPlane
     }
 }
 
-template <class T, int ORDER, int TY>
+// SLOPES: slope arrays beside the cells; without them each face forms its cells' slopes.
+template <class T, int ORDER, int TY, bool SLOPES = true>
 struct SmemM {
     static constexpr int H = ORDER == 2 ? 2 : 1;
     static constexpr int SX = TX + 2 * H;
     static constexpr int SY = TY + 2 * H;
     static constexpr int kPrim = NF * SY * SX;
-    static constexpr int kSlx = ORDER == 2 ? NF * TY * (TX + 2) : 0;
-    static constexpr int kSly = ORDER == 2 ? NF * (TY + 2) * TX : 0;
+    static constexpr int kSlx = ORDER == 2 && SLOPES ? NF * TY * (TX + 2) : 0;
+    static constexpr int kSly = ORDER == 2 && SLOPES ? NF * (TY + 2) * TX : 0;
     static constexpr int kFx = NF * TY * (TX + 1);
     static constexpr int kFy = NF * (TY + 1) * TX;
+    static constexpr int kCell = NF * TX * TY;
     static constexpr size_t bytes = sizeof(T) * (kPrim + kSlx + kSly + kFx + kFy);
 };
+// The HLLD step's tile in integers: no slopes, the cells' own values beside them.  Its float tile
+// (for ranges the integers cannot hold) works without slope arrays, in the same room: 69 KB, three
+// CTAs per SM.  The HLLC-MHD step always works in floating point, with slope arrays (88 KB, two).
+template <int ORDER, int TY, bool HLLD>
+constexpr size_t step_bytes() {
+    using I = SmemM<double, ORDER, TY, false>;
+    return HLLD ? I::bytes + sizeof(double) * I::kCell : SmemM<double, ORDER, TY>::bytes;
+}
 
 struct MhdTileResult {
     double umax_x, umax_y;
@@ -123,16 +134,188 @@ struct MhdTileResult {
     unsigned int nfl_r, nfl_p, nbad;
 };
 
+// One face of a tile: faces 0 .. NFX-1 have an x normal, the rest a y normal.
+template <int TY>
+struct FaceM {
+    static constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
+    bool isx, used;
+    int lx, ly;
+    // used: inside the grid, and next to a cell that the step updates
+    __device__ FaceM(const Params& P, int tx0, int ty0, int i) {
+        isx = i < NFX;
+        if (isx) {
+            ly = i / (TX + 1);
+            lx = i - ly * (TX + 1);
+            used = tx0 + lx <= P.N && ty0 + ly < P.M;
+        } else {
+            const int j = i - NFX;
+            ly = j / TX;
+            lx = j - ly * TX;
+            used = tx0 + lx < P.N && ty0 + ly <= P.M;
+        }
+        if (used && P.frozen)
+            used = cell_active(P, tx0 + (isx ? lx - 1 : lx), ty0 + (isx ? ly : ly - 1)) ||
+                   cell_active(P, tx0 + lx, ty0 + ly);
+    }
+    // field of the local frame's component f: x-face (n, t) = (x, y); y-face (n, t) = (y, x)
+    __device__ __forceinline__ int field(int f) const {
+        return isx || f < 2 || f == 6 ? f : (f < 4 ? 5 - f : 9 - f);
+    }
+    template <class T>
+    __device__ __forceinline__ void store(T* fx, T* fy, const FluxM<T>& F) const {
+        constexpr int sx = TY * (TX + 1), sy = (TY + 1) * TX;
+        T* fo = isx ? fx + ly * (TX + 1) + lx : fy + ly * TX + lx;
+        const int st = isx ? sx : sy;
+        fo[0 * st] = F.m;
+        fo[1 * st] = F.e;
+        fo[2 * st] = isx ? F.mn : F.mt;
+        fo[3 * st] = isx ? F.mt : F.mn;
+        fo[4 * st] = isx ? F.bn : F.bt;
+        fo[5 * st] = isx ? F.bt : F.bn;
+        fo[6 * st] = F.bz;
+    }
+};
+
+struct SpeedsM {
+    double x, y;
+    __device__ __forceinline__ void take(bool isx, double UU) {
+        if (isx) x = max_nonneg(x, UU);
+        else y = max_nonneg(y, UU);
+    }
+};
+
+// the flux in floating point between two states of the local frame
+template <class T>
+__device__ __forceinline__ FluxM<T> float_flux(const Params& P, const T* qa, const T* qb, T& UU) {
+    Side<T> A, B;
+    side(A, qa[0], qa[1], qa[2], qa[3], qa[4], qa[5], qa[6], P);
+    side(B, qb[0], qb[1], qb[2], qb[3], qb[4], qb[5], qb[6], P);
+    return hlld_local(A, B, P.method, P, UU);
+}
+// the states on either side of a face, c + d/2 and c - d/2; rho and p fall back to the cell's
+template <class T>
+__device__ __forceinline__ void side_states(int f, T ca, T da, T cb, T db, T& a, T& b) {
+    a = fma(0.5, da, ca);
+    b = fma(-0.5, db, cb);
+    if (f < 2) {
+        a = le_zero(a) ? ca : a;
+        b = le_zero(b) ? cb : b;
+    }
+}
+
+// ---- U: update (kernel.cu:2606-2660 in Heaviside-Lorentz field units) --------------------------
+// cell: the tile's own values, rows RS and fields FS apart; jump: b_x across a cell in x and b_y
+// in y, from its neighbours.
+template <class T, int TY, int RS, int FS, class IN, class OUT, class JUMP>
+__device__ __forceinline__ void update_cells(const Params& P, const IN& in, const OUT& out, int tx0,
+                                             int ty0, double T_do, int dt_only, const T* cell,
+                                             const JUMP& jump, const T* fx, const T* fy,
+                                             MhdTileResult& res, double* aux) {
+    const int N = P.N, M = P.M;
+    const double kx = imul<true>(T_do, P.inv_dx), ky = imul<true>(T_do, P.inv_dy);
+    const double hkx = half_exact(kx), hky = half_exact(ky);  // 0.5 kx, 0.5 ky
+    const bool axi = P.geometry == GD_AXISYM;
+    bool any_active = false;
+    unsigned int nfl_r = 0, nfl_p = 0, nbad = 0;
+    for (int i = threadIdx.x; i < TX * TY; i += NT) {
+        const int ly = i / TX, lx = i - ly * TX;
+        const int gx = tx0 + lx, gy = ty0 + ly;
+        if (gx >= N || gy >= M) continue;
+        const T* c = cell + ly * RS + lx;
+        const T r = c[0], p = c[FS], u = c[2 * FS], v = c[3 * FS];
+        const T bx = c[4 * FS], by = c[5 * FS], bz = c[6 * FS];
+        const long long k = (long long)gy * N + gx;
+        if (P.frozen && !cell_active(P, gx, gy)) {  // the faces' own test
+            if (!dt_only) copy_cell(in, out, k);
+            continue;
+        }
+        any_active = true;
+        if (dt_only) continue;
+        const T* fxc = fx + ly * (TX + 1) + lx;
+        const T* fyc = fy + ly * TX + lx;
+        T d[NF];
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const T* a = fxc + f * TY * (TX + 1);
+            const T* b = fyc + f * (TY + 1) * TX;
+            d[f] = fma(kx, a[1] - a[0], ky * (b[TX] - b[0]));
+        }
+        // Powell divergence from cell-centred field: dx dy div b (kernel.cu:2568-2604)
+        T divb = fma(hkx, jump.x(lx, ly), mulx<true>(hky, jump.y(lx, ly)));  // T_do * div b
+        const double iy = axi ? rcp_fast(P.y0 + gy * P.dy) : 0.0;
+        if (axi) divb = fma(T_do * by, iy, divb);                 // kernel.cu:2615
+        if constexpr (std::is_same<T, double>::value) {
+            if (aux != nullptr) {
+                const long long KK = (long long)N * M;
+#pragma unroll
+                for (int f = 0; f < NF; ++f) aux[f * KK + k] = d[f];
+                aux[7 * KK + k] = divb;
+            }
+        }
+        const T ub = fma(u, bx, v * by);
+        const T bb = fma(bz, bz, fma(by, by, bx * bx));
+        const T K1 = fma(r, fma(u, u, v * v), bb);  // twice the kinetic and field energy
+        T r2 = r - d[0];
+        T mx2 = fma(r, u, -fma(bx, divb, d[2]));
+        T my2 = fma(r, v, -fma(by, divb, d[3]));
+        T bx2 = bx - fma(u, divb, d[4]);
+        const T by2 = by - fma(v, divb, d[5]);
+        const T bz2 = bz - d[6];
+        T dE = fma(ub, divb, d[1]);
+        if (axi) {
+            // geometric sources / y (kernel.cu:2619-2648) in field units b
+            const double ty = T_do * iy;
+            r2 = fma(-ty * r, v, r2);
+            mx2 = fma(-ty, fma(r * u, v, -bx * by), mx2);
+            my2 = fma(-ty, fma(r * v, v, fma(bz, bz, -by * by)), my2);
+            bx2 = fma(-ty, fma(v, bx, -by * u), bx2);
+            dE = fma(ty, fma(fma(p, P.g_gm1, 0.5 * (K1 + bb)), v, -by * ub), dE);
+        }
+        if (le_zero(r2)) { r2 = r; ++nfl_r; }
+        const T inv = rcp_fast(r2);
+        const T u2 = mx2 * inv, v2 = my2 * inv;
+        // p' = p - (gamma - 1) (d_E - (K - K') / 2): no sum of the whole energy to round
+        const T K2 = fma(r2, fma(u2, u2, v2 * v2), fma(bz2, bz2, fma(by2, by2, bx2 * bx2)));
+        T p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, dE, p));
+        if (le_zero(p2)) { p2 = cst<T>(0.000001); ++nfl_p; }
+        if (!finite_bits(r2) || !finite_bits(p2) || !finite_bits(u2) || !finite_bits(v2) ||
+            !finite_bits(bx2) || !finite_bits(by2) || !finite_bits(bz2))
+            ++nbad;
+        store_state2(out, k, 0, r2, p2);
+        store_state2(out, k, 2, u2, v2);
+        store_state(out, k, 4, bx2 * kSpi4);
+        store_state(out, k, 5, by2 * kSpi4);
+        store_state(out, k, 6, bz2 * kSpi4);
+    }
+    res.any_active = any_active;
+    res.nfl_r = nfl_r;
+    res.nfl_p = nfl_p;
+    res.nbad = nbad;
+}
+
+template <class T, int SX, int FS>
+struct JumpFloat {
+    const T* own;  // the tile's first cell
+    __device__ __forceinline__ T x(int lx, int ly) const {
+        const T* c = own + 4 * FS + ly * SX + lx;
+        return c[1] - c[-1];
+    }
+    __device__ __forceinline__ T y(int lx, int ly) const {
+        const T* c = own + 5 * FS + ly * SX + lx;
+        return c[SX] - c[-SX];
+    }
+};
+
 // One TX x TY tile at (tx0, ty0): load, slopes, faces, update.  IN/OUT are CPlanes/Planes
 // for T = double and DualCPlanes/DualPlanes for T = Dual.
 // flux component slots in smem: 0 mass, 1 energy, 2 mom x, 3 mom y, 4 bx, 5 by, 6 bz
 // `aux` (T = double only; may be null) receives, per cell, the flux differences d[0..6]
 // and the Powell term divb that the update used (planes of N*M), for the adjoint.
-template <class T, int ORDER, int TY, class IN, class OUT>
-__device__ __forceinline__ void mhd_tile(const Params& P, const IN& in, const OUT& out, int tx0,
+template <class T, int ORDER, int TY, bool SLOPES, class IN, class OUT>
+__device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& out, int tx0,
                                          int ty0, double T_do, int dt_only, T* smem,
-                                         MhdTileResult& res, double* aux = nullptr) {
-    using S = SmemM<T, ORDER, TY>;
+                                         MhdTileResult& res, double* aux) {
+    using S = SmemM<T, ORDER, TY, SLOPES>;
     constexpr int H = S::H, SX = S::SX, SY = S::SY;
     T* prim = smem;
     T* slx = prim + S::kPrim;
@@ -167,7 +350,7 @@ __device__ __forceinline__ void mhd_tile(const Params& P, const IN& in, const OU
 
     // ---- S: slopes ---------------------------------------------------------------------------
     // a thread takes a run of G cells, so neighbouring slopes share their difference
-    if (ORDER == 2) {
+    if (ORDER == 2 && SLOPES) {
         constexpr int GX = (TX + 2) % 3 == 0 ? 3 : 2, GY = (TY + 2) % 3 == 0 ? 3 : 2;
         constexpr int NGX = (TX + 2) / GX, NGY = (TY + 2) / GY;
         static_assert((TX + 2) % GX == 0 && (TY + 2) % GY == 0, "slope runs tile the rows");
@@ -207,181 +390,248 @@ __device__ __forceinline__ void mhd_tile(const Params& P, const IN& in, const OU
     }
 
     // ---- F: faces ----------------------------------------------------------------------------
-    double umax_x = 0.0, umax_y = 0.0;
-    constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
-    for (int i = tid; i < NFX + NFY; i += NT) {
-        const bool isx = i < NFX;
-        int lx, ly;
-        if (isx) {
-            ly = i / (TX + 1);
-            lx = i - ly * (TX + 1);
-            if (tx0 + lx > N || ty0 + ly >= M) continue;
-        } else {
-            const int j = i - NFX;
-            ly = j / TX;
-            lx = j - ly * TX;
-            if (tx0 + lx >= N || ty0 + ly > M) continue;
-        }
-        const int ax = isx ? lx - 1 : lx, ay = isx ? ly : ly - 1;
-        if (P.frozen && !cell_active(P, tx0 + ax, ty0 + ay) &&
-            !cell_active(P, tx0 + lx, ty0 + ly))
-            continue;
-        const T* pa = prim + (ay + H) * SX + (ax + H);
-        const T* pb = pa + (isx ? 1 : SX);
-        T qa[NF], qb[NF];
+    SpeedsM u{0.0, 0.0};
+    for (int i = tid; i < FaceM<TY>::NFX + FaceM<TY>::NFY; i += NT) {
+        const FaceM<TY> w(P, tx0, ty0, i);
+        if (!w.used) continue;
+        const int lx = w.lx, ly = w.ly;
+        const T* pb = prim + (ly + H) * SX + (lx + H);
+        const T* pa = pb - (w.isx ? 1 : SX);
+        T qa[NF], qb[NF], UU;
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-            const T ca = pa[f * SY * SX], cb = pb[f * SY * SX];
+            const int g = w.field(f);
+            qa[f] = pa[g * SY * SX];
+            qb[f] = pb[g * SY * SX];
             if (ORDER == 2) {
                 T da, db;
-                if (isx) {
-                    da = slx[(f * TY + ly) * (TX + 2) + lx];
-                    db = slx[(f * TY + ly) * (TX + 2) + lx + 1];
+                if (!SLOPES) {
+                    const int st = w.isx ? 1 : SX;
+                    const T *ga = pa + g * SY * SX, *gb = pb + g * SY * SX, d = gb[0] - ga[0];
+                    da = minmod(ga[0] - ga[-st], d);
+                    db = minmod(d, gb[st] - gb[0]);
+                } else if (w.isx) {
+                    da = slx[(g * TY + ly) * (TX + 2) + lx];
+                    db = slx[(g * TY + ly) * (TX + 2) + lx + 1];
                 } else {
-                    da = sly[(f * (TY + 2) + ly) * TX + lx];
-                    db = sly[(f * (TY + 2) + ly + 1) * TX + lx];
+                    da = sly[(g * (TY + 2) + ly) * TX + lx];
+                    db = sly[(g * (TY + 2) + ly + 1) * TX + lx];
                 }
-                T a = fma(0.5, da, ca), b = fma(-0.5, db, cb);
-                if (f < 2) {
-                    a = le_zero(a) ? ca : a;
-                    b = le_zero(b) ? cb : b;
-                }
-                qa[f] = a;
-                qb[f] = b;
-            } else {
-                qa[f] = ca;
-                qb[f] = cb;
+                side_states(f, qa[f], da, qb[f], db, qa[f], qb[f]);
             }
         }
-        // local frame: x-face (n, t) = (x, y); y-face (n, t) = (y, x); z stays z
-        Side<T> A, B;
-        side(A, qa[0], qa[1], isx ? qa[2] : qa[3], isx ? qa[3] : qa[2], isx ? qa[4] : qa[5],
-             isx ? qa[5] : qa[4], qa[6], P);
-        side(B, qb[0], qb[1], isx ? qb[2] : qb[3], isx ? qb[3] : qb[2], isx ? qb[4] : qb[5],
-             isx ? qb[5] : qb[4], qb[6], P);
-        T UU;
-        const FluxM<T> F = hlld_local(A, B, P.method, P, UU);
-        if (isx) {
-            T* fo = fx + ly * (TX + 1) + lx;
-            constexpr int st = TY * (TX + 1);
-            fo[0 * st] = F.m;
-            fo[1 * st] = F.e;
-            fo[2 * st] = F.mn;
-            fo[3 * st] = F.mt;
-            fo[4 * st] = F.bn;
-            fo[5 * st] = F.bt;
-            fo[6 * st] = F.bz;
-            umax_x = max_nonneg(umax_x, value_of(UU));
-        } else {
-            T* fo = fy + ly * TX + lx;
-            constexpr int st = (TY + 1) * TX;
-            fo[0 * st] = F.m;
-            fo[1 * st] = F.e;
-            fo[2 * st] = F.mt;
-            fo[3 * st] = F.mn;
-            fo[4 * st] = F.bt;
-            fo[5 * st] = F.bn;
-            fo[6 * st] = F.bz;
-            umax_y = max_nonneg(umax_y, value_of(UU));
+        w.store(fx, fy, float_flux(P, qa, qb, UU));
+        u.take(w.isx, value_of(UU));
+    }
+    __syncthreads();
+
+    const T* own = prim + H * SX + H;
+    update_cells<T, TY, SX, SY * SX>(P, in, out, tx0, ty0, T_do, dt_only, own,
+                                     JumpFloat<T, SX, SY * SX>{own}, fx, fy, res, aux);
+    res.umax_x = u.x;
+    res.umax_y = u.y;
+}
+
+// ---- The same tile with its face work in 64-bit integers (HLLD) --------------------------------
+//
+// HLLD takes about 150 binary64 operations a face; on the FP64 pipe, at 64 cycles of a sub-
+// partition each, they held the tile to 35 000 cycles per 32 cells.  Here the cells of the tile
+// and its halo are integers in units of the tile's own largest density, pressure, velocity and
+// field (fx::TopsM), slopes and face states are adds and selects, and the flux is fx::hlld.  The
+// FP64 pipe keeps the conversion of the fluxes and the update.
+template <int ORDER, int TY>
+struct MemInt {
+    using S = SmemM<double, ORDER, TY, false>;
+    fx::i64* q;    // [NF][SY][SX]
+    double* cell;  // [NF][TY][TX]
+    double *fx, *fy;
+    __device__ explicit MemInt(double* smem)
+        : q(reinterpret_cast<fx::i64*>(smem)), cell(smem + S::kPrim), fx(cell + S::kCell),
+          fy(fx + S::kFx) {}
+};
+
+// The faces of a thread that the integer solver left (bit k: the k-th), in floating point; speed:
+// those whose wave speed is missing too.  Out of line and after the loop over the faces, so that
+// it takes no registers from it.
+template <int ORDER, int TY>
+__device__ __noinline__ void faces_left(const Params& P, double* smem, const fx::TopsM& X, int tx0,
+                                        int ty0, unsigned int left, unsigned int speed,
+                                        SpeedsM& u) {
+    using S = SmemM<double, ORDER, TY, false>;
+    const MemInt<ORDER, TY> t(smem);
+    while (left) {
+        const int k = __ffs((int)left) - 1;
+        left &= left - 1;
+        const FaceM<TY> w(P, tx0, ty0, threadIdx.x + k * NT);
+        const int st = w.isx ? 1 : S::SX;
+        double qa[NF], qb[NF], UU;
+#pragma unroll 1
+        for (int f = 0; f < NF; ++f) {
+            const int ue = (f == 0 ? X.r : (f == 1 ? X.p : (f < 4 ? X.v : X.b))) - 60;
+            const fx::i64* q = t.q + (w.field(f) * S::SY + w.ly + S::H) * S::SX + w.lx + S::H;
+            const double ca = fx::to_double(q[-st], ue), cb = fx::to_double(q[0], ue);
+            qa[f] = ca;
+            qb[f] = cb;
+            if (ORDER == 2) {
+                const double d = cb - ca;
+                side_states(f, ca, minmod(ca - fx::to_double(q[-2 * st], ue), d), cb,
+                            minmod(d, fx::to_double(q[st], ue) - cb), qa[f], qb[f]);
+            }
+        }
+        w.store(t.fx, t.fy, float_flux(P, qa, qb, UU));
+        if (speed & (1u << k)) u.take(w.isx, UU);
+    }
+}
+
+template <int SX, int FS>
+struct JumpInt {
+    const fx::i64* own;
+    int ue;
+    __device__ __forceinline__ double x(int lx, int ly) const {
+        const fx::i64* c = own + 4 * FS + ly * SX + lx;
+        return fx::to_double(c[1] - c[-1], ue);
+    }
+    __device__ __forceinline__ double y(int lx, int ly) const {
+        const fx::i64* c = own + 5 * FS + ly * SX + lx;
+        return fx::to_double(c[SX] - c[-SX], ue);
+    }
+};
+
+// Returns false, with nothing written, where the tile's cells cannot be held in common units.
+// Every thread of the block must call it, and all get the same answer.
+template <int ORDER, int TY>
+__device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in, const Planes& out,
+                                             int tx0, int ty0, double T_do, int dt_only,
+                                             double* smem, MhdTileResult& res, double* aux) {
+    using S = SmemM<double, ORDER, TY, false>;
+    using fx::i64;
+    constexpr int H = S::H, SX = S::SX, SY = S::SY, FS = SY * SX, NC = (FS + NT - 1) / NT;
+    const MemInt<ORDER, TY> t(smem);
+    // the largest and (negated) the smallest exponents of rho and p, the largest of v and b
+    constexpr int NK = 6;
+    __shared__ unsigned int keys[NK][NT / 32];
+    const int tid = threadIdx.x, N = P.N, M = P.M;
+
+    double v[NC][NF];
+    unsigned int key[NK] = {0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int i = tid + c * NT;
+        const int ly = i / SX, lx = i - ly * SX;
+        const bool xh = lx < H || lx >= TX + H, yh = ly < H || ly >= TY + H;
+        const int gx = tx0 + lx - H, gy = ty0 + ly - H;
+        const bool some = i < FS && !(xh && yh) && gx >= -2 && gx < N + 2 && gy >= -2 &&
+                          gy < M + 2 && !((gx < 0 || gx >= N) && (gy < 0 || gy >= M));
+#pragma unroll
+        for (int f = 0; f < NF; ++f) v[c][f] = 0.0;  // never used
+        if (some) {
+            load_state(P, in, gx, gy, v[c]);
+#pragma unroll
+            for (int f = 4; f < NF; ++f) v[c][f] = __dmul_rn(v[c][f], kInvSpi4);
+            const unsigned int r = fx::signed_exp_field(v[c][0]), p = fx::signed_exp_field(v[c][1]);
+            key[0] = max(key[0], r);
+            key[1] = max(key[1], 0xfffu - r);
+            key[2] = max(key[2], p);
+            key[3] = max(key[3], 0xfffu - p);
+            key[4] = max(key[4], max(fx::exp_field(v[c][2]), fx::exp_field(v[c][3])));
+#pragma unroll
+            for (int f = 4; f < NF; ++f) key[5] = max(key[5], fx::exp_field(v[c][f]));
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NK; ++k) {
+        const unsigned int m = __reduce_max_sync(0xffffffffu, key[k]);
+        if ((tid & 31) == 0) keys[k][tid >> 5] = m;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NK; ++k)
+        key[k] = __reduce_max_sync(0xffffffffu, keys[k][tid & (NT / 32 - 1)]);
+    fx::TopsM X;
+    if (!fx::tops_of(0xfffu - key[1], key[0], 0xfffu - key[3], key[2], key[4], key[5], P.gas, X))
+        return false;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const int i = tid + c * NT;
+        if (i >= FS) break;
+        const int ly = i / SX, lx = i - ly * SX;
+        const bool own = lx >= H && lx < TX + H && ly >= H && ly < TY + H;
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            t.q[f * FS + i] =
+                fx::to_units(v[c][f], f == 0 ? X.r : (f == 1 ? X.p : (f < 4 ? X.v : X.b)));
+            if (own) t.cell[(f * TY + ly - H) * TX + lx - H] = v[c][f];
         }
     }
     __syncthreads();
 
-    // ---- U: update (kernel.cu:2606-2660 in Heaviside-Lorentz field units) ----------------------
-    const double kx = imul<true>(T_do, P.inv_dx), ky = imul<true>(T_do, P.inv_dy);
-    const double hkx = half_exact(kx), hky = half_exact(ky);  // 0.5 kx, 0.5 ky
-    const bool axi = P.geometry == GD_AXISYM;
-    bool any_active = false;
-    unsigned int nfl_r = 0, nfl_p = 0, nbad = 0;
-    for (int i = tid; i < TX * TY; i += NT) {
-        const int ly = i / TX, lx = i - ly * TX;
-        const int gx = tx0 + lx, gy = ty0 + ly;
-        if (gx >= N || gy >= M) continue;
-        const T* c = prim + (ly + H) * SX + (lx + H);
-        constexpr int PS = SY * SX;
-        const T r = c[0], p = c[PS], u = c[2 * PS], v = c[3 * PS];
-        const T bx = c[4 * PS], by = c[5 * PS], bz = c[6 * PS];
-        const long long k = (long long)gy * N + gx;
-        if (P.frozen && !cell_active(P, gx, gy)) {  // the faces' own test
-            if (!dt_only) copy_cell(in, out, k);
-            continue;
-        }
-        any_active = true;
-        if (dt_only) continue;
-        const T* fxc = fx + ly * (TX + 1) + lx;
-        const T* fyc = fy + ly * TX + lx;
-        T d[NF];
+    SpeedsM u{0.0, 0.0};
+    unsigned int left = 0, speed = 0, bit = 1;
+    for (int i = tid; i < FaceM<TY>::NFX + FaceM<TY>::NFY; i += NT, bit <<= 1) {
+        const FaceM<TY> w(P, tx0, ty0, i);
+        if (!w.used) continue;
+        const int st = w.isx ? 1 : SX;
+        const i64* q = t.q + (w.ly + H) * SX + w.lx + H;
+        i64 a[NF], b[NF];
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-            const T* a = fxc + f * TY * (TX + 1);
-            const T* b = fyc + f * (TY + 1) * TX;
-            d[f] = fma(kx, a[1] - a[0], ky * (b[TX] - b[0]));
-        }
-        // Powell divergence from cell-centred field: dx dy div b (kernel.cu:2568-2604)
-        const T bxE = c[4 * PS + 1], bxW = c[4 * PS - 1];
-        const T byN = c[5 * PS + SX], byS = c[5 * PS - SX];
-        T divb = fma(hkx, bxE - bxW, mulx<true>(hky, byN - byS));  // T_do * div b
-        const double iy = axi ? rcp_fast(P.y0 + gy * P.dy) : 0.0;
-        if (axi) divb = fma(T_do * by, iy, divb);                 // kernel.cu:2615
-        if constexpr (std::is_same<T, double>::value) {
-            if (aux != nullptr) {
-                const long long KK = (long long)N * M;
-#pragma unroll
-                for (int f = 0; f < NF; ++f) aux[f * KK + k] = d[f];
-                aux[7 * KK + k] = divb;
+            const i64* p = q + w.field(f) * FS;
+            const i64 ca = p[-st], cb = p[0];
+            a[f] = 2 * ca;
+            b[f] = 2 * cb;
+            if (ORDER == 2) {  // between the cell and the middle to its neighbour: rho, p > 0
+                const i64 d = cb - ca;
+                a[f] += fx::minmod(ca - p[-2 * st], d);
+                b[f] -= fx::minmod(d, p[st] - cb);
             }
         }
-        const T ub = fma(u, bx, v * by);
-        const T bb = fma(bz, bz, fma(by, by, bx * bx));
-        const T E = fma(p, P.inv_gm1, 0.5 * fma(r, fma(u, u, v * v), bb));
-        T r2 = r - d[0];
-        T mx2 = fma(r, u, -fma(bx, divb, d[2]));
-        T my2 = fma(r, v, -fma(by, divb, d[3]));
-        T bx2 = bx - fma(u, divb, d[4]);
-        const T by2 = by - fma(v, divb, d[5]);
-        const T bz2 = bz - d[6];
-        T E2 = E - fma(ub, divb, d[1]);
-        if (axi) {
-            // geometric sources / y (kernel.cu:2619-2648) in field units b
-            const double ty = T_do * iy;
-            r2 = fma(-ty * r, v, r2);
-            mx2 = fma(-ty, fma(r * u, v, -bx * by), mx2);
-            my2 = fma(-ty, fma(r * v, v, fma(bz, bz, -by * by)), my2);
-            bx2 = fma(-ty, fma(v, bx, -by * u), bx2);
-            E2 = fma(-ty, fma(E + p + 0.5 * bb, v, -by * ub), E2);
+        const fx::StatesM A{a[0], a[1], a[2], a[3], a[4], a[5], a[6]};
+        const fx::StatesM B{b[0], b[1], b[2], b[3], b[4], b[5], b[6]};
+        double UU;
+        const fx::FanM fan = fx::fan_of(A, B, X, P.gas, UU);
+        if (!fan.ok) {
+            left |= bit;
+            speed |= bit;
+            continue;
         }
-        if (le_zero(r2)) { r2 = r; ++nfl_r; }
-        const T inv = rcp_fast(r2);
-        const T u2 = mx2 * inv, v2 = my2 * inv;
-        T p2 = (E2 - 0.5 * fma(r2, fma(u2, u2, v2 * v2), fma(bz2, bz2, fma(by2, by2, bx2 * bx2)))) * P.gm1;
-        if (le_zero(p2)) { p2 = cst<T>(0.000001); ++nfl_p; }
-        if (!finite_bits(r2) || !finite_bits(p2) || !finite_bits(u2) || !finite_bits(v2) ||
-            !finite_bits(bx2) || !finite_bits(by2) || !finite_bits(bz2))
-            ++nbad;
-        store_state2(out, k, 0, r2, p2);
-        store_state2(out, k, 2, u2, v2);
-        store_state(out, k, 4, bx2 * kSpi4);
-        store_state(out, k, 5, by2 * kSpi4);
-        store_state(out, k, 6, bz2 * kSpi4);
+        u.take(w.isx, UU);
+        if (dt_only) continue;
+        fx::FluxI F;
+        if (fx::hlld(fan, A, B, X, P.gas, F))
+            w.store(t.fx, t.fy, FluxM<double>{F.m, F.mn, F.mt, F.e, F.bn, F.bt, F.bz});
+        else
+            left |= bit;
     }
-    res.umax_x = umax_x;
-    res.umax_y = umax_y;
-    res.any_active = any_active;
-    res.nfl_r = nfl_r;
-    res.nfl_p = nfl_p;
-    res.nbad = nbad;
+    if (left) faces_left<ORDER, TY>(P, smem, X, tx0, ty0, left, speed, u);
+    __syncthreads();
+
+    update_cells<double, TY, TX, TX * TY>(P, in, out, tx0, ty0, T_do, dt_only, t.cell,
+                                          JumpInt<SX, FS>{t.q + H * SX + H, X.b - 60}, t.fx, t.fy,
+                                          res, aux);
+    res.umax_x = u.x;
+    res.umax_y = u.y;
+    return true;
 }
 
-template <int ORDER, int TY>
-__global__ void __launch_bounds__(NT, 2) mhd_fast_kernel(Params P, CPlanes in, Planes out,
+template <int ORDER, int TY, bool HLLD>
+__global__ void __launch_bounds__(NT, HLLD ? 3 : 2) mhd_fast_kernel(const __grid_constant__ Params P,
+                                                      const __grid_constant__ CPlanes in,
+                                                      const __grid_constant__ Planes out,
                                                       const double* __restrict__ T_do_ptr,
                                                       unsigned long long* T_bits, Scalars* rot,
                                                       Scalars* ctr, int dt_only, double* aux) {
     extern __shared__ __align__(16) double smem[];
     MhdTileResult r;
-    mhd_tile<double, ORDER, TY>(P, in, out, blockIdx.x * TX, (blockIdx.y + P.tile_row0) * TY,
-                                *T_do_ptr, dt_only,
-                                smem, r, aux);
+    const int tx0 = blockIdx.x * TX, ty0 = (blockIdx.y + P.tile_row0) * TY;
+    const double T_do = *T_do_ptr;
+    if constexpr (HLLD) {  // in integers where the tile's range allows it
+        if (!mhd_tile_int<ORDER, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux)) {
+            __syncthreads();
+            mhd_tile<double, ORDER, TY, false>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux);
+        }
+    } else {
+        mhd_tile<double, ORDER, TY, true>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux);
+    }
     if (ctr != nullptr && (r.nfl_r | r.nfl_p | r.nbad)) {
         if (r.nfl_r) atomicAdd(&ctr->rho_floor, (unsigned long long)r.nfl_r);
         if (r.nfl_p) atomicAdd(&ctr->p_floor, (unsigned long long)r.nfl_p);
@@ -392,19 +642,20 @@ __global__ void __launch_bounds__(NT, 2) mhd_fast_kernel(Params P, CPlanes in, P
 
 // Tangent of one step: (U, dU) -> (U', dU') with the dt read from *T_do_ptr (held fixed).
 template <int ORDER, int TY>
-__global__ void __launch_bounds__(NT) mhd_tangent_kernel(Params P, CPlanes in, CPlanes din,
+__global__ void __launch_bounds__(NT) mhd_tangent_kernel(const __grid_constant__ Params P,
+                                                         CPlanes in, CPlanes din,
                                                          Planes out, Planes dout,
                                                          const double* __restrict__ T_do_ptr) {
     extern __shared__ __align__(16) double smem[];
     MhdTileResult r;
     const DualCPlanes I{in, din};
     const DualPlanes O{out, dout};
-    mhd_tile<Dual, ORDER, TY>(P, I, O, blockIdx.x * TX, blockIdx.y * TY, *T_do_ptr, 0,
-                              reinterpret_cast<Dual*>(smem), r);
+    mhd_tile<Dual, ORDER, TY, true>(P, I, O, blockIdx.x * TX, blockIdx.y * TY, *T_do_ptr, 0,
+                              reinterpret_cast<Dual*>(smem), r, nullptr);
 }
 
-// 32 x 8 tiles: 88 KB of shared memory and at most 128 registers, so two CTAs (16 warps) are
-// resident per SM; the halo costs 3 % more faces than 32 x 16 tiles at one CTA per SM.
+// 32 x 8 tiles: three CTAs (24 warps) of the integer HLLD tile are resident per SM at 80 registers
+// and 69 KB of shared memory, two of the floating-point one at 128 and 88 KB.
 constexpr int kTY = 8;
 constexpr int kTYDual = 8;
 
@@ -413,8 +664,12 @@ cudaError_t launch_t(const Params& P, const CPlanes& in, const Planes& out, cons
                      unsigned long long* T_bits, Scalars* rot, Scalars* ctr, int dt_only,
                      cudaStream_t st, double* aux = nullptr) {
     dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + kTY - 1) / kTY);
-    mhd_fast_kernel<ORDER, kTY><<<grid, NT, SmemM<double, ORDER, kTY>::bytes, st>>>(
-        P, in, out, T_do, T_bits, rot, ctr, dt_only, aux);
+    if (P.method == GD_METHOD_HLLD)
+        mhd_fast_kernel<ORDER, kTY, true><<<grid, NT, step_bytes<ORDER, kTY, true>(), st>>>(
+            P, in, out, T_do, T_bits, rot, ctr, dt_only, aux);
+    else
+        mhd_fast_kernel<ORDER, kTY, false><<<grid, NT, step_bytes<ORDER, kTY, false>(), st>>>(
+            P, in, out, T_do, T_bits, rot, ctr, dt_only, aux);
     return cudaGetLastError();
 }
 
@@ -428,18 +683,22 @@ cudaError_t launch_tangent_t(const Params& P, const CPlanes& in, const CPlanes& 
     return cudaGetLastError();
 }
 
+template <int ORDER, bool HLLD>
+cudaError_t set_room() {
+    return cudaFuncSetAttribute(mhd_fast_kernel<ORDER, kTY, HLLD>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)step_bytes<ORDER, kTY, HLLD>());
+}
+
 }  // namespace
 
 int mhd_tile_height() { return kTY; }
 
 cudaError_t prepare_mhd_fast() {
-    cudaError_t e = cudaFuncSetAttribute(mhd_fast_kernel<1, kTY>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)SmemM<double, 1, kTY>::bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(mhd_fast_kernel<2, kTY>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)SmemM<double, 2, kTY>::bytes);
+    cudaError_t e = set_room<1, true>();
+    if (e == cudaSuccess) e = set_room<1, false>();
+    if (e == cudaSuccess) e = set_room<2, true>();
+    if (e == cudaSuccess) e = set_room<2, false>();
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(mhd_tangent_kernel<1, kTYDual>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -497,13 +756,20 @@ __global__ void mhd_face_probe_kernel(Params P, long long n, int axis,
         qa[f] = __dmul_rn(a[f + 1], kInvSpi4);
         qb[f] = __dmul_rn(b[f + 1], kInvSpi4);
     }
-    Side<double> A, B;
-    side(A, qa[0], qa[1], isx ? qa[2] : qa[3], isx ? qa[3] : qa[2], isx ? qa[4] : qa[5],
-         isx ? qa[5] : qa[4], qa[6], P);
-    side(B, qb[0], qb[1], isx ? qb[2] : qb[3], isx ? qb[3] : qb[2], isx ? qb[4] : qb[5],
-         isx ? qb[5] : qb[4], qb[6], P);
+    double la[NF], lb[NF];  // in the face's frame
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        const int g = isx || f < 2 || f == 6 ? f : (f < 4 ? 5 - f : 9 - f);
+        la[f] = qa[g];
+        lb[f] = qb[g];
+    }
     double UU;
-    const FluxM<double> F = hlld_local(A, B, P.method, P, UU);
+    fx::FluxI G;
+    FluxM<double> F;
+    if (P.method == GD_METHOD_HLLD && fx::hlld_face(la, lb, P.gas, G, UU))
+        F = FluxM<double>{G.m, G.mn, G.mt, G.e, G.bn, G.bt, G.bz};
+    else
+        F = float_flux(P, la, lb, UU);
     double* o = flux + 8 * i;
     o[0] = F.m;
     o[1] = isx ? F.mn : F.mt;

@@ -1,0 +1,374 @@
+// gd_fixed_mhd.cuh -- the HLLD face flux in scaled 64-bit integers (see gd_fixed.cuh).
+//
+// The states, speeds and guards of hlld_local (gd_mhd_flux.cuh; Gas_Dinamic.cu:964-1510), with
+// the fluxes of the star states in the form the jump conditions across S_K give them.  K is the
+// side the flux is taken from, m = rho (S - u), q = S_M / (S - S_M), b the HLL mean normal field:
+//   mass F = rho q (S - u), normal momentum F S_M + p_T* - b_K^2, p_T* = p_T + m (S_M - u),
+//   tangential F v* + m (v* - v) - b_K b_t, field S b* - (S - u) b_t - v b_K,
+//   energy q (S - u) (p gamma / (gamma - 1) + rho (u^2 + v^2) / 2 + |b|^2 + rho S (S_M - u))
+//          + b (q (v.b - v*.b*) - v*.b*) + (b - b_K) v.b,
+// and S** (U** - U*) on top between the Alfven waves.  Only K's star state is formed unless the
+// face lies between the Alfven waves.
+//
+// Units: velocities 2^(E - 61) as for HLLC; fields 2^(X.b - 61), below 2^60; rho v^2 quantities
+// 2^(ER + 2E - 59) and 2^(ER + 2E - 60), ER the larger density's exponent.  Squares of the field
+// move to those by a shift: |b|^2 / 2 <= rho c_f^2 bounds them there.
+#pragma once
+
+#include "gd_fixed.cuh"
+
+namespace gd {
+namespace fx {
+
+struct TopsM {
+    int r, p, v, b;
+};
+// fields are held with two bits of room above their largest value
+constexpr int kFieldRoom = 2;
+
+struct StatesM {
+    i64 r, p, un, ut, bn, bt, bz;
+};
+
+// x 2^-s for either sign of s; a left shift's result fits
+GD_HD i64 shift(i64 x, int s) {
+    return (i64)((u64)x << imin(imax(-s, 0), 62)) >> imin(imax(s, 0), 63);
+}
+GD_HD i64 iabs(i64 x) { return x < 0 ? -x : x; }
+// |x| < 2^61 (and a little beyond on the negative side)
+GD_HD bool below61(i64 x) { return (uint32_t)(hi32(x) + (1 << 29)) < (1u << 30); }
+
+// whether x >= 0 shifted by shift(x, s) stays below 2^61
+GD_HD bool fits(i64 x, int s) { return s >= 0 || x >> imax(61 + s, 0) == 0; }
+
+// sqrt(x) 2^(29 + h) of x 2^(2 h) in [2^61, 2^63): the root (w, in [2^59, 2^61)) and, where asked,
+// the reciprocal root times 2^(91 - h).  As sqrt_over: e = 1 - x y^2 for the FP32 seed y.
+template <bool RECIP>
+GD_HD i64 sqrt_norm(i64 x, i64& rs) {
+    const uint32_t y = (uint32_t)(rsqrt_seed((float)hi32(x)) * 35184363700224.0f);  // 2^45 - 2^23
+    const i64 w = mul32(x, y);
+    const i64 e = (1LL << 58) - mul32(w, y);
+    const int32_t es = (int32_t)(e >> 15);
+    const i64 g = (e << 3) + (wide(es, 3 * es) >> 27);
+    if (RECIP) rs = ((i64)((u64)y << 30)) + mul32(g, y);
+    return w + (mulk<0, 0, false>(w, g << 21) >> 19);
+}
+// sqrt(x) 2^31 for 0 <= x < 2^63
+GD_HD i64 sqrt31(i64 x) {
+    const int z = (clz64((u64)x) - 1) & ~1;
+    i64 none;
+    const i64 w = sqrt_norm<false>((i64)((u64)x << z), none);
+    return (w << 2) >> (z >> 1);
+}
+
+// What a side gives: density, pressure, |b|^2 and b_n^2 in units of 2^(2 X.b - 58), and the fast
+// speed w 2^(k - 60).
+struct SideM {
+    Pos R, P;
+    i64 bb, n2, w;
+    int k;
+};
+GD_HD SideM side_of(const StatesM& s, const TopsM& X, const Gas& G) {
+    SideM S;
+    S.R = pos_of(s.r, X.r);
+    S.P = pos_of(s.p, X.p);
+    S.n2 = mulk<0, 0>(s.bn, s.bn);
+    const i64 t2 = mulk<0, 0>(s.bt, s.bt) + mulk<0, 0>(s.bz, s.bz);
+    S.bb = S.n2 + t2;
+    // gamma p, |b|^2 and the tangential part in one unit 2^U, below 2^61 and the larger above 2^59
+    const i64 gp = mulk<0, 0>(S.P.m, G.g);
+    const int ug = S.P.e + G.ge - 60;
+    const int z = clz32((uint32_t)hi32(S.bb)) - 2;
+    const int ub = 2 * X.b - 58 - z;
+    const int U = imax(ug, ub) + 1;
+    const i64 g1 = gp >> imin(U - ug, 63);
+    const int sb = imin(U - ub, 63);
+    const i64 b1 = (S.bb << z) >> sb, t1 = (t2 << z) >> sb;
+    // a^2 - 4 gamma p b_n^2 with a = gamma p + |b|^2, as a sum: four times it
+    const i64 d = g1 - b1;
+    const i64 disc = mulk<1, 1>(d, d) + mulk<2, 2>(g1, t1);
+    const i64 x = (g1 + b1 + sqrt31(disc)) >> 1;
+    const int lz = clz32((uint32_t)hi32(x));
+    S.w = sqrt_over(x << (lz - 2), U - lz + 62, S.R, S.k);
+    return S;
+}
+
+// The star state of one side: v - v0, w, b_t, b_z behind the fast wave (Gas_Dinamic.cu:1306-1350).
+// am = |rho (S - u)|, ad = |S - S_M|, as = |S - u|; bn2 the square of the mean normal field in
+// units of 2^(ER + 2E - 59), sh the shift that brings products of two fields to them, thr the
+// guard's 1e-5 in them.  False where a ratio leaves its range.
+struct StarM {
+    i64 dv, dw, bt, bz;
+};
+GD_HD bool star_of(i64 am, i64 ad, i64 as, i64 SMu, i64 bn, i64 bn2, int sh, i64 thr, i64 bt,
+                   i64 bz, StarM& T) {
+    const i64 tt = mulk<2, 1>(am, ad) - bn2;
+    const i64 at = iabs(tt);
+    if (at < thr) {
+        T.dv = T.dw = T.bt = T.bz = 0;
+        return true;
+    }
+    if (hi32(at) == 0) return false;
+    int lz;
+    const i64 it = rcp(at, lz);
+    const i64 num = mulk<2, 1>(am, as) - bn2;
+    const i64 x1 = shift(mulk<0, 0>(bn, bt), sh), x2 = shift(mulk<0, 0>(bn, bz), sh);
+    if (!(iabs(num >> 1) < 2 * (at >> 1) && iabs(x1) < at && iabs(x2) < at)) return false;
+    const i64 k1 = mulk<0, 2>(x1 << (lz - 2), it), k2 = mulk<0, 2>(x2 << (lz - 2), it);
+    const i64 d = mulk<0, 2>((num >> 1) << (lz - 2), it);
+    const i64 dv = mulk<2, 1>(k1, SMu) << 1, dw = mulk<2, 1>(k2, SMu) << 1;
+    const i64 ct = mulk<2, 1>(d, bt) << 2, cz = mulk<2, 1>(d, bz) << 2;
+    const bool neg = tt < 0;
+    T.dv = neg ? dv : -dv;
+    T.dw = neg ? dw : -dw;
+    T.bt = neg ? -ct : ct;
+    T.bz = neg ? -cz : cz;
+    return true;
+}
+
+// rho* = am / ad, and its root s 2^(k - 60) (and reciprocal root rs 2^(-60 - k))
+GD_HD Pos star_density(i64 am, i64 iad, int lz, int ER) {
+    const i64 t = mulk<2, 2>(am, iad);
+    const int z = clz32((uint32_t)hi32(t));
+    return Pos{t << (z - 1), ER + lz - z + 1};
+}
+template <bool RECIP>
+GD_HD i64 root_of(Pos R, int& k, i64& rs) {
+    const int odd = R.e & 1;
+    k = (R.e + odd) >> 1;
+    return sqrt_norm<RECIP>(R.m >> odd, rs);
+}
+
+// The larger wave speed of the face between A and B, and all speeds.
+struct FanM {
+    SideM A, B;
+    i64 uA, uB, vA, vB, SL, SR;
+    int E, ER, kmin;
+    bool ok;
+};
+GD_HD FanM fan_of(const StatesM& a, const StatesM& b, const TopsM& X, const Gas& G, double& UU) {
+    FanM f;
+    f.A = side_of(a, X, G);
+    f.B = side_of(b, X, G);
+    const int kmax = imax(f.A.k, f.B.k);
+    f.kmin = imin(f.A.k, f.B.k);
+    f.ER = imax(f.A.R.e, f.B.R.e);
+    const int32_t h1 = hi32(a.un), h2 = hi32(b.un), h3 = hi32(a.ut), h4 = hi32(b.ut);
+    const int lz = clz32((uint32_t)((h1 ^ (h1 >> 31)) | (h2 ^ (h2 >> 31)) | (h3 ^ (h3 >> 31)) |
+                                    (h4 ^ (h4 >> 31))));
+    f.E = imax(kmax + 2, X.v + imax(4 - lz, 0));
+    const int dr = f.A.R.e - f.B.R.e;
+    f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 8 && (uint32_t)(dr + 3) <= 6u;
+    if (!f.ok) return f;
+    const i64 cA = f.A.w >> (f.E - 1 - f.A.k), cB = f.B.w >> (f.E - 1 - f.B.k);
+    const i64 c = cA > cB ? cA : cB;
+    const int sh = imin(f.E - X.v, 63);
+    f.uA = a.un >> sh;
+    f.uB = b.un >> sh;
+    f.vA = a.ut >> sh;
+    f.vB = b.ut >> sh;
+    f.SL = (f.uA < f.uB ? f.uA : f.uB) - c;
+    f.SR = (f.uA > f.uB ? f.uA : f.uB) + c;
+    UU = to_double(-f.SL > f.SR ? -f.SL : f.SR, f.E - 61);
+    return f;
+}
+
+struct FluxI {
+    double m, mn, mt, e, bn, bt, bz;
+};
+
+// m 2^(e - 62) in units of 2^u, at least 1, or the largest integer where it does not fit
+GD_HD i64 threshold(i64 m, int e, int u) {
+    const int s = u - e + 62;
+    return s < 0 ? 0x7fffffffffffffffLL : (m >> imin(s, 62)) | 1;
+}
+
+GD_HD bool hlld(const FanM& f, const StatesM& a, const StatesM& b, const TopsM& X, const Gas& G,
+                FluxI& F) {
+    const int E = f.E, ER = f.ER, XB = 2 * X.b;
+    const i64 suA = f.SL - f.uA, suB = f.SR - f.uB;
+    const i64 mA = mulk<0, 0>(f.A.R.m, suA) >> (ER - f.A.R.e);
+    const i64 mB = mulk<0, 0>(f.B.R.m, suB) >> (ER - f.B.R.e);
+    // total pressures in units of 2^(ER + 2E - 60)
+    const int sp = ER + 2 * E + 2, sq = ER + 2 * E - 1 - XB;
+    const i64 ptA = (f.A.P.m >> imin(sp - f.A.P.e, 63)) + shift(f.A.bb, sq);
+    const i64 ptB = (f.B.P.m >> imin(sp - f.B.P.e, 63)) + shift(f.B.bb, sq);
+    const i64 N = mulk<1, 3>(mB, f.uB) - mulk<1, 3>(mA, f.uA) + (ptA - ptB);
+    int lz;
+    const i64 iD = rcp(mB - mA, lz);
+    i64 SM = mulk<0, 2>(N << (lz - 2), iD);
+    // the mean normal field
+    int lzs;
+    const i64 iS = rcp(f.SR - f.SL, lzs);
+    const i64 bs = mulk<2, 1>(f.SR, b.bn) - mulk<2, 1>(f.SL, a.bn);
+    i64 bn = mulk<0, 2>(bs << (lzs - 2), iS) << 1;
+
+    const bool takeL = f.SL >= 0 || N >= 0;
+    const bool star = takeL ? f.SL < 0 : f.SR > 0;
+    const Pos R{takeL ? f.A.R.m : f.B.R.m, takeL ? f.A.R.e : f.B.R.e};
+    const Pos Pk{takeL ? f.A.P.m : f.B.P.m, takeL ? f.A.P.e : f.B.P.e};
+    const i64 bbK = takeL ? f.A.bb : f.B.bb, n2K = takeL ? f.A.n2 : f.B.n2;
+    const i64 un = takeL ? f.uA : f.uB, ut = takeL ? f.vA : f.vB;
+    const i64 bnK = takeL ? a.bn : b.bn, btK = takeL ? a.bt : b.bt, bzK = takeL ? a.bz : b.bz;
+    const i64 m = takeL ? mA : mB, ptK = (takeL ? ptA : ptB) >> 1;
+    const i64 S = takeL ? f.SL : f.SR, su = takeL ? suA : suB;
+
+    const int sh = ER + 2 * E - 1 - XB;  // products of fields to units of 2^(ER + 2E - 59)
+    const i64 ub = mulk<2, 1>(un, bnK) + mulk<2, 1>(ut, btK);  // units 2^(E + X.b - 61)
+    i64 qs = un, qsg = 0, sb = ub, S2 = 0;
+    StarM K{0, 0, btK, bzK};
+    Pos RK = R;
+    i64 sK = 0, am = 0, bn2 = 0, thr = 0;
+    int kK = 0;
+    bool alfven = false;
+    if (star) {
+        if (E - f.kmin > 4) return false;
+        const i64 ad = takeL ? SM - S : S - SM;
+        if (hi32(ad) <= 0) return false;
+        int lza;
+        const i64 iA = rcp(ad, lza);
+        const i64 q = mulk<0, 2>(SM << (lza - 2), iA);
+        qsg = takeL ? -q : q;  // S_M / (S - S_M), at most 1 in size, in units of 2^-60
+        qs = mulk<2, 1>(qsg, su) << 1;
+        am = iabs(m);
+        bn2 = shift(mulk<0, 0>(bn, bn), sh);
+        thr = threshold(0x53e2d6238da3c211LL, -17, ER + 2 * E - 59);  // 1e-5
+        if (!star_of(am, ad, iabs(su), SM - un, bn, bn2, sh, thr, btK, bzK, K)) return false;
+        RK = star_density(am, iA, lza, ER);
+        i64 rs;
+        sK = root_of<true>(RK, kK, rs);
+        const i64 abn = iabs(bn);
+        // |b| / sqrt(rho*), where |b| > 1e-6 (Gas_Dinamic.cu:1352-1369)
+        const i64 va = abn > threshold(0x431bde82d7b634daLL, -20, X.b - 61)
+                           ? shift(mulk<1, 2>(abn, rs), kK + E - 1 - X.b) : 0;
+        S2 = takeL ? SM - va : SM + va;
+        alfven = takeL ? S2 < 0 : S2 > 0;
+    } else {  // the physical flux of K: no mean of both sides in it
+        SM = un;
+        bn = bnK;
+    }
+    const i64 SMu = SM - un, vK = ut + K.dv;
+    if (!(below61(vK) && below61(K.dw) && below61(K.bt) && below61(K.bz))) return false;
+    if (star) sb = mulk<2, 1>(SM, bn) + mulk<2, 1>(vK, K.bt) + mulk<2, 1>(K.dw, K.bz);
+
+    const int32_t qh = hi32(qs);
+    const int z = clz32((uint32_t)(qh ^ (qh >> 31))) - 1;
+    const i64 qn = qs << z;
+    const i64 M = mulk<0, 0>(R.m, qn);
+    const int em = R.e + E - 59 - z;
+    F.m = to_double(M, em);
+    const int dR = ER - R.e;
+    const i64 n2s = shift(n2K, sh), bnt = shift(mulk<0, 0>(bnK, btK), sh);
+    const i64 mn = ptK + (mulk<1, 2>(M, SM) >> imin(z + dR, 63)) + mulk<2, 1>(m, SMu) - n2s;
+    i64 mt = (mulk<1, 2>(M, vK) >> imin(z + dR, 63)) + mulk<2, 1>(m, K.dv) - bnt;
+    i64 ft = mulk<2, 1>(S, K.bt) - mulk<1, 2>(su, btK) - mulk<2, 1>(ut, bnK);
+    i64 fz = mulk<2, 1>(S, K.bz) - mulk<1, 2>(su, bzK);
+    const i64 H = mulk<1, 1>(un, un) + mulk<1, 1>(ut, ut) + mulk<2, 1>(S, SMu);
+    const i64 B = sra(mulk<0, 0>(Pk.m, G.gg), ER + 2 * E - Pk.e - G.gge + G.room) +
+                  ((mulk<0, 1>(R.m, H) >> dR) + shift(bbK, ER + 2 * E - 2 - XB) >> G.room);
+    const i64 y = (mulk<2, 1>(qsg, ub - sb) << 1) - sb;
+    // units 2^(ER + 3E - 61)
+    const i64 e0 = mulk<0, 2>(qn, B);
+    if (!(below61(B) && fits(iabs(e0), z - 2 - G.room))) return false;
+    i64 e = shift(e0, z - 2 - G.room) +
+            shift(mulk<2, 0>(bn, y) + mulk<2, 0>(bn - bnK, ub), ER + 2 * E - 1 - XB);
+
+    if (alfven) {
+        // the other side's star state and the states between the Alfven waves
+        // (Gas_Dinamic.cu:1371-1430); v3 = vO + w (vK - vO) + ..., w = sK / (sK + sO)
+        const i64 unO = takeL ? f.uB : f.uA, utO = takeL ? f.vB : f.vA;
+        const i64 btO = takeL ? b.bt : a.bt, bzO = takeL ? b.bz : a.bz;
+        const i64 amO = iabs(takeL ? mB : mA), asO = iabs(takeL ? suB : suA);
+        const i64 adO = takeL ? f.SR - SM : SM - f.SL;
+        if (hi32(adO) <= 0) return false;
+        StarM O;
+        if (!star_of(amO, adO, asO, SM - unO, bn, bn2, sh, thr, btO, bzO, O)) return false;
+        const i64 vO = utO + O.dv;
+        if (!(below61(vO) && below61(O.dw) && below61(O.bt) && below61(O.bz))) return false;
+        int lzO, kO, lzt;
+        const i64 iO = rcp(adO, lzO);
+        i64 none;
+        const i64 sO = root_of<false>(star_density(amO, iO, lzO, ER), kO, none);
+        const int kk = imax(kK, kO) + 1;
+        const i64 aK = sK >> imin(kk - kK, 63), aO = sO >> imin(kk - kO, 63);
+        const i64 iT = rcp(aK + aO, lzt);
+        const i64 w = mulk<0, 2>(aK << (lzt - 2), iT);
+        const bool flip = takeL != (bn > 0);  // sign of b times that of O - K in R - L
+        const int sv = E + kk + 3 - lzt - X.b;
+        const i64 xt = shift(mulk<1, 2>(O.bt - K.bt, iT), sv);
+        const i64 xz = shift(mulk<1, 2>(O.bz - K.bz, iT), sv);
+        const i64 v3 = vO + (mulk<2, 1>(w, vK - vO) << 1) + (flip ? -xt : xt);
+        const i64 w3 = O.dw + (mulk<2, 1>(w, K.dw - O.dw) << 1) + (flip ? -xz : xz);
+        const i64 wo = mulk<2, 2>(w, aO);
+        const int sc = X.b - kk - E - 1;
+        const i64 ct = mulk<2, 1>(wo, vO - vK), cz = mulk<2, 1>(wo, O.dw - K.dw);
+        // root(rho) times the jump of v may be far above a weak field
+        if (!fits(iabs(ct) | iabs(cz), sc)) return false;
+        const i64 yt = shift(ct, sc), yz = shift(cz, sc);
+        const i64 bt3 = K.bt + (mulk<2, 1>(w, O.bt - K.bt) << 1) + (flip ? -yt : yt);
+        const i64 bz3 = K.bz + (mulk<2, 1>(w, O.bz - K.bz) << 1) + (flip ? -yz : yz);
+        if (!(below61(v3) && below61(w3) && below61(bt3) && below61(bz3) && below61(S2)))
+            return false;
+        const i64 sb3 = mulk<2, 1>(SM, bn) + mulk<2, 1>(v3, bt3) + mulk<2, 1>(w3, bz3);
+        mt += shift(mulk<2, 1>(mulk<0, 0>(RK.m, S2), v3 - vK), ER - RK.e);
+        ft += mulk<2, 1>(S2, bt3 - K.bt);
+        fz += mulk<2, 1>(S2, bz3 - K.bz);
+        const i64 de = shift(mulk<1, 2>(mulk<2, 0>(sK, sb - sb3), S2), ER + E - kK - X.b - 2);
+        e += flip ? de : -de;
+    }
+    F.mn = to_double(mn, ER + 2 * E - 59);
+    F.mt = to_double(mt, ER + 2 * E - 59);
+    F.e = to_double(e, ER + 3 * E - 61);
+    F.bt = to_double(ft, E + X.b - 61);
+    F.bz = to_double(fz, E + X.b - 61);
+    F.bn = -to_double(mulk<2, 1>(-f.SL > f.SR ? -f.SL : f.SR, b.bn - a.bn), E + X.b - 61);
+    return true;
+}
+
+// Whether the cells can be held in the units of TopsM (b1: the largest field's exponent field).
+GD_HD bool tops_of(uint32_t r0, uint32_t r1, uint32_t p0, uint32_t p1, uint32_t v1, uint32_t b1,
+                   const Gas& G, TopsM& X) {
+    Tops Y;
+    const bool ok = tops_of(r0, r1, p0, p1, v1, G, Y);
+    X.r = Y.r;
+    X.p = Y.p;
+    X.v = Y.v;
+    X.b = imax((int)b1 - 1023, -300) + kFieldRoom;
+    return ok && b1 <= 1023 + kRange;
+}
+
+// Flux and larger wave speed of one face given by its states {rho, p, un, ut, bn, bt, bz}.
+GD_HD bool hlld_face(const double* L, const double* R, const Gas& G, FluxI& F, double& UU) {
+    uint32_t r0 = ~0u, r1 = 0, p0 = ~0u, p1 = 0, v1 = 0, b1 = 0;
+    for (int k = 0; k < 2; ++k) {
+        const double* q = k ? R : L;
+        const uint32_t r = signed_exp_field(q[0]), p = signed_exp_field(q[1]);
+        r0 = r < r0 ? r : r0;
+        r1 = r > r1 ? r : r1;
+        p0 = p < p0 ? p : p0;
+        p1 = p > p1 ? p : p1;
+        for (int f = 2; f < 7; ++f) {
+            const uint32_t x = exp_field(q[f]);
+            if (f < 4) v1 = x > v1 ? x : v1;
+            else b1 = x > b1 ? x : b1;
+        }
+    }
+    TopsM X;
+    if (!tops_of(r0, r1, p0, p1, v1, b1, G, X)) return false;
+    StatesM s[2];
+    for (int k = 0; k < 2; ++k) {
+        const double* q = k ? R : L;
+        s[k].r = 2 * to_units(q[0], X.r);
+        s[k].p = 2 * to_units(q[1], X.p);
+        s[k].un = 2 * to_units(q[2], X.v);
+        s[k].ut = 2 * to_units(q[3], X.v);
+        s[k].bn = 2 * to_units(q[4], X.b);
+        s[k].bt = 2 * to_units(q[5], X.b);
+        s[k].bz = 2 * to_units(q[6], X.b);
+    }
+    const FanM f = fan_of(s[0], s[1], X, G, UU);
+    return f.ok && hlld(f, s[0], s[1], X, G, F);
+}
+
+}  // namespace fx
+}  // namespace gd
