@@ -81,6 +81,27 @@ gd_status validate(const gd_config* c) {
     return GD_OK;
 }
 
+// The bounds of cell_active's FP32 test.  Each FP32 coordinate is within e = 2^-21 (|x0| + N dx) of
+// the true one (three roundings of 2^-24 of at most that size), so for a point of the sphere
+// (radius R) the square differs by at most m = 2 R (ex + ey) + (ex + ey)^2 + 2^-21 R^2; a point
+// beyond it stays beyond R^2 - m, one within it within R^2 + m, if R > ex + ey.  Twice that is
+// kept clear.  Indexes above 2^24 are not exact in FP32: the exact test decides alone then.
+void frozen_bounds(const gd_config& c, Params& P) {
+    P.f_x0 = (float)c.x0;
+    P.f_y0 = (float)c.y0;
+    P.f_dx = (float)c.dx;
+    P.f_dy = (float)c.dy;
+    P.f_in = -1.0f;
+    P.f_out = INFINITY;
+    const double u = 1.0 / (1 << 21), R = c.frozen_radius;
+    const double ex = u * (std::fabs(c.x0) + c.N * c.dx), ey = u * (std::fabs(c.y0) + c.M * c.dy);
+    const double m = 2.0 * (2.0 * R * (ex + ey) + (ex + ey) * (ex + ey) + u * R * R);
+    if (c.N > (1 << 24) || c.M > (1 << 24) || !(R > ex + ey)) return;
+    if (!(R * R > 1e-30 && R * R < 1e30 && c.dx > 1e-30 && c.dy > 1e-30)) return;
+    P.f_in = (float)(R * R - m);
+    P.f_out = (float)(R * R + m);
+}
+
 Params make_params(const gd_config& c) {
     Params P{};
     P.N = c.N;
@@ -98,6 +119,7 @@ Params make_params(const gd_config& c) {
     P.krit = c.krit;
     P.frozen_radius = c.frozen_radius;
     P.frozen = c.frozen_radius > 0.0 ? 1 : 0;
+    frozen_bounds(c, P);
     P.scheme = c.scheme;
     P.x_max = c.x_max;
     P.y_max = c.y_max;

@@ -546,7 +546,7 @@ __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in,
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < NK; ++k)
-        key[k] = __reduce_max_sync(0xffffffffu, keys[k][tid & (NT / 32 - 1)]);
+        key[k] = __reduce_max_sync(0xffffffffu, keys[k][(tid & 31) % (NT / 32)]);
     fx::TopsM X;
     if (!fx::tops_of(0xfffu - key[1], key[0], 0xfffu - key[3], key[2], key[4], key[5], P.gas, X))
         return false;

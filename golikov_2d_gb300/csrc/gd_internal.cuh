@@ -34,6 +34,8 @@ struct Params {
     double gamma, krit;
     double frozen_radius;
     int frozen;           // frozen_radius > 0 (tested on the integer pipe)
+    // the frozen test in FP32 (cell_active): squares above f_out are outside, below f_in inside
+    float f_x0, f_y0, f_dx, f_dy, f_in, f_out;
     int scheme;           // GD_SCHEME_*
     double x_max, y_max;  // domain extents of the Hancock schemes' cell coordinates
     // A launch of the fast step over a band of tile rows (gd_step_host): the band starts at
@@ -596,10 +598,17 @@ __device__ __forceinline__ void fetch_cell(const Params& P, const CPlanes& in, i
     if (bc >= 0) ghost_transform<NF>(v, bc, P.ambient_p);
 }
 
-// Inside the grid and not frozen (kernel.cu:2205, 2218: dist = sqrt(x*x + y*y) < ddist).
+// Inside the grid and not frozen (kernel.cu:2205, 2218: dist = sqrt(x*x + y*y) < ddist).  The
+// distance in FP32 decides away from the sphere; the shell that its error leaves open (frozen_bounds
+// in gd_api.cu) takes the reference's own arithmetic.  The exact test costs about 20 FP64
+// operations, and a face asks for both its cells.
 __device__ __forceinline__ bool cell_active(const Params& P, int gx, int gy) {
     if (gx < 0 || gx >= P.N || gy < 0 || gy >= P.M) return false;
     if (!P.frozen) return true;
+    const float fx = fmaf((float)gx, P.f_dx, P.f_x0), fy = fmaf((float)gy, P.f_dy, P.f_y0);
+    const float s = fmaf(fx, fx, fy * fy);
+    if (s > P.f_out) return true;
+    if (s < P.f_in) return false;
     const double x = P.x0 + gx * P.dx, y = P.y0 + gy * P.dy;
     // explicit roundings: every build and every call site decides alike (the parity build,
     // without contraction, computes the same sum)
