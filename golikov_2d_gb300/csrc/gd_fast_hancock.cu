@@ -25,6 +25,7 @@
 // divisions, slopes minmod(a - b, b - c) instead of h minmod((a - b)/h, (b - c)/h), the
 // neighbour's prediction at its own radius y_{m+-1} instead of y -+ dy, and the face solved
 // once (its two sides see the same flux up to rounding of the solver's symmetry).
+#include "gd_fixed_mhd.cuh"
 #include "gd_hancock_cell.cuh"
 #include "gd_internal.cuh"
 #include "gd_kernels.h"
@@ -105,8 +106,82 @@ __device__ __forceinline__ void mean_half(const double* Q, const double* D, doub
     }
 }
 
+// One face of a tile: faces 0 .. NFX-1 have an x normal, the rest a y normal.
+struct FaceH {
+    bool isx, used;  // used: next to a cell that the step updates
+    int pa, pb, out;  // the predictions on either side, and the place among the tile's fluxes
+    __device__ FaceH(const unsigned char* flag, int i) {
+        isx = i < NFX;
+        if (isx) {
+            const int ly = i / (TX + 1), lx = i - ly * (TX + 1);
+            used = (lx > 0 && flag[ly * TX + lx - 1] == 2) || (lx < TX && flag[ly * TX + lx] == 2);
+            pa = (ly + 1) * PX + lx;  // cell lx-1 of the tile
+            pb = pa + 1;
+            out = i;
+        } else {
+            const int j = i - NFX, ly = j / TX, lx = j - ly * TX;
+            used = (ly > 0 && flag[(ly - 1) * TX + lx] == 2) || (ly < TY && flag[ly * TX + lx] == 2);
+            pa = ly * PX + lx + 1;  // cell (lx, ly-1) of the tile
+            pb = pa + PX;
+            out = j;
+        }
+    }
+    // its states A + D/2 and A - D/2 in the local frame: x-face (n, t) = (x, y), y-face (y, x)
+    __device__ __forceinline__ void states(const double* pA, const double* D, double* qa,
+                                           double* qb) const {
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            const int g = (isx || f < 2 || f == 6 ? f : (f < 4 ? 5 - f : 9 - f)) * (PY * PX);
+            const double Aa = pA[g + pa], Ab = pA[g + pb];
+            qa[f] = fma(0.5, D[g + pa], Aa);
+            qb[f] = fma(-0.5, D[g + pb], Ab);
+            if (f < 2) {
+                qa[f] = le_zero(qa[f]) ? Aa : qa[f];
+                qb[f] = le_zero(qb[f]) ? Ab : qb[f];
+            }
+        }
+    }
+    template <class F>
+    __device__ __forceinline__ void store(double* fx, double* fy, const F& f) const {
+        double* fo = (isx ? fx : fy) + out;
+        const int st = isx ? NFX : NFY;
+        fo[0 * st] = f.m;
+        fo[1 * st] = f.e;
+        fo[2 * st] = isx ? f.mn : f.mt;
+        fo[3 * st] = isx ? f.mt : f.mn;
+        fo[4 * st] = isx ? f.bn : f.bt;
+        fo[5 * st] = isx ? f.bt : f.bn;
+        fo[6 * st] = f.bz;
+    }
+};
+
+// The faces of a thread that the integer solver left (bit k: the k-th), in floating point; speed:
+// those whose wave speed is missing too.
+__device__ __noinline__ void faces_left(const Params& P, double* smem, const unsigned char* flag,
+                                        unsigned int left, unsigned int speed, double& umax_x,
+                                        double& umax_y) {
+    const double *pA = smem + kUnion, *pDX = pA + kPred, *pDY = pDX + kPred;
+    while (left) {
+        const int k = __ffs((int)left) - 1;
+        left &= left - 1;
+        const FaceH w(flag, threadIdx.x + k * NT);
+        double qa[NF], qb[NF], UU;
+        w.states(pA, w.isx ? pDX : pDY, qa, qb);
+        Side<double> A, B;
+        side(A, qa[0], qa[1], qa[2], qa[3], qa[4], qa[5], qa[6], P);
+        side(B, qb[0], qb[1], qb[2], qb[3], qb[4], qb[5], qb[6], P);
+        w.store(smem, smem + kFx, hlld_local(A, B, GD_METHOD_HLLD, P, UU));
+        if (speed >> k & 1) {
+            if (w.isx) umax_x = max_nonneg(umax_x, UU);
+            else umax_y = max_nonneg(umax_y, UU);
+        }
+    }
+}
+
 template <bool VYP>
-__global__ void __launch_bounds__(NT) hancock_tile_kernel(Params P, CPlanes in, Planes out,
+__global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_constant__ Params P,
+                                                          const __grid_constant__ CPlanes in,
+                                                          const __grid_constant__ Planes out,
                                                           const double* __restrict__ T_do_ptr,
                                                           unsigned long long* T_bits,
                                                           Scalars* rot, Scalars* ctr,
@@ -234,71 +309,34 @@ __global__ void __launch_bounds__(NT) hancock_tile_kernel(Params P, CPlanes in, 
     }
     __syncthreads();
 
-    // ---- F: each face of an updated cell once -------------------------------------------
+    // ---- F: each face of an updated cell once: HLLD in 64-bit integers (gd_fixed_mhd.cuh), the
+    // two states of a face in units of their own; the corrector and the predictor keep the FP64
+    // pipe (the flux took 240 of the step's 671 FP64 operations a cell)
     double umax_x = 0.0, umax_y = 0.0;
-    for (int i = tid; i < NFX + NFY; i += NT) {
-        const bool isx = i < NFX;
-        int lx, ly, pa, pb;
-        if (isx) {
-            ly = i / (TX + 1);
-            lx = i - ly * (TX + 1);
-            const bool need = (lx > 0 && flag[ly * TX + lx - 1] == 2) ||
-                              (lx < TX && flag[ly * TX + lx] == 2);
-            if (!need) continue;
-            pa = (ly + 1) * PX + lx;  // cell lx-1 of the tile
-            pb = pa + 1;
-        } else {
-            const int j = i - NFX;
-            ly = j / TX;
-            lx = j - ly * TX;
-            const bool need = (ly > 0 && flag[(ly - 1) * TX + lx] == 2) ||
-                              (ly < TY && flag[ly * TX + lx] == 2);
-            if (!need) continue;
-            pa = ly * PX + lx + 1;  // cell (lx, ly-1) of the tile
-            pb = pa + PX;
+    unsigned int left = 0, speed = 0, bit = 1;
+    for (int i = tid; i < NFX + NFY; i += NT, bit <<= 1) {
+        const FaceH w(flag, i);
+        if (!w.used) continue;
+        double qa[NF], qb[NF], UU;
+        w.states(pA, w.isx ? pDX : pDY, qa, qb);
+        fx::StatesM A, B;
+        fx::TopsM X;
+        fx::FanM fan;
+        if (fx::face_units(qa, qb, P.gas, A, B, X)) fan = fx::fan_of(A, B, X, P.gas, UU);
+        else fan.ok = false;
+        if (!fan.ok) {
+            left |= bit;
+            speed |= bit;
+            continue;
         }
-        const double* D = isx ? pDX : pDY;
-        double qa[NF], qb[NF];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            const double Aa = pA[f * PY * PX + pa], Ab = pA[f * PY * PX + pb];
-            qa[f] = fma(0.5, D[f * PY * PX + pa], Aa);
-            qb[f] = fma(-0.5, D[f * PY * PX + pb], Ab);
-            if (f < 2) {
-                qa[f] = le_zero(qa[f]) ? Aa : qa[f];
-                qb[f] = le_zero(qb[f]) ? Ab : qb[f];
-            }
-        }
-        // local frame: x-face (n, t) = (x, y); y-face (n, t) = (y, x); z stays z
-        Side<double> A, B;
-        side(A, qa[0], qa[1], isx ? qa[2] : qa[3], isx ? qa[3] : qa[2], isx ? qa[4] : qa[5],
-             isx ? qa[5] : qa[4], qa[6], P);
-        side(B, qb[0], qb[1], isx ? qb[2] : qb[3], isx ? qb[3] : qb[2], isx ? qb[4] : qb[5],
-             isx ? qb[5] : qb[4], qb[6], P);
-        double UU;
-        const FluxM<double> F = hlld_local(A, B, GD_METHOD_HLLD, P, UU);
-        if (isx) {
-            double* fo = fx + ly * (TX + 1) + lx;
-            fo[0 * NFX] = F.m;
-            fo[1 * NFX] = F.e;
-            fo[2 * NFX] = F.mn;
-            fo[3 * NFX] = F.mt;
-            fo[4 * NFX] = F.bn;
-            fo[5 * NFX] = F.bt;
-            fo[6 * NFX] = F.bz;
-            umax_x = max_nonneg(umax_x, UU);
-        } else {
-            double* fo = fy + ly * TX + lx;
-            fo[0 * NFY] = F.m;
-            fo[1 * NFY] = F.e;
-            fo[2 * NFY] = F.mt;
-            fo[3 * NFY] = F.mn;
-            fo[4 * NFY] = F.bt;
-            fo[5 * NFY] = F.bn;
-            fo[6 * NFY] = F.bz;
-            umax_y = max_nonneg(umax_y, UU);
-        }
+        if (w.isx) umax_x = max_nonneg(umax_x, UU);
+        else umax_y = max_nonneg(umax_y, UU);
+        if (dt_only) continue;
+        fx::FluxI F;
+        if (fx::hlld(fan, A, B, X, P.gas, F)) w.store(fx, fy, F);
+        else left |= bit;
     }
+    if (left) faces_left(P, smem, flag, left, speed, umax_x, umax_y);
     __syncthreads();
 
     // ---- U: corrector (kernel.cu:3256-3281, Pdiv = 0) --------------------------------------

@@ -337,37 +337,37 @@ GD_HD bool tops_of(uint32_t r0, uint32_t r1, uint32_t p0, uint32_t p1, uint32_t 
     return ok && b1 <= 1023 + kRange;
 }
 
-// Flux and larger wave speed of one face given by its states {rho, p, un, ut, bn, bt, bz}.
+// The two states {rho, p, un, ut, bn, bt, bz} of a face in units of their own; false where the
+// integer solver does not take them.
+GD_HD bool face_units(const double* L, const double* R, const Gas& G, StatesM& A, StatesM& B,
+                      TopsM& X) {
+    const uint32_t rL = signed_exp_field(L[0]), rR = signed_exp_field(R[0]);
+    const uint32_t pL = signed_exp_field(L[1]), pR = signed_exp_field(R[1]);
+    uint32_t v1 = 0, b1 = 0;
+#pragma unroll
+    for (int f = 2; f < 7; ++f) {
+        const uint32_t x = exp_field(L[f]), y = exp_field(R[f]), m = x > y ? x : y;
+        if (f < 4) v1 = m > v1 ? m : v1;
+        else b1 = m > b1 ? m : b1;
+    }
+    if (!tops_of(rL < rR ? rL : rR, rL < rR ? rR : rL, pL < pR ? pL : pR, pL < pR ? pR : pL, v1,
+                 b1, G, X))
+        return false;
+    A = StatesM{2 * to_units(L[0], X.r), 2 * to_units(L[1], X.p), 2 * to_units(L[2], X.v),
+                2 * to_units(L[3], X.v), 2 * to_units(L[4], X.b), 2 * to_units(L[5], X.b),
+                2 * to_units(L[6], X.b)};
+    B = StatesM{2 * to_units(R[0], X.r), 2 * to_units(R[1], X.p), 2 * to_units(R[2], X.v),
+                2 * to_units(R[3], X.v), 2 * to_units(R[4], X.b), 2 * to_units(R[5], X.b),
+                2 * to_units(R[6], X.b)};
+    return true;
+}
+// Flux and larger wave speed of that face.
 GD_HD bool hlld_face(const double* L, const double* R, const Gas& G, FluxI& F, double& UU) {
-    uint32_t r0 = ~0u, r1 = 0, p0 = ~0u, p1 = 0, v1 = 0, b1 = 0;
-    for (int k = 0; k < 2; ++k) {
-        const double* q = k ? R : L;
-        const uint32_t r = signed_exp_field(q[0]), p = signed_exp_field(q[1]);
-        r0 = r < r0 ? r : r0;
-        r1 = r > r1 ? r : r1;
-        p0 = p < p0 ? p : p0;
-        p1 = p > p1 ? p : p1;
-        for (int f = 2; f < 7; ++f) {
-            const uint32_t x = exp_field(q[f]);
-            if (f < 4) v1 = x > v1 ? x : v1;
-            else b1 = x > b1 ? x : b1;
-        }
-    }
+    StatesM A, B;
     TopsM X;
-    if (!tops_of(r0, r1, p0, p1, v1, b1, G, X)) return false;
-    StatesM s[2];
-    for (int k = 0; k < 2; ++k) {
-        const double* q = k ? R : L;
-        s[k].r = 2 * to_units(q[0], X.r);
-        s[k].p = 2 * to_units(q[1], X.p);
-        s[k].un = 2 * to_units(q[2], X.v);
-        s[k].ut = 2 * to_units(q[3], X.v);
-        s[k].bn = 2 * to_units(q[4], X.b);
-        s[k].bt = 2 * to_units(q[5], X.b);
-        s[k].bz = 2 * to_units(q[6], X.b);
-    }
-    const FanM f = fan_of(s[0], s[1], X, G, UU);
-    return f.ok && hlld(f, s[0], s[1], X, G, F);
+    if (!face_units(L, R, G, A, B, X)) return false;
+    const FanM f = fan_of(A, B, X, G, UU);
+    return f.ok && hlld(f, A, B, X, G, F);
 }
 
 }  // namespace fx
