@@ -36,6 +36,7 @@ gd_status cuda_status(cudaError_t e) { return e == cudaSuccess ? GD_OK : gd::cud
 struct gd_batch {
     int ngrids = 0;
     int order = 2;
+    bool hllc_only = true;
     int nf = 4;
     std::vector<gd_config> cfgs;
     std::vector<Params> params;
@@ -77,7 +78,7 @@ gd_status step_persistent(gd_batch* b, int variant, int dt_only, Scalars* sc_ove
                           cudaStream_t st) {
     GD_TRY(gd::launch_euler_batch(variant, b->order, b->d_grids[variant], b->d_items[variant],
                                   b->nitems[variant], b->cur, dt_only, sc_override,
-                                  b->ctas[variant], st));
+                                  b->ctas[variant], b->hllc_only, st));
     b->launches += 1;
     return GD_OK;
 }
@@ -124,6 +125,7 @@ gd_status gd_batch_create(const gd_config* cfgs, int ngrids, gd_batch** out) {
     if (!b) return GD_ERR_INVALID_ARG;
     b->ngrids = ngrids;
     b->order = cfgs[0].order;
+    for (int g = 0; g < ngrids; ++g) b->hllc_only = b->hllc_only && cfgs[g].method == GD_METHOD_HLLC;
     b->cfgs.assign(cfgs, cfgs + ngrids);
     size_t off = 0;
     for (int g = 0; g < ngrids; ++g) {

@@ -557,8 +557,8 @@ __device__ __noinline__ void faces_left(const Params& P, double* smem, const fx:
 }
 
 // Every face of a tile held in integers.  dt_only: the wave speeds alone.
-template <int ORDER, int TX, int TY>
-__device__ __forceinline__ void faces_hllc(const Params& P, double* smem, const fx::Tops& X,
+template <bool HLL, int ORDER, int TX, int TY>
+__device__ __forceinline__ void faces_int(const Params& P, double* smem, const fx::Tops& X,
                                            int tx0, int ty0, int dt_only, Speeds& u) {
     using S = Shape<ORDER, TX, TY>;
     using fx::i64;
@@ -585,7 +585,7 @@ __device__ __forceinline__ void faces_hllc(const Params& P, double* smem, const 
         }
         const fx::States s{a[0], b[0], a[1], b[1], a[2], b[2], a[3], b[3]};
         double UU;
-        const fx::Fan fan = fx::fan_of(s, X, P.gas, UU);
+        const fx::Fan fan = fx::fan_of<HLL>(s, X, P.gas, UU);
         if (!fan.ok) {
             left |= bit;
             speed |= bit;
@@ -594,15 +594,18 @@ __device__ __forceinline__ void faces_hllc(const Params& P, double* smem, const 
         u.take(w.isx, UU);
         if (dt_only) continue;
         double m, mn, mt, e;
-        if (fx::hllc(fan, s, X, P.gas, m, mn, mt, e)) w.store(t.fx, t.fy, m, e, mn, mt);
+        const bool done = HLL ? fx::hll(fan, s, X, P.gas, m, mn, mt, e)
+                              : fx::hllc(fan, s, X, P.gas, m, mn, mt, e);
+        if (done) w.store(t.fx, t.fy, m, e, mn, mt);
         else left |= bit;
     }
     if (left) faces_left<ORDER, TX, TY>(P, smem, X, tx0, ty0, left, speed, u);
 }
 
 // Returns false, with nothing written, where the tile's cells cannot be held in common units.
-// Every thread of the block must call it, and all get the same answer.
-template <int ORDER, int TX, int TY>
+// Every thread of the block must call it, and all get the same answer.  METHODS: 1 HLLC, 2 HLL, 3
+// the one of P (both solvers in the function).
+template <int METHODS, int ORDER, int TX, int TY>
 __device__ __forceinline__ bool euler_tile_int(const Params& P, const CPlanes& in, const Planes& out,
                                             int tx0, int ty0, double T_do, int dt_only,
                                             double* smem, TileResult& res, double* aux) {
@@ -662,7 +665,10 @@ __device__ __forceinline__ bool euler_tile_int(const Params& P, const CPlanes& i
     }
     __syncthreads();
     Speeds fastest{0.0, 0.0};
-    faces_hllc<ORDER, TX, TY>(P, smem, X, tx0, ty0, dt_only, fastest);
+    if (METHODS == 2 || (METHODS == 3 && P.method == GD_METHOD_HLL))
+        faces_int<true, ORDER, TX, TY>(P, smem, X, tx0, ty0, dt_only, fastest);
+    else
+        faces_int<false, ORDER, TX, TY>(P, smem, X, tx0, ty0, dt_only, fastest);
     __syncthreads();
     update_cells<double, ORDER, TX, TY, TX, TX * TY>(P, out, tx0, ty0, T_do, dt_only, t.cell, t.fx,
                                                      t.fy, res, aux);
@@ -671,13 +677,13 @@ __device__ __forceinline__ bool euler_tile_int(const Params& P, const CPlanes& i
     return true;
 }
 
-// A tile of the step: in integers where the method is HLLC and the tile's range allows it.
-template <int ORDER, int TX, int TY>
+// A tile of the step: in integers where the tile's range allows it.
+template <int METHODS, int ORDER, int TX, int TY>
 __device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, const Planes& out,
                                           int tx0, int ty0, double T_do, int dt_only,
                                           double* smem, TileResult& res, double* aux) {
-    if (P.method != GD_METHOD_HLL && euler_tile_int<ORDER, TX, TY>(P, in, out, tx0, ty0, T_do,
-                                                                   dt_only, smem, res, aux))
+    if (euler_tile_int<METHODS, ORDER, TX, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, res,
+                                               aux))
         return;
     __syncthreads();
     euler_tile<double, ORDER, TX, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, res, aux);
@@ -691,7 +697,7 @@ __device__ __forceinline__ void add_counters(Scalars* ctr, const TileResult& r) 
     }
 }
 
-template <int ORDER, int TX, int TY>
+template <int METHODS, int ORDER, int TX, int TY>
 __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_fast_kernel(const __grid_constant__ Params P,
                                                         const __grid_constant__ CPlanes in,
                                                         const __grid_constant__ Planes out,
@@ -701,7 +707,7 @@ __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_fast_kernel(const __g
                                                         double* aux) {
     extern __shared__ double smem[];
     TileResult r;
-    step_tile<ORDER, TX, TY>(P, in, out, blockIdx.x * TX, (blockIdx.y + P.tile_row0) * TY,
+    step_tile<METHODS, ORDER, TX, TY>(P, in, out, blockIdx.x * TX, (blockIdx.y + P.tile_row0) * TY,
                              *T_do_ptr, dt_only, smem, r, aux);
     add_counters(ctr, r);
     block_dt_and_rotate<NT>(P, r.umax_x, r.umax_y, r.any_active, T_bits, rot, P.tile_nblocks);
@@ -730,7 +736,9 @@ __global__ void __launch_bounds__(NT) euler_tangent_kernel(Params P, CPlanes in,
 // With dt_only, tiles only min-combine their dt (no state write, no rotation).
 // `sc_override` (may be null) replaces every grid's scalars (the autotuner times steps
 // without touching the real dt and time).
-template <int ORDER, int TX, int TY>
+// METHODS 1: every grid's method is HLLC (a second solver in the kernel costs it 40 registers'
+// spills: 7.40 against 7.69 ms per pass of 128 grids); 3: any.
+template <int METHODS, int ORDER, int TX, int TY>
 __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_batch_kernel(const BatchGrid* __restrict__ grids,
                                                          const int2* __restrict__ items,
                                                          int nitems, int cur, int dt_only,
@@ -758,22 +766,25 @@ __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_batch_kernel(const Ba
         const int tx0 = (tile % g.tiles_x) * TX, ty0 = (tile / g.tiles_x) * TY;
         const double T_do = g.sc->T_do;
         TileResult r;
-        step_tile<ORDER, TX, TY>(g.P, in, out, tx0, ty0, T_do, dt_only, smem, r, nullptr);
+        step_tile<METHODS, ORDER, TX, TY>(g.P, in, out, tx0, ty0, T_do, dt_only, smem, r, nullptr);
         add_counters(dt_only ? nullptr : g.sc, r);
         block_dt_and_rotate<NT>(g.P, r.umax_x, r.umax_y, r.any_active, &g.sc->T_bits,
                                 dt_only ? nullptr : g.sc, (unsigned int)g.ntiles);
     }
 }
 
+template <class K>
+cudaError_t set_room(K* kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
 template <int ORDER, int TX, int TY>
 cudaError_t set_attrs() {
-    cudaError_t e = cudaFuncSetAttribute(euler_fast_kernel<ORDER, TX, TY>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)Shape<ORDER, TX, TY>::bytes);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(euler_batch_kernel<ORDER, TX, TY>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)Shape<ORDER, TX, TY>::bytes);
+    constexpr size_t n = Shape<ORDER, TX, TY>::bytes;
+    cudaError_t e = set_room(euler_fast_kernel<1, ORDER, TX, TY>, n);
+    if (e == cudaSuccess) e = set_room(euler_fast_kernel<2, ORDER, TX, TY>, n);
+    if (e == cudaSuccess) e = set_room(euler_batch_kernel<1, ORDER, TX, TY>, n);
+    if (e == cudaSuccess) e = set_room(euler_batch_kernel<3, ORDER, TX, TY>, n);
+    return e;
 }
 
 template <int ORDER, int TX, int TY>
@@ -781,16 +792,27 @@ cudaError_t launch_single(const Params& P, const CPlanes& in, const Planes& out,
                           const double* T_do, unsigned long long* T_bits, Scalars* rot,
                           Scalars* ctr, int dt_only, cudaStream_t st, double* aux = nullptr) {
     dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + TY - 1) / TY);
-    euler_fast_kernel<ORDER, TX, TY><<<grid, NT, Shape<ORDER, TX, TY>::bytes, st>>>(
-        P, in, out, T_do, T_bits, rot, ctr, dt_only, aux);
+    constexpr size_t n = Shape<ORDER, TX, TY>::bytes;
+    if (P.method == GD_METHOD_HLL)
+        euler_fast_kernel<2, ORDER, TX, TY><<<grid, NT, n, st>>>(P, in, out, T_do, T_bits, rot,
+                                                                 ctr, dt_only, aux);
+    else
+        euler_fast_kernel<1, ORDER, TX, TY><<<grid, NT, n, st>>>(P, in, out, T_do, T_bits, rot,
+                                                                 ctr, dt_only, aux);
     return cudaGetLastError();
 }
 
 template <int ORDER, int TX, int TY>
 cudaError_t launch_batch(const BatchGrid* grids, const int2* items, int nitems, int cur,
-                         int dt_only, Scalars* sc_override, int ctas, cudaStream_t st) {
-    euler_batch_kernel<ORDER, TX, TY><<<ctas, NT, Shape<ORDER, TX, TY>::bytes, st>>>(
-        grids, items, nitems, cur, dt_only, sc_override);
+                         int dt_only, Scalars* sc_override, int ctas, bool hllc_only,
+                         cudaStream_t st) {
+    constexpr size_t n = Shape<ORDER, TX, TY>::bytes;
+    if (hllc_only)
+        euler_batch_kernel<1, ORDER, TX, TY><<<ctas, NT, n, st>>>(grids, items, nitems, cur,
+                                                                  dt_only, sc_override);
+    else
+        euler_batch_kernel<3, ORDER, TX, TY><<<ctas, NT, n, st>>>(grids, items, nitems, cur,
+                                                                  dt_only, sc_override);
     return cudaGetLastError();
 }
 
@@ -825,7 +847,7 @@ namespace {
 template <int ORDER, int TX, int TY>
 int blocks_per_sm() {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, euler_batch_kernel<ORDER, TX, TY>, NT,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, euler_batch_kernel<3, ORDER, TX, TY>, NT,
                                                       Shape<ORDER, TX, TY>::bytes) != cudaSuccess)
         return 1;
     return n > 0 ? n : 1;
@@ -910,13 +932,13 @@ cudaError_t launch_euler_fast_aux(const Params& P, const CPlanes& in, const Plan
 
 cudaError_t launch_euler_batch(int variant, int order, const BatchGrid* grids, const int2* items,
                                int nitems, int cur, int dt_only, Scalars* sc_override, int ctas,
-                               cudaStream_t st) {
+                               bool hllc_only, cudaStream_t st) {
     if (order == 1) {
         GD_EULER_DISPATCH(1, variant, launch_batch,
-                          (grids, items, nitems, cur, dt_only, sc_override, ctas, st));
+                          (grids, items, nitems, cur, dt_only, sc_override, ctas, hllc_only, st));
     }
     GD_EULER_DISPATCH(2, variant, launch_batch,
-                      (grids, items, nitems, cur, dt_only, sc_override, ctas, st));
+                      (grids, items, nitems, cur, dt_only, sc_override, ctas, hllc_only, st));
 }
 
 
@@ -937,7 +959,8 @@ __global__ void euler_face_probe_kernel(Params P, long long n, int axis,
     const double qb[NF] = {b[0], b[1], isx ? b[2] : b[3], isx ? b[3] : b[2]};
     double UU, f[NF];
     FluxE<double> F;
-    if (P.method != GD_METHOD_HLL && fx::hllc_face(qa, qb, P.gas, f, UU))
+    if (P.method == GD_METHOD_HLL ? fx::euler_face<true>(qa, qb, P.gas, f, UU)
+                                  : fx::euler_face<false>(qa, qb, P.gas, f, UU))
         F = FluxE<double>{f[0], f[1], f[2], f[3]};
     else
         F = flux_of(P, qa, qb, UU);

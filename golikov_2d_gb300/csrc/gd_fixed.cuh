@@ -113,6 +113,14 @@ GD_HD int imin(int a, int b) { return a < b ? a : b; }
 // arithmetic shift right by any n >= 0
 GD_HD i64 sra(i64 x, int n) { return x >> (n < 63 ? n : 63); }
 
+// x 2^-s for either sign of s; a left shift's result fits
+GD_HD i64 shift(i64 x, int s) {
+    return (i64)((u64)x << imin(imax(-s, 0), 62)) >> imin(imax(s, 0), 63);
+}
+GD_HD i64 iabs(i64 x) { return x < 0 ? -x : x; }
+// whether x >= 0 shifted by shift(x, s) stays below 2^61
+GD_HD bool fits(i64 x, int s) { return s >= 0 || x >> imax(61 + s, 0) == 0; }
+
 GD_HD float rsqrt_seed(float x) {
 #if defined(__CUDA_ARCH__)
     float r;
@@ -187,13 +195,15 @@ GD_HD i64 sqrt_over(i64 am, int ea, Pos r, int& k) {
 
 // The constants a face solver needs of gamma, as m 2^(e - 62).
 struct Gas {
-    i64 g, gg;    // gamma, gamma / (gamma - 1)
-    int ge, gge;
+    i64 g, gg, gi;  // gamma, gamma / (gamma - 1), 1 / (gamma - 1)
+    int ge, gge, gie;
     int room;     // extra bits that gamma / (gamma - 1) p takes beside rho c^2; -1: no integer path
 };
 inline Gas gas_of(double gamma) {
     Gas G;
-    const Pos a = pos_of(gamma), b = pos_of(gamma / (gamma - 1.0));
+    const Pos a = pos_of(gamma), b = pos_of(gamma / (gamma - 1.0)), c = pos_of(1.0 / (gamma - 1.0));
+    G.gi = c.m;
+    G.gie = c.e;
     G.g = a.m;
     G.ge = a.e;
     G.gg = b.m;
@@ -258,6 +268,8 @@ struct Fan {
 // ok is false where a scale would leave a quantity fewer bits than binary64 does: accepted are
 // sound speeds within a factor of about 4 of each other, and normal velocities to about 64 of
 // them.  UU: the larger wave speed.
+// HLL: the fan min(u) - max(c), max(u) + max(c) of kernel.cu:1516-1517 instead of Davis'.
+template <bool HLL = false>
 GD_HD Fan fan_of(const States& q, const Tops& X, const Gas& G, double& UU) {
     Fan f;
     f.RL = pos_of(q.rL, X.r);
@@ -274,7 +286,11 @@ GD_HD Fan fan_of(const States& q, const Tops& X, const Gas& G, double& UU) {
     f.E = imax(kmax + 2, X.v + imax(4 - lz, 0));
     f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 8;
     if (!f.ok) return f;
-    const i64 cL = wL >> (f.E - 1 - kL), cR = wR >> (f.E - 1 - kR);
+    i64 cL = wL >> (f.E - 1 - kL), cR = wR >> (f.E - 1 - kR);
+    if (HLL) {
+        cL = cL > cR ? cL : cR;
+        cR = cL;
+    }
     const int sh = imin(f.E - X.v, 63);
     f.uL = q.uL >> sh;
     f.uR = q.uR >> sh;
@@ -353,6 +369,48 @@ GD_HD bool hllc(const Fan& f, const States& s, const Tops& X, const Gas& G, doub
     return true;
 }
 
+// HLL flux of that face (kernel.cu:1485-1609) with fan_of<true>.  With the fan cut at the face,
+// D_L <= 0 <= D_R, and a = D_R / (D_R - D_L), the average (D_R F_L - D_L F_R + D_L D_R (U_R - U_L))
+// / (D_R - D_L) is a (F_L - D_L U_L) + (1 - a) (F_R - D_R U_R), and on one side of the face
+// a = 1 or 0 gives the physical flux: no difference of the two sides' states is formed.  False,
+// with nothing to use, where the energy would not fit its unit.
+GD_HD bool hll(const Fan& f, const States& s, const Tops& X, const Gas& G, double& Fm, double& Fn,
+               double& Ft, double& Fe) {
+    const int E = f.E, ER = imax(f.RL.e, f.RR.e);
+    const i64 DL = f.SL < 0 ? f.SL : 0, DR = f.SR > 0 ? f.SR : 0;
+    int lz;
+    const i64 iD = rcp(DR - DL, lz);
+    const i64 one = 1LL << 60;
+    i64 a = mulk<0, 2>(DR << (lz - 2), iD);  // units of 2^-60
+    a = f.SL >= 0 ? one : (f.SR <= 0 ? 0 : a);
+    const i64 b = one - a;
+    const i64 gL = f.uL - DL, gR = f.uR - DR;
+    // a rho_L (u_L - D_L) and b rho_R (u_R - D_R), units 2^(ER + E - 59)
+    const i64 A = mulk<2, 2>(a, mulk<0, 0>(f.RL.m, gL) >> imin(ER - f.RL.e, 63));
+    const i64 B = mulk<2, 2>(b, mulk<0, 0>(f.RR.m, gR) >> imin(ER - f.RR.e, 63));
+    Fm = to_double(A + B, ER + E - 59);
+    // a p_L and b p_R, units 2^(ER + 2E - 60); over gamma - 1 with G.room bits of room
+    const int sp = ER + 2 * E;
+    const i64 pL = mulk<2, 2>(a, f.PL.m >> imin(sp + 2 - f.PL.e, 63));
+    const i64 pR = mulk<2, 2>(b, f.PR.m >> imin(sp + 2 - f.PR.e, 63));
+    Fn = to_double(mulk<2, 2>(A, f.uL) + mulk<2, 2>(B, f.uR) + pL + pR, ER + 2 * E - 60);
+    const i64 TL = mulk<2, 1>(A, s.vL), TR = mulk<2, 1>(B, s.vR);
+    Ft = to_double(TL + TR, ER + E + X.v - 59);
+    // energy: p (u - D) / (gamma - 1) + p u + rho (u - D) (u^2 + v^2) / 2, units
+    // 2^(ER + 3E - 62 + room)
+    const i64 qL = mulk<2, 2>(a, sra(mulk<0, 0>(f.PL.m, G.gi), sp - f.PL.e - G.gie + G.room));
+    const i64 qR = mulk<2, 2>(b, sra(mulk<0, 0>(f.PR.m, G.gi), sp - f.PR.e - G.gie + G.room));
+    const int z = clz32((uint32_t)(hi32(qL) | hi32(qR))) - 1;
+    const i64 h = mulk<0, 1>(qL << z, gL) + mulk<0, 1>(qR << z, gR);
+    const i64 t = mulk<1, 1>(TL, s.vL) + mulk<1, 1>(TR, s.vR);
+    const int st = 2 * (E - X.v) - 3;
+    if (!(fits(iabs(h), z - 4) && fits(iabs(t), st))) return false;
+    const i64 k = mulk<2, 2>(A, mulk<2, 2>(f.uL, f.uL)) + mulk<2, 2>(B, mulk<2, 2>(f.uR, f.uR)) +
+                  mulk<3, 2>(pL, f.uL) + mulk<3, 2>(pR, f.uR) + shift(t, st);
+    Fe = to_double(shift(h, z - 4) + (k >> G.room), ER + 3 * E - 62 + G.room);
+    return true;
+}
+
 // Exponent field of x (0x7ff for infinities and NaN), and with its sign bit above it.
 GD_HD uint32_t exp_field(double x) {
     uint32_t hi, lo;
@@ -375,9 +433,10 @@ GD_HD bool tops_of(uint32_t r0, uint32_t r1, uint32_t p0, uint32_t p1, uint32_t 
     return G.room >= 0 && r0 >= low && r1 <= high && r1 - r0 <= kSpan && p0 >= low &&
            p1 <= high && p1 - p0 <= kSpan && v1 <= high;
 }
-// The flux and the larger wave speed of one face given by its two states; false where the
-// integer solver does not take it.
-GD_HD bool hllc_face(const double* L, const double* R, const Gas& G, double* F, double& UU) {
+// The flux (HLL or HLLC) and the larger wave speed of one face given by its two states; false
+// where the integer solver does not take it.
+template <bool HLL>
+GD_HD bool euler_face(const double* L, const double* R, const Gas& G, double* F, double& UU) {
     const uint32_t rL = signed_exp_field(L[0]), rR = signed_exp_field(R[0]);
     const uint32_t pL = signed_exp_field(L[1]), pR = signed_exp_field(R[1]);
     const uint32_t v0 = imax(exp_field(L[2]), exp_field(L[3]));
@@ -389,8 +448,10 @@ GD_HD bool hllc_face(const double* L, const double* R, const Gas& G, double* F, 
     const States s{2 * to_units(L[0], X.r), 2 * to_units(R[0], X.r), 2 * to_units(L[1], X.p),
                    2 * to_units(R[1], X.p), 2 * to_units(L[2], X.v), 2 * to_units(R[2], X.v),
                    2 * to_units(L[3], X.v), 2 * to_units(R[3], X.v)};
-    const Fan f = fan_of(s, X, G, UU);
-    return f.ok && hllc(f, s, X, G, F[0], F[1], F[2], F[3]);
+    const Fan f = fan_of<HLL>(s, X, G, UU);
+    if (!f.ok) return false;
+    if (!HLL) return hllc(f, s, X, G, F[0], F[1], F[2], F[3]);
+    return hll(f, s, X, G, F[0], F[1], F[2], F[3]);
 }
 
 }  // namespace fx

@@ -30,16 +30,8 @@ struct StatesM {
     i64 r, p, un, ut, bn, bt, bz;
 };
 
-// x 2^-s for either sign of s; a left shift's result fits
-GD_HD i64 shift(i64 x, int s) {
-    return (i64)((u64)x << imin(imax(-s, 0), 62)) >> imin(imax(s, 0), 63);
-}
-GD_HD i64 iabs(i64 x) { return x < 0 ? -x : x; }
 // |x| < 2^61 (and a little beyond on the negative side)
 GD_HD bool below61(i64 x) { return (uint32_t)(hi32(x) + (1 << 29)) < (1u << 30); }
-
-// whether x >= 0 shifted by shift(x, s) stays below 2^61
-GD_HD bool fits(i64 x, int s) { return s >= 0 || x >> imax(61 + s, 0) == 0; }
 
 // sqrt(x) 2^(29 + h) of x 2^(2 h) in [2^61, 2^63): the root (w, in [2^59, 2^61)) and, where asked,
 // the reciprocal root times 2^(91 - h).  As sqrt_over: e = 1 - x y^2 for the FP32 seed y.

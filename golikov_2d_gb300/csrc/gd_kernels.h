@@ -59,10 +59,11 @@ cudaError_t launch_batch_set_time(BatchGrid* grids, int ngrids, double T_do, dou
                                   cudaStream_t st);
 cudaError_t launch_batch_reset_T(BatchGrid* grids, int ngrids, cudaStream_t st);
 cudaError_t launch_batch_dt_commit(BatchGrid* grids, int ngrids, cudaStream_t st);
-// Persistent batched step over the (grid, tile) list `items` with `ctas` CTAs.
+// Persistent batched step over the (grid, tile) list `items` with `ctas` CTAs; hllc_only: no grid
+// of it uses HLL.
 cudaError_t launch_euler_batch(int variant, int order, const BatchGrid* grids, const int2* items,
                                int nitems, int cur, int dt_only, Scalars* sc_override, int ctas,
-                               cudaStream_t st);
+                               bool hllc_only, cudaStream_t st);
 
 // Tangent (forward-mode JVP) of one fast MHD step with the dt read from *T_do:
 // (in, din) -> (out, dout).
