@@ -631,8 +631,11 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
 // Called by one thread of each block after the block's dt is combined: the last block of
 // the launch to arrive performs the funk_time rotation on `sc` (T_do <- T, TT += T_do,
 // T <- 1e7, ++step).  `nblocks` blocks report per launch; 0 means every block of the grid.
-__device__ __forceinline__ void rotate_if_last(Scalars* sc, unsigned int nblocks) {
-    __threadfence();
+// `combined`: this block lowered T (what it wrote has to be seen before its ticket; a block that
+// wrote nothing to T has nothing to order).
+__device__ __forceinline__ void rotate_if_last(Scalars* sc, unsigned int nblocks,
+                                               bool combined = true) {
+    if (combined) __threadfence();
     const unsigned int nb = nblocks ? nblocks : gridDim.x * gridDim.y * gridDim.z;
     const unsigned int ticket = atomicAdd(&sc->done, 1u);
     if (ticket == nb - 1) {
@@ -650,6 +653,16 @@ __device__ __forceinline__ void rotate_if_last(Scalars* sc, unsigned int nblocks
     }
 }
 
+// Whether krad / u is sure to be above T (all positive; FP32 quotient, 2^-20 off at most, with a
+// margin of 2^-12).  False where a value is outside FP32's range.
+__device__ __forceinline__ bool dt_above(double krad, unsigned long long u, double T) {
+    const double v = from_bits((long long)u);
+    if (!(in_f32_range(krad) && in_f32_range(v) && in_f32_range(T))) return false;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(seed_f32(v)));
+    return seed_f32(krad) * r > seed_f32(T) * 1.000244140625f;
+}
+
 // Reduces the per-thread maximum wave speeds of x and y faces over the block, turns them
 // into the block's dt (min over faces of krit*rad/UU, capped at 1000) and min-combines it
 // into *T_bits.  `any_active` says whether the block contains a non-frozen cell.  Then,
@@ -664,6 +677,10 @@ __device__ void block_dt_and_rotate(const Params& P, double umax_x, double umax_
     __shared__ unsigned long long red[2][NTHREADS / 32];
     __shared__ int act[NTHREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // the minimum so far, no smaller than it will be: a block above it has nothing to combine,
+    // and needs neither the two divisions nor the fence, which one thread made all others wait for
+    unsigned long long T_seen = 0;
+    if (threadIdx.x == 0) T_seen = *(volatile unsigned long long*)T_bits;
     unsigned long long ax = warp_max_u64(abs_bits(umax_x));
     unsigned long long ay = warp_max_u64(abs_bits(umax_y));
     int a = __any_sync(0xffffffffu, any_active);
@@ -681,7 +698,10 @@ __device__ void block_dt_and_rotate(const Params& P, double umax_x, double umax_
             my = red[1][w] > my ? red[1][w] : my;
             any |= act[w];
         }
-        if (any) {
+        const double Ts = from_bits((long long)T_seen);
+        const bool combine = any && !(dt_above(P.krad_x, mx, Ts) && dt_above(P.krad_y, my, Ts) &&
+                                      Ts < kCellTmin0);
+        if (combine) {
             double t = kCellTmin0;
             const double ux = from_bits((long long)mx), uy = from_bits((long long)my);
             if (mx != 0) {
@@ -694,7 +714,7 @@ __device__ void block_dt_and_rotate(const Params& P, double umax_x, double umax_
             }
             atomicMin(T_bits, (unsigned long long)bits(t));
         }
-        if (sc != nullptr) rotate_if_last(sc, nblocks);
+        if (sc != nullptr) rotate_if_last(sc, nblocks, combine);
     }
 }
 
