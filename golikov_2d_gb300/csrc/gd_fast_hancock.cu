@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
         else umax_y = max_nonneg(umax_y, UU);
         if (dt_only) continue;
         fx::FluxI F;
-        if (fx::hlld(fan, A, B, X, P.gas, F)) w.store(fx, fy, F);
+        if (fx::mhd_flux<true>(fan, A, B, X, P.gas, F)) w.store(fx, fy, F);
         else left |= bit;
     }
     if (left) faces_left(P, smem, flag, left, speed, umax_x, umax_y);

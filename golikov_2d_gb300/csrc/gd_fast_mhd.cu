@@ -119,13 +119,12 @@ struct SmemM {
     static constexpr int kCell = NF * TX * TY;
     static constexpr size_t bytes = sizeof(T) * (kPrim + kSlx + kSly + kFx + kFy);
 };
-// The HLLD step's tile in integers: no slopes, the cells' own values beside them.  Its float tile
-// (for ranges the integers cannot hold) works without slope arrays, in the same room: 69 KB, three
-// CTAs per SM.  The HLLC-MHD step always works in floating point, with slope arrays (88 KB, two).
-template <int ORDER, int TY, bool HLLD>
+// The step's tile in integers: no slopes, the cells' own values beside them.  Its float tile (for
+// ranges the integers cannot hold) works without slope arrays, in the same room.
+template <int ORDER, int TY>
 constexpr size_t step_bytes() {
     using I = SmemM<double, ORDER, TY, false>;
-    return HLLD ? I::bytes + sizeof(double) * I::kCell : SmemM<double, ORDER, TY>::bytes;
+    return I::bytes + sizeof(double) * I::kCell;
 }
 
 struct MhdTileResult {
@@ -432,12 +431,12 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
     res.umax_y = u.y;
 }
 
-// ---- The same tile with its face work in 64-bit integers (HLLD) --------------------------------
+// ---- The same tile with its face work in 64-bit integers --------------------------------------
 //
 // HLLD takes about 150 binary64 operations a face; on the FP64 pipe, at 64 cycles of a sub-
 // partition each, they held the tile to 35 000 cycles per 32 cells.  Here the cells of the tile
 // and its halo are integers in units of the tile's own largest density, pressure, velocity and
-// field (fx::TopsM), slopes and face states are adds and selects, and the flux is fx::hlld.  The
+// field (fx::TopsM), slopes and face states are adds and selects, and the flux is fx::mhd_flux.  The
 // FP64 pipe keeps the conversion of the fluxes and the update.
 template <int ORDER, int TY>
 struct MemInt {
@@ -499,7 +498,7 @@ struct JumpInt {
 
 // Returns false, with nothing written, where the tile's cells cannot be held in common units.
 // Every thread of the block must call it, and all get the same answer.
-template <int ORDER, int TY>
+template <bool HLLD, int ORDER, int TY>
 __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in, const Planes& out,
                                              int tx0, int ty0, double T_do, int dt_only,
                                              double* smem, MhdTileResult& res, double* aux) {
@@ -597,7 +596,7 @@ __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in,
         u.take(w.isx, UU);
         if (dt_only) continue;
         fx::FluxI F;
-        if (fx::hlld(fan, A, B, X, P.gas, F))
+        if (fx::mhd_flux<HLLD>(fan, A, B, X, P.gas, F))
             w.store(t.fx, t.fy, FluxM<double>{F.m, F.mn, F.mt, F.e, F.bn, F.bt, F.bz});
         else
             left |= bit;
@@ -614,7 +613,7 @@ __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in,
 }
 
 template <int ORDER, int TY, bool HLLD>
-__global__ void __launch_bounds__(NT, HLLD ? 3 : 2) mhd_fast_kernel(const __grid_constant__ Params P,
+__global__ void __launch_bounds__(NT, 3) mhd_fast_kernel(const __grid_constant__ Params P,
                                                       const __grid_constant__ CPlanes in,
                                                       const __grid_constant__ Planes out,
                                                       const double* __restrict__ T_do_ptr,
@@ -624,13 +623,10 @@ __global__ void __launch_bounds__(NT, HLLD ? 3 : 2) mhd_fast_kernel(const __grid
     MhdTileResult r;
     const int tx0 = blockIdx.x * TX, ty0 = (blockIdx.y + P.tile_row0) * TY;
     const double T_do = *T_do_ptr;
-    if constexpr (HLLD) {  // in integers where the tile's range allows it
-        if (!mhd_tile_int<ORDER, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux)) {
-            __syncthreads();
-            mhd_tile<double, ORDER, TY, false>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux);
-        }
-    } else {
-        mhd_tile<double, ORDER, TY, true>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux);
+    // in integers where the tile's range allows it
+    if (!mhd_tile_int<HLLD, ORDER, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux)) {
+        __syncthreads();
+        mhd_tile<double, ORDER, TY, false>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux);
     }
     if (ctr != nullptr && (r.nfl_r | r.nfl_p | r.nbad)) {
         if (r.nfl_r) atomicAdd(&ctr->rho_floor, (unsigned long long)r.nfl_r);
@@ -654,8 +650,7 @@ __global__ void __launch_bounds__(NT) mhd_tangent_kernel(const __grid_constant__
                               reinterpret_cast<Dual*>(smem), r, nullptr);
 }
 
-// 32 x 8 tiles: three CTAs (24 warps) of the integer HLLD tile are resident per SM at 80 registers
-// and 69 KB of shared memory, two of the floating-point one at 128 and 88 KB.
+// 32 x 8 tiles: three CTAs (24 warps) per SM at 80 registers and 69 KB of shared memory.
 constexpr int kTY = 8;
 constexpr int kTYDual = 8;
 
@@ -665,10 +660,10 @@ cudaError_t launch_t(const Params& P, const CPlanes& in, const Planes& out, cons
                      cudaStream_t st, double* aux = nullptr) {
     dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + kTY - 1) / kTY);
     if (P.method == GD_METHOD_HLLD)
-        mhd_fast_kernel<ORDER, kTY, true><<<grid, NT, step_bytes<ORDER, kTY, true>(), st>>>(
+        mhd_fast_kernel<ORDER, kTY, true><<<grid, NT, step_bytes<ORDER, kTY>(), st>>>(
             P, in, out, T_do, T_bits, rot, ctr, dt_only, aux);
     else
-        mhd_fast_kernel<ORDER, kTY, false><<<grid, NT, step_bytes<ORDER, kTY, false>(), st>>>(
+        mhd_fast_kernel<ORDER, kTY, false><<<grid, NT, step_bytes<ORDER, kTY>(), st>>>(
             P, in, out, T_do, T_bits, rot, ctr, dt_only, aux);
     return cudaGetLastError();
 }
@@ -687,7 +682,7 @@ template <int ORDER, bool HLLD>
 cudaError_t set_room() {
     return cudaFuncSetAttribute(mhd_fast_kernel<ORDER, kTY, HLLD>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)step_bytes<ORDER, kTY, HLLD>());
+                                (int)step_bytes<ORDER, kTY>());
 }
 
 }  // namespace
@@ -766,7 +761,8 @@ __global__ void mhd_face_probe_kernel(Params P, long long n, int axis,
     double UU;
     fx::FluxI G;
     FluxM<double> F;
-    if (P.method == GD_METHOD_HLLD && fx::hlld_face(la, lb, P.gas, G, UU))
+    if (P.method == GD_METHOD_HLLD ? fx::mhd_face<true>(la, lb, P.gas, G, UU)
+                                   : fx::mhd_face<false>(la, lb, P.gas, G, UU))
         F = FluxM<double>{G.m, G.mn, G.mt, G.e, G.bn, G.bt, G.bz};
     else
         F = float_flux(P, la, lb, UU);

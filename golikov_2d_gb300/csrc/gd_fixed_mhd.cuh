@@ -1,4 +1,5 @@
-// gd_fixed_mhd.cuh -- the HLLD face flux in scaled 64-bit integers (see gd_fixed.cuh).
+// gd_fixed_mhd.cuh -- the HLLD and HLLC-MHD face fluxes in scaled 64-bit integers (see
+// gd_fixed.cuh).
 //
 // The states, speeds and guards of hlld_local (gd_mhd_flux.cuh; Gas_Dinamic.cu:964-1510), with
 // the fluxes of the star states in the form the jump conditions across S_K give them.  K is the
@@ -8,7 +9,9 @@
 //   energy q (S - u) (p gamma / (gamma - 1) + rho (u^2 + v^2) / 2 + |b|^2 + rho S (S_M - u))
 //          + b (q (v.b - v*.b*) - v*.b*) + (b - b_K) v.b,
 // and S** (U** - U*) on top between the Alfven waves.  Only K's star state is formed unless the
-// face lies between the Alfven waves.
+// face lies between the Alfven waves.  HLLC-MHD (Gas_Dinamic.cu:1137-1302) is the same with v*, b*
+// and v*.b* of the HLL state of the fan, which the two sides' m and iS = 1 / (S_R - S_L) give:
+//   b_t* = [(S_R - u_R) b_t,R + v_R b_R - (L)] iS,  v* = [m_R v_R + b_R b_t,R - (L)] / (m_R - m_L).
 //
 // Units: velocities 2^(E - 61) as for HLLC; fields 2^(X.b - 61), below 2^60; rho v^2 quantities
 // 2^(ER + 2E - 59) and 2^(ER + 2E - 60), ER the larger density's exponent.  Squares of the field
@@ -175,7 +178,11 @@ GD_HD i64 threshold(i64 m, int e, int u) {
     return s < 0 ? 0x7fffffffffffffffLL : (m >> imin(s, 62)) | 1;
 }
 
-GD_HD bool hlld(const FanM& f, const StatesM& a, const StatesM& b, const TopsM& X, const Gas& G,
+// x << (lz - 2) fits, x >= 0
+GD_HD bool scales(i64 x, int lz) { return x >> imin(65 - lz, 63) == 0; }
+
+template <bool HLLD>
+GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const TopsM& X, const Gas& G,
                 FluxI& F) {
     const int E = f.E, ER = f.ER, XB = 2 * X.b;
     const i64 suA = f.SL - f.uA, suB = f.SR - f.uB;
@@ -222,26 +229,50 @@ GD_HD bool hlld(const FanM& f, const StatesM& a, const StatesM& b, const TopsM& 
         const i64 q = mulk<0, 2>(SM << (lza - 2), iA);
         qsg = takeL ? -q : q;  // S_M / (S - S_M), at most 1 in size, in units of 2^-60
         qs = mulk<2, 1>(qsg, su) << 1;
-        am = iabs(m);
-        bn2 = shift(mulk<0, 0>(bn, bn), sh);
-        thr = threshold(0x53e2d6238da3c211LL, -17, ER + 2 * E - 59);  // 1e-5
-        if (!star_of(am, ad, iabs(su), SM - un, bn, bn2, sh, thr, btK, bzK, K)) return false;
-        RK = star_density(am, iA, lza, ER);
-        i64 rs;
-        sK = root_of<true>(RK, kK, rs);
-        const i64 abn = iabs(bn);
-        // |b| / sqrt(rho*), where |b| > 1e-6 (Gas_Dinamic.cu:1352-1369)
-        const i64 va = abn > threshold(0x431bde82d7b634daLL, -20, X.b - 61)
-                           ? shift(mulk<1, 2>(abn, rs), kK + E - 1 - X.b) : 0;
-        S2 = takeL ? SM - va : SM + va;
-        alfven = takeL ? S2 < 0 : S2 > 0;
+        if constexpr (HLLD) {
+            am = iabs(m);
+            bn2 = shift(mulk<0, 0>(bn, bn), sh);
+            thr = threshold(0x53e2d6238da3c211LL, -17, ER + 2 * E - 59);  // 1e-5
+            if (!star_of(am, ad, iabs(su), SM - un, bn, bn2, sh, thr, btK, bzK, K)) return false;
+            RK = star_density(am, iA, lza, ER);
+            i64 rs;
+            sK = root_of<true>(RK, kK, rs);
+            const i64 abn = iabs(bn);
+            // |b| / sqrt(rho*), where |b| > 1e-6 (Gas_Dinamic.cu:1352-1369)
+            const i64 va = abn > threshold(0x431bde82d7b634daLL, -20, X.b - 61)
+                               ? shift(mulk<1, 2>(abn, rs), kK + E - 1 - X.b) : 0;
+            S2 = takeL ? SM - va : SM + va;
+            alfven = takeL ? S2 < 0 : S2 > 0;
+        } else {
+            // the fan's HLL state: v*, b*, and v*.b* with its own u and w
+            const i64 nA = f.A.n2, nB = f.B.n2;  // b_n^2
+            const i64 tA = mulk<0, 0>(a.bn, a.bt), tB = mulk<0, 0>(b.bn, b.bt);
+            const i64 zA = mulk<0, 0>(a.bn, a.bz), zB = mulk<0, 0>(b.bn, b.bz);
+            const i64 N1 = N + (shift(nB - nA, sq) << 1);
+            const i64 N2 = mulk<1, 3>(mB, f.vB) - mulk<1, 3>(mA, f.vA) + (shift(tB - tA, sq) << 1);
+            const i64 N3 = shift(zB - zA, sq) << 1;
+            const i64 Tt = mulk<1, 2>(suB, b.bt) + mulk<2, 1>(f.vB, b.bn) -
+                           (mulk<1, 2>(suA, a.bt) + mulk<2, 1>(f.vA, a.bn));
+            const i64 Tz = mulk<1, 2>(suB, b.bz) - mulk<1, 2>(suA, a.bz);
+            if (!(scales(iabs(N1) | iabs(N2) | iabs(N3), lz) &&
+                  scales(iabs(Tt) | iabs(Tz), lzs)))
+                return false;
+            const i64 u1 = mulk<0, 2>(N1 << (lz - 2), iD), vs = mulk<0, 2>(N2 << (lz - 2), iD);
+            const i64 ws = mulk<0, 2>(N3 << (lz - 2), iD);
+            K.bt = mulk<0, 2>(Tt << (lzs - 2), iS) << 1;
+            K.bz = mulk<0, 2>(Tz << (lzs - 2), iS) << 1;
+            K.dv = vs - ut;
+            if (!(below61(u1) && below61(ws) && below61(vs) && below61(K.bt) && below61(K.bz)))
+                return false;
+            sb = mulk<2, 1>(u1, bn) + mulk<2, 1>(vs, K.bt) + mulk<2, 1>(ws, K.bz);
+        }
     } else {  // the physical flux of K: no mean of both sides in it
         SM = un;
         bn = bnK;
     }
     const i64 SMu = SM - un, vK = ut + K.dv;
     if (!(below61(vK) && below61(K.dw) && below61(K.bt) && below61(K.bz))) return false;
-    if (star) sb = mulk<2, 1>(SM, bn) + mulk<2, 1>(vK, K.bt) + mulk<2, 1>(K.dw, K.bz);
+    if (HLLD && star) sb = mulk<2, 1>(SM, bn) + mulk<2, 1>(vK, K.bt) + mulk<2, 1>(K.dw, K.bz);
 
     const int32_t qh = hi32(qs);
     const int z = clz32((uint32_t)(qh ^ (qh >> 31))) - 1;
@@ -265,7 +296,7 @@ GD_HD bool hlld(const FanM& f, const StatesM& a, const StatesM& b, const TopsM& 
     i64 e = shift(e0, z - 2 - G.room) +
             shift(mulk<2, 0>(bn, y) + mulk<2, 0>(bn - bnK, ub), ER + 2 * E - 1 - XB);
 
-    if (alfven) {
+    if (HLLD && alfven) {
         // the other side's star state and the states between the Alfven waves
         // (Gas_Dinamic.cu:1371-1430); v3 = vO + w (vK - vO) + ..., w = sK / (sK + sO)
         const i64 unO = takeL ? f.uB : f.uA, utO = takeL ? f.vB : f.vA;
@@ -354,12 +385,13 @@ GD_HD bool face_units(const double* L, const double* R, const Gas& G, StatesM& A
     return true;
 }
 // Flux and larger wave speed of that face.
-GD_HD bool hlld_face(const double* L, const double* R, const Gas& G, FluxI& F, double& UU) {
+template <bool HLLD>
+GD_HD bool mhd_face(const double* L, const double* R, const Gas& G, FluxI& F, double& UU) {
     StatesM A, B;
     TopsM X;
     if (!face_units(L, R, G, A, B, X)) return false;
     const FanM f = fan_of(A, B, X, G, UU);
-    return f.ok && hlld(f, A, B, X, G, F);
+    return f.ok && mhd_flux<HLLD>(f, A, B, X, G, F);
 }
 
 }  // namespace fx
