@@ -93,6 +93,12 @@ __device__ __forceinline__ void mean_half(const double* Q, const double* D, doub
                                           double* h) {
 #pragma unroll
     for (int f = 0; f < 2; ++f) {
+        // |D| < 2 Q (always, for a minmod slope between positive cells): neither state is <= 0
+        if (gt_zero(Q[f]) && mag_lt(D[f], twice_exact(Q[f]))) {
+            m[f] = Q[f];
+            h[f] = half_exact(D[f]);
+            continue;
+        }
         double a = fma(0.5, D[f], Q[f]), b = fma(-0.5, D[f], Q[f]);
         a = le_zero(a) ? Q[f] : a;
         b = le_zero(b) ? Q[f] : b;
@@ -201,7 +207,6 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
     const int tid = threadIdx.x;
     const int N = P.N, M = P.M;
     const int tx0 = 2 + blockIdx.x * TX, ty0 = 2 + (blockIdx.y + P.tile_row0) * TY;
-    const double ig = P.inv_gm1;
 
     // ---- L: state of the tile + 2 halo; corner blocks the stencils never reach are skipped
     for (int i = tid; i < RY * RX; i += NT) {
@@ -239,6 +244,17 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
     int my_flag = 0;
     if (gx < N - 2 && gy < M - 2) my_flag = hancock_frozen_fast(P, colx[cx], rowy[cy + 1]) ? 1 : 2;
     flag[tid] = (unsigned char)my_flag;
+    // a tile inside the frozen sphere has nothing to predict or solve (7 % of the wind's tiles)
+    const bool any_active = __syncthreads_or(my_flag == 2) != 0;
+    if (!any_active) {
+        if (my_flag == 1 && !dt_only) {
+            const long long k = (long long)gy * N + gx;
+#pragma unroll
+            for (int f = 0; f < NF; ++f) store_f(out, f, k, load_f(in, f, k));
+        }
+        block_dt_and_rotate<NT>(P, 0.0, 0.0, false, T_bits, rot, nblocks);
+        return;
+    }
 
     // ---- P: predictions of the tile + 1 halo (not its corners) ---------------------------
     const double T_do = *T_do_ptr;
@@ -284,7 +300,7 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
         const double sty = st * rowiy[py];
         const double r = Q[0], p = Q[1], u = Q[2], v = Q[3], bx = Q[4], by = Q[5], bz = Q[6];
         const double bb = fma(bz, bz, fma(by, by, bx * bx));
-        const double U = fma(p, ig, 0.5 * fma(r, fma(u, u, v * v), bb));
+        const double K1 = fma(r, fma(u, u, v * v), bb);  // twice the kinetic and field energy
         double r2 = fma(-sty * r, v, r - d[0]);
         r2 = le_zero(r2) ? r : r2;
         const double ir2 = rcp_fast(r2);
@@ -293,16 +309,17 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
         const double bx2 = fma(-sty, fma(v, bx, -by * u), bx - d[4]);
         const double by2 = by - d[5];
         const double bz2 = bz - d[6];
-        const double E2 =
-            fma(-sty, fma(U + p + 0.5 * bb, v, -by * fma(u, bx, v * by)), U - d[1]);
-        double p2 = (E2 - 0.5 * fma(r2, fma(u2, u2, v2 * v2),
-                                    fma(bz2, bz2, fma(by2, by2, bx2 * bx2)))) * P.gm1;
+        // p' = p - (gamma - 1) (d_E - (K - K') / 2)
+        const double dE = fma(sty, fma(fma(p, P.g_gm1, half_exact(K1 + bb)), v,
+                                       -by * fma(u, bx, v * by)), d[1]);
+        const double K2 = fma(r2, fma(u2, u2, v2 * v2), fma(bz2, bz2, fma(by2, by2, bx2 * bx2)));
+        double p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, dE, p));
         p2 = le_zero(p2) ? 0.000001 : p2;
         const double QQ[NF] = {r2, p2, u2, v2, bx2, by2, bz2};
         const int o = py * PX + px;
 #pragma unroll
         for (int f = 0; f < NF; ++f) {
-            pA[f * PY * PX + o] = 0.5 * (Q[f] + QQ[f]);
+            pA[f * PY * PX + o] = half_exact(Q[f] + QQ[f]);
             pDX[f * PY * PX + o] = DX[f];
             pDY[f * PY * PX + o] = DY[f];
         }
@@ -360,7 +377,7 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
         }
         const double r = A[0], p = A[1], u = A[2], v = A[3], bx = A[4], by = A[5], bz = A[6];
         const double bb = fma(bz, bz, fma(by, by, bx * bx));
-        const double U = fma(p, ig, 0.5 * fma(r, fma(u, u, v * v), bb));
+        const double K1 = fma(r, fma(u, u, v * v), bb);
         double r2 = fma(-hTy * r, v, r - d[0]);
         if (le_zero(r2)) {
             r2 = r;
@@ -372,10 +389,10 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
         const double bx2 = fma(-hTy, fma(v, bx, -by * u), bx - d[4]);
         const double by2 = by - d[5];
         const double bz2 = bz - d[6];
-        const double E2 =
-            fma(-hTy, fma(U + p + 0.5 * bb, v, -by * fma(u, bx, v * by)), U - d[1]);
-        double p2 = (E2 - 0.5 * fma(r2, fma(u2, u2, v2 * v2),
-                                    fma(bz2, bz2, fma(by2, by2, bx2 * bx2)))) * P.gm1;
+        const double dE = fma(hTy, fma(fma(p, P.g_gm1, half_exact(K1 + bb)), v,
+                                       -by * fma(u, bx, v * by)), d[1]);
+        const double K2 = fma(r2, fma(u2, u2, v2 * v2), fma(bz2, bz2, fma(by2, by2, bx2 * bx2)));
+        double p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, dE, p));
         if (le_zero(p2)) {
             p2 = 0.000001;
             ++nfl_p;
@@ -397,7 +414,6 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
         if (nfl_p) atomicAdd(&ctr->p_floor, (unsigned long long)nfl_p);
         if (nbad) atomicAdd(&ctr->nonfinite, (unsigned long long)nbad);
     }
-    const bool any_active = __syncthreads_or(my_flag == 2) != 0;
     block_dt_and_rotate<NT>(P, umax_x, umax_y, any_active, T_bits, rot, nblocks);
 }
 
