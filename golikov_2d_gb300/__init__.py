@@ -105,6 +105,11 @@ class gd_tecplot_opts(ctypes.Structure):
 
 _lib = None
 
+# PyBytes_FromStringAndSize: with no string, a bytes object whose contents are still to be written
+_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.argtypes = [ctypes.c_void_p, ctypes.c_ssize_t]
+_new_bytes.restype = ctypes.py_object
+
 
 def lib_path() -> str:
     return LIB_PATH
@@ -196,11 +201,30 @@ def _check(status: int, what: str) -> None:
         raise GdError(status, what)
 
 
+# torch's raw handle of the calling thread's current stream, looked up once: the public
+# torch.cuda.current_stream() builds a Stream object, a third of the cost of a small call here
+_raw_stream = None
+
+
+def _current_stream() -> int:
+    global _raw_stream
+    import torch
+    handle = torch.cuda.current_stream().cuda_stream  # initialises CUDA as well
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    device = getattr(torch._C, "_cuda_getDevice", None)
+    if raw is not None and device is not None:
+        _raw_stream = lambda: raw(device())  # noqa: E731
+    return handle
+
+
 def _stream_handle(stream) -> int | None:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream or None
+        return (_raw_stream or _current_stream)() or None
     return getattr(stream, "cuda_stream", stream) or None
+
+
+def _ptr(t) -> int | None:
+    return None if t is None else t.data_ptr()
 
 
 @dataclass
@@ -267,10 +291,9 @@ class Solver:
                     stream=None) -> None:
         """gd_step_ref: Kernel_TVD / add2 / Ker_Dekard on CUDA tensors; `method` is the
         reference's code (METHOD_*) or METHOD_CONFIG."""
-        p = lambda t: None if t is None else t.data_ptr()
-        _check(self.lib.gd_step_ref(self.handle, p(s), p(u), p(b), p(s2), p(u2), p(b2), p(T),
-                                    p(T_do), int(i), int(method), _stream_handle(stream)),
-               "gd_step_ref")
+        _check(self.lib.gd_step_ref(self.handle, _ptr(s), _ptr(u), _ptr(b), _ptr(s2), _ptr(u2),
+                                    _ptr(b2), _ptr(T), _ptr(T_do), int(i), int(method),
+                                    _stream_handle(stream)), "gd_step_ref")
 
     def funk_time(self, T, T_do, TT, i, stream=None) -> None:
         _check(self.lib.gd_funk_time(self.handle, T.data_ptr(), T_do.data_ptr(), TT.data_ptr(),
@@ -290,6 +313,8 @@ class Solver:
 
     @staticmethod
     def _ptrs(s, u, b):
+        if getattr(s, "is_cuda", False):
+            return False, (s.data_ptr(), u.data_ptr(), _ptr(b))
         import numpy as np
         if isinstance(s, np.ndarray):
             arrs = [s, u, b]
@@ -297,8 +322,7 @@ class Solver:
                 if a is not None:
                     assert a.dtype == np.float64 and a.flags.c_contiguous
             return True, [None if a is None else a.ctypes.data for a in arrs]
-        host = not s.is_cuda
-        return host, [None if t is None else t.data_ptr() for t in (s, u, b)]
+        return True, [_ptr(t) for t in (s, u, b)]
 
     def set_time(self, T_do: float, TT: float = 0.0, stream=None) -> None:
         _check(self.lib.gd_set_time(self.handle, float(T_do), float(TT), _stream_handle(stream)),
@@ -353,8 +377,7 @@ class Solver:
                                        _stream_handle(stream)), "gd_adj_forward")
 
     def _vec_call(self, fn, what, ins, outs, stream):
-        ptr = lambda t: None if t is None else t.data_ptr()  # Euler: no field tensors
-        p = [ptr(t) for t in ins] + [ptr(t) for t in outs]
+        p = [_ptr(t) for t in ins] + [_ptr(t) for t in outs]  # Euler: no field tensors
         _check(fn(self.handle, *p, _stream_handle(stream)), what)
 
     def adj_backward(self, gs, gu, gb, os_, ou, ob, stream=None) -> None:
@@ -392,10 +415,13 @@ class Solver:
     def _fetch(self, fn, what, *args, stream=None) -> bytes:
         n = ctypes.c_size_t(0)
         _check(fn(self.handle, *args, None, 0, ctypes.byref(n), _stream_handle(stream)), what)
-        buf = ctypes.create_string_buffer(n.value)
-        _check(fn(self.handle, *args, buf, n.value, ctypes.byref(n), _stream_handle(stream)),
-               what)
-        return buf.raw[:n.value]
+        # the text is written into the bytes object itself: a ctypes buffer is zeroed first and
+        # copied twice on the way out
+        size = n.value
+        out = _new_bytes(None, size)
+        _check(fn(self.handle, *args, ctypes.cast(ctypes.c_char_p(out), ctypes.c_void_p), size,
+                  ctypes.byref(n), _stream_handle(stream)), what)
+        return out if n.value == size else out[:n.value]
 
     def format_text(self, stream=None) -> bytes:
         """The restart text of the resident state ("x y rho p vx vy Bx By Bz" per cell)."""
