@@ -34,7 +34,8 @@ namespace gd {
 namespace {
 
 constexpr int TX = 32;
-constexpr int NT = 256;
+constexpr int NT = 384;     // threads of the step
+constexpr int NTDual = 256;  // and of its tangent
 constexpr int NF = 7;  // rho, p, vx, vy, bx, by, bz
 
 // ---- state access: planes of doubles for the step, value + tangent planes for the JVP ----
@@ -205,7 +206,7 @@ __device__ __forceinline__ void side_states(int f, T ca, T da, T cb, T db, T& a,
 // ---- U: update (kernel.cu:2606-2660 in Heaviside-Lorentz field units) --------------------------
 // cell: the tile's own values, rows RS and fields FS apart; jump: b_x across a cell in x and b_y
 // in y, from its neighbours.
-template <class T, int TY, int RS, int FS, class IN, class OUT, class JUMP>
+template <class T, int BT, int TY, int RS, int FS, class IN, class OUT, class JUMP>
 __device__ __forceinline__ void update_cells(const Params& P, const IN& in, const OUT& out, int tx0,
                                              int ty0, double T_do, int dt_only, const T* cell,
                                              const JUMP& jump, const T* fx, const T* fy,
@@ -216,7 +217,7 @@ __device__ __forceinline__ void update_cells(const Params& P, const IN& in, cons
     const bool axi = P.geometry == GD_AXISYM;
     bool any_active = false;
     unsigned int nfl_r = 0, nfl_p = 0, nbad = 0;
-    for (int i = threadIdx.x; i < TX * TY; i += NT) {
+    for (int i = threadIdx.x; i < TX * TY; i += BT) {
         const int ly = i / TX, lx = i - ly * TX;
         const int gx = tx0 + lx, gy = ty0 + ly;
         if (gx >= N || gy >= M) continue;
@@ -310,7 +311,7 @@ struct JumpFloat {
 // flux component slots in smem: 0 mass, 1 energy, 2 mom x, 3 mom y, 4 bx, 5 by, 6 bz
 // `aux` (T = double only; may be null) receives, per cell, the flux differences d[0..6]
 // and the Powell term divb that the update used (planes of N*M), for the adjoint.
-template <class T, int ORDER, int TY, bool SLOPES, class IN, class OUT>
+template <class T, int BT, int ORDER, int TY, bool SLOPES, class IN, class OUT>
 __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& out, int tx0,
                                          int ty0, double T_do, int dt_only, T* smem,
                                          MhdTileResult& res, double* aux) {
@@ -326,7 +327,7 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
     const int N = P.N, M = P.M;
 
     // ---- L: tile + cross halo, field to Heaviside-Lorentz units --------------------------
-    for (int i = tid; i < SY * SX; i += NT) {
+    for (int i = tid; i < SY * SX; i += BT) {
         const int ly = i / SX, lx = i - ly * SX;
         const bool xh = lx < H || lx >= TX + H, yh = ly < H || ly >= TY + H;
         if (xh && yh) continue;
@@ -349,11 +350,11 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
 
     // ---- S: slopes ---------------------------------------------------------------------------
     // a thread takes a run of G cells, so neighbouring slopes share their difference
-    if (ORDER == 2 && SLOPES) {
+    if constexpr (ORDER == 2 && SLOPES) {
         constexpr int GX = (TX + 2) % 3 == 0 ? 3 : 2, GY = (TY + 2) % 3 == 0 ? 3 : 2;
         constexpr int NGX = (TX + 2) / GX, NGY = (TY + 2) / GY;
         static_assert((TX + 2) % GX == 0 && (TY + 2) % GY == 0, "slope runs tile the rows");
-        for (int i = tid; i < TY * NGX; i += NT) {
+        for (int i = tid; i < TY * NGX; i += BT) {
             const int ly = i / NGX, c0 = (i - ly * NGX) * GX;
             const T* row = prim + (ly + H) * SX + (c0 - 1 + H);
 #pragma unroll
@@ -369,7 +370,7 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
                 }
             }
         }
-        for (int i = tid; i < NGY * TX; i += NT) {
+        for (int i = tid; i < NGY * TX; i += BT) {
             const int g = i / TX, lx = i - g * TX, r0 = g * GY;
             const T* col = prim + (r0 - 1 + H) * SX + (lx + H);
 #pragma unroll
@@ -390,7 +391,7 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
 
     // ---- F: faces ----------------------------------------------------------------------------
     SpeedsM u{0.0, 0.0};
-    for (int i = tid; i < FaceM<TY>::NFX + FaceM<TY>::NFY; i += NT) {
+    for (int i = tid; i < FaceM<TY>::NFX + FaceM<TY>::NFY; i += BT) {
         const FaceM<TY> w(P, tx0, ty0, i);
         if (!w.used) continue;
         const int lx = w.lx, ly = w.ly;
@@ -425,7 +426,7 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
     __syncthreads();
 
     const T* own = prim + H * SX + H;
-    update_cells<T, TY, SX, SY * SX>(P, in, out, tx0, ty0, T_do, dt_only, own,
+    update_cells<T, BT, TY, SX, SY * SX>(P, in, out, tx0, ty0, T_do, dt_only, own,
                                      JumpFloat<T, SX, SY * SX>{own}, fx, fy, res, aux);
     res.umax_x = u.x;
     res.umax_y = u.y;
@@ -604,7 +605,7 @@ __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in,
     if (left) faces_left<ORDER, TY>(P, smem, X, tx0, ty0, left, speed, u);
     __syncthreads();
 
-    update_cells<double, TY, TX, TX * TY>(P, in, out, tx0, ty0, T_do, dt_only, t.cell,
+    update_cells<double, NT, TY, TX, TX * TY>(P, in, out, tx0, ty0, T_do, dt_only, t.cell,
                                           JumpInt<SX, FS>{t.q + H * SX + H, X.b - 60}, t.fx, t.fy,
                                           res, aux);
     res.umax_x = u.x;
@@ -613,7 +614,7 @@ __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in,
 }
 
 template <int ORDER, int TY, bool HLLD>
-__global__ void __launch_bounds__(NT, 3) mhd_fast_kernel(const __grid_constant__ Params P,
+__global__ void __launch_bounds__(NT, 2) mhd_fast_kernel(const __grid_constant__ Params P,
                                                       const __grid_constant__ CPlanes in,
                                                       const __grid_constant__ Planes out,
                                                       const double* __restrict__ T_do_ptr,
@@ -626,7 +627,7 @@ __global__ void __launch_bounds__(NT, 3) mhd_fast_kernel(const __grid_constant__
     // in integers where the tile's range allows it
     if (!mhd_tile_int<HLLD, ORDER, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux)) {
         __syncthreads();
-        mhd_tile<double, ORDER, TY, false>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux);
+        mhd_tile<double, NT, ORDER, TY, false>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux);
     }
     if (ctr != nullptr && (r.nfl_r | r.nfl_p | r.nbad)) {
         if (r.nfl_r) atomicAdd(&ctr->rho_floor, (unsigned long long)r.nfl_r);
@@ -638,7 +639,7 @@ __global__ void __launch_bounds__(NT, 3) mhd_fast_kernel(const __grid_constant__
 
 // Tangent of one step: (U, dU) -> (U', dU') with the dt read from *T_do_ptr (held fixed).
 template <int ORDER, int TY>
-__global__ void __launch_bounds__(NT) mhd_tangent_kernel(const __grid_constant__ Params P,
+__global__ void __launch_bounds__(NTDual) mhd_tangent_kernel(const __grid_constant__ Params P,
                                                          CPlanes in, CPlanes din,
                                                          Planes out, Planes dout,
                                                          const double* __restrict__ T_do_ptr) {
@@ -646,12 +647,16 @@ __global__ void __launch_bounds__(NT) mhd_tangent_kernel(const __grid_constant__
     MhdTileResult r;
     const DualCPlanes I{in, din};
     const DualPlanes O{out, dout};
-    mhd_tile<Dual, ORDER, TY, true>(P, I, O, blockIdx.x * TX, blockIdx.y * TY, *T_do_ptr, 0,
+    mhd_tile<Dual, NTDual, ORDER, TY, true>(P, I, O, blockIdx.x * TX, blockIdx.y * TY, *T_do_ptr, 0,
                               reinterpret_cast<Dual*>(smem), r, nullptr);
 }
 
-// 32 x 8 tiles: three CTAs (24 warps) per SM at 80 registers and 69 KB of shared memory.
-constexpr int kTY = 8;
+// 32 x 11 tiles of 384 threads, two CTAs (24 warps) per SM at 80 registers and 93 KB of shared
+// memory: the tile's 747 faces are two rounds of 384 threads (97 % of them busy), and the face code
+// (45 KB) is fetched by 12 warps together.  32 x 8 with 256 threads, three CTAs: 2.25 rounds, 27 %
+// of the instruction fetches missing; 1.82 against 1.66 ms per pass of 1024^2, 3.05 against 3.00
+// for the wind.
+constexpr int kTY = 11;
 constexpr int kTYDual = 8;
 
 template <int ORDER>
@@ -673,7 +678,7 @@ cudaError_t launch_tangent_t(const Params& P, const CPlanes& in, const CPlanes& 
                              const Planes& out, const Planes& dout, const double* T_do,
                              cudaStream_t st) {
     dim3 grid((P.N + TX - 1) / TX, (P.M + kTYDual - 1) / kTYDual);
-    mhd_tangent_kernel<ORDER, kTYDual><<<grid, NT, SmemM<Dual, ORDER, kTYDual>::bytes, st>>>(
+    mhd_tangent_kernel<ORDER, kTYDual><<<grid, NTDual, SmemM<Dual, ORDER, kTYDual>::bytes, st>>>(
         P, in, din, out, dout, T_do);
     return cudaGetLastError();
 }
