@@ -11,7 +11,7 @@
 //      recompute pass), lambda'.  Outputs: the direct adjoint of the cell state, the adjoint
 //      of d[7] and of divb.
 //   B  per face, then per cell (adj_face_kernel, adj_gather_kernel): every face recomputes
-//      its forward states and HLLD flux once and runs the flux's reverse sweep on
+//      its forward states and the flux's star states and runs the flux's reverse sweep on
 //      Fbar = k (dbar_low - dbar_high); the adjoints of the two face states are gathered
 //      into the cells through the reconstruction (c +- slope/2, minmod choice, rho/p
 //      fallback) and the Powell central difference, in a fixed order (deterministic).
@@ -142,12 +142,20 @@ __global__ void __launch_bounds__(NT) adj_update_kernel(Params P, CPlanes U, con
 // Reverse sweep of one HLLD face flux (method 3) in the local frame.
 // Inputs: the two face states A (low) and B (high) as (r, p, un, ut, bn, bt, bz) and the
 // adjoint of the flux (m, mn, mt, e, bn, bt, bz).  Writes the adjoints of A and B to Ab, Bb.
-// The forward part repeats hlld_local<double> of gd_fast_mhd.cu operation for operation.
-// The reverse does per-side work only where the adjoint can be non-zero: the flux's base
-// terms and the energy enter through the upwind side K alone (the side whose state or star
-// state gives the flux), the fast speed through the side of max(cf) alone, and only K's
-// star energy and its sb term reach the flux; those chains run once, on the selected
-// side's values, and their results are added to that side.
+//
+// The derivative is that of the forward's flux on the branch it takes; what is differentiated
+// is the shortest form of that flux, not the forward's chain of operations.  K is the upwind
+// side, O the other one, m = r (S - un), d = SM - un, D = S - SM, and X the state the flux
+// belongs to (K's star state, or the double star).  The jump relations across S and across
+// the Alfven wave hold identically for the solver's star formulas, so that with
+// phi = rK SM and P* = pT + m d the flux is
+//   m = phi,  mn = phi SM + P* - bnK^2,  mt = phi v - bn b + (bn - bnK) bt,
+//   bt: SM b - bn v + (bn - bnK) ut,  bz: SM z - bn w,  e = SM (e + P*) - bn sb + (bn - bnK) wK
+// with v, w, b, z, sb, e those of X.  Neither S nor the Alfven speeds appear any more; the
+// other side's star state is needed for the double star alone; v* and b* of one wave share
+// their reverse products; the reverse of a quotient n / q is that of n - q x = 0 (no chain
+// through the reciprocal).  A side whose star guard fails (|tt| < 1e-5) has v* = ut and
+// w* = b* = z* = 0; the three terms by which its flux then differs are added apart.
 // ---------------------------------------------------------------------------------------
 struct SideV {
     double r, p, un, ut, bn, bt, bz;
@@ -198,6 +206,47 @@ __device__ __forceinline__ void side_tail(const SideV& S, SideB& b, double* qb) 
     qb[6] = fma(2.0 * bbb, S.bz, b.bz);
 }
 
+// star state of one side: m, D = S - SM, d = SM - un as above, bbn = bn^2
+struct StarV {
+    double it, h, c, q;  // 1 / tt, d / tt, bn d / tt, 1 + m d / tt (all 0 where the guard fails)
+    double v, w, b, z;
+    bool g;
+};
+
+__device__ __forceinline__ StarV star_fwd(double m, double D, double d, double bn, double bbn,
+                                          double ut, double bt, double bz) {
+    StarV s;
+    const double tt = fma(m, D, -bbn);
+    s.g = mag_ge(tt, kMag1em5);
+    s.it = s.g ? rcp_fast(tt) : 0.0;
+    s.h = d * s.it;
+    s.c = bn * s.h;
+    s.q = s.g ? fma(m, s.h, 1.0) : 0.0;
+    s.v = fma(-s.c, bt, ut);
+    s.w = -s.c * bz;
+    s.b = bt * s.q;
+    s.z = bz * s.q;
+    return s;
+}
+
+// its reverse: (vb, wb, bb, zb) onto the side's ut, bt, bz and onto m, D, d, bn
+__device__ __forceinline__ void star_rev(const StarV& s, double m, double D, double bn, double bt,
+                                         double bz, double vb, double wb, double bb, double zb,
+                                         SideB& Q, double& mb, double& Db, double& db,
+                                         double& bnb) {
+    const double cb = fma(vb, bt, wb * bz);  // minus the adjoint of c
+    const double qb = fma(bb, bt, zb * bz);
+    Q.ut += vb;
+    Q.bt = fma(bb, s.q, fma(-vb, s.c, Q.bt));
+    Q.bz = fma(zb, s.q, fma(-wb, s.c, Q.bz));
+    const double n = fma(qb, m, -cb * bn) * s.it;
+    db += n;
+    const double ttb = -n * s.h;
+    mb = fma(ttb, D, fma(qb, s.h, mb));
+    Db = fma(ttb, m, Db);
+    bnb = fma(-2.0 * ttb, bn, fma(-cb, s.h, bnb));
+}
+
 // Fb = (m, mn, mt, e, bn, bt, bz); qa_b, qb_b receive (r, p, un, ut, bn, bt, bz).
 __device__ __forceinline__ void hlld_vjp(const double* qa, const double* qb, const double* Fb,
                                          const Params& P, double* qa_b, double* qb_b) {
@@ -207,476 +256,260 @@ __device__ __forceinline__ void hlld_vjp(const double* qa, const double* qb, con
     // ---- forward, shared part
     const bool minA = !dlt(B.un, A.un);              // uminN = A.un (else B.un)
     const bool maxB = dlt(A.un, B.un);               // umaxN = B.un (else A.un)
-    const double uminN = minA ? A.un : B.un;
-    const double umaxN = maxB ? B.un : A.un;
     const bool cfB = mag_lt(A.cf, B.cf);
     const double cmax = cfB ? B.cf : A.cf;
-    const double SL = uminN - cmax, SR = umaxN + cmax;
+    const double SL = (minA ? A.un : B.un) - cmax, SR = (maxB ? B.un : A.un) + cmax;
     const double suL = SL - A.un, suR = SR - B.un;
     const double mL = A.r * suL, mR = B.r * suR;
     const double iden = rcp_fast(mR - mL);
-    const double SMn = (fma(mR, B.un, -mL * A.un) - B.pT) + A.pT;
-    const double SM = SMn * iden;
-    const double PTTn = fma(mL * mR, B.un - A.un, fma(mR, A.pT, -mL * B.pT));
-    const double PTT = PTTn * iden;
+    const double du = B.un - A.un;
+    const double dA = fma(mR, du, A.pT - B.pT) * iden;  // SM - A.un
+    const double SM = A.un + dA;
     const bool UUR = mag_lt(SL, SR);
-    const double UU = dabs(UUR ? SR : SL);
-    const double iS = rcp_fast(SR - SL);
-    const double bnn = fma(SR, B.bn, -SL * A.bn);
-    const double bn = bnn * iS;
-    const double iL = rcp_fast(SL - SM), iR = rcp_fast(SR - SM);
-    const double rLL = mL * iL, rRR = mR * iR;
-    const double bbn = bn * bn;
-    // star states
-    const double ttL = fma(mL, SL - SM, -bbn);
-    const bool gL = mag_ge(ttL, kMag1em5);
-    double itL = 0, cL = 0, dL = 0, vLL, wLL, btL, bzL;
-    if (gL) {
-        itL = rcp_fast(ttL);
-        cL = bn * (SM - A.un) * itL;
-        dL = fma(mL, suL, -bbn) * itL;
-        vLL = fma(-cL, A.bt, A.ut);
-        wLL = -cL * A.bz;
-        btL = A.bt * dL;
-        bzL = A.bz * dL;
-    } else {
-        vLL = A.ut; wLL = 0.0; btL = 0.0; bzL = 0.0;
-    }
-    const double ttR = fma(mR, SR - SM, -bbn);
-    const bool gR = mag_ge(ttR, kMag1em5);
-    double itR = 0, cR = 0, dR = 0, vRR, wRR, btR, bzR;
-    if (gR) {
-        itR = rcp_fast(ttR);
-        cR = bn * (SM - B.un) * itR;
-        dR = fma(mR, suR, -bbn) * itR;
-        vRR = fma(-cR, B.bt, B.ut);
-        wRR = -cR * B.bz;
-        btR = B.bt * dR;
-        bzR = B.bz * dR;
-    } else {
-        vRR = B.ut; wRR = 0.0; btR = 0.0; bzR = 0.0;
-    }
-    const double SMbn = SM * bn;
-    double isLL, isRR, sLL, sRR;
-    rsqrt_and_sqrt(rLL, isLL, sLL);
-    rsqrt_and_sqrt(rRR, isRR, sRR);
-    const bool bnz = mag_ge(bn, kMag1em6 + 1);
-    const double abn = dabs(bn);
-    const double SLL = bnz ? fma(-abn, isLL, SM) : SM;
-    const double SRR = bnz ? fma(abn, isRR, SM) : SM;
-    const int idbn = bnz ? (gt_zero(bn) ? 1 : -1) : 0;
     const bool takeL = ge_zero(SL) || ge_zero(SM);
-    int level;
-    if (takeL) level = ge_zero(SL) ? 0 : (ge_zero(SLL) ? 1 : 2);
-    else level = gt_zero(SRR) ? 2 : (gt_zero(SR) ? 1 : 0);
-    // the upwind side K: its state, star state and energies
+    // the upwind side K and the other side O
     const double Kr = takeL ? A.r : B.r, Kp = takeL ? A.p : B.p;
     const double Kun = takeL ? A.un : B.un, Kut = takeL ? A.ut : B.ut;
     const double Kbn = takeL ? A.bn : B.bn, Kbt = takeL ? A.bt : B.bt;
     const double Kbz = takeL ? A.bz : B.bz, KpT = takeL ? A.pT : B.pT;
     const double Kbb = takeL ? A.bb : B.bb;
-    const double S = takeL ? SL : SR;
-    const double su = takeL ? suL : suR;
-    const double iK = takeL ? iL : iR;
-    const double rK = takeL ? rLL : rRR;
-    const double vK = takeL ? vLL : vRR;
-    const double wK = takeL ? wLL : wRR;
-    const double btK = takeL ? btL : btR;
-    const double bzK = takeL ? bzL : bzR;
+    const double Or = takeL ? B.r : A.r, Out = takeL ? B.ut : A.ut;
+    const double Obn = takeL ? B.bn : A.bn, Obt = takeL ? B.bt : A.bt;
+    const double Obz = takeL ? B.bz : A.bz;
+    const double SK = takeL ? SL : SR, SO = takeL ? SR : SL;
+    const double suK = takeL ? suL : suR, suO = takeL ? suR : suL;
+    const double mK = takeL ? mL : mR, mO = takeL ? mR : mL;
+    const double dB = dA - du;
+    const double dK = takeL ? dA : dB, dO = takeL ? dB : dA;
+    const double DK = suK - dK;
+    const double iS = rcp_fast(SR - SL);
+    const double bn = fma(SR, B.bn, -SL * A.bn) * iS;
+    const double bbn = bn * bn;
+    const double iK = rcp_fast(DK);
+    const double rK = mK * iK;
+    double isK, sK;
+    rsqrt_and_sqrt(rK, isK, sK);
+    const bool bnz = mag_ge(bn, kMag1em6 + 1);
+    const double SA = bnz ? fma(takeL ? -dabs(bn) : dabs(bn), isK, SM) : SM;  // Alfven speed
+    int level;
+    if (takeL) level = ge_zero(SL) ? 0 : (ge_zero(SA) ? 1 : 2);
+    else level = gt_zero(SA) ? 2 : (gt_zero(SR) ? 1 : 0);
     const double vsq = fma(Kun, Kun, Kut * Kut);
     const double KE = fma(Kp, P.inv_gm1, 0.5 * fma(Kr, vsq, Kbb));
-    const double sbK = fma(wK, bzK, fma(vK, btK, SMbn));
     const double wKf = fma(Kun, Kbn, Kut * Kbt);
-    const double eKn = fma(KE, su, fma(PTT, SM, -KpT * Kun)) + bn * (wKf - sbK);
-    const double eK = eKn * iK;
-    // double-star (only needed for level 2)
-    double is = 0, vL3 = 0, wL3 = 0, s2 = 0, bt3 = 0, bz3 = 0, sb3 = 0, sK = 0, e3 = 0, S2 = 0;
-    if (level == 2) {
-        is = rcp_fast(sLL + sRR);
-        vL3 = (fma(sLL, vLL, sRR * vRR) + sgn_select(btR - btL, idbn)) * is;
-        wL3 = (fma(sLL, wLL, sRR * wRR) + sgn_select(bzR - bzL, idbn)) * is;
-        s2 = sgn_select(sLL * sRR, idbn);
-        bt3 = fma(s2, vRR - vLL, fma(sLL, btR, sRR * btL)) * is;
-        bz3 = fma(s2, wRR - wLL, fma(sLL, bzR, sRR * bzL)) * is;
-        sb3 = fma(wL3, bz3, fma(vL3, bt3, SMbn));
-        sK = takeL ? -sLL : sRR;
-        e3 = fma(sgn_select(sK, idbn), sbK - sb3, eK);
-        S2 = takeL ? SLL : SRR;
-    }
 
     // ---- reverse ------------------------------------------------------------------------
-    SideB Ab = {}, Bb = {};
-    // adjoints of the K side's state and energy (added to its side at the end)
-    double kr = 0, kun = 0, kut = 0, kE = 0, kbt = 0, kbz = 0, kbn = 0, kpT = 0;
-    // adjoints of intermediates
-    double SLb = 0, SRb = 0, SMb = 0, PTTb = 0, UUb = 0, bnb = 0;
-    double rLLb = 0, rRRb = 0, iLb = 0, iRb = 0;
-    double vLLb = 0, wLLb = 0, btLb = 0, bzLb = 0, vRRb = 0, wRRb = 0, btRb = 0, bzRb = 0;
-    double sLLb = 0, sRRb = 0, SLLb = 0, SRRb = 0, SMbnb = 0;
     const double Fm = Fb[0], Fmn = Fb[1], Fmt = Fb[2], Fe = Fb[3], Fbn = Fb[4], Fbt = Fb[5],
                  Fbz = Fb[6];
-    // F.bn = -UU (B.bn - A.bn)
-    UUb = -Fbn * (B.bn - A.bn);
-    Bb.bn = -Fbn * UU;
-    Ab.bn = Fbn * UU;
-    double Sb = 0, rKb = 0, vKb = 0, wKb = 0, eKb = 0, btKb = 0, bzKb = 0, sbKb = 0;
-    if (level >= 1) {
-        if (level == 2) {
-            // F.mt += S2 rK (vL3 - vK); F.e += S2 (e3 - eK); F.bt += S2 (bt3 - btK);
-            // F.bz += S2 (bz3 - bzK)
-            const double S2b = Fmt * rK * (vL3 - vK) + Fe * (e3 - eK) + Fbt * (bt3 - btK) +
-                               Fbz * (bz3 - bzK);
-            rKb += Fmt * S2 * (vL3 - vK);
-            double vL3b = Fmt * S2 * rK;
-            vKb -= Fmt * S2 * rK;
-            double e3b = Fe * S2;
-            eKb -= Fe * S2;
-            double bt3b = Fbt * S2;
-            btKb -= Fbt * S2;
-            double bz3b = Fbz * S2;
-            bzKb -= Fbz * S2;
-            if (takeL) SLLb += S2b; else SRRb += S2b;
-            // e3 = eK + sgn(sK) (sbK - sb3)
-            eKb += e3b;
-            const double sKv = sgn_select(sK, idbn);
-            const double sKvb = e3b * (sbK - sb3);
-            sbKb += e3b * sKv;
-            double sb3b = -e3b * sKv;
-            const double sKb = sgn_select(sKvb, idbn);
-            if (takeL) sLLb -= sKb; else sRRb += sKb;
-            // sb3 = wL3 bz3 + vL3 bt3 + SMbn
-            double wL3b = sb3b * bz3;
-            bz3b += sb3b * wL3;
-            vL3b += sb3b * bt3;
-            bt3b += sb3b * vL3;
-            SMbnb += sb3b;
-            // bz3 = (s2 (wRR - wLL) + sLL bzR + sRR bzL) is
-            double isb = bz3b * (bz3 * (sLL + sRR));  // bz3 / is = numerator
-            {
-                const double nb = bz3b * is;
-                double s2b = nb * (wRR - wLL);
-                wRRb += nb * s2;
-                wLLb -= nb * s2;
-                sLLb += nb * bzR;
-                bzRb += nb * sLL;
-                sRRb += nb * bzL;
-                bzLb += nb * sRR;
-                // bt3 = (s2 (vRR - vLL) + sLL btR + sRR btL) is
-                isb += bt3b * (bt3 * (sLL + sRR));
-                const double mb = bt3b * is;
-                s2b += mb * (vRR - vLL);
-                vRRb += mb * s2;
-                vLLb -= mb * s2;
-                sLLb += mb * btR;
-                btRb += mb * sLL;
-                sRRb += mb * btL;
-                btLb += mb * sRR;
-                // s2 = sgn(sLL sRR)
-                const double pb = sgn_select(s2b, idbn);
-                sLLb += pb * sRR;
-                sRRb += pb * sLL;
-            }
-            // wL3 = (sLL wLL + sRR wRR + sgn(bzR - bzL)) is
-            {
-                isb += wL3b * (wL3 * (sLL + sRR));
-                const double nb = wL3b * is;
-                sLLb += nb * wLL;
-                wLLb += nb * sLL;
-                sRRb += nb * wRR;
-                wRRb += nb * sRR;
-                const double tb = sgn_select(nb, idbn);
-                bzRb += tb;
-                bzLb -= tb;
-            }
-            // vL3 = (sLL vLL + sRR vRR + sgn(btR - btL)) is
-            {
-                isb += vL3b * (vL3 * (sLL + sRR));
-                const double nb = vL3b * is;
-                sLLb += nb * vLL;
-                vLLb += nb * sLL;
-                sRRb += nb * vRR;
-                vRRb += nb * sRR;
-                const double tb = sgn_select(nb, idbn);
-                btRb += tb;
-                btLb -= tb;
-            }
-            // is = 1 / (sLL + sRR)
-            const double db = -isb * is * is;
-            sLLb += db;
-            sRRb += db;
-        }
-        // level-1 terms: F.m += S (rK - K.r); F.mn += S (rK SM - K.r K.un);
-        // F.mt += S (rK vK - K.r K.ut); F.e += S (eK - K.E); F.bt += S (btK - K.bt);
-        // F.bz += S (bzK - K.bz)
-        Sb += Fm * (rK - Kr) + Fmn * fma(rK, SM, -Kr * Kun) + Fmt * fma(rK, vK, -Kr * Kut) +
-              Fe * (eK - KE) + Fbt * (btK - Kbt) + Fbz * (bzK - Kbz);
-        rKb += S * (Fm + Fmn * SM + Fmt * vK);
-        SMb += S * Fmn * rK;
-        vKb += S * Fmt * rK;
-        eKb += S * Fe;
-        btKb += S * Fbt;
-        bzKb += S * Fbz;
-        kr = -S * (Fm + Fmn * Kun + Fmt * Kut);
-        kun = -S * Fmn * Kr;
-        kut = -S * Fmt * Kr;
-        kE = -S * Fe;
-        kbt = -S * Fbt;
-        kbz = -S * Fbz;
-    }
-    // eK = eKn iK, eKn = K.E su + PTT SM - K.pT K.un + bn (wKf - sbK)
-    const double iKb = eKb * eKn;
-    {
-        const double nb = eKb * iK;
-        kE += nb * su;
-        const double sub = nb * KE;
-        PTTb += nb * SM;
-        SMb += nb * PTT;
-        kpT -= nb * Kun;
-        kun -= nb * KpT;
-        bnb += nb * (wKf - sbK);
-        const double wKfb = nb * bn;
-        sbKb -= nb * bn;
-        // wKf = K.un K.bn + K.ut K.bt
-        kun += wKfb * Kbn;
-        kbn += wKfb * Kun;
-        kut += wKfb * Kbt;
-        kbt += wKfb * Kut;
-        // su = S - K.un
-        Sb += sub;
-        kun -= sub;
-    }
-    // sbK = wK bzK + vK btK + SMbn
-    wKb += sbKb * bzK;
-    bzKb += sbKb * wK;
-    vKb += sbKb * btK;
-    btKb += sbKb * vK;
-    SMbnb += sbKb;
-    // distribute the K-selected adjoints
-    if (takeL) {
-        SLb += Sb; rLLb += rKb; vLLb += vKb; wLLb += wKb; btLb += btKb; bzLb += bzKb;
-        iLb += iKb;
-    } else {
-        SRb += Sb; rRRb += rKb; vRRb += vKb; wRRb += wKb; btRb += btKb; bzRb += bzKb;
-        iRb += iKb;
-    }
-    // SLL = SM - abn isLL ; SRR = SM + abn isRR  (if bnz, else = SM)
-    double isLLb = 0, isRRb = 0;
-    SMb += SLLb + SRRb;
-    if (bnz) {
-        const double abnb = fma(SRRb, isRR, -SLLb * isLL);
-        isLLb = -SLLb * abn;
-        isRRb = SRRb * abn;
-        bnb += sgn_select(abnb, idbn);
-    }
-    // sLL = rLL isLL, isLL = rsqrt(rLL)  =>  d sLL / d rLL = 0.5 isLL
-    rLLb += sLLb * 0.5 * isLL;
-    rRRb += sRRb * 0.5 * isRR;
-    rLLb += isLLb * (-0.5) * isLL * isLL * isLL;
-    rRRb += isRRb * (-0.5) * isRR * isRR * isRR;
-    // SMbn = SM bn
-    SMb += SMbnb * bn;
-    bnb += SMbnb * SM;
-    // star states L
-    double bbnb = 0;
-    if (gL) {
-        // vLL = A.ut - cL A.bt ; wLL = -cL A.bz ; btL = A.bt dL ; bzL = A.bz dL
-        Ab.ut += vLLb;
-        const double cLb = -vLLb * A.bt - wLLb * A.bz;
-        Ab.bt += -vLLb * cL + btLb * dL;
-        Ab.bz += -wLLb * cL + bzLb * dL;
-        const double dLb = btLb * A.bt + bzLb * A.bz;
-        // dL = (mL suL - bbn) itL ; cL = bn (SM - A.un) itL
-        const double itLb = dLb * fma(mL, suL, -bbn) + cLb * bn * (SM - A.un);
-        const double dnb = dLb * itL;
-        double mLb_s = dnb * suL;
-        double suLb_s = dnb * mL;
-        bbnb -= dnb;
-        const double cnb = cLb * itL;
-        bnb += cnb * (SM - A.un);
-        SMb += cnb * bn;
-        Ab.un -= cnb * bn;
-        // itL = 1 / ttL ; ttL = mL (SL - SM) - bbn
-        const double ttLb = -itLb * itL * itL;
-        mLb_s += ttLb * (SL - SM);
-        SLb += ttLb * mL;
-        SMb -= ttLb * mL;
-        bbnb -= ttLb;
-        // mL and suL adjoints
-        Ab.r += mLb_s * suL;
-        suLb_s += mLb_s * A.r;
-        SLb += suLb_s;
-        Ab.un -= suLb_s;
-    } else {
-        Ab.ut += vLLb;
-    }
-    if (gR) {
-        Bb.ut += vRRb;
-        const double cRb = -vRRb * B.bt - wRRb * B.bz;
-        Bb.bt += -vRRb * cR + btRb * dR;
-        Bb.bz += -wRRb * cR + bzRb * dR;
-        const double dRb = btRb * B.bt + bzRb * B.bz;
-        const double itRb = dRb * fma(mR, suR, -bbn) + cRb * bn * (SM - B.un);
-        const double dnb = dRb * itR;
-        double mRb_s = dnb * suR;
-        double suRb_s = dnb * mR;
-        bbnb -= dnb;
-        const double cnb = cRb * itR;
-        bnb += cnb * (SM - B.un);
-        SMb += cnb * bn;
-        Bb.un -= cnb * bn;
-        const double ttRb = -itRb * itR * itR;
-        mRb_s += ttRb * (SR - SM);
-        SRb += ttRb * mR;
-        SMb -= ttRb * mR;
-        bbnb -= ttRb;
-        Bb.r += mRb_s * suR;
-        suRb_s += mRb_s * B.r;
-        SRb += suRb_s;
-        Bb.un -= suRb_s;
-    } else {
-        Bb.ut += vRRb;
-    }
-    // bbn = bn^2
-    bnb += 2.0 * bbnb * bn;
-    // rLL = mL iL ; rRR = mR iR ; iL = 1 / (SL - SM) ; iR = 1 / (SR - SM)
-    double mLb = rLLb * iL, mRb = rRRb * iR;
-    iLb += rLLb * mL;
-    iRb += rRRb * mR;
-    {
-        const double dLb = -iLb * iL * iL;
-        SLb += dLb;
-        SMb -= dLb;
-        const double dRb = -iRb * iR * iR;
-        SRb += dRb;
-        SMb -= dRb;
-    }
-    // bn = bnn iS (the star bt, bz of the HLLC-MHD branch are not used by HLLD)
-    const double iSb = bnb * bnn;
-    {
-        const double nb = bnb * iS;  // bnn = SR B.bn - SL A.bn
-        SRb += nb * B.bn;
-        Bb.bn += nb * SR;
-        SLb -= nb * A.bn;
-        Ab.bn -= nb * SL;
-    }
-    // iS = 1 / (SR - SL)
-    {
-        const double db = -iSb * iS * iS;
-        SRb += db;
-        SLb -= db;
-    }
-    // UU = max(|SL|, |SR|)
-    {
-        const double Sx = UUR ? SR : SL;
-        const double t = lt_zero(Sx) ? from_bits(bits(UUb) ^ (long long)0x8000000000000000ULL)
-                                     : UUb;  // sign(Sx) UUb on the integer pipe
-        add_to(UUR, SRb, SLb, t);
-    }
-    // PTT = PTTn iden ; SM = SMn iden
-    const double idenb = PTTb * PTTn + SMb * SMn;
-    {
-        const double nb = PTTb * iden;  // PTTn = mL mR (B.un - A.un) + mR A.pT - mL B.pT
-        mLb += nb * (mR * (B.un - A.un) - B.pT);
-        mRb += nb * (mL * (B.un - A.un) + A.pT);
-        Bb.un += nb * mL * mR;
-        Ab.un -= nb * mL * mR;
-        Ab.pT += nb * mR;
-        Bb.pT -= nb * mL;
-    }
-    {
-        const double nb = SMb * iden;  // SMn = mR B.un - mL A.un - B.pT + A.pT
-        mRb += nb * B.un;
-        Bb.un += nb * mR;
-        mLb -= nb * A.un;
-        Ab.un -= nb * mL;
-        Bb.pT -= nb;
-        Ab.pT += nb;
-    }
-    // iden = 1 / (mR - mL)
-    {
-        const double db = -idenb * iden * iden;
-        mRb += db;
-        mLb -= db;
-    }
-    // mL = A.r suL, mR = B.r suR ; suL = SL - A.un ; suR = SR - B.un
-    Ab.r += mLb * suL;
-    const double suLb = mLb * A.r;
-    Bb.r += mRb * suR;
-    const double suRb = mRb * B.r;
-    SLb += suLb;
-    Ab.un -= suLb;
-    SRb += suRb;
-    Bb.un -= suRb;
-    // SL = uminN - cmax ; SR = umaxN + cmax
-    const double cmaxb = SRb - SLb;
-    if (minA) Ab.un += SLb; else Bb.un += SLb;
-    if (maxB) Bb.un += SRb; else Ab.un += SRb;
-
-    // ---- the K side's base flux and energy ----------------------------------------------
-    {
-        // F7 = un bz ; F6 = un bt - ut bn
-        kun += Fbz * Kbz;
-        kbz += Fbz * Kun;
-        kun += Fbt * Kbt;
-        kbt += Fbt * Kun;
-        kut -= Fbt * Kbn;
-        kbn -= Fbt * Kut;
-        // F4 = (E + pT) un - bn (ut bt + un bn)
-        const double w = fma(Kut, Kbt, Kun * Kbn);
-        kE += Fe * Kun;
-        kpT += Fe * Kun;
-        kun += Fe * (KE + KpT);
-        kbn -= Fe * w;
-        const double wb = -Fe * Kbn;
-        kut += wb * Kbt;
-        kbt += wb * Kut;
-        kun += wb * Kbn;
-        kbn += wb * Kun;
-        // F0 = r un ; F1 = F0 un + pT - bn^2 ; F2 = F0 ut - bn bt
+    SideB k = {}, o = {};
+    double KEb, wKfb;               // adjoints of K's energy and of its u.b
+    double SKb = 0.0, SOb = 0.0;    // of the two outer speeds
+    if (level == 0) {
+        // F0 = r un ; F1 = F0 un + pT - bn^2 ; F2 = F0 ut - bn bt ; F5 = un bt - ut bn ;
+        // F6 = un bz ; F3 = (E + pT) un - bn (ut bt + un bn)
         const double F0 = Kr * Kun;
         const double F0b = fma(Fmt, Kut, fma(Fmn, Kun, Fm));
-        kut += Fmt * F0;
-        kbn -= Fmt * Kbt;
-        kbt -= Fmt * Kbn;
-        kun += Fmn * F0;
-        kpT += Fmn;
-        kbn -= 2.0 * Fmn * Kbn;
-        kr += F0b * Kun;
-        kun += F0b * Kr;
-        // E = p inv_gm1 + 0.5 (r (un^2 + ut^2) + bb)
-        const double kinb = 0.5 * kE;
-        kr += kinb * vsq;
-        kun += kinb * 2.0 * Kr * Kun;
-        kut += kinb * 2.0 * Kr * Kut;
-        add_to(takeL, Ab.r, Bb.r, kr);
-        add_to(takeL, Ab.un, Bb.un, kun);
-        add_to(takeL, Ab.ut, Bb.ut, kut);
-        add_to(takeL, Ab.bn, Bb.bn, kbn);
-        add_to(takeL, Ab.bt, Bb.bt, kbt);
-        add_to(takeL, Ab.bz, Bb.bz, kbz);
-        add_to(takeL, Ab.pT, Bb.pT, kpT);
-        // the side's p and bb adjoints are still zero: assign
-        const double kp = kE * P.inv_gm1;
-        Ab.p = takeL ? kp : 0.0;
-        Bb.p = takeL ? 0.0 : kp;
-        Ab.bb = takeL ? kinb : 0.0;
-        Bb.bb = takeL ? 0.0 : kinb;
+        KEb = Fe * Kun;
+        wKfb = -Fe * Kbn;
+        k.r = F0b * Kun;
+        k.un = fma(F0b, Kr, fma(Fmn, F0, fma(Fbt, Kbt, fma(Fbz, Kbz, Fe * (KE + KpT)))));
+        k.ut = fma(Fmt, F0, -Fbt * Kbn);
+        k.pT = Fmn + KEb;
+        k.bn = -fma(2.0 * Fmn, Kbn, fma(Fmt, Kbt, fma(Fbt, Kut, Fe * wKf)));
+        k.bt = fma(Fbt, Kun, -Fmt * Kbn);
+        k.bz = Fbz * Kun;
+    } else {
+        const StarV sk = star_fwd(mK, DK, dK, bn, bbn, Kut, Kbt, Kbz);
+        const double PT = fma(mK, dK, KpT);
+        const double phi = rK * SM;
+        const double SMbn = SM * bn;
+        const double sbK = fma(sk.w, sk.z, fma(sk.v, sk.b, SMbn));
+        const double wsb = wKf - sbK;
+        const double eK = fma(bn, wsb, fma(KE, suK, fma(PT, SM, -KpT * Kun))) * iK;
+        // X: the double star at level 2, else K's star state
+        double Xv = sk.v, Xw = sk.w, Xb = sk.b, Xz = sk.z, Xsb = sbK, Xe = eK;
+        StarV so;
+        double DO = 0, iO = 0, rO = 0, isO = 0, sO = 0, is = 0, dv = 0, dw = 0, v3 = 0, w3 = 0;
+        // sign(bn) towards O
+        const int sg = bnz ? ((gt_zero(bn) == takeL) ? 1 : -1) : 0;
+        if (level == 2) {
+            DO = suO - dO;
+            iO = rcp_fast(DO);
+            rO = mO * iO;
+            rsqrt_and_sqrt(rO, isO, sO);
+            so = star_fwd(mO, DO, dO, bn, bbn, Out, Obt, Obz);
+            is = rcp_fast(sK + sO);
+            dv = so.v - sk.v;
+            dw = so.w - sk.w;
+            v3 = fma(sO, dv, sgn_select(so.b - sk.b, sg)) * is;  // from K's star state
+            w3 = fma(sO, dw, sgn_select(so.z - sk.z, sg)) * is;
+            const double ss = sgn_select(sK, sg);
+            Xv = sk.v + v3;
+            Xw = sk.w + w3;
+            Xb = fma(ss, v3, sk.b);
+            Xz = fma(ss, w3, sk.z);
+            Xsb = fma(Xw, Xz, fma(Xv, Xb, SMbn));
+            Xe = fma(ss, Xsb - sbK, eK);
+        }
+        const double eb = Fe * SM;
+        const double dbn = bn - Kbn;
+        const double t0 = fma(Fmt, Kbt, fma(Fbt, Kut, Fe * wKf));
+        double SMb = fma(phi, Fmn, fma(Xb, Fbt, fma(Xz, Fbz, Fe * (Xe + PT))));
+        double PTb = Fmn + eb;
+        double bnb = t0 - fma(Xb, Fmt, fma(Xv, Fbt, fma(Xw, Fbz, Xsb * Fe)));
+        double vb = fma(phi, Fmt, -bn * Fbt), wb = -bn * Fbz;
+        double bb = fma(SM, Fbt, -bn * Fmt), zb = SM * Fbz;
+        double sbb = -bn * Fe;
+        double rKb = fma(Fmn, SM, fma(Fmt, Xv, Fm));  // of phi
+        SMb = fma(rKb, rK, SMb);
+        rKb *= SM;
+        wKfb = dbn * Fe;
+        k.bn = -fma(2.0 * Fmn, Kbn, t0);
+        k.bt = dbn * Fmt;
+        k.ut = dbn * Fbt;
+        double mKb = 0.0, mOb = 0.0, suKb = 0.0;
+        if (!sk.g) {
+            bnb = fma(-Fmt, Kbt, bnb);
+            k.bt -= fma(Fmt, bn, Fbt * suK);
+            k.bz = -Fbz * suK;
+            suKb = -fma(Fbt, Kbt, Fbz * Kbz);
+        }
+        if (level == 2) {
+            // e3 = eK + sg sK (sb3 - sbK), sb3 = w3 z3 + v3 b3 + SM bn
+            const double t = sgn_select(eb, sg);
+            double sKb = t * (Xsb - sbK);
+            sbb = fma(t, sK, sbb);
+            wb = fma(sbb, Xz, wb);
+            zb = fma(sbb, Xw, zb);
+            vb = fma(sbb, Xb, vb);
+            bb = fma(sbb, Xv, bb);
+            SMb = fma(sbb, bn, SMb);
+            bnb = fma(sbb, SM, bnb);
+            sbb = -t * sK;
+            // (sK + sO) v3 = sK vK + sO vO + sg (bO - bK), b3 = bK + sg sK (v3 - vK): with
+            // al = (v - sO sg b) / (sK + sO), be = (v + sK sg b) / (sK + sO) of the adjoints,
+            // sK += (vK - v3) al, sO += (vO - v3) be, vK = sK al, vO = sO be, bK = -sg al,
+            // bO = sg be; the same for w, z
+            vb *= is;
+            wb *= is;
+            bb = sgn_select(bb, sg) * is;
+            zb = sgn_select(zb, sg) * is;
+            const double av = fma(-sO, bb, vb), bv = fma(sK, bb, vb);
+            const double aw = fma(-sO, zb, wb), bw = fma(sK, zb, wb);
+            sKb = fma(-v3, av, fma(-w3, aw, sKb));
+            const double sOb = fma(dv - v3, bv, (dw - w3) * bw);
+            vb = sK * av;
+            wb = sK * aw;
+            bb = sgn_select(av, -sg);
+            zb = sgn_select(aw, -sg);
+            // s = sqrt(r*): ds = 0.5 / s dr ; r* = m / D
+            rKb = fma(0.5 * sKb, isK, rKb);
+            mOb = 0.5 * sOb * isO * iO;
+            double DOb = -mOb * rO, dOb = 0.0;
+            star_rev(so, mO, DO, bn, Obt, Obz, sO * bv, sO * bw, sgn_select(bv, sg),
+                     sgn_select(bw, sg), o, mOb, DOb, dOb, bnb);
+            SOb = DOb;
+            SMb += dOb - DOb;
+            o.un = -dOb;
+        }
+        // D eK = E su + P* SM - pT un + bn (wKf - sbK)
+        const double nb = eb * iK;
+        KEb = nb * suK;
+        suKb = fma(nb, KE, suKb);
+        PTb = fma(nb, SM, PTb);
+        SMb = fma(nb, PT, SMb);
+        bnb = fma(nb, wsb, bnb);
+        const double nbn = nb * bn;
+        wKfb += nbn;
+        sbb -= nbn;
+        double DKb = -nb * eK, dKb = 0.0;
+        // sbK = wK zK + vK bK + SM bn
+        wb = fma(sbb, sk.z, wb);
+        zb = fma(sbb, sk.w, zb);
+        vb = fma(sbb, sk.b, vb);
+        bb = fma(sbb, sk.v, bb);
+        SMb = fma(sbb, bn, SMb);
+        bnb = fma(sbb, SM, bnb);
+        // rK = m / D ; the star state ; P* = pT + m d
+        mKb = rKb * iK;
+        DKb = fma(-mKb, rK, DKb);
+        star_rev(sk, mK, DK, bn, Kbt, Kbz, vb, wb, bb, zb, k, mKb, DKb, dKb, bnb);
+        mKb = fma(PTb, dK, mKb);
+        dKb = fma(PTb, mK, dKb);
+        SKb = DKb;
+        SMb += dKb - DKb;
+        // mR (SM - uR) + pR = mL (SM - uL) + pL
+        const double ns = SMb * iden;
+        const double nK = takeL ? -ns : ns;
+        mKb = fma(-nK, dK, mKb);
+        mOb = fma(nK, dO, mOb);
+        // m = r su, su = S - un
+        suKb = fma(mKb, Kr, suKb);
+        const double suOb = mOb * Or;
+        k.r = mKb * suK;
+        o.r = mOb * suO;
+        k.un = fma(nK, mK, -fma(nb, KpT, dKb)) - suKb;
+        o.un = fma(-nK, mO, o.un) - suOb;
+        k.pT = PTb - fma(nb, Kun, nK);
+        o.pT = nK;
+        SKb += suKb;
+        SOb += suOb;
+        // (SR - SL) bn = SR bR - SL bL
+        const double nn = bnb * iS;
+        const double nB = takeL ? -nn : nn;
+        SKb = fma(nB, Kbn - bn, SKb);
+        SOb = fma(-nB, Obn - bn, SOb);
+        k.bn = fma(nB, SK, k.bn);
+        o.bn = -nB * SO;
     }
+    // E = p inv_gm1 + 0.5 (r (un^2 + ut^2) + bb) ; wKf = un bn + ut bt
+    const double kin = 0.5 * KEb, rE = Kr * KEb;
+    k.p = KEb * P.inv_gm1;
+    k.bb = kin;
+    k.r = fma(kin, vsq, k.r);
+    k.un = fma(wKfb, Kbn, fma(rE, Kun, k.un));
+    k.ut = fma(wKfb, Kbt, fma(rE, Kut, k.ut));
+    k.bn = fma(wKfb, Kun, k.bn);
+    k.bt = fma(wKfb, Kut, k.bt);
+    // F.bn = -UU (B.bn - A.bn), UU = max(|SL|, |SR|)
+    const double UU = dabs(UUR ? SR : SL);
+    const double UUb = -Fbn * (B.bn - A.bn);
+    double SLb = takeL ? SKb : SOb, SRb = takeL ? SOb : SKb;
+    {
+        add_to(UUR, SRb, SLb, sgn_select(UUb, lt_zero(UUR ? SR : SL) ? -1 : 1));
+    }
+    // back to A and B
+    SideB Ab, Bb;
+    Ab.r = takeL ? k.r : o.r;      Bb.r = takeL ? o.r : k.r;
+    Ab.p = takeL ? k.p : 0.0;      Bb.p = takeL ? 0.0 : k.p;
+    Ab.un = takeL ? k.un : o.un;   Bb.un = takeL ? o.un : k.un;
+    Ab.ut = takeL ? k.ut : o.ut;   Bb.ut = takeL ? o.ut : k.ut;
+    Ab.bn = takeL ? k.bn : o.bn;   Bb.bn = takeL ? o.bn : k.bn;
+    Ab.bt = takeL ? k.bt : o.bt;   Bb.bt = takeL ? o.bt : k.bt;
+    Ab.bz = takeL ? k.bz : o.bz;   Bb.bz = takeL ? o.bz : k.bz;
+    Ab.pT = takeL ? k.pT : o.pT;   Bb.pT = takeL ? o.pT : k.pT;
+    Ab.bb = takeL ? k.bb : 0.0;    Bb.bb = takeL ? 0.0 : k.bb;
+    Ab.bn = fma(Fbn, UU, Ab.bn);
+    Bb.bn = fma(-Fbn, UU, Bb.bn);
+    // SL = uminN - cmax ; SR = umaxN + cmax
+    const double cmaxb = SRb - SLb;
+    add_to(minA, Ab.un, Bb.un, SLb);
+    add_to(!maxB, Ab.un, Bb.un, SRb);
     // ---- the fast speed of the side of max(cf) ------------------------------------------
     {
         const double Ccf = cfB ? B.cf : A.cf, Crs = cfB ? B.rs : A.rs;
         const double Crq = cfB ? B.rq : A.rq, Ca = cfB ? B.a : A.a, Cgp = cfB ? B.gp : A.gp;
         const double Cbn2 = cfB ? B.bn2 : A.bn2, Cdisc = cfB ? B.disc : A.disc;
         // cf = X rsqrt(X r) = sqrt(X / r): d/dX = 0.5 rs, d/dr = -0.5 cf / r = -0.5 cf^2 rs
-        const double Xb = cmaxb * 0.5 * Crs;
-        const double rb = -0.5 * cmaxb * (Ccf * Ccf) * Crs;
+        const double Xh = 0.25 * cmaxb * Crs;  // half the adjoint of X
+        const double rb = -2.0 * Xh * (Ccf * Ccf);
         // X = 0.5 (a + sq), sq = sqrt(disc), disc = a^2 - 4 gp bn2 (clamped at 0)
-        double ab = 0.5 * Xb, gpb = 0.0, bn2b = 0.0;
+        double ab = Xh, gpb = 0.0, bn2b = 0.0;
         if ((bits(Cdisc) << 1) != 0) {
-            const double discb = (0.5 * Xb) * 0.5 * Crq;
-            ab = fma(discb * 2.0, Ca, ab);
-            gpb = -discb * 4.0 * Cbn2;
-            bn2b = -discb * 4.0 * Cgp;
+            const double sb = Xh * Crq;  // twice the adjoint of disc
+            ab = fma(sb, Ca, ab);
+            gpb = -2.0 * sb * Cbn2;
+            bn2b = -2.0 * sb * Cgp;
         }
         gpb += ab;  // a = gp + bb
         add_to(!cfB, Ab.r, Bb.r, rb);
@@ -692,8 +525,10 @@ __device__ __forceinline__ void hlld_vjp(const double* qa, const double* qb, con
 // ---------------------------------------------------------------------------------------
 // Pass B: face adjoints (each face once), then the gather into cells.
 //
-// B1 adj_face_kernel: one thread per face.  It reconstructs the face's two states from the
-// four cells along its normal, recomputes the HLLD flux and runs its reverse sweep on
+// B1 adj_face_kernel: one thread per face.  Bound by the FP64 pipe: 374 us for the 2 x 1024^2
+// faces of a 1024^2 grid, 552 us when the sweep reversed the forward's chain of operations (512
+// FP64 operations per face).  It reconstructs the face's two states from the
+// four cells along its normal, recomputes the flux's star states and runs its reverse sweep on
 // Fbar = k (dbar_low - dbar_high).  The adjoint of the low-side state (the upper face state
 // of the low cell) goes to that cell's "up" plane, the adjoint of the high-side state (the
 // lower face state of the high cell) to that cell's "dn" plane: every entry has exactly one
@@ -715,7 +550,12 @@ __device__ __forceinline__ void hlld_vjp(const double* qa, const double* qb, con
 constexpr int kFaceAdj = 15;
 constexpr int kSel = kFaceAdj + 4 * NF;
 constexpr int kScratchPlanes = kSel + 3;  // 18 bytes per cell fit in three planes of doubles
-constexpr int FBX = 32, FBY = 4;  // 128-thread blocks of both kernels
+constexpr int FBX = 32, FBY = 4;  // 128-thread blocks of the gather
+// B1: 64-thread blocks at five per SM (168 registers, 0.25 KB of spills per thread) take 5.90 ms
+// for ten reverse steps on 1024^2 cells; 5.95 ms without the bound (208 registers), 5.99 ms at
+// six, 6.15 ms at eight per SM; 128-thread blocks 6.06 ms (208 registers), 5.99 ms at three per
+// SM; 32-thread blocks 6.12 ms.
+constexpr int kFaceRows = 2;
 
 // periodic index for any i
 __device__ __forceinline__ int wrap(int i, int n) {
@@ -740,13 +580,15 @@ __device__ __forceinline__ double slope_sel(double cm, double c, double cp, int&
     return s;
 }
 
-__global__ void __launch_bounds__(FBX * FBY) adj_face_kernel(Params P, CPlanes U, double* scratch,
-                                                             const double* __restrict__ T_do_ptr) {
+__global__ void __launch_bounds__(FBX * kFaceRows, 5) adj_face_kernel(
+    Params P, CPlanes U, double* scratch, const double* __restrict__ T_do_ptr) {
     const int N = P.N, M = P.M;
     const long long K = (long long)N * M;
-    const bool isx = blockIdx.z == 0;
-    const int ix = blockIdx.x * FBX + threadIdx.x;  // x-face index (x) or column (y)
-    const int iy = blockIdx.y * FBY + threadIdx.y;  // row (x) or y-face index (y)
+    const bool isx = blockIdx.y == 0;
+    // blocks of a row first, then rows, in one grid dimension (the second one is too short)
+    const unsigned nbx = (unsigned)((N + FBX - 1) / FBX);
+    const int ix = (int)(blockIdx.x % nbx) * FBX + threadIdx.x;         // x-face index or column
+    const int iy = (int)(blockIdx.x / nbx) * kFaceRows + threadIdx.y;  // row or y-face index
     if (ix >= N || iy >= M) return;
     const double T_do = *T_do_ptr;
     const double kk = T_do * (isx ? P.inv_dx : P.inv_dy);  // the forward's scaling
@@ -890,7 +732,7 @@ int grid_cells(long long K) {
 // Branch switches between two runs (gd_adj_switches).  A central difference of runs from
 // U0 + eps v and U0 - eps v is the derivative of the branch both take only where every
 // non-smooth choice comes out the same in both.  Per face, the choices its flux depends on,
-// computed with the forward's own operations (as adj_face_kernel repeats them): the minmod
+// computed from the FP64 quantities that adj_face_kernel takes its branches by: the minmod
 // pick of its low cell's slope (every cell's slope is counted at exactly one face per
 // direction), the rho / p fallbacks of its two face states, and the HLLD choices: which
 // side gives min(u), max(u), max(cf) and max(|S|) (speeds), the upwind side and the region
@@ -931,7 +773,7 @@ __device__ __forceinline__ FaceCode face_code(const Params& P, const CPlanes& U,
     SideV A, B;
     side_fwd(A, la, P);
     side_fwd(B, lb, P);
-    // the forward part of hlld_vjp up to the region, operation for operation
+    // the forward part of hlld_vjp up to the region, for both sides
     const bool minA = !dlt(B.un, A.un);
     const bool maxB = dlt(A.un, B.un);
     const double uminN = minA ? A.un : B.un;
@@ -942,7 +784,7 @@ __device__ __forceinline__ FaceCode face_code(const Params& P, const CPlanes& U,
     const double suL = SL - A.un, suR = SR - B.un;
     const double mL = A.r * suL, mR = B.r * suR;
     const double iden = rcp_fast(mR - mL);
-    const double SM = ((fma(mR, B.un, -mL * A.un) - B.pT) + A.pT) * iden;
+    const double SM = A.un + fma(mR, B.un - A.un, A.pT - B.pT) * iden;
     const bool UUR = mag_lt(SL, SR);
     const double iS = rcp_fast(SR - SL);
     const double bn = fma(SR, B.bn, -SL * A.bn) * iS;
@@ -1116,7 +958,8 @@ cudaError_t launch_adjoint_step(const Params& P, const CPlanes& U, const double*
     adj_update_kernel<<<grid_cells(K), NT, 0, st>>>(P, U, aux, lam_out, scratch);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    adj_face_kernel<<<dim3(gxb, gyb, 2), blk, 0, st>>>(P, U, scratch, T_do);
+    const unsigned fyb = (unsigned)((P.M + kFaceRows - 1) / kFaceRows);
+    adj_face_kernel<<<dim3(gxb * fyb, 2), dim3(FBX, kFaceRows), 0, st>>>(P, U, scratch, T_do);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     adj_gather_kernel<<<dim3(gxb, gyb, 1), blk, 0, st>>>(P, scratch, lam_in, T_do);
