@@ -42,11 +42,14 @@
 namespace gd {
 namespace {
 
-constexpr int NT = 256;
+constexpr int kNT = 256;  // threads of a tile: single-grid step, tangent
 constexpr int NF = 4;
 // CTAs per SM that the shared memory of a tile shape leaves room for
 template <int TX, int TY>
 constexpr int kCtas = TX * TY > 256 ? 2 : 4;
+// threads of a tile in the batch kernel (see there)
+template <int TX, int TY>
+constexpr int kNTBatch = TX * TY > 256 ? 256 : 192;
 
 template <class T>
 struct FluxE {
@@ -358,7 +361,7 @@ __device__ __forceinline__ Dual mul_rn(double a, Dual b) { return a * b; }
 
 // ---- U: conservative update of the tile's cells ---------------------------------------------
 // cell: the tile's own values, rows RS and fields FS apart.
-template <class T, int ORDER, int TX, int TY, int RS, int FS, class OUT>
+template <class T, int ORDER, int TX, int TY, int NT, int RS, int FS, class OUT>
 __device__ __forceinline__ void update_cells(const Params& P, const OUT& out, int tx0, int ty0,
                                              double T_do, int dt_only, const T* cell, const T* fx,
                                              const T* fy, TileResult& res, double* aux) {
@@ -427,7 +430,7 @@ __device__ __forceinline__ void update_cells(const Params& P, const OUT& out, in
 // Not inlined: the single-grid kernel and the persistent batch kernel call one compiled
 // function per tile shape, so a grid's arithmetic, and its bits, do not depend on which
 // schedule advanced it (inlined into each, the compiler may fuse the two differently).
-template <class T, int ORDER, int TX, int TY, class IN, class OUT>
+template <class T, int ORDER, int TX, int TY, int NT, class IN, class OUT>
 __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT& out, int tx0,
                                         int ty0, double T_do, int dt_only, T* smem,
                                         TileResult& res, double* aux) {
@@ -508,7 +511,7 @@ __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT
     }
     __syncthreads();
 
-    update_cells<T, ORDER, TX, TY, SX, SY * SX>(P, out, tx0, ty0, T_do, dt_only,
+    update_cells<T, ORDER, TX, TY, NT, SX, SY * SX>(P, out, tx0, ty0, T_do, dt_only,
                                                 prim + H * SX + H, fx, fy, res, aux);
     res.umax_x = fastest.x;
     res.umax_y = fastest.y;
@@ -525,7 +528,7 @@ __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT
 // The faces of a thread that the integer solver left (bit k: the k-th), in floating point.  Out of
 // line, and after the loop over the faces: a second solver inside it would take registers from
 // every face for what a few need.  speed: the faces whose wave speed is missing too.
-template <int ORDER, int TX, int TY>
+template <int ORDER, int TX, int TY, int NT>
 __device__ __noinline__ void faces_left(const Params& P, double* smem, const fx::Tops& X, int tx0,
                                         int ty0, unsigned int left, unsigned int speed,
                                         Speeds& u) {
@@ -557,7 +560,7 @@ __device__ __noinline__ void faces_left(const Params& P, double* smem, const fx:
 }
 
 // Every face of a tile held in integers.  dt_only: the wave speeds alone.
-template <bool HLL, int ORDER, int TX, int TY>
+template <bool HLL, int ORDER, int TX, int TY, int NT>
 __device__ __forceinline__ void faces_int(const Params& P, double* smem, const fx::Tops& X,
                                            int tx0, int ty0, int dt_only, Speeds& u) {
     using S = Shape<ORDER, TX, TY>;
@@ -599,13 +602,13 @@ __device__ __forceinline__ void faces_int(const Params& P, double* smem, const f
         if (done) w.store(t.fx, t.fy, m, e, mn, mt);
         else left |= bit;
     }
-    if (left) faces_left<ORDER, TX, TY>(P, smem, X, tx0, ty0, left, speed, u);
+    if (left) faces_left<ORDER, TX, TY, NT>(P, smem, X, tx0, ty0, left, speed, u);
 }
 
 // Returns false, with nothing written, where the tile's cells cannot be held in common units.
 // Every thread of the block must call it, and all get the same answer.  METHODS: 1 HLLC, 2 HLL, 3
 // the one of P (both solvers in the function).
-template <int METHODS, int ORDER, int TX, int TY>
+template <int METHODS, int ORDER, int TX, int TY, int NT>
 __device__ __forceinline__ bool euler_tile_int(const Params& P, const CPlanes& in, const Planes& out,
                                             int tx0, int ty0, double T_do, int dt_only,
                                             double* smem, TileResult& res, double* aux) {
@@ -666,11 +669,11 @@ __device__ __forceinline__ bool euler_tile_int(const Params& P, const CPlanes& i
     __syncthreads();
     Speeds fastest{0.0, 0.0};
     if (METHODS == 2 || (METHODS == 3 && P.method == GD_METHOD_HLL))
-        faces_int<true, ORDER, TX, TY>(P, smem, X, tx0, ty0, dt_only, fastest);
+        faces_int<true, ORDER, TX, TY, NT>(P, smem, X, tx0, ty0, dt_only, fastest);
     else
-        faces_int<false, ORDER, TX, TY>(P, smem, X, tx0, ty0, dt_only, fastest);
+        faces_int<false, ORDER, TX, TY, NT>(P, smem, X, tx0, ty0, dt_only, fastest);
     __syncthreads();
-    update_cells<double, ORDER, TX, TY, TX, TX * TY>(P, out, tx0, ty0, T_do, dt_only, t.cell, t.fx,
+    update_cells<double, ORDER, TX, TY, NT, TX, TX * TY>(P, out, tx0, ty0, T_do, dt_only, t.cell, t.fx,
                                                      t.fy, res, aux);
     res.umax_x = fastest.x;
     res.umax_y = fastest.y;
@@ -678,15 +681,15 @@ __device__ __forceinline__ bool euler_tile_int(const Params& P, const CPlanes& i
 }
 
 // A tile of the step: in integers where the tile's range allows it.
-template <int METHODS, int ORDER, int TX, int TY>
+template <int METHODS, int ORDER, int TX, int TY, int NT>
 __device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, const Planes& out,
                                           int tx0, int ty0, double T_do, int dt_only,
                                           double* smem, TileResult& res, double* aux) {
-    if (euler_tile_int<METHODS, ORDER, TX, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, res,
+    if (euler_tile_int<METHODS, ORDER, TX, TY, NT>(P, in, out, tx0, ty0, T_do, dt_only, smem, res,
                                                aux))
         return;
     __syncthreads();
-    euler_tile<double, ORDER, TX, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, res, aux);
+    euler_tile<double, ORDER, TX, TY, NT>(P, in, out, tx0, ty0, T_do, dt_only, smem, res, aux);
 }
 
 __device__ __forceinline__ void add_counters(Scalars* ctr, const TileResult& r) {
@@ -698,7 +701,7 @@ __device__ __forceinline__ void add_counters(Scalars* ctr, const TileResult& r) 
 }
 
 template <int METHODS, int ORDER, int TX, int TY>
-__global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_fast_kernel(const __grid_constant__ Params P,
+__global__ void __launch_bounds__(kNT, kCtas<TX, TY>) euler_fast_kernel(const __grid_constant__ Params P,
                                                         const __grid_constant__ CPlanes in,
                                                         const __grid_constant__ Planes out,
                                                         const double* __restrict__ T_do_ptr,
@@ -707,10 +710,10 @@ __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_fast_kernel(const __g
                                                         double* aux) {
     extern __shared__ double smem[];
     TileResult r;
-    step_tile<METHODS, ORDER, TX, TY>(P, in, out, blockIdx.x * TX, (blockIdx.y + P.tile_row0) * TY,
+    step_tile<METHODS, ORDER, TX, TY, kNT>(P, in, out, blockIdx.x * TX, (blockIdx.y + P.tile_row0) * TY,
                              *T_do_ptr, dt_only, smem, r, aux);
     add_counters(ctr, r);
-    block_dt_and_rotate<NT>(P, r.umax_x, r.umax_y, r.any_active, T_bits, rot, P.tile_nblocks);
+    block_dt_and_rotate<kNT>(P, r.umax_x, r.umax_y, r.any_active, T_bits, rot, P.tile_nblocks);
 }
 
 // Tangent of one step: (U, dU) -> (U', dU') with the dt read from *T_do_ptr (held fixed):
@@ -719,14 +722,14 @@ __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_fast_kernel(const __g
 // one).
 constexpr int kTanTX = 32, kTanTY = 8;
 template <int ORDER>
-__global__ void __launch_bounds__(NT) euler_tangent_kernel(Params P, CPlanes in, CPlanes din,
+__global__ void __launch_bounds__(kNT) euler_tangent_kernel(Params P, CPlanes in, CPlanes din,
                                                            Planes out, Planes dout,
                                                            const double* __restrict__ T_do_ptr) {
     extern __shared__ __align__(16) double smem[];
     TileResult r;
     const DualIn I{in, din};
     const DualOut O{out, dout};
-    euler_tile<Dual, ORDER, kTanTX, kTanTY>(P, I, O, blockIdx.x * kTanTX, blockIdx.y * kTanTY,
+    euler_tile<Dual, ORDER, kTanTX, kTanTY, kNT>(P, I, O, blockIdx.x * kTanTX, blockIdx.y * kTanTY,
                                             *T_do_ptr, 0, reinterpret_cast<Dual*>(smem), r,
                                             nullptr);
 }
@@ -743,10 +746,13 @@ __device__ __forceinline__ void async_copy4(void* to, const void* from) {
 }
 __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// METHODS 1: every grid's method is HLLC (a second solver in the kernel costs it 40 registers'
-// spills: 7.40 against 7.69 ms per pass of 128 grids); 3: any.
+// One pass of 128 grids: 6.54 ms with 192 threads per tile (80 registers, no spills); 6.80 ms with
+// 256 (64 registers: the descriptors and the prefetch on top of the step spill), 6.66 ms with
+// 160.  The single-grid step, which holds less, is the other way round (4.79 against 4.92 ms for
+// two steps at 4096^2).  Tiles of 512 cells, two per SM, have the registers at 256 threads.
+// METHODS 1: every grid's method is HLLC (6.54 against 6.59 ms with both solvers); 3: any.
 template <int METHODS, int ORDER, int TX, int TY>
-__global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_batch_kernel(const BatchGrid* __restrict__ grids,
+__global__ void __launch_bounds__(kNTBatch<TX, TY>, kCtas<TX, TY>) euler_batch_kernel(const BatchGrid* __restrict__ grids,
                                                          const int2* __restrict__ items,
                                                          int nitems, int cur, int dt_only,
                                                          Scalars* sc_override) {
@@ -756,7 +762,7 @@ __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_batch_kernel(const Ba
     __shared__ BatchGrid grid_of[2];
     __shared__ __align__(8) int2 item_of[2];
     constexpr int kWords = sizeof(BatchGrid) / 4;
-    static_assert(sizeof(BatchGrid) % 4 == 0 && kWords <= NT, "one word a thread");
+    static_assert(sizeof(BatchGrid) % 4 == 0 && kWords <= kNTBatch<TX, TY>, "one word a thread");
     const int stride = gridDim.x;
     if (threadIdx.x < 2 && blockIdx.x + threadIdx.x * stride < nitems)
         item_of[threadIdx.x] = items[blockIdx.x + threadIdx.x * stride];
@@ -793,9 +799,9 @@ __global__ void __launch_bounds__(NT, kCtas<TX, TY>) euler_batch_kernel(const Ba
         const int tx0 = (tile % g.tiles_x) * TX, ty0 = (tile / g.tiles_x) * TY;
         const double T_do = sc->T_do;
         TileResult r;
-        step_tile<METHODS, ORDER, TX, TY>(g.P, in, out, tx0, ty0, T_do, dt_only, smem, r, nullptr);
+        step_tile<METHODS, ORDER, TX, TY, kNTBatch<TX, TY>>(g.P, in, out, tx0, ty0, T_do, dt_only, smem, r, nullptr);
         add_counters(dt_only ? nullptr : sc, r);
-        block_dt_and_rotate<NT>(g.P, r.umax_x, r.umax_y, r.any_active, &sc->T_bits,
+        block_dt_and_rotate<kNTBatch<TX, TY>>(g.P, r.umax_x, r.umax_y, r.any_active, &sc->T_bits,
                                 dt_only ? nullptr : sc, (unsigned int)g.ntiles);
     }
 }
@@ -821,10 +827,10 @@ cudaError_t launch_single(const Params& P, const CPlanes& in, const Planes& out,
     dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + TY - 1) / TY);
     constexpr size_t n = Shape<ORDER, TX, TY>::bytes;
     if (P.method == GD_METHOD_HLL)
-        euler_fast_kernel<2, ORDER, TX, TY><<<grid, NT, n, st>>>(P, in, out, T_do, T_bits, rot,
+        euler_fast_kernel<2, ORDER, TX, TY><<<grid, kNT, n, st>>>(P, in, out, T_do, T_bits, rot,
                                                                  ctr, dt_only, aux);
     else
-        euler_fast_kernel<1, ORDER, TX, TY><<<grid, NT, n, st>>>(P, in, out, T_do, T_bits, rot,
+        euler_fast_kernel<1, ORDER, TX, TY><<<grid, kNT, n, st>>>(P, in, out, T_do, T_bits, rot,
                                                                  ctr, dt_only, aux);
     return cudaGetLastError();
 }
@@ -835,10 +841,10 @@ cudaError_t launch_batch(const BatchGrid* grids, const int2* items, int nitems, 
                          cudaStream_t st) {
     constexpr size_t n = Shape<ORDER, TX, TY>::bytes;
     if (hllc_only)
-        euler_batch_kernel<1, ORDER, TX, TY><<<ctas, NT, n, st>>>(grids, items, nitems, cur,
+        euler_batch_kernel<1, ORDER, TX, TY><<<ctas, kNTBatch<TX, TY>, n, st>>>(grids, items, nitems, cur,
                                                                   dt_only, sc_override);
     else
-        euler_batch_kernel<3, ORDER, TX, TY><<<ctas, NT, n, st>>>(grids, items, nitems, cur,
+        euler_batch_kernel<3, ORDER, TX, TY><<<ctas, kNTBatch<TX, TY>, n, st>>>(grids, items, nitems, cur,
                                                                   dt_only, sc_override);
     return cudaGetLastError();
 }
@@ -874,7 +880,7 @@ namespace {
 template <int ORDER, int TX, int TY>
 int blocks_per_sm() {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, euler_batch_kernel<3, ORDER, TX, TY>, NT,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, euler_batch_kernel<3, ORDER, TX, TY>, kNTBatch<TX, TY>,
                                                       Shape<ORDER, TX, TY>::bytes) != cudaSuccess)
         return 1;
     return n > 0 ? n : 1;
@@ -940,10 +946,10 @@ cudaError_t launch_euler_tangent(const Params& P, const CPlanes& in, const CPlan
                                  cudaStream_t st) {
     const dim3 grid((P.N + kTanTX - 1) / kTanTX, (P.M + kTanTY - 1) / kTanTY);
     if (P.order == 1)
-        euler_tangent_kernel<1><<<grid, NT, 2 * Shape<1, kTanTX, kTanTY>::bytes, st>>>(
+        euler_tangent_kernel<1><<<grid, kNT, 2 * Shape<1, kTanTX, kTanTY>::bytes, st>>>(
             P, in, din, out, dout, T_do);
     else
-        euler_tangent_kernel<2><<<grid, NT, 2 * Shape<2, kTanTX, kTanTY>::bytes, st>>>(
+        euler_tangent_kernel<2><<<grid, kNT, 2 * Shape<2, kTanTX, kTanTY>::bytes, st>>>(
             P, in, din, out, dout, T_do);
     return cudaGetLastError();
 }
