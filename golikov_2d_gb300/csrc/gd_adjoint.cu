@@ -32,7 +32,8 @@ constexpr int NT = 256;
 // Pass A: transpose of the cell update (Cartesian).
 // aux layout per cell: d[0..6] (slot order m, e, mx, my, bx, by, bz), divb.  Adjoint
 // scratch per cell: qbar[0..6] (field order rho, p, vx, vy, bx, by, bz, field in b units),
-// dbar[0..6] (slot order), divbbar.
+// dbar[0..6] (slot order), divbbar.  Bound by the FP64 pipe: 40 us at 512^2, 49 us before the
+// squares of both kinetic energies shared one factor (62 FP64 operations per cell, 100 before).
 // ---------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(NT) adj_update_kernel(Params P, CPlanes U, const double* aux,
                                                         CPlanes lam_out, double* scratch) {
@@ -50,7 +51,8 @@ __global__ void __launch_bounds__(NT) adj_update_kernel(Params P, CPlanes U, con
         // forward (same operations as the tile update)
         const double ub = fma(u, bx, imul(v, by));
         const double bb = fma(bz, bz, fma(by, by, imul(bx, bx)));
-        const double K1 = fma(r, fma(u, u, imul(v, v)), bb);
+        const double V1 = fma(u, u, imul(v, v));
+        const double K1 = fma(r, V1, bb);
         double r2 = r - d[0];
         const bool rfl = le_zero(r2);
         if (rfl) r2 = r;
@@ -62,68 +64,32 @@ __global__ void __launch_bounds__(NT) adj_update_kernel(Params P, CPlanes U, con
         const double dE = fma(ub, divb, d[1]);
         const double inv = rcp_fast(r2);
         const double u2 = imul(mx2, inv), v2 = imul(my2, inv);
-        const double K2 = fma(r2, fma(u2, u2, imul(v2, v2)),
-                              fma(bz2, bz2, fma(by2, by2, imul(bx2, bx2))));
+        const double V2 = fma(u2, u2, imul(v2, v2));
+        const double K2 = fma(r2, V2, fma(bz2, bz2, fma(by2, by2, imul(bx2, bx2))));
         const double p2 = fma(P.hgm1, K1 - K2, fma(-P.gm1, dE, p));
         const bool pfl = le_zero(p2);
-        // reverse
-        double r2b = lam_out.f[0][k], p2b = lam_out.f[1][k];
-        double u2b = lam_out.f[2][k], v2b = lam_out.f[3][k];
-        double bx2b = imul(lam_out.f[4][k], kSpi4), by2b = imul(lam_out.f[5][k], kSpi4);
-        double bz2b = imul(lam_out.f[6][k], kSpi4);
-        double E2b = 0.0;
-        if (!pfl) {
-            E2b = p2b * P.gm1;
-            const double Xb = -0.5 * p2b * P.gm1;
-            r2b += Xb * fma(u2, u2, v2 * v2);
-            u2b += Xb * 2.0 * r2 * u2;
-            v2b += Xb * 2.0 * r2 * v2;
-            bx2b += Xb * 2.0 * bx2;
-            by2b += Xb * 2.0 * by2;
-            bz2b += Xb * 2.0 * bz2;
-        }
+        // reverse.  p2 = p - gm1 dE + hgm1 (K1 - K2); gm1 = 2 hgm1 and r2 u2 = mx2 make one
+        // factor w = gm1 p2b serve dE and every square of K1 and K2
+        const double p2b = pfl ? 0.0 : lam_out.f[1][k];
+        const double w = p2b * P.gm1, h = p2b * P.hgm1;
+        const double u2b = fma(-w, mx2, lam_out.f[2][k]), v2b = fma(-w, my2, lam_out.f[3][k]);
+        const double bx2b = fma(-w, bx2, imul(lam_out.f[4][k], kSpi4));
+        const double by2b = fma(-w, by2, imul(lam_out.f[5][k], kSpi4));
+        const double bz2b = fma(-w, bz2, imul(lam_out.f[6][k], kSpi4));
+        // u2 = mx2 / r2, v2 = my2 / r2
         const double mx2b = imul(u2b, inv), my2b = imul(v2b, inv);
-        const double invb = u2b * mx2 + v2b * my2;
-        r2b += -invb * inv * inv;
-        double rb = 0.0, pb = 0.0, ub_ = 0.0, vb = 0.0, bxb = 0.0, byb = 0.0, bzb = 0.0;
-        double db[NF] = {0, 0, 0, 0, 0, 0, 0};
-        double divbb = 0.0, Eb = 0.0, ubb = 0.0;
-        rb += r2b;
-        if (!rfl) db[0] -= r2b;
-        Eb += E2b;
-        ubb -= E2b * divb;
-        divbb -= E2b * ub;
-        db[1] -= E2b;
-        bzb += bz2b;
-        db[6] -= bz2b;
-        byb += by2b;
-        vb -= by2b * divb;
-        divbb -= by2b * v;
-        db[5] -= by2b;
-        bxb += bx2b;
-        ub_ -= bx2b * divb;
-        divbb -= bx2b * u;
-        db[4] -= bx2b;
-        rb += my2b * v;
-        vb += my2b * r;
-        byb -= my2b * divb;
-        divbb -= my2b * by;
-        db[3] -= my2b;
-        rb += mx2b * u;
-        ub_ += mx2b * r;
-        bxb -= mx2b * divb;
-        divbb -= mx2b * bx;
-        db[2] -= mx2b;
-        pb += Eb * P.inv_gm1;
-        rb += 0.5 * Eb * fma(u, u, v * v);
-        ub_ += Eb * r * u;
-        vb += Eb * r * v;
-        const double bbb = 0.5 * Eb;
-        bxb += 2.0 * bbb * bx + ubb * u;
-        byb += 2.0 * bbb * by + ubb * v;
-        bzb += 2.0 * bbb * bz;
-        ub_ += ubb * bx;
-        vb += ubb * by;
+        const double r2b = fma(-mx2b, u2, fma(-my2b, v2, fma(-h, V2, lam_out.f[0][k])));
+        const double db[NF] = {rfl ? 0.0 : -r2b, -w, -mx2b, -my2b, -bx2b, -by2b, -bz2b};
+        const double pb = p2b;
+        const double wr = w * r, wd = -w * divb;  // wd: adjoint of u . b
+        const double rb = fma(mx2b, u, fma(my2b, v, fma(h, V1, r2b)));
+        const double ub_ = fma(wr, u, fma(mx2b, r, fma(-bx2b, divb, wd * bx)));
+        const double vb = fma(wr, v, fma(my2b, r, fma(-by2b, divb, wd * by)));
+        const double bxb = fma(w, bx, fma(wd, u, fma(-mx2b, divb, bx2b)));
+        const double byb = fma(w, by, fma(wd, v, fma(-my2b, divb, by2b)));
+        const double bzb = fma(w, bz, bz2b);
+        const double divbb =
+            -fma(w, ub, fma(bx2b, u, fma(by2b, v, fma(mx2b, bx, my2b * by))));
         double* s = scratch;
         s[0 * K + k] = rb;
         s[1 * K + k] = pb;
@@ -525,8 +491,8 @@ __device__ __forceinline__ void hlld_vjp(const double* qa, const double* qb, con
 // ---------------------------------------------------------------------------------------
 // Pass B: face adjoints (each face once), then the gather into cells.
 //
-// B1 adj_face_kernel: one thread per face.  Bound by the FP64 pipe: 374 us for the 2 x 1024^2
-// faces of a 1024^2 grid, 552 us when the sweep reversed the forward's chain of operations (512
+// B1 adj_face_kernel: one thread per face.  Bound by the FP64 pipe: 357 us for the 2 x 512^2
+// faces of a 512^2 grid, 552 us when the sweep reversed the forward's chain of operations (512
 // FP64 operations per face).  It reconstructs the face's two states from the
 // four cells along its normal, recomputes the flux's star states and runs its reverse sweep on
 // Fbar = k (dbar_low - dbar_high).  The adjoint of the low-side state (the upper face state
@@ -545,14 +511,15 @@ __device__ __forceinline__ void hlld_vjp(const double* qa, const double* qb, con
 // B2 adj_gather_kernel: one thread per cell.  The cell's state adjoint collects the value
 // parts of its two face states per direction, its own slope adjoint through its minmod
 // choice, its neighbours' slope adjoints where their minmod choice used it, and the Powell
-// terms of its neighbours, in a fixed order (deterministic).
+// terms of its neighbours, in a fixed order (deterministic).  Bound by the FP64 pipe: 52 us at
+// 512^2, 69 us with the slope adjoints of all three cells formed before the choices.
 // ---------------------------------------------------------------------------------------
 constexpr int kFaceAdj = 15;
 constexpr int kSel = kFaceAdj + 4 * NF;
 constexpr int kScratchPlanes = kSel + 3;  // 18 bytes per cell fit in three planes of doubles
 constexpr int FBX = 32, FBY = 4;  // 128-thread blocks of the gather
-// B1: 64-thread blocks at five per SM (168 registers, 0.25 KB of spills per thread) take 5.90 ms
-// for ten reverse steps on 1024^2 cells; 5.95 ms without the bound (208 registers), 5.99 ms at
+// B1: 64-thread blocks at five per SM (168 registers, 0.25 KB of spills per thread) took 5.90 ms
+// for ten reverse steps on 512^2 cells; 5.95 ms without the bound (208 registers), 5.99 ms at
 // six, 6.15 ms at eight per SM; 128-thread blocks 6.06 ms (208 registers), 5.99 ms at three per
 // SM; 32-thread blocks 6.12 ms.
 constexpr int kFaceRows = 2;
@@ -681,28 +648,25 @@ __global__ void __launch_bounds__(FBX * FBY) adj_gather_kernel(Params P,
         for (int f = 0; f < NF; ++f) {
             const double* upf = up + (size_t)f * K;
             const double* dnf = dn + (size_t)f * K;
-            // twice the slope adjoint of cell t: up - dn of that cell, a fallback face state
-            // dropping its term; 0.5 a - 0.5 b rounds as 0.5 (a - b) (scaling by 2^-1 is
-            // exact), so the factor goes last
-            double sb2[3];
             int s[3];
+            bool fu[3], fd[3];
 #pragma unroll
             for (int t = 0; t < 3; ++t) {
                 const int b = sel[(size_t)f * K + kc[t]];
                 s[t] = (b & 3) - 1;
-                const bool fu = (b & 4) != 0;
-                const bool fd = f < 2 && fbl[(size_t)f * K + kc[t]] != 0;
-                sb2[t] = (fu ? 0.0 : upf[kc[t]]) - (fd ? 0.0 : dnf[kc[t]]);
+                fu[t] = (b & 4) != 0;
+                fd[t] = f < 2 && fbl[(size_t)f * K + kc[t]] != 0;
             }
-            // value parts of the cell's two face states
-            double acc = upf[k] + dnf[k];
-            // own slope: left difference (c - c_{-1}) -> +1, right (c_{+1} - c) -> -1
-            if (s[1] != 0) acc = fma(s[1] == -1 ? 0.5 : -0.5, sb2[1], acc);
-            // neighbour -1 took its right difference (c - c_{-1})
-            if (s[0] == 1) acc = fma(0.5, sb2[0], acc);
-            // neighbour +1 took its left difference (c_{+1} - c)
-            if (s[2] == -1) acc = fma(-0.5, sb2[2], acc);
-            lam[f] += acc;
+            // The slope adjoint of a cell is half of up - dn, a fallback face state dropping its
+            // term.  Value parts and the cell's own slope (left difference c - c_{-1} -> +1,
+            // right one -> -1): up (1 +- 1/2) + dn (1 -+ 1/2).
+            double acc = fma(fu[1] || s[1] == 0 ? 1.0 : (s[1] == -1 ? 1.5 : 0.5), upf[k], lam[f]);
+            acc = fma(fd[1] || s[1] == 0 ? 1.0 : (s[1] == -1 ? 0.5 : 1.5), dnf[k], acc);
+            // neighbour -1 took its right difference (c - c_{-1}); neighbour +1 its left one
+            const bool a = s[0] == 1, c = s[2] == -1;
+            const double x = (a && !fu[0] ? upf[kc[0]] : 0.0) - (a && !fd[0] ? dnf[kc[0]] : 0.0);
+            const double y = (c && !fu[2] ? upf[kc[2]] : 0.0) - (c && !fd[2] ? dnf[kc[2]] : 0.0);
+            lam[f] = fma(0.5, x - y, acc);
         }
     }
     // Powell: divb_c' = 0.5 kx (bx_{c'+1} - bx_{c'-1}) + 0.5 ky (by_{c'+N} - by_{c'-N})
