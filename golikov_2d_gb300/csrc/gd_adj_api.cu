@@ -289,7 +289,12 @@ gd_status gd_tangent(gd_ctx* ctx, const double* vs, const double* vu, const doub
         const Planes uo = planes_at(u[c ^ 1], nf, K), to = planes_at(t[c ^ 1], nf, K);
         GD_TRY(nf == 7 ? gd::launch_mhd_tangent(ctx->P, ui, ti, uo, to, a->dts + k, st)
                        : gd::launch_euler_tangent(ctx->P, ui, ti, uo, to, a->dts + k, st));
-        ctx->launches += 1;
+        // The values are the recorded run's: the tangent kernel's own, in FP64 throughout, part
+        // from the step's by rounding, and a run through ties and shocks makes that 3e-4 of the
+        // derivative after 100 steps.
+        GD_TRY(step_aux(ctx, ctx->P, ui, uo, a->dts + k, (unsigned long long*)a->tbits, nullptr,
+                        nullptr, nullptr, st));
+        ctx->launches += 2;
         c ^= 1;
     }
     GD_TRY(gd::launch_soa_to_aos(cplanes_at(t[c], nf, K), os, ou, ob, K, nf, st));

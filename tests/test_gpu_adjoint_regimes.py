@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 import golikov_2d_gb300 as g
+from golikov_2d_gb300 import problems
 from test_gpu_adjoint_ragged import dev, host, smooth_state
 
 pytestmark = pytest.mark.gpu
@@ -47,6 +48,35 @@ def test_dot_product_in_every_region_of_the_fan(cuda, regime):
     def call(fn, xs):
         out = [torch.zeros_like(dev(x)) for x in xs]
         fn(*[dev(x) for x in xs], *out)
+        torch.cuda.synchronize()
+        return [host(o) for o in out]
+
+    dot = lambda p, q: sum(float((x * y).sum()) for x, y in zip(p, q))
+    lhs, rhs = dot(lam, call(sol.tangent, v)), dot(call(sol.adj_backward, lam), v)
+    assert np.isfinite(lhs) and abs(lhs - rhs) <= 1e-10 * max(abs(lhs), abs(rhs)), (lhs, rhs)
+    sol.close()
+
+
+@pytest.mark.parametrize("flow", ["orszag_tang", "kelvin_helmholtz"])
+def test_tangent_follows_the_recorded_run(cuda, flow):
+    """A long run from an initial state full of exact ties: the tangent takes the branches of the
+    recorded states, not of states of its own that drift from them by rounding."""
+    import torch
+    cfg, s, u, b = getattr(problems, flow)(256, 256)
+    sol = g.Solver(cfg)
+    sol.import_state(s, u, b)
+    sol.set_time(0.0, 0.0)
+    sol.init_dt()
+    sol.adj_forward(100, 10)
+    rng = np.random.default_rng(3)
+    ins = [x for x in (s, u, b) if x is not None]
+    lam, v = ([rng.standard_normal(x.shape) for x in ins] for _ in range(2))
+
+    def call(fn, xs):
+        xs = [dev(x) for x in xs]
+        out = [torch.zeros_like(x) for x in xs]
+        pad = [None] * (3 - len(xs))
+        fn(*xs, *pad, *out, *pad)
         torch.cuda.synchronize()
         return [host(o) for o in out]
 
