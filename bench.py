@@ -13,7 +13,7 @@ funk_time rotation) over the whole grid.  Metric: FP64 cell-updates/s, whole job
             region.
 * roofline  HBM roofline of the step kernel: algorithmic bytes per launch (each state field
             read once and written once, 8 B each) / average launch time, against the
-            measured HBM bandwidth.  The step is FP64-issue bound on GB300; the "fp64"
+            measured HBM bandwidth.  The step is bound by FP64 and integer issue; the "fp64"
             object reports that fraction against the FP64 FMA rate measured in this run.
 * cpu_baseline  the oracle (the project's C restatement of the reference step, OpenMP over
             all host cores) timed on a bounded sample of the same workload.
@@ -114,24 +114,6 @@ def ncu_fp64_per_cell(workload):
                 return float(parts[2])
             except ValueError:
                 return None
-    return None
-
-
-def int_products_per_cell(workload):
-    """Binary64 products per cell the step kernel forms on the integer pipes (gd_swfp.cuh),
-    from the `int_products=<n>` token of the workload's line in profiles/ncu_traffic.txt."""
-    p = os.path.join(ROOT, "profiles", "ncu_traffic.txt")
-    if not os.path.exists(p):
-        return None
-    for line in open(p):
-        parts = line.split()
-        if parts and parts[0] == workload:
-            for tok in parts[3:]:
-                if tok.startswith("int_products="):
-                    try:
-                        return float(tok.split("=", 1)[1])
-                    except ValueError:
-                        return None
     return None
 
 
@@ -259,17 +241,6 @@ def fp64_roofline(g, workload, cells_per_s, torch, sm_mhz=None):
         out.update({"ops_per_cell": per_cell, "achieved": ach, "frac": ach / pipe_peak_ops,
                     "frac_of_dfma_loop": ach / (probe / 2.0),
                     "ops_source": OPS_SOURCE})
-        ip = int_products_per_cell(workload)
-        if ip is not None:
-            # the binary64 arithmetic of a cell is the FP64-pipe operations plus the products
-            # formed on the integer pipes (bit-identical to FP64 multiplies)
-            b64 = (per_cell + ip) * cells_per_s
-            out.update({"int_pipe_products_per_cell": ip,
-                        "binary64_ops_per_cell": per_cell + ip,
-                        "binary64_achieved": b64,
-                        "binary64_vs_fp64_pipe_peak": b64 / pipe_peak_ops,
-                        "int_products_source": "count of integer-pipe products in the kernel "
-                                               "source per cell, profiles/ncu_traffic.txt"})
     return out
 
 
@@ -1181,7 +1152,7 @@ def run_gb300(args):
                      "frac": achieved / peak_gbs,
                      "traffic": traffic, "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
                      "algorithmic_bytes_per_launch": alg_bytes,
-                     "note": "FP64-issue bound on GB300; see fp64"},
+                     "note": "bound by FP64 and integer issue on GB300; see fp64"},
         "fp64": fp64,
         "clocks": clocks,
         "e2e": e2e,
