@@ -244,8 +244,14 @@ gd_status gd_create(const gd_config* cfg, gd_ctx** out) {
                 ctx->side = new (std::nothrow) gd::HancockStreams{nullptr, nullptr, nullptr};
                 if (!ctx->side) e = cudaErrorMemoryAllocation;
             }
+            // At the tiles' priority the band's blocks are handed out after all of theirs (the tile
+            // kernel starts first, without the event): 0.43 ms of mostly idle SMs at a step's end
+            // at 3226 x 1792.  Above it they run beside the first tiles: dt pass and step 8.42 ->
+            // 7.78 ms.
+            int least = 0, greatest = 0;
+            if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
             if (e == cudaSuccess)
-                e = cudaStreamCreateWithFlags(&ctx->side->stream, cudaStreamNonBlocking);
+                e = cudaStreamCreateWithPriority(&ctx->side->stream, cudaStreamNonBlocking, greatest);
             if (e == cudaSuccess)
                 e = cudaEventCreateWithFlags(&ctx->side->fork, cudaEventDisableTiming);
             if (e == cudaSuccess)
