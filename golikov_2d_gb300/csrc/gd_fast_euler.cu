@@ -49,6 +49,13 @@ namespace gd {
 namespace {
 
 constexpr int kNT = 256;  // threads of a tile: single-grid step, tangent
+// Threads of a tile of the 16x16 shape where every tile has an SM to itself (152 of them): the
+// step is then one tile's latency, and 576 threads take its 544 faces in one round instead of
+// three: 11.7 against 13.5 us at 64x48, 12.1 against 13.9 at 192x192 (144 tiles; 288 threads:
+// 12.8).  From two tiles per SM on (156 tiles: 18.9 against 16.4 us) the 256-thread tiles share
+// an SM better.  The threads of a tile change no result: faces and cells are independent.
+constexpr int kNTFew = 576;
+constexpr long long kFewTiles = 152;
 constexpr int NF = 4;
 // CTAs per SM that the shared memory of a tile shape leaves room for
 template <int TX, int TY>
@@ -706,8 +713,8 @@ __device__ __forceinline__ void add_counters(Scalars* ctr, const TileResult& r) 
     }
 }
 
-template <int METHODS, int ORDER, int TX, int TY>
-__global__ void __launch_bounds__(kNT, kCtas<TX, TY>) euler_fast_kernel(const __grid_constant__ Params P,
+template <int METHODS, int ORDER, int TX, int TY, int NT>
+__global__ void __launch_bounds__(NT, NT == kNT ? kCtas<TX, TY> : 1) euler_fast_kernel(const __grid_constant__ Params P,
                                                         const __grid_constant__ CPlanes in,
                                                         const __grid_constant__ Planes out,
                                                         const double* __restrict__ T_do_ptr,
@@ -716,10 +723,10 @@ __global__ void __launch_bounds__(kNT, kCtas<TX, TY>) euler_fast_kernel(const __
                                                         double* aux) {
     extern __shared__ double smem[];
     TileResult r;
-    step_tile<METHODS, ORDER, TX, TY, kNT>(P, in, out, blockIdx.x * TX, (blockIdx.y + P.tile_row0) * TY,
+    step_tile<METHODS, ORDER, TX, TY, NT>(P, in, out, blockIdx.x * TX, (blockIdx.y + P.tile_row0) * TY,
                              *T_do_ptr, dt_only, smem, r, aux);
     add_counters(ctr, r);
-    block_dt_and_rotate<kNT>(P, r.umax_x, r.umax_y, r.any_active, T_bits, rot, P.tile_nblocks);
+    block_dt_and_rotate<NT>(P, r.umax_x, r.umax_y, r.any_active, T_bits, rot, P.tile_nblocks);
 }
 
 // Tangent of one step: (U, dU) -> (U', dU') with the dt read from *T_do_ptr (held fixed):
@@ -819,25 +826,43 @@ cudaError_t set_room(K* kernel, size_t bytes) {
 template <int ORDER, int TX, int TY>
 cudaError_t set_attrs() {
     constexpr size_t n = Shape<ORDER, TX, TY>::bytes;
-    cudaError_t e = set_room(euler_fast_kernel<1, ORDER, TX, TY>, n);
-    if (e == cudaSuccess) e = set_room(euler_fast_kernel<2, ORDER, TX, TY>, n);
+    cudaError_t e = set_room(euler_fast_kernel<1, ORDER, TX, TY, kNT>, n);
+    if (e == cudaSuccess) e = set_room(euler_fast_kernel<2, ORDER, TX, TY, kNT>, n);
+    if constexpr (TX == 16 && TY == 16) {
+        if (e == cudaSuccess) e = set_room(euler_fast_kernel<1, ORDER, TX, TY, kNTFew>, n);
+        if (e == cudaSuccess) e = set_room(euler_fast_kernel<2, ORDER, TX, TY, kNTFew>, n);
+    }
     if (e == cudaSuccess) e = set_room(euler_batch_kernel<1, ORDER, TX, TY>, n);
     if (e == cudaSuccess) e = set_room(euler_batch_kernel<3, ORDER, TX, TY>, n);
     return e;
+}
+
+template <int ORDER, int TX, int TY, int NT>
+void launch_tiles(const Params& P, dim3 grid, const CPlanes& in, const Planes& out,
+                  const double* T_do, unsigned long long* T_bits, Scalars* rot, Scalars* ctr,
+                  int dt_only, cudaStream_t st, double* aux) {
+    constexpr size_t n = Shape<ORDER, TX, TY>::bytes;
+    if (P.method == GD_METHOD_HLL)
+        euler_fast_kernel<2, ORDER, TX, TY, NT><<<grid, NT, n, st>>>(P, in, out, T_do, T_bits, rot,
+                                                                     ctr, dt_only, aux);
+    else
+        euler_fast_kernel<1, ORDER, TX, TY, NT><<<grid, NT, n, st>>>(P, in, out, T_do, T_bits, rot,
+                                                                     ctr, dt_only, aux);
 }
 
 template <int ORDER, int TX, int TY>
 cudaError_t launch_single(const Params& P, const CPlanes& in, const Planes& out,
                           const double* T_do, unsigned long long* T_bits, Scalars* rot,
                           Scalars* ctr, int dt_only, cudaStream_t st, double* aux = nullptr) {
-    dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + TY - 1) / TY);
-    constexpr size_t n = Shape<ORDER, TX, TY>::bytes;
-    if (P.method == GD_METHOD_HLL)
-        euler_fast_kernel<2, ORDER, TX, TY><<<grid, kNT, n, st>>>(P, in, out, T_do, T_bits, rot,
-                                                                 ctr, dt_only, aux);
-    else
-        euler_fast_kernel<1, ORDER, TX, TY><<<grid, kNT, n, st>>>(P, in, out, T_do, T_bits, rot,
-                                                                 ctr, dt_only, aux);
+    const dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + TY - 1) / TY);
+    if constexpr (TX == 16 && TY == 16) {
+        if ((long long)grid.x * grid.y <= kFewTiles) {
+            launch_tiles<ORDER, TX, TY, kNTFew>(P, grid, in, out, T_do, T_bits, rot, ctr, dt_only,
+                                                st, aux);
+            return cudaGetLastError();
+        }
+    }
+    launch_tiles<ORDER, TX, TY, kNT>(P, grid, in, out, T_do, T_bits, rot, ctr, dt_only, st, aux);
     return cudaGetLastError();
 }
 

@@ -117,3 +117,16 @@ def test_one_solver_batches_equal_mixed_ones_and_single_grids(cuda):
     out = gpu_run(cfg, s, u, None, 12)
     assert np.array_equal(out[0], runs["mixed"][1][0])
     assert np.array_equal(out[1], runs["mixed"][1][1])
+
+
+def test_threads_of_a_tile_change_no_result(cuda):
+    """A batch runs its tiles with 192 threads, a single grid with 576 up to 152 tiles and with
+    256 beyond: the same bits on both sides of that line."""
+    grids = problems.batch_four_quadrant(8, lo=150, hi=250, seed=9)
+    tiles = [-(-c.N // 16) * -(-c.M // 16) for c, *_ in grids]
+    assert min(tiles) <= 152 < max(tiles)
+    batch, _ = run_batch(grids, 5)
+    for (cfg, s, u, b), (s2, u2, st) in zip(grids, batch):
+        ss, us, _, sst = gpu_run(cfg, s, u, b, 5)
+        assert np.array_equal(ss, s2) and np.array_equal(us, u2)
+        assert sst.t == st.t and sst.dt == st.dt
