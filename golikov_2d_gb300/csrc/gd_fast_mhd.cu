@@ -37,7 +37,12 @@ namespace gd {
 namespace {
 
 constexpr int TX = 32;
-constexpr int NT = 384;     // threads of the step
+constexpr int kNT = 384;  // threads of the step (see kTY)
+// Threads where every tile has an SM to itself (152 of them): the step is one tile's latency, and
+// 768 threads take its 747 faces in one round: 29.1 against 32.4 us at 64x48, 28.4 against 31.9 at
+// 320x165 (150 tiles).  At 160 tiles 50.0 against 47.0: there the 384-thread tiles stay.
+constexpr int kNTFew = 768;
+constexpr long long kFewTiles = 152;
 constexpr int NTDual = 256;  // and of its tangent
 constexpr int NF = 7;  // rho, p, vx, vy, bx, by, bz
 
@@ -456,7 +461,7 @@ struct MemInt {
 // The faces of a thread that the integer solver left (bit k: the k-th), in floating point; speed:
 // those whose wave speed is missing too.  Out of line and after the loop over the faces, so that
 // it takes no registers from it.
-template <int ORDER, int TY>
+template <int ORDER, int TY, int NT>
 __device__ __noinline__ void faces_left(const Params& P, double* smem, const fx::TopsM& X, int tx0,
                                         int ty0, unsigned int left, unsigned int speed,
                                         SpeedsM& u) {
@@ -502,7 +507,7 @@ struct JumpInt {
 
 // Returns false, with nothing written, where the tile's cells cannot be held in common units.
 // Every thread of the block must call it, and all get the same answer.
-template <bool HLLD, int ORDER, int TY>
+template <bool HLLD, int ORDER, int TY, int NT>
 __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in, const Planes& out,
                                              int tx0, int ty0, double T_do, int dt_only,
                                              double* smem, MhdTileResult& res, double* aux) {
@@ -605,7 +610,7 @@ __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in,
         else
             left |= bit;
     }
-    if (left) faces_left<ORDER, TY>(P, smem, X, tx0, ty0, left, speed, u);
+    if (left) faces_left<ORDER, TY, NT>(P, smem, X, tx0, ty0, left, speed, u);
     __syncthreads();
 
     update_cells<double, NT, TY, TX, TX * TY>(P, in, out, tx0, ty0, T_do, dt_only, t.cell,
@@ -616,8 +621,8 @@ __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in,
     return true;
 }
 
-template <int ORDER, int TY, bool HLLD>
-__global__ void __launch_bounds__(NT, 2) mhd_fast_kernel(const __grid_constant__ Params P,
+template <int ORDER, int TY, bool HLLD, int NT>
+__global__ void __launch_bounds__(NT, NT == kNT ? 2 : 1) mhd_fast_kernel(const __grid_constant__ Params P,
                                                       const __grid_constant__ CPlanes in,
                                                       const __grid_constant__ Planes out,
                                                       const double* __restrict__ T_do_ptr,
@@ -628,7 +633,7 @@ __global__ void __launch_bounds__(NT, 2) mhd_fast_kernel(const __grid_constant__
     const int tx0 = blockIdx.x * TX, ty0 = (blockIdx.y + P.tile_row0) * TY;
     const double T_do = *T_do_ptr;
     // in integers where the tile's range allows it
-    if (!mhd_tile_int<HLLD, ORDER, TY>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux)) {
+    if (!mhd_tile_int<HLLD, ORDER, TY, NT>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux)) {
         __syncthreads();
         mhd_tile<double, NT, ORDER, TY, false>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux);
     }
@@ -662,17 +667,28 @@ __global__ void __launch_bounds__(NTDual) mhd_tangent_kernel(const __grid_consta
 constexpr int kTY = 11;
 constexpr int kTYDual = 8;
 
+template <int ORDER, int NT>
+void launch_tiles(const Params& P, dim3 grid, const CPlanes& in, const Planes& out,
+                  const double* T_do, unsigned long long* T_bits, Scalars* rot, Scalars* ctr,
+                  int dt_only, cudaStream_t st, double* aux) {
+    constexpr size_t n = step_bytes<ORDER, kTY>();
+    if (P.method == GD_METHOD_HLLD)
+        mhd_fast_kernel<ORDER, kTY, true, NT><<<grid, NT, n, st>>>(P, in, out, T_do, T_bits, rot,
+                                                                   ctr, dt_only, aux);
+    else
+        mhd_fast_kernel<ORDER, kTY, false, NT><<<grid, NT, n, st>>>(P, in, out, T_do, T_bits, rot,
+                                                                    ctr, dt_only, aux);
+}
+
 template <int ORDER>
 cudaError_t launch_t(const Params& P, const CPlanes& in, const Planes& out, const double* T_do,
                      unsigned long long* T_bits, Scalars* rot, Scalars* ctr, int dt_only,
                      cudaStream_t st, double* aux = nullptr) {
-    dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + kTY - 1) / kTY);
-    if (P.method == GD_METHOD_HLLD)
-        mhd_fast_kernel<ORDER, kTY, true><<<grid, NT, step_bytes<ORDER, kTY>(), st>>>(
-            P, in, out, T_do, T_bits, rot, ctr, dt_only, aux);
+    const dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + kTY - 1) / kTY);
+    if ((long long)grid.x * grid.y <= kFewTiles)
+        launch_tiles<ORDER, kNTFew>(P, grid, in, out, T_do, T_bits, rot, ctr, dt_only, st, aux);
     else
-        mhd_fast_kernel<ORDER, kTY, false><<<grid, NT, step_bytes<ORDER, kTY>(), st>>>(
-            P, in, out, T_do, T_bits, rot, ctr, dt_only, aux);
+        launch_tiles<ORDER, kNT>(P, grid, in, out, T_do, T_bits, rot, ctr, dt_only, st, aux);
     return cudaGetLastError();
 }
 
@@ -688,9 +704,12 @@ cudaError_t launch_tangent_t(const Params& P, const CPlanes& in, const CPlanes& 
 
 template <int ORDER, bool HLLD>
 cudaError_t set_room() {
-    return cudaFuncSetAttribute(mhd_fast_kernel<ORDER, kTY, HLLD>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)step_bytes<ORDER, kTY>());
+    constexpr int n = (int)step_bytes<ORDER, kTY>();
+    constexpr auto what = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(mhd_fast_kernel<ORDER, kTY, HLLD, kNT>, what, n);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(mhd_fast_kernel<ORDER, kTY, HLLD, kNTFew>, what, n);
+    return e;
 }
 
 }  // namespace

@@ -130,3 +130,16 @@ def test_threads_of_a_tile_change_no_result(cuda):
         ss, us, _, sst = gpu_run(cfg, s, u, b, 5)
         assert np.array_equal(ss, s2) and np.array_equal(us, u2)
         assert sst.t == st.t and sst.dt == st.dt
+
+
+@pytest.mark.parametrize("N,M", [(320, 165), (320, 176)])
+@pytest.mark.parametrize("solver", ["hlld", "hllc_mhd"])
+def test_mhd_step_on_both_sides_of_152_tiles(cuda, oracle_lib, solver, N, M):
+    """768 threads per tile up to 152 tiles of 32 x 11, 384 beyond (150 and 160 tiles here)."""
+    physics, method = METHODS[solver]
+    cfg = config(physics, method, N, M)
+    s, u, b = state(physics, N * M, 3.0, (1.0, 1.0), 1.0, 17)
+    so, uo, bo, To = oracle_lib.step(grid_of(cfg), s, u, b, 1e-4)
+    sg, ug, bg, Tg = gpu_step_ref(cfg, s, u, b, 1e-4)
+    assert max_rel_l1(cfg, (sg, ug, bg), (so, uo, bo)) <= PER_STEP_TOL
+    assert abs(Tg - To) <= 1e-12 * To
