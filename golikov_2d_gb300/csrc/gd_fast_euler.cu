@@ -16,11 +16,11 @@
 // slopes and face states are integer adds, the flux an integer chain; only the flux results
 // and the update are FP64.  It takes a tile whose densities' and pressures' exponents each
 // span at most 8 and redoes single faces in FP64 where the fan leaves the integers' range.
-// euler_tile is the FP64 body for every other tile, and the tangent's (Dual): its standalone products run
-// on the integer pipes (mulx: the FP64 multiply's bits), the sound speeds and reciprocals take
-// two FP64 operations each, and the HLLC star state takes S_M and q from one reciprocal.
-// One step at 4096^2: 1.69 ms in integers (43.7 FP64 operations per cell, FP64 pipe 68 %, ALU
-// 65 %, issue 61 %), 3.86 ms in FP64 (102.9 per cell, 73 %).
+// euler_tile is the FP64 body for every other tile, and the tangent's (Dual): its standalone
+// products run on the integer pipes (mulx: the FP64 multiply's bits), the sound speeds and
+// reciprocals take two FP64 operations each, and the HLLC star state takes S_M and q from one
+// reciprocal.  One step at 4096^2: 1.70 ms in integers (43.6 FP64 operations per cell, FP64 pipe
+// 69 %, ALU 69 %, issue 65 %), 3.86 ms in FP64 (102.9 per cell, 73 %).
 //
 // Each tile shape is a separate template instantiation; the compiler may fuse multiply-adds
 // differently in each, so shapes agree to rounding (~1e-14 relative per step), not bit for
