@@ -48,7 +48,10 @@
 namespace gd {
 namespace {
 
-constexpr int kNT = 256;  // threads of a tile: single-grid step, tangent
+constexpr int kNT = 256;  // threads of a tile: single-grid step
+// The tangent's 552 faces in two rounds: 20 tangent steps at 512^2 take 5.55 ms, 5.79 with 256
+// threads, 6.17 with 384.
+constexpr int kNTTan = 288;
 // Threads of a tile of the 16x16 shape where every tile has an SM to itself (152 of them): the
 // step is then one tile's latency, and 576 threads take its 544 faces in one round instead of
 // three: 11.7 against 13.5 us at 64x48, 12.1 against 13.9 at 192x192 (144 tiles; 288 threads:
@@ -735,14 +738,14 @@ __global__ void __launch_bounds__(NT, NT == kNT ? kCtas<TX, TY> : 1) euler_fast_
 // one).
 constexpr int kTanTX = 32, kTanTY = 8;
 template <int ORDER>
-__global__ void __launch_bounds__(kNT) euler_tangent_kernel(Params P, CPlanes in, CPlanes din,
+__global__ void __launch_bounds__(kNTTan) euler_tangent_kernel(Params P, CPlanes in, CPlanes din,
                                                            Planes out, Planes dout,
                                                            const double* __restrict__ T_do_ptr) {
     extern __shared__ __align__(16) double smem[];
     TileResult r;
     const DualIn I{in, din};
     const DualOut O{out, dout};
-    euler_tile<Dual, ORDER, kTanTX, kTanTY, kNT>(P, I, O, blockIdx.x * kTanTX, blockIdx.y * kTanTY,
+    euler_tile<Dual, ORDER, kTanTX, kTanTY, kNTTan>(P, I, O, blockIdx.x * kTanTX, blockIdx.y * kTanTY,
                                             *T_do_ptr, 0, reinterpret_cast<Dual*>(smem), r,
                                             nullptr);
 }
@@ -977,10 +980,10 @@ cudaError_t launch_euler_tangent(const Params& P, const CPlanes& in, const CPlan
                                  cudaStream_t st) {
     const dim3 grid((P.N + kTanTX - 1) / kTanTX, (P.M + kTanTY - 1) / kTanTY);
     if (P.order == 1)
-        euler_tangent_kernel<1><<<grid, kNT, 2 * Shape<1, kTanTX, kTanTY>::bytes, st>>>(
+        euler_tangent_kernel<1><<<grid, kNTTan, 2 * Shape<1, kTanTX, kTanTY>::bytes, st>>>(
             P, in, din, out, dout, T_do);
     else
-        euler_tangent_kernel<2><<<grid, kNT, 2 * Shape<2, kTanTX, kTanTY>::bytes, st>>>(
+        euler_tangent_kernel<2><<<grid, kNTTan, 2 * Shape<2, kTanTX, kTanTY>::bytes, st>>>(
             P, in, din, out, dout, T_do);
     return cudaGetLastError();
 }

@@ -43,7 +43,9 @@ constexpr int kNT = 384;  // threads of the step (see kTY)
 // 320x165 (150 tiles).  At 160 tiles 50.0 against 47.0: there the 384-thread tiles stay.
 constexpr int kNTFew = 768;
 constexpr long long kFewTiles = 152;
-constexpr int NTDual = 256;  // and of its tangent
+// The tangent's: one CTA per SM.  20 tangent steps at 512^2 take 18.4 ms with 256 threads, 17.8
+// with 288, 17.3 with 384, 17.9 with 576.
+constexpr int NTDual = 384;
 constexpr int NF = 7;  // rho, p, vx, vy, bx, by, bz
 
 // ---- state access: planes of doubles for the step, value + tangent planes for the JVP ----
