@@ -221,6 +221,9 @@ struct Tops {
 };
 constexpr int kSpan = 8;        // exponents that the densities, and the pressures, may span
 constexpr int kRange = 128;     // exponents of densities, pressures (both signs) and velocities
+// Below 2^-300 a velocity or field that is not 0 goes to the floating-point solver: with densities
+// and fan speeds down to 2^-128 every result stays above 2^-1022.
+constexpr int kLow = 300;
 // x in units of 2^(top - 60), |x| < 2^(top + 1)
 GD_HD i64 to_units(double x, int top) {
     uint32_t hi, lo;
@@ -230,15 +233,12 @@ GD_HD i64 to_units(double x, int top) {
     const i64 v = (i64)((((u64)((h << 8) | (lo >> 24)) << 32) | (lo << 8)) >> imin(top - e, 63));
     return (int32_t)hi < 0 ? -v : v;
 }
-// x 2^ue as a double
+// x 2^ue as a double, a normal number (or 0): ue is added to the exponent field.  The same bits on
+// the host, so that what is checked there is what the kernels compute.
 GD_HD double to_double(i64 x, int ue) {
-#if defined(__CUDA_ARCH__)
     uint32_t hi, lo;
-    swfp::halves(__ll2double_rn(x), hi, lo);
+    swfp::halves((double)x, hi, lo);
     return swfp::from_halves(x == 0 ? 0u : hi + ((uint32_t)ue << 20), lo);
-#else
-    return std::ldexp((double)x, ue);
-#endif
 }
 // 0 unless a and b have the same sign, else the one of smaller magnitude
 GD_HD i64 minmod(i64 a, i64 b) {
@@ -411,17 +411,22 @@ GD_HD bool hll(const Fan& f, const States& s, const Tops& X, const Gas& G, doubl
     return true;
 }
 
-// Exponent field of x (0x7ff for infinities and NaN), and with its sign bit above it.
+// Exponent field of x (0x7ff for infinities and NaN, 1 for subnormal numbers), and with its sign
+// bit above it.
 GD_HD uint32_t exp_field(double x) {
     uint32_t hi, lo;
     swfp::halves(x, hi, lo);
-    return (hi >> 20) & 0x7ffu;
+    const uint32_t e = (hi >> 20) & 0x7ffu;
+    return e == 0 && ((hi << 1) | lo) != 0 ? 1u : e;
 }
 GD_HD uint32_t signed_exp_field(double x) {
     uint32_t hi, lo;
     swfp::halves(x, hi, lo);
     return hi >> 20;
 }
+// Whether the largest velocity or field, of exponent field e, gives a unit: 0, or not so small
+// that a product with it could fall below the normal numbers (to_double).
+GD_HD bool unit_of(uint32_t e) { return e == 0 || (e >= 1023 - kLow && e <= 1023 + kRange); }
 // Whether cells whose densities have exponent fields (sign bit included) in [r0, r1], pressures
 // in [p0, p1] and velocities up to v1 can be held in the units of Tops.
 GD_HD bool tops_of(uint32_t r0, uint32_t r1, uint32_t p0, uint32_t p1, uint32_t v1, const Gas& G,
@@ -429,9 +434,9 @@ GD_HD bool tops_of(uint32_t r0, uint32_t r1, uint32_t p0, uint32_t p1, uint32_t 
     const uint32_t low = 1023 - kRange, high = 1023 + kRange;
     X.r = (int)r1 - 1023;
     X.p = (int)p1 - 1023;
-    X.v = imax((int)v1 - 1023, -900);  // zeros and subnormals come out as 0
+    X.v = imax((int)v1 - 1023, -kLow);
     return G.room >= 0 && r0 >= low && r1 <= high && r1 - r0 <= kSpan && p0 >= low &&
-           p1 <= high && p1 - p0 <= kSpan && v1 <= high;
+           p1 <= high && p1 - p0 <= kSpan && unit_of(v1);
 }
 // The flux (HLL or HLLC) and the larger wave speed of one face given by its two states; false
 // where the integer solver does not take it.

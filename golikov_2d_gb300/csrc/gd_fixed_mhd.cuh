@@ -356,8 +356,8 @@ GD_HD bool tops_of(uint32_t r0, uint32_t r1, uint32_t p0, uint32_t p1, uint32_t 
     X.r = Y.r;
     X.p = Y.p;
     X.v = Y.v;
-    X.b = imax((int)b1 - 1023, -300) + kFieldRoom;
-    return ok && b1 <= 1023 + kRange;
+    X.b = imax((int)b1 - 1023, -kLow) + kFieldRoom;
+    return ok && unit_of(b1);
 }
 
 // The two states {rho, p, un, ut, bn, bt, bz} of a face in units of their own; false where the
