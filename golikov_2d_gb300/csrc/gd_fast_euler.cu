@@ -11,20 +11,17 @@
 // The reference computes every face twice, once from each neighbour (kernel.cu:3560-3586);
 // here each face is computed once and used with opposite signs by its two cells.
 //
-// Two bodies of a tile.  euler_tile_int runs S and F in scaled 64-bit integers (gd_fixed.cuh):
-// the tile's density, pressure and velocity units are powers of two over its largest values,
-// slopes and face states are integer adds, the flux an integer chain; only the flux results
-// and the update are FP64.  It takes a tile whose densities' and pressures' exponents each
-// span at most 8 and redoes single faces in FP64 where the fan leaves the integers' range.
-// euler_tile is the FP64 body for every other tile, and the tangent's (Dual): its standalone
-// products run on the integer pipes (mulx: the FP64 multiply's bits), the sound speeds and
-// reciprocals take two FP64 operations each, and the HLLC star state takes S_M and q from one
-// reciprocal.  One step at 4096^2: 1.70 ms in integers (43.6 FP64 operations per cell, FP64 pipe
-// 69 %, ALU 69 %, issue 65 %), 3.86 ms in FP64 (102.9 per cell, 73 %).
+// S and F of the step run in scaled 64-bit integers (gd_fixed.cuh): a tile's cells are held as
+// significands and exponents, each face takes powers of two over its own stencil as units, slopes
+// and face states are integer adds, the flux an integer chain; only the flux results and the update
+// are FP64.  A face whose densities' or pressures' exponents span more than 8, or whose fan leaves
+// the integers' range, is solved in FP64 from the cells themselves.  The tangent's tile (Dual) is
+// floating point throughout: its standalone products run on the integer pipes (mulx: the FP64
+// multiply's bits), the sound speeds and reciprocals take two FP64 operations each, and the HLLC
+// star state takes S_M and q from one reciprocal.
 //
-// Each tile shape is a separate template instantiation; the compiler may fuse multiply-adds
-// differently in each, so shapes agree to rounding (~1e-14 relative per step), not bit for
-// bit.  A given shape is deterministic.
+// A face's arithmetic depends on its stencil alone and every operation of the update is written
+// out, so that tile shapes, thread counts and kernels agree bit for bit.
 //
 // Two kernels share the tile body: euler_fast_kernel (one grid, one CTA per tile) and
 // euler_batch_kernel (a persistent launch that walks the tiles of many independent grids,
@@ -191,10 +188,10 @@ struct Shape {
     static constexpr int kSly = ORDER == 2 ? NF * (TY + 2) * TX : 0;
     static constexpr int kFx = NF * TY * (TX + 1);
     static constexpr int kFy = NF * (TY + 1) * TX;
-    static constexpr int kFloat = kPrim + kSlx + kSly + kFx + kFy;
-    static constexpr int kInt = kPrim + NF * TY * TX + kFx + kFy;  // TileMemInt
-    static constexpr int doubles = kFloat > kInt ? kFloat : kInt;
-    static constexpr size_t bytes = sizeof(double) * doubles;
+    static constexpr int kKey = SY * SX;
+    static constexpr int kCell = NF * TY * TX;
+    static constexpr size_t bytes = sizeof(double) * (kKey + kPrim + kCell + kFx + kFy);
+    static constexpr size_t dual_bytes = 2 * sizeof(double) * (kPrim + kSlx + kSly + kFx + kFy);
 };
 
 // Value and tangent planes (the tangent step of the adjoint checks).
@@ -250,17 +247,19 @@ struct TileMem {
         : prim(smem), slx(prim + S::kPrim), sly(slx + S::kSlx), fx(sly + S::kSly),
           fy(fx + S::kFx) {}
 };
-// The same of a tile held in integers: no slopes, and the cells' own values beside them.
+// The step's: the cells' significands and keys (gd_fixed.cuh), and the tile's own values.
 template <int ORDER, int TX, int TY>
 struct TileMemInt {
     using S = Shape<ORDER, TX, TY>;
+    using Key = fx::Keys<NF>;
+    static_assert(sizeof(Key) == sizeof(double), "keys take one double a cell");
+    Key* key;      // [SY][SX]
     fx::i64* q;    // [NF][SY][SX]
     double* cell;  // [NF][TY][TX]
     double *fx, *fy;
     __device__ explicit TileMemInt(double* smem)
-        : q(reinterpret_cast<fx::i64*>(smem)), cell(smem + S::kPrim), fx(cell + NF * TY * TX),
-          fy(fx + S::kFx) {}
-    static_assert(S::kPrim + NF * TY * TX + S::kFx + S::kFy <= S::doubles, "fits the tile's room");
+        : key(reinterpret_cast<Key*>(smem)), q(reinterpret_cast<fx::i64*>(smem + S::kKey)),
+          cell(smem + S::kKey + S::kPrim), fx(cell + S::kCell), fy(fx + S::kFx) {}
 };
 
 // One face of a tile: faces 0 .. NFX-1 have an x normal, the rest a y normal.
@@ -439,13 +438,7 @@ __device__ __forceinline__ void update_cells(const Params& P, const OUT& out, in
     res.nbad = nbad;
 }
 
-// One TX x TY tile whose lower-left cell is (tx0, ty0).  Reads `in`, writes `out`, returns
-// the per-thread wave-speed maxima and counters.  Every thread of the block must call it.
-// `aux` (may be null): per cell, the flux differences d[0..3] of the update, planes of N*M
-// (the adjoint's recording).
-// Not inlined: the single-grid kernel and the persistent batch kernel call one compiled
-// function per tile shape, so a grid's arithmetic, and its bits, do not depend on which
-// schedule advanced it (inlined into each, the compiler may fuse the two differently).
+// The tangent's tile: slopes in shared memory, faces in floating point on Dual values.
 template <class T, int ORDER, int TX, int TY, int NT, class IN, class OUT>
 __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT& out, int tx0,
                                         int ty0, double T_do, int dt_only, T* smem,
@@ -533,179 +526,125 @@ __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT
     res.umax_y = fastest.y;
 }
 
-// ---- The same tile with its face work in 64-bit integers --------------------------------------
+// ---- The step's tile: face work in 64-bit integers --------------------------------------------
 //
-// The cells of the tile and its halo are held as integers in units of one power of two for the
-// densities, one for the pressures and one for the velocities (fx::Tops), taken from the tile's
-// own largest values.  Slopes, minmod and face states are then plain 64-bit adds and selects, and
-// the HLLC flux is fx::hllc: the FP64 pipe is left with the conversion of the fluxes and the
-// update (about 40 instructions a cell instead of 103).
+// The cells of the tile and its halo are held as significands and exponents (gd_fixed.cuh); a face
+// shifts its stencil to units of its own.  Slopes, minmod and face states are then plain 64-bit
+// adds and selects, and the HLLC flux is fx::hllc: the FP64 pipe is left with the conversion of
+// the fluxes and the update (about 40 instructions a cell instead of 103).
 
-// The faces of a thread that the integer solver left (bit k: the k-th), in floating point.  Out of
-// line, and after the loop over the faces: a second solver inside it would take registers from
-// every face for what a few need.  speed: the faces whose wave speed is missing too.
+// One compiled body for every kernel, so that a face left to floating point has the same bits
+// whichever kernel solves it.
+__device__ __noinline__ FluxE<double> float_flux(const Params& P, const double* qa,
+                                                 const double* qb, double& UU) {
+    return flux_of(P, qa, qb, UU);
+}
+
+// The faces of a thread that the integer solver left (bit k: the k-th), in floating point from the
+// cells themselves.  Out of line, and after the loop over the faces: a second solver inside it
+// would take registers from every face for what a few need.  speed: the faces whose wave speed is
+// missing too.
 template <int ORDER, int TX, int TY, int NT>
-__device__ __noinline__ void faces_left(const Params& P, double* smem, const fx::Tops& X, int tx0,
+__device__ __noinline__ void faces_left(const Params& P, const CPlanes& in, double* smem, int tx0,
                                         int ty0, unsigned int left, unsigned int speed,
                                         Speeds& u) {
-    using S = Shape<ORDER, TX, TY>;
     const TileMemInt<ORDER, TX, TY> t(smem);
     while (left) {
         const int k = __ffs((int)left) - 1;
         left &= left - 1;
         const Face<TX, TY> w(P, tx0, ty0, threadIdx.x + k * NT);
-        const int st = w.isx ? 1 : S::SX;
-        double qa[NF], qb[NF], UU;
+        const int gx = tx0 + w.lx, gy = ty0 + w.ly, sx = w.isx ? 1 : 0, sy = w.isx ? 0 : 1;
+        double c[4][NF], qa[NF], qb[NF], UU;
+        load_cell(P, in, gx - sx, gy - sy, c[1]);
+        load_cell(P, in, gx, gy, c[2]);
+        if (ORDER == 2) {
+            load_cell(P, in, gx - 2 * sx, gy - 2 * sy, c[0]);
+            load_cell(P, in, gx + sx, gy + sy, c[3]);
+        }
+#pragma unroll
         for (int f = 0; f < NF; ++f) {
-            const int g = f < 2 ? f : (w.isx ? f : 5 - f);
-            const int ue = (f == 0 ? X.r : (f == 1 ? X.p : X.v)) - 60;
-            const fx::i64* q = t.q + (g * S::SY + w.ly + S::H) * S::SX + w.lx + S::H;
-            const double ca = fx::to_double(q[-st], ue), cb = fx::to_double(q[0], ue);
-            qa[f] = ca;
-            qb[f] = cb;
+            qa[f] = c[1][f];
+            qb[f] = c[2][f];
             if (ORDER == 2) {
-                const double d = cb - ca;
-                side_states(f, ca, minmod(ca - fx::to_double(q[-2 * st], ue), d), cb,
-                            minmod(d, fx::to_double(q[st], ue) - cb), qa[f], qb[f]);
+                const double d = qb[f] - qa[f];
+                side_states(f, qa[f], minmod(qa[f] - c[0][f], d), qb[f],
+                            minmod(d, c[3][f] - qb[f]), qa[f], qb[f]);
             }
         }
-        const FluxE<double> F = flux_of(P, qa, qb, UU);
+        const double la[NF] = {qa[0], qa[1], w.isx ? qa[2] : qa[3], w.isx ? qa[3] : qa[2]};
+        const double lb[NF] = {qb[0], qb[1], w.isx ? qb[2] : qb[3], w.isx ? qb[3] : qb[2]};
+        const FluxE<double> F = float_flux(P, la, lb, UU);
         w.store(t.fx, t.fy, F.m, F.e, F.mn, F.mt);
         if (speed & (1u << k)) u.take(w.isx, UU);
     }
 }
 
-// Every face of a tile held in integers.  dt_only: the wave speeds alone.
+// Every face of a tile.  dt_only: the wave speeds alone.
 template <bool HLL, int ORDER, int TX, int TY, int NT>
-__device__ __forceinline__ void faces_int(const Params& P, double* smem, const fx::Tops& X,
-                                           int tx0, int ty0, int dt_only, Speeds& u) {
+__device__ __forceinline__ void faces(const Params& P, const CPlanes& in, double* smem, int tx0,
+                                      int ty0, int dt_only, Speeds& u) {
     using S = Shape<ORDER, TX, TY>;
     using fx::i64;
-    constexpr int FS = S::SY * S::SX;
     const TileMemInt<ORDER, TX, TY> t(smem);
     unsigned int left = 0, speed = 0, bit = 1;
     for (int i = threadIdx.x; i < Face<TX, TY>::NFX + Face<TX, TY>::NFY; i += NT, bit <<= 1) {
         const Face<TX, TY> w(P, tx0, ty0, i);
         if (!w.used) continue;
-        const int st = w.isx ? 1 : S::SX;
-        const i64* q = t.q + (w.ly + S::H) * S::SX + w.lx + S::H;
+        const int c = (w.ly + S::H) * S::SX + w.lx + S::H, st = w.isx ? 1 : S::SX;
         i64 a[NF], b[NF];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            const i64* p = q + (f < 2 ? f * FS : (w.isx ? f : 5 - f) * FS);
-            const i64 ca = p[-st], cb = p[0];
-            a[f] = 2 * ca;
-            b[f] = 2 * cb;
-            if (ORDER == 2) {  // between the cell and the middle to its neighbour: rho, p > 0
-                const i64 d = cb - ca;
-                a[f] += fx::minmod(ca - p[-2 * st], d);
-                b[f] -= fx::minmod(d, p[st] - cb);
-            }
-        }
-        const fx::States s{a[0], b[0], a[1], b[1], a[2], b[2], a[3], b[3]};
-        double UU;
-        const fx::Fan fan = fx::fan_of<HLL>(s, X, P.gas, UU);
-        if (!fan.ok) {
-            left |= bit;
-            speed |= bit;
-            continue;
-        }
-        u.take(w.isx, UU);
-        if (dt_only) continue;
-        double m, mn, mt, e;
-        const bool done = HLL ? fx::hll(fan, s, X, P.gas, m, mn, mt, e)
-                              : fx::hllc(fan, s, X, P.gas, m, mn, mt, e);
-        if (done) w.store(t.fx, t.fy, m, e, mn, mt);
-        else left |= bit;
+        int top[NF];
+        double F[NF], UU;
+        bool speed_ok = false, done = false;
+        if (P.gas.room >= 0 && fx::face_states<NF, ORDER>(t.q + c, st, S::SY * S::SX, t.key + c, st,
+                                                          w.isx, a, b, top))
+            done = fx::euler_flux<HLL>(a, b, top, P.gas, F, UU, speed_ok, dt_only);
+        if (speed_ok) u.take(w.isx, UU);
+        else speed |= bit;
+        if (!done) left |= bit;
+        else if (!dt_only) w.store(t.fx, t.fy, F[0], F[3], F[1], F[2]);
     }
-    if (left) faces_left<ORDER, TX, TY, NT>(P, smem, X, tx0, ty0, left, speed, u);
+    if (left) faces_left<ORDER, TX, TY, NT>(P, in, smem, tx0, ty0, left, speed, u);
 }
 
-// Returns false, with nothing written, where the tile's cells cannot be held in common units.
-// Every thread of the block must call it, and all get the same answer.  METHODS: 1 HLLC, 2 HLL, 3
-// the one of P (both solvers in the function).
+// One TX x TY tile of the step whose lower-left cell is (tx0, ty0).  Reads `in`, writes `out`,
+// returns the per-thread wave-speed maxima and counters.  Every thread of the block must call it.
+// `aux` (may be null): per cell, the flux differences d[0..3] of the update, planes of N*M
+// (the adjoint's recording).  METHODS: 1 HLLC, 2 HLL, 3 the one of P (both solvers in the
+// function).
 template <int METHODS, int ORDER, int TX, int TY, int NT>
-__device__ __forceinline__ bool euler_tile_int(const Params& P, const CPlanes& in, const Planes& out,
-                                            int tx0, int ty0, double T_do, int dt_only,
-                                            double* smem, TileResult& res, double* aux) {
+__device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, const Planes& out,
+                                          int tx0, int ty0, double T_do, int dt_only,
+                                          double* smem, TileResult& res, double* aux) {
     using S = Shape<ORDER, TX, TY>;
-    constexpr int H = S::H, SX = S::SX, SY = S::SY, NC = (SY * SX + NT - 1) / NT;
+    constexpr int H = S::H, SX = S::SX, SY = S::SY;
     const TileMemInt<ORDER, TX, TY> t(smem);
-    // keys of the tile's exponents: the largest and (negated) the smallest of rho and p, and the
-    // largest of the velocities
-    __shared__ unsigned int keys[5][NT / 32];
-    const int tid = threadIdx.x, N = P.N, M = P.M;
-
-    double v[NC][NF];
-    unsigned int key[5] = {0, 0, 0, 0, 0};
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        const int i = tid + c * NT;
+    const int N = P.N, M = P.M;
+    for (int i = threadIdx.x; i < SY * SX; i += NT) {
         const int ly = i / SX, lx = i - ly * SX;
         const bool xh = lx < H || lx >= TX + H, yh = ly < H || ly >= TY + H;
         const int gx = tx0 + lx - H, gy = ty0 + ly - H;
-        const bool some = i < SY * SX && !(xh && yh) && gx >= -2 && gx < N + 2 && gy >= -2 &&
-                          gy < M + 2 && !((gx < 0 || gx >= N) && (gy < 0 || gy >= M));
+        if ((xh && yh) || gx < -2 || gx >= N + 2 || gy < -2 || gy >= M + 2 ||
+            ((gx < 0 || gx >= N) && (gy < 0 || gy >= M)))
+            continue;  // no face reads it
+        double v[NF];
+        load_cell(P, in, gx, gy, v);
+        fx::cell_units<NF>(v, t.q + i, SY * SX, t.key[i]);
+        if (!xh && !yh) {
 #pragma unroll
-        for (int f = 0; f < NF; ++f) v[c][f] = 0.0;  // never used
-        if (some) {
-            load_cell(P, in, gx, gy, v[c]);
-            const unsigned int r = fx::signed_exp_field(v[c][0]), p = fx::signed_exp_field(v[c][1]);
-            key[0] = max(key[0], r);
-            key[1] = max(key[1], 0xfffu - r);
-            key[2] = max(key[2], p);
-            key[3] = max(key[3], 0xfffu - p);
-            key[4] = max(key[4], max(fx::exp_field(v[c][2]), fx::exp_field(v[c][3])));
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        const unsigned int m = __reduce_max_sync(0xffffffffu, key[k]);
-        if ((tid & 31) == 0) keys[k][tid >> 5] = m;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 5; ++k)
-        key[k] = __reduce_max_sync(0xffffffffu, keys[k][(tid & 31) % (NT / 32)]);
-    fx::Tops X;
-    if (!fx::tops_of(0xfffu - key[1], key[0], 0xfffu - key[3], key[2], key[4], P.gas, X))
-        return false;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        const int i = tid + c * NT;
-        if (i >= SY * SX) break;
-        const int ly = i / SX, lx = i - ly * SX;
-        const bool own = lx >= H && lx < TX + H && ly >= H && ly < TY + H;
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            t.q[f * SY * SX + i] = fx::to_units(v[c][f], f == 0 ? X.r : (f == 1 ? X.p : X.v));
-            if (own) t.cell[(f * TY + ly - H) * TX + lx - H] = v[c][f];
+            for (int f = 0; f < NF; ++f) t.cell[(f * TY + ly - H) * TX + lx - H] = v[f];
         }
     }
     __syncthreads();
     Speeds fastest{0.0, 0.0};
     if (METHODS == 2 || (METHODS == 3 && P.method == GD_METHOD_HLL))
-        faces_int<true, ORDER, TX, TY, NT>(P, smem, X, tx0, ty0, dt_only, fastest);
+        faces<true, ORDER, TX, TY, NT>(P, in, smem, tx0, ty0, dt_only, fastest);
     else
-        faces_int<false, ORDER, TX, TY, NT>(P, smem, X, tx0, ty0, dt_only, fastest);
+        faces<false, ORDER, TX, TY, NT>(P, in, smem, tx0, ty0, dt_only, fastest);
     __syncthreads();
     update_cells<double, ORDER, TX, TY, NT, TX, TX * TY>(P, out, tx0, ty0, T_do, dt_only, t.cell, t.fx,
                                                      t.fy, res, aux);
     res.umax_x = fastest.x;
     res.umax_y = fastest.y;
-    return true;
-}
-
-// A tile of the step: in integers where the tile's range allows it.
-template <int METHODS, int ORDER, int TX, int TY, int NT>
-__device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, const Planes& out,
-                                          int tx0, int ty0, double T_do, int dt_only,
-                                          double* smem, TileResult& res, double* aux) {
-    if (euler_tile_int<METHODS, ORDER, TX, TY, NT>(P, in, out, tx0, ty0, T_do, dt_only, smem, res,
-                                               aux))
-        return;
-    __syncthreads();
-    euler_tile<double, ORDER, TX, TY, NT>(P, in, out, tx0, ty0, T_do, dt_only, smem, res, aux);
 }
 
 __device__ __forceinline__ void add_counters(Scalars* ctr, const TileResult& r) {
@@ -943,11 +882,11 @@ cudaError_t prepare_euler_fast() {
     if (e == cudaSuccess)  // Dual tiles: twice the bytes of the double ones
         e = cudaFuncSetAttribute(euler_tangent_kernel<1>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(2 * Shape<1, kTanTX, kTanTY>::bytes));
+                                 (int)(Shape<1, kTanTX, kTanTY>::dual_bytes));
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(euler_tangent_kernel<2>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(2 * Shape<2, kTanTX, kTanTY>::bytes));
+                                 (int)(Shape<2, kTanTX, kTanTY>::dual_bytes));
     if (e == cudaSuccess) e = set_attrs<2, 32, 16>();
     if (e == cudaSuccess) e = set_attrs<1, 32, 8>();
     if (e == cudaSuccess) e = set_attrs<2, 32, 8>();
@@ -980,10 +919,10 @@ cudaError_t launch_euler_tangent(const Params& P, const CPlanes& in, const CPlan
                                  cudaStream_t st) {
     const dim3 grid((P.N + kTanTX - 1) / kTanTX, (P.M + kTanTY - 1) / kTanTY);
     if (P.order == 1)
-        euler_tangent_kernel<1><<<grid, kNTTan, 2 * Shape<1, kTanTX, kTanTY>::bytes, st>>>(
+        euler_tangent_kernel<1><<<grid, kNTTan, Shape<1, kTanTX, kTanTY>::dual_bytes, st>>>(
             P, in, din, out, dout, T_do);
     else
-        euler_tangent_kernel<2><<<grid, kNTTan, 2 * Shape<2, kTanTX, kTanTY>::bytes, st>>>(
+        euler_tangent_kernel<2><<<grid, kNTTan, Shape<2, kTanTX, kTanTY>::dual_bytes, st>>>(
             P, in, din, out, dout, T_do);
     return cudaGetLastError();
 }
@@ -1030,7 +969,7 @@ __global__ void euler_face_probe_kernel(Params P, long long n, int axis,
                                   : fx::euler_face<false>(qa, qb, P.gas, f, UU))
         F = FluxE<double>{f[0], f[1], f[2], f[3]};
     else
-        F = flux_of(P, qa, qb, UU);
+        F = float_flux(P, qa, qb, UU);
     double* o = flux + 4 * i;
     o[0] = F.m;
     o[1] = F.e;

@@ -342,22 +342,17 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
         if (!w.used) continue;
         double qa[NF], qb[NF], UU;
         w.states(pA, w.isx ? pDX : pDY, qa, qb);
-        fx::StatesM A, B;
-        fx::TopsM X;
-        fx::FanM fan;
-        if (fx::face_units(qa, qb, P.gas, A, B, X)) fan = fx::fan_of(A, B, X, P.gas, UU);
-        else fan.ok = false;
-        if (!fan.ok) {
-            left |= bit;
-            speed |= bit;
-            continue;
-        }
-        if (w.isx) umax_x = max_nonneg(umax_x, UU);
-        else umax_y = max_nonneg(umax_y, UU);
-        if (dt_only) continue;
+        fx::i64 a[NF], b[NF];
+        int top[NF];
         fx::FluxI F;
-        if (fx::mhd_flux<true>(fan, A, B, X, P.gas, F)) w.store(fx, fy, F);
-        else left |= bit;
+        bool speed_ok = false, done = false;
+        if (fx::face_units(qa, qb, P.gas, a, b, top))
+            done = fx::mhd_face_flux<true>(a, b, top, P.gas, F, UU, speed_ok, dt_only);
+        if (!speed_ok) speed |= bit;
+        else if (w.isx) umax_x = max_nonneg(umax_x, UU);
+        else umax_y = max_nonneg(umax_y, UU);
+        if (!done) left |= bit;
+        else if (!dt_only) w.store(fx, fy, F);
     }
     if (left) faces_left(P, smem, flag, left, speed, umax_x, umax_y);
     __syncthreads();

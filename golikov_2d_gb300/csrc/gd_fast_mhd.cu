@@ -2,12 +2,12 @@
 // MHD, face-once tiles (same phase structure as gd_fast_euler.cu: load, slopes, faces,
 // update), and its forward-mode tangent.
 //
-// Two bodies of a tile, as in gd_fast_euler.cu.  mhd_tile_int runs slopes and faces in scaled
-// 64-bit integers (gd_fixed_mhd.cuh), where the tile's densities, pressures and fields allow:
-// 91 FP64 operations per cell against 448, one HLLD step at 1024^2 0.37 against 0.98 ms.
-// mhd_tile is the FP64 body for the other tiles; it and its flux are templates on the scalar
-// type, and `Dual` (gd_dual.cuh) gives the tangent (JVP), with the dt held fixed and
-// derivatives taken along the branches the values take.
+// The step's slopes and faces run in scaled 64-bit integers (gd_fixed_mhd.cuh), as in
+// gd_fast_euler.cu: 91 FP64 operations per cell against 448.  A face whose states or fan leave the
+// integers' range is solved in FP64 from the cells themselves.  The tangent's tile is floating
+// point throughout; it and the flux are templates on the scalar type, and `Dual` (gd_dual.cuh)
+// gives the tangent (JVP), with the dt held fixed and derivatives taken along the branches the
+// values take.
 //
 // Field units.  The reference stores Gaussian B and divides by sqrt(4 pi) inside every flux
 // call (Gas_Dinamic.cu:970-976), multiplying the field fluxes back (:1497-1499).  Here the
@@ -116,27 +116,34 @@ __device__ __forceinline__ void copy_cell(const DualCPlanes& in, const DualPlane
     }
 }
 
-// SLOPES: slope arrays beside the cells; without them each face forms its cells' slopes.
-template <class T, int ORDER, int TY, bool SLOPES = true>
+// The tangent's tile.
+template <class T, int ORDER, int TY>
 struct SmemM {
     static constexpr int H = ORDER == 2 ? 2 : 1;
     static constexpr int SX = TX + 2 * H;
     static constexpr int SY = TY + 2 * H;
     static constexpr int kPrim = NF * SY * SX;
-    static constexpr int kSlx = ORDER == 2 && SLOPES ? NF * TY * (TX + 2) : 0;
-    static constexpr int kSly = ORDER == 2 && SLOPES ? NF * (TY + 2) * TX : 0;
+    static constexpr int kSlx = ORDER == 2 ? NF * TY * (TX + 2) : 0;
+    static constexpr int kSly = ORDER == 2 ? NF * (TY + 2) * TX : 0;
     static constexpr int kFx = NF * TY * (TX + 1);
     static constexpr int kFy = NF * (TY + 1) * TX;
-    static constexpr int kCell = NF * TX * TY;
     static constexpr size_t bytes = sizeof(T) * (kPrim + kSlx + kSly + kFx + kFy);
 };
-// The step's tile in integers: no slopes, the cells' own values beside them.  Its float tile (for
-// ranges the integers cannot hold) works without slope arrays, in the same room.
+// The step's tile: the cells' significands and keys (gd_fixed.cuh), the tile's own values, and
+// b_x beside the tile in x and b_y in y.
 template <int ORDER, int TY>
-constexpr size_t step_bytes() {
-    using I = SmemM<double, ORDER, TY, false>;
-    return I::bytes + sizeof(double) * I::kCell;
-}
+struct ShapeInt {
+    static constexpr int H = ORDER == 2 ? 2 : 1;
+    static constexpr int SX = TX + 2 * H;
+    static constexpr int SY = TY + 2 * H;
+    static constexpr int kKey = 2 * SY * SX;
+    static constexpr int kPrim = NF * SY * SX;
+    static constexpr int kCell = NF * TX * TY;
+    static constexpr int kEdge = 2 * (TX + TY);
+    static constexpr int kFx = NF * TY * (TX + 1);
+    static constexpr int kFy = NF * (TY + 1) * TX;
+    static constexpr size_t bytes = sizeof(double) * (kKey + kPrim + kCell + kEdge + kFx + kFy);
+};
 
 struct MhdTileResult {
     double umax_x, umax_y;
@@ -215,7 +222,8 @@ __device__ __forceinline__ void side_states(int f, T ca, T da, T cb, T db, T& a,
 
 // ---- U: update (kernel.cu:2606-2660 in Heaviside-Lorentz field units) --------------------------
 // cell: the tile's own values, rows RS and fields FS apart; jump: b_x across a cell in x and b_y
-// in y, from its neighbours.
+// in y, from its neighbours.  `aux` (T = double only; may be null) receives, per cell, the flux
+// differences d[0..6] and the Powell term divb that the update used (planes of N*M), for the adjoint.
 template <class T, int BT, int TY, int RS, int FS, class IN, class OUT, class JUMP>
 __device__ __forceinline__ void update_cells(const Params& P, const IN& in, const OUT& out, int tx0,
                                              int ty0, double T_do, int dt_only, const T* cell,
@@ -316,16 +324,14 @@ struct JumpFloat {
     }
 };
 
-// One TX x TY tile at (tx0, ty0): load, slopes, faces, update.  IN/OUT are CPlanes/Planes
-// for T = double and DualCPlanes/DualPlanes for T = Dual.
+// The tangent's TX x TY tile at (tx0, ty0): load, slopes, faces, update, with IN/OUT
+// DualCPlanes/DualPlanes for T = Dual.
 // flux component slots in smem: 0 mass, 1 energy, 2 mom x, 3 mom y, 4 bx, 5 by, 6 bz
-// `aux` (T = double only; may be null) receives, per cell, the flux differences d[0..6]
-// and the Powell term divb that the update used (planes of N*M), for the adjoint.
-template <class T, int BT, int ORDER, int TY, bool SLOPES, class IN, class OUT>
+template <class T, int BT, int ORDER, int TY, class IN, class OUT>
 __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& out, int tx0,
                                          int ty0, double T_do, int dt_only, T* smem,
                                          MhdTileResult& res, double* aux) {
-    using S = SmemM<T, ORDER, TY, SLOPES>;
+    using S = SmemM<T, ORDER, TY>;
     constexpr int H = S::H, SX = S::SX, SY = S::SY;
     T* prim = smem;
     T* slx = prim + S::kPrim;
@@ -360,7 +366,7 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
 
     // ---- S: slopes ---------------------------------------------------------------------------
     // a thread takes a run of G cells, so neighbouring slopes share their difference
-    if constexpr (ORDER == 2 && SLOPES) {
+    if constexpr (ORDER == 2) {
         constexpr int GX = (TX + 2) % 3 == 0 ? 3 : 2, GY = (TY + 2) % 3 == 0 ? 3 : 2;
         constexpr int NGX = (TX + 2) / GX, NGY = (TY + 2) / GY;
         static_assert((TX + 2) % GX == 0 && (TY + 2) % GY == 0, "slope runs tile the rows");
@@ -415,12 +421,7 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
             qb[f] = pb[g * SY * SX];
             if (ORDER == 2) {
                 T da, db;
-                if (!SLOPES) {
-                    const int st = w.isx ? 1 : SX;
-                    const T *ga = pa + g * SY * SX, *gb = pb + g * SY * SX, d = gb[0] - ga[0];
-                    da = minmod(ga[0] - ga[-st], d);
-                    db = minmod(d, gb[st] - gb[0]);
-                } else if (w.isx) {
+                if (w.isx) {
                     da = slx[(g * TY + ly) * (TX + 2) + lx];
                     db = slx[(g * TY + ly) * (TX + 2) + lx + 1];
                 } else {
@@ -442,135 +443,118 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
     res.umax_y = u.y;
 }
 
-// ---- The same tile with its face work in 64-bit integers --------------------------------------
+// ---- The step's tile: face work in 64-bit integers --------------------------------------------
 //
 // HLLD takes about 150 binary64 operations a face; on the FP64 pipe, at 64 cycles of a sub-
 // partition each, they held the tile to 35 000 cycles per 32 cells.  Here the cells of the tile
-// and its halo are integers in units of the tile's own largest density, pressure, velocity and
-// field (fx::TopsM), slopes and face states are adds and selects, and the flux is fx::mhd_flux.  The
-// FP64 pipe keeps the conversion of the fluxes and the update.
+// and its halo are significands and exponents (gd_fixed.cuh), a face shifts its stencil to units of
+// its own, slopes and face states are adds and selects, and the flux is fx::mhd_flux.  The FP64 pipe
+// keeps the conversion of the fluxes and the update.
 template <int ORDER, int TY>
 struct MemInt {
-    using S = SmemM<double, ORDER, TY, false>;
+    using S = ShapeInt<ORDER, TY>;
+    using Key = fx::Keys<NF>;
+    static_assert(sizeof(Key) == 2 * sizeof(double), "keys take two doubles a cell");
+    Key* key;      // [SY][SX]
     fx::i64* q;    // [NF][SY][SX]
     double* cell;  // [NF][TY][TX]
+    double* edgex;  // [2][TY]  b_x of the cells at x = -1 and TX
+    double* edgey;  // [2][TX]  b_y of the cells at y = -1 and TY
     double *fx, *fy;
     __device__ explicit MemInt(double* smem)
-        : q(reinterpret_cast<fx::i64*>(smem)), cell(smem + S::kPrim), fx(cell + S::kCell),
-          fy(fx + S::kFx) {}
+        : key(reinterpret_cast<Key*>(smem)), q(reinterpret_cast<fx::i64*>(smem + S::kKey)),
+          cell(smem + S::kKey + S::kPrim), edgex(cell + S::kCell), edgey(edgex + 2 * TY),
+          fx(edgey + 2 * TX), fy(fx + S::kFx) {}
 };
 
-// The faces of a thread that the integer solver left (bit k: the k-th), in floating point; speed:
-// those whose wave speed is missing too.  Out of line and after the loop over the faces, so that
-// it takes no registers from it.
+// One compiled body for every kernel, so that a face left to floating point has the same bits
+// whichever kernel solves it.
+__device__ __noinline__ FluxM<double> float_flux_of(const Params& P, const double* qa,
+                                                    const double* qb, double& UU) {
+    return float_flux(P, qa, qb, UU);
+}
+__device__ __forceinline__ void load_cell(const Params& P, const CPlanes& in, int gx, int gy,
+                                          double* v) {
+    load_state(P, in, gx, gy, v);
+#pragma unroll
+    for (int f = 4; f < NF; ++f) v[f] = __dmul_rn(v[f], kInvSpi4);
+}
+
+// The faces of a thread that the integer solver left (bit k: the k-th), in floating point from the
+// cells themselves; speed: those whose wave speed is missing too.  Out of line and after the loop
+// over the faces, so that it takes no registers from it.
 template <int ORDER, int TY, int NT>
-__device__ __noinline__ void faces_left(const Params& P, double* smem, const fx::TopsM& X, int tx0,
+__device__ __noinline__ void faces_left(const Params& P, const CPlanes& in, double* smem, int tx0,
                                         int ty0, unsigned int left, unsigned int speed,
                                         SpeedsM& u) {
-    using S = SmemM<double, ORDER, TY, false>;
     const MemInt<ORDER, TY> t(smem);
     while (left) {
         const int k = __ffs((int)left) - 1;
         left &= left - 1;
         const FaceM<TY> w(P, tx0, ty0, threadIdx.x + k * NT);
-        const int st = w.isx ? 1 : S::SX;
-        double qa[NF], qb[NF], UU;
-#pragma unroll 1
-        for (int f = 0; f < NF; ++f) {
-            const int ue = (f == 0 ? X.r : (f == 1 ? X.p : (f < 4 ? X.v : X.b))) - 60;
-            const fx::i64* q = t.q + (w.field(f) * S::SY + w.ly + S::H) * S::SX + w.lx + S::H;
-            const double ca = fx::to_double(q[-st], ue), cb = fx::to_double(q[0], ue);
-            qa[f] = ca;
-            qb[f] = cb;
-            if (ORDER == 2) {
-                const double d = cb - ca;
-                side_states(f, ca, minmod(ca - fx::to_double(q[-2 * st], ue), d), cb,
-                            minmod(d, fx::to_double(q[st], ue) - cb), qa[f], qb[f]);
-            }
+        const int gx = tx0 + w.lx, gy = ty0 + w.ly, sx = w.isx ? 1 : 0, sy = w.isx ? 0 : 1;
+        double c[4][NF], qa[NF], qb[NF], UU;
+        load_cell(P, in, gx - sx, gy - sy, c[1]);
+        load_cell(P, in, gx, gy, c[2]);
+        if (ORDER == 2) {
+            load_cell(P, in, gx - 2 * sx, gy - 2 * sy, c[0]);
+            load_cell(P, in, gx + sx, gy + sy, c[3]);
         }
-        w.store(t.fx, t.fy, float_flux(P, qa, qb, UU));
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            double a = c[1][f], b = c[2][f];
+            if (ORDER == 2) {
+                const double d = b - a;
+                side_states(f, a, minmod(a - c[0][f], d), b, minmod(d, c[3][f] - b), a, b);
+            }
+            qa[w.field(f)] = a;  // the swap is its own inverse
+            qb[w.field(f)] = b;
+        }
+        w.store(t.fx, t.fy, float_flux_of(P, qa, qb, UU));
         if (speed & (1u << k)) u.take(w.isx, UU);
     }
 }
 
-template <int SX, int FS>
-struct JumpInt {
-    const fx::i64* own;
-    int ue;
+template <int TY>
+struct JumpCells {
+    const double *cell, *edgex, *edgey;
     __device__ __forceinline__ double x(int lx, int ly) const {
-        const fx::i64* c = own + 4 * FS + ly * SX + lx;
-        return fx::to_double(c[1] - c[-1], ue);
+        const double* c = cell + 4 * TX * TY + ly * TX + lx;
+        return (lx < TX - 1 ? c[1] : edgex[TY + ly]) - (lx > 0 ? c[-1] : edgex[ly]);
     }
     __device__ __forceinline__ double y(int lx, int ly) const {
-        const fx::i64* c = own + 5 * FS + ly * SX + lx;
-        return fx::to_double(c[SX] - c[-SX], ue);
+        const double* c = cell + 5 * TX * TY + ly * TX + lx;
+        return (ly < TY - 1 ? c[TX] : edgey[TX + lx]) - (ly > 0 ? c[-TX] : edgey[lx]);
     }
 };
 
-// Returns false, with nothing written, where the tile's cells cannot be held in common units.
-// Every thread of the block must call it, and all get the same answer.
+// One tile of the step.  Every thread of the block must call it.
 template <bool HLLD, int ORDER, int TY, int NT>
-__device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in, const Planes& out,
-                                             int tx0, int ty0, double T_do, int dt_only,
-                                             double* smem, MhdTileResult& res, double* aux) {
-    using S = SmemM<double, ORDER, TY, false>;
+__device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, const Planes& out,
+                                          int tx0, int ty0, double T_do, int dt_only,
+                                          double* smem, MhdTileResult& res, double* aux) {
+    using S = ShapeInt<ORDER, TY>;
     using fx::i64;
-    constexpr int H = S::H, SX = S::SX, SY = S::SY, FS = SY * SX, NC = (FS + NT - 1) / NT;
+    constexpr int H = S::H, SX = S::SX, SY = S::SY, FS = SY * SX;
     const MemInt<ORDER, TY> t(smem);
-    // the largest and (negated) the smallest exponents of rho and p, the largest of v and b
-    constexpr int NK = 6;
-    __shared__ unsigned int keys[NK][NT / 32];
     const int tid = threadIdx.x, N = P.N, M = P.M;
-
-    double v[NC][NF];
-    unsigned int key[NK] = {0, 0, 0, 0, 0, 0};
+    for (int i = tid; i < FS; i += NT) {
+        const int ly = i / SX - H, lx = i % SX - H;
+        const bool xh = lx < 0 || lx >= TX, yh = ly < 0 || ly >= TY;
+        const int gx = tx0 + lx, gy = ty0 + ly;
+        if ((xh && yh) || gx < -2 || gx >= N + 2 || gy < -2 || gy >= M + 2 ||
+            ((gx < 0 || gx >= N) && (gy < 0 || gy >= M)))
+            continue;  // no face reads it
+        double v[NF];
+        load_cell(P, in, gx, gy, v);
+        fx::cell_units<NF>(v, t.q + i, FS, t.key[i]);
+        if (!xh && !yh) {
 #pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        const int i = tid + c * NT;
-        const int ly = i / SX, lx = i - ly * SX;
-        const bool xh = lx < H || lx >= TX + H, yh = ly < H || ly >= TY + H;
-        const int gx = tx0 + lx - H, gy = ty0 + ly - H;
-        const bool some = i < FS && !(xh && yh) && gx >= -2 && gx < N + 2 && gy >= -2 &&
-                          gy < M + 2 && !((gx < 0 || gx >= N) && (gy < 0 || gy >= M));
-#pragma unroll
-        for (int f = 0; f < NF; ++f) v[c][f] = 0.0;  // never used
-        if (some) {
-            load_state(P, in, gx, gy, v[c]);
-#pragma unroll
-            for (int f = 4; f < NF; ++f) v[c][f] = __dmul_rn(v[c][f], kInvSpi4);
-            const unsigned int r = fx::signed_exp_field(v[c][0]), p = fx::signed_exp_field(v[c][1]);
-            key[0] = max(key[0], r);
-            key[1] = max(key[1], 0xfffu - r);
-            key[2] = max(key[2], p);
-            key[3] = max(key[3], 0xfffu - p);
-            key[4] = max(key[4], max(fx::exp_field(v[c][2]), fx::exp_field(v[c][3])));
-#pragma unroll
-            for (int f = 4; f < NF; ++f) key[5] = max(key[5], fx::exp_field(v[c][f]));
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < NK; ++k) {
-        const unsigned int m = __reduce_max_sync(0xffffffffu, key[k]);
-        if ((tid & 31) == 0) keys[k][tid >> 5] = m;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < NK; ++k)
-        key[k] = __reduce_max_sync(0xffffffffu, keys[k][(tid & 31) % (NT / 32)]);
-    fx::TopsM X;
-    if (!fx::tops_of(0xfffu - key[1], key[0], 0xfffu - key[3], key[2], key[4], key[5], P.gas, X))
-        return false;
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        const int i = tid + c * NT;
-        if (i >= FS) break;
-        const int ly = i / SX, lx = i - ly * SX;
-        const bool own = lx >= H && lx < TX + H && ly >= H && ly < TY + H;
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            t.q[f * FS + i] =
-                fx::to_units(v[c][f], f == 0 ? X.r : (f == 1 ? X.p : (f < 4 ? X.v : X.b)));
-            if (own) t.cell[(f * TY + ly - H) * TX + lx - H] = v[c][f];
+            for (int f = 0; f < NF; ++f) t.cell[(f * TY + ly) * TX + lx] = v[f];
+        } else if (lx == -1 || lx == TX) {
+            t.edgex[(lx == TX ? TY : 0) + ly] = v[4];
+        } else if (ly == -1 || ly == TY) {
+            t.edgey[(ly == TY ? TX : 0) + lx] = v[5];
         }
     }
     __syncthreads();
@@ -580,47 +564,29 @@ __device__ __forceinline__ bool mhd_tile_int(const Params& P, const CPlanes& in,
     for (int i = tid; i < FaceM<TY>::NFX + FaceM<TY>::NFY; i += NT, bit <<= 1) {
         const FaceM<TY> w(P, tx0, ty0, i);
         if (!w.used) continue;
-        const int st = w.isx ? 1 : SX;
-        const i64* q = t.q + (w.ly + H) * SX + w.lx + H;
+        const int c = (w.ly + H) * SX + w.lx + H, st = w.isx ? 1 : SX;
         i64 a[NF], b[NF];
-#pragma unroll
-        for (int f = 0; f < NF; ++f) {
-            const i64* p = q + w.field(f) * FS;
-            const i64 ca = p[-st], cb = p[0];
-            a[f] = 2 * ca;
-            b[f] = 2 * cb;
-            if (ORDER == 2) {  // between the cell and the middle to its neighbour: rho, p > 0
-                const i64 d = cb - ca;
-                a[f] += fx::minmod(ca - p[-2 * st], d);
-                b[f] -= fx::minmod(d, p[st] - cb);
-            }
-        }
-        const fx::StatesM A{a[0], a[1], a[2], a[3], a[4], a[5], a[6]};
-        const fx::StatesM B{b[0], b[1], b[2], b[3], b[4], b[5], b[6]};
+        int top[NF];
         double UU;
-        const fx::FanM fan = fx::fan_of(A, B, X, P.gas, UU);
-        if (!fan.ok) {
-            left |= bit;
-            speed |= bit;
-            continue;
-        }
-        u.take(w.isx, UU);
-        if (dt_only) continue;
         fx::FluxI F;
-        if (fx::mhd_flux<HLLD>(fan, A, B, X, P.gas, F))
+        bool speed_ok = false, done = false;
+        if (P.gas.room >= 0 &&
+            fx::face_states<NF, ORDER>(t.q + c, st, FS, t.key + c, st, w.isx, a, b, top))
+            done = fx::mhd_face_flux<HLLD>(a, b, top, P.gas, F, UU, speed_ok, dt_only);
+        if (speed_ok) u.take(w.isx, UU);
+        else speed |= bit;
+        if (!done) left |= bit;
+        else if (!dt_only)
             w.store(t.fx, t.fy, FluxM<double>{F.m, F.mn, F.mt, F.e, F.bn, F.bt, F.bz});
-        else
-            left |= bit;
     }
-    if (left) faces_left<ORDER, TY, NT>(P, smem, X, tx0, ty0, left, speed, u);
+    if (left) faces_left<ORDER, TY, NT>(P, in, smem, tx0, ty0, left, speed, u);
     __syncthreads();
 
     update_cells<double, NT, TY, TX, TX * TY>(P, in, out, tx0, ty0, T_do, dt_only, t.cell,
-                                          JumpInt<SX, FS>{t.q + H * SX + H, X.b - 60}, t.fx, t.fy,
+                                          JumpCells<TY>{t.cell, t.edgex, t.edgey}, t.fx, t.fy,
                                           res, aux);
     res.umax_x = u.x;
     res.umax_y = u.y;
-    return true;
 }
 
 template <int ORDER, int TY, bool HLLD, int NT>
@@ -632,13 +598,8 @@ __global__ void __launch_bounds__(NT, NT == kNT ? 2 : 1) mhd_fast_kernel(const _
                                                       Scalars* ctr, int dt_only, double* aux) {
     extern __shared__ __align__(16) double smem[];
     MhdTileResult r;
-    const int tx0 = blockIdx.x * TX, ty0 = (blockIdx.y + P.tile_row0) * TY;
-    const double T_do = *T_do_ptr;
-    // in integers where the tile's range allows it
-    if (!mhd_tile_int<HLLD, ORDER, TY, NT>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux)) {
-        __syncthreads();
-        mhd_tile<double, NT, ORDER, TY, false>(P, in, out, tx0, ty0, T_do, dt_only, smem, r, aux);
-    }
+    step_tile<HLLD, ORDER, TY, NT>(P, in, out, blockIdx.x * TX, (blockIdx.y + P.tile_row0) * TY,
+                                   *T_do_ptr, dt_only, smem, r, aux);
     if (ctr != nullptr && (r.nfl_r | r.nfl_p | r.nbad)) {
         if (r.nfl_r) atomicAdd(&ctr->rho_floor, (unsigned long long)r.nfl_r);
         if (r.nfl_p) atomicAdd(&ctr->p_floor, (unsigned long long)r.nfl_p);
@@ -657,7 +618,7 @@ __global__ void __launch_bounds__(NTDual) mhd_tangent_kernel(const __grid_consta
     MhdTileResult r;
     const DualCPlanes I{in, din};
     const DualPlanes O{out, dout};
-    mhd_tile<Dual, NTDual, ORDER, TY, true>(P, I, O, blockIdx.x * TX, blockIdx.y * TY, *T_do_ptr, 0,
+    mhd_tile<Dual, NTDual, ORDER, TY>(P, I, O, blockIdx.x * TX, blockIdx.y * TY, *T_do_ptr, 0,
                               reinterpret_cast<Dual*>(smem), r, nullptr);
 }
 
@@ -673,7 +634,7 @@ template <int ORDER, int NT>
 void launch_tiles(const Params& P, dim3 grid, const CPlanes& in, const Planes& out,
                   const double* T_do, unsigned long long* T_bits, Scalars* rot, Scalars* ctr,
                   int dt_only, cudaStream_t st, double* aux) {
-    constexpr size_t n = step_bytes<ORDER, kTY>();
+    constexpr size_t n = ShapeInt<ORDER, kTY>::bytes;
     if (P.method == GD_METHOD_HLLD)
         mhd_fast_kernel<ORDER, kTY, true, NT><<<grid, NT, n, st>>>(P, in, out, T_do, T_bits, rot,
                                                                    ctr, dt_only, aux);
@@ -706,7 +667,7 @@ cudaError_t launch_tangent_t(const Params& P, const CPlanes& in, const CPlanes& 
 
 template <int ORDER, bool HLLD>
 cudaError_t set_room() {
-    constexpr int n = (int)step_bytes<ORDER, kTY>();
+    constexpr int n = (int)ShapeInt<ORDER, kTY>::bytes;
     constexpr auto what = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(mhd_fast_kernel<ORDER, kTY, HLLD, kNT>, what, n);
     if (e == cudaSuccess)
@@ -794,7 +755,7 @@ __global__ void mhd_face_probe_kernel(Params P, long long n, int axis,
                                    : fx::mhd_face<false>(la, lb, P.gas, G, UU))
         F = FluxM<double>{G.m, G.mn, G.mt, G.e, G.bn, G.bt, G.bz};
     else
-        F = float_flux(P, la, lb, UU);
+        F = float_flux_of(P, la, lb, UU);
     double* o = flux + 8 * i;
     o[0] = F.m;
     o[1] = isx ? F.mn : F.mt;

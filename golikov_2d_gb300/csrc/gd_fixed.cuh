@@ -5,10 +5,9 @@
 // 59 64-bit adds, 25 wide multiply-adds per clock and SM; all three run side by side).  A face
 // flux is a short chain of products and sums of quantities of a few known sizes, so it can be
 // formed in integers: each quantity is a signed 64-bit integer times a power of two chosen per
-// face from the exponents of its inputs (one for all velocities, one per density, ...).  A
-// sum is then one 64-bit add, a product mulk() below, and nothing is rounded to 53 bits before
-// the result is.  Units keep 57 bits or more below the face's velocity, momentum and energy
-// scales, against the 53 of a binary64 rounding.
+// face from the exponents of its cells (one per state component, one for the face's normal
+// velocities and speeds, ...).  A sum is then one 64-bit add, a product mulk() below, and nothing
+// is rounded to 53 bits before the result is.
 //
 // Host-compilable, so that the same arithmetic is checked on the CPU against 113-bit floats.
 #pragma once
@@ -213,33 +212,6 @@ inline Gas gas_of(double gamma) {
     return G;
 }
 
-// The top exponents of a set of cells: densities, pressures and velocities are held in units of
-// 2^(r - 60), 2^(p - 60) and 2^(v - 60), below 2^61 each.  Densities and pressures within 2^8 of
-// each other (kSpan) are held exactly; a velocity is cut below 2^-60 of the largest.
-struct Tops {
-    int r, p, v;
-};
-constexpr int kSpan = 8;        // exponents that the densities, and the pressures, may span
-constexpr int kRange = 128;     // exponents of densities, pressures (both signs) and velocities
-// Below 2^-300 a velocity or field that is not 0 goes to the floating-point solver: with densities
-// and fan speeds down to 2^-128 every result stays above 2^-1022.
-constexpr int kLow = 300;
-// x in units of 2^(top - 60), |x| < 2^(top + 1)
-GD_HD i64 to_units(double x, int top) {
-    uint32_t hi, lo;
-    swfp::halves(x, hi, lo);
-    const int e = (int)((hi >> 20) & 0x7ffu) - 1023;
-    const uint32_t h = (hi & 0xfffffu) | 0x100000u;
-    const i64 v = (i64)((((u64)((h << 8) | (lo >> 24)) << 32) | (lo << 8)) >> imin(top - e, 63));
-    return (int32_t)hi < 0 ? -v : v;
-}
-// x 2^ue as a double, a normal number (or 0): ue is added to the exponent field.  The same bits on
-// the host, so that what is checked there is what the kernels compute.
-GD_HD double to_double(i64 x, int ue) {
-    uint32_t hi, lo;
-    swfp::halves((double)x, hi, lo);
-    return swfp::from_halves(x == 0 ? 0u : hi + ((uint32_t)ue << 20), lo);
-}
 // 0 unless a and b have the same sign, else the one of smaller magnitude
 GD_HD i64 minmod(i64 a, i64 b) {
     const bool lt = a < b, neg = hi32(a) < 0;
@@ -247,7 +219,178 @@ GD_HD i64 minmod(i64 a, i64 b) {
     return (hi32(a) ^ hi32(b)) < 0 ? 0 : m;
 }
 
-// The two sides of a face in its local frame, in units of half those of Tops (below 2^62).
+GD_HD uint32_t rotate(uint32_t x, int n) {  // by 0 or 16 bits
+#if defined(__CUDA_ARCH__)
+    return __funnelshift_l(x, x, n);
+#else
+    return n ? x << 16 | x >> 16 : x;
+#endif
+}
+
+// ---- cells and the states of a face ------------------------------------------------------------
+//
+// A cell is held as the signed significands of its values, x = q 2^(e - 60) with q below 2^61, and
+// the exponent fields e, packed 16 bits each (Keys).  A face takes, per component, the unit
+// 2^(top - 60) from the cells of its own stencil, so that a shift is all that separates a cell from
+// the face's integers: what a face computes depends on its stencil alone, and a small component
+// beside large ones, or a quiet cell in a tile with a shock, keeps its digits.
+constexpr int kSpan = 8;     // exponents that the face's densities, and the pressures, may span
+constexpr int kRange = 128;  // exponents of densities, pressures (both signs) and velocities
+// Below 2^-300 a velocity or field that is not 0 goes to the floating-point solver: with densities
+// and fan speeds down to 2^-128 every result stays above 2^-1022.
+constexpr int kLow = 300;
+constexpr uint32_t kNoKey = 0x7ff;  // key of a value that the integers do not take
+
+// {rho, p}, {vx, vy}, {bx, by}, {bz, 0}
+template <int NF>
+struct alignas(NF == 4 ? 8 : 16) Keys {
+    static constexpr int W = NF == 4 ? 2 : 4;
+    uint32_t w[W];
+};
+// the larger and the smaller of both 16-bit halves
+GD_HD uint32_t max2(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+    return __vmaxu2(a, b);
+#else
+    const uint32_t l = (a & 0xffffu) > (b & 0xffffu) ? a : b, h = (a >> 16) > (b >> 16) ? a : b;
+    return (l & 0xffffu) | (h & 0xffff0000u);
+#endif
+}
+GD_HD uint32_t min2(uint32_t a, uint32_t b) {
+#if defined(__CUDA_ARCH__)
+    return __vminu2(a, b);
+#else
+    const uint32_t l = (a & 0xffffu) < (b & 0xffffu) ? a : b, h = (a >> 16) < (b >> 16) ? a : b;
+    return (l & 0xffffu) | (h & 0xffff0000u);
+#endif
+}
+// x / 2^n below, n any number that is not negative
+GD_HD i64 asr(i64 x, uint32_t n) {
+#if defined(__CUDA_ARCH__)
+    i64 r;
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(n));  // amounts beyond 63 act as 63
+    return r;
+#else
+    return x >> (n < 63 ? n : 63);
+#endif
+}
+// The significand and the key of a cell's value: a density or pressure (POSITIVE), or a component
+// of a vector.
+template <bool POSITIVE>
+GD_HD uint32_t cell_units(double x, i64& q) {
+    uint32_t hi, lo;
+    swfp::halves(x, hi, lo);
+    const uint32_t e = (hi >> 20) & 0x7ffu;
+    const uint32_t h = (hi & 0xfffffu) | (e ? 0x100000u : 0u);
+    const i64 m = (i64)(((u64)((h << 8) | (lo >> 24)) << 32) | (lo << 8));
+    q = (int32_t)hi < 0 ? -m : m;
+    if (POSITIVE) return (hi >> 20) - 1u < 0x7feu ? e : kNoKey;  // zeros and negatives out
+    return e >= 1023 - kLow || m == 0 ? e : kNoKey;
+}
+template <int NF>
+GD_HD void cell_units(const double* v, i64* q, int fs, Keys<NF>& k) {
+    uint32_t e[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+        e[f] = f < 2 ? cell_units<true>(v[f], q[f * fs]) : cell_units<false>(v[f], q[f * fs]);
+#pragma unroll
+    for (int w = 0; w < Keys<NF>::W; ++w) k.w[w] = e[2 * w] | (e[2 * w + 1] << 16);
+}
+// the field of the local frame's component f: x-face (n, t) = (x, y); y-face (n, t) = (y, x)
+GD_HD int face_field(int f, bool isx) {
+    return isx || f < 2 || f == 6 ? f : (f < 4 ? 5 - f : 9 - f);
+}
+
+// c + d/2 and c - d/2 of the cells on either side of a face, d the minmod slopes (ORDER 1: c), per
+// component of the face's local frame in units of 2^(top - 61), below 2^62.  q, key: the cell above
+// the face; its neighbours along the normal are st (in key: kst) apart, its fields fs.  False where
+// a cell of the stencil is out of the integers' range.
+//
+// The unit is that of the two cells beside the face, up to 3 exponents above them if the outer
+// cells are larger.  An outer cell beyond that stays as it is, at 8 times the inner cells' exponent
+// or above: its difference keeps the sign and stays the larger one, which is all minmod asks of it.
+template <int NF, int ORDER>
+GD_HD bool face_states(const i64* q, int st, int fs, const Keys<NF>* key, int kst, bool isx, i64* a,
+                       i64* b, int* top) {
+    constexpr int W = Keys<NF>::W;
+    const Keys<NF> ka = key[-kst], kb = key[0];
+    Keys<NF> k1, k2, kt;  // the outer cells, the units
+    uint32_t high = 0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+        const uint32_t m = max2(ka.w[w], kb.w[w]);
+        kt.w[w] = m;
+        if (ORDER == 2) {
+            k1.w[w] = key[-2 * kst].w[w];
+            k2.w[w] = key[kst].w[w];
+            const uint32_t o = max2(k1.w[w], k2.w[w]);
+            high = max2(high, o);
+            kt.w[w] = max2(m, min2(o, m + 0x30003u));
+        }
+        high = max2(high, m);
+    }
+    const uint32_t low = min2(ka.w[0], kb.w[0]);
+    constexpr uint32_t kH = (1023 + kRange) * 0x10001u, kL = (1023 - kRange) * 0x10001u;
+    constexpr uint32_t kS = kSpan * 0x10001u;
+    if (max2(high, kH) != kH || min2(low, kL) != kL || max2(kt.w[0] - low, kS) != kS) return false;
+    // shifts, and the units, in the local frame
+    uint32_t sa[W], sb[W], s1[W], s2[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+        uint32_t t = kt.w[w];
+        sa[w] = t - ka.w[w];
+        sb[w] = t - kb.w[w];
+        if (ORDER == 2) {
+            s1[w] = t - min2(k1.w[w], t);
+            s2[w] = t - min2(k2.w[w], t);
+        }
+        if (w == 1 || w == 2) {
+            const int r = isx ? 0 : 16;
+            t = rotate(t, r);
+            sa[w] = rotate(sa[w], r);
+            sb[w] = rotate(sb[w], r);
+            if (ORDER == 2) {
+                s1[w] = rotate(s1[w], r);
+                s2[w] = rotate(s2[w], r);
+            }
+        }
+        kt.w[w] = t;
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f) {
+        const int w = f >> 1, h = 16 * (f & 1);
+        const i64* p = q + face_field(f, isx) * fs;
+        const i64 ca = asr(p[-st], sa[w] >> h & 0xffffu), cb = asr(p[0], sb[w] >> h & 0xffffu);
+        a[f] = 2 * ca;
+        b[f] = 2 * cb;
+        if (ORDER == 2) {  // between the cell and the middle to its neighbour: rho, p > 0
+            const i64 d = cb - ca;
+            a[f] += minmod(ca - asr(p[-2 * st], s1[w] >> h & 0xffffu), d);
+            b[f] -= minmod(d, asr(p[st], s2[w] >> h & 0xffffu) - cb);
+        }
+        top[f] = (int)(kt.w[w] >> h & 0xffffu) - 1023;
+    }
+    return true;
+}
+
+// x 2^ue as a double, a normal number (or 0): ue is added to the exponent field.  The same bits on
+// the host, so that what is checked there is what the kernels compute.
+GD_HD double to_double(i64 x, int ue) {
+    uint32_t hi, lo;
+    swfp::halves((double)x, hi, lo);
+    return swfp::from_halves(x == 0 ? 0u : hi + ((uint32_t)ue << 20), lo);
+}
+// The least E >= top for which both x 2^(top - 61) and y 2^(top - 61) are below 2^(E - 1)
+GD_HD int scale_of(i64 x, i64 y, int top) {
+    const int32_t h = hi32(x), k = hi32(y);
+    return top + imax(4 - clz32((uint32_t)((h ^ (h >> 31)) | (k ^ (k >> 31)))), 0);
+}
+
+// The two sides of a face in its local frame, per component (rho, p, normal and tangential
+// velocity) in units of 2^(X - 61), below 2^62.
+struct Tops {
+    int r, p, n, t;
+};
 struct States {
     i64 rL, rR, pL, pR, uL, uR, vL, vR;
 };
@@ -281,9 +424,7 @@ GD_HD Fan fan_of(const States& q, const Tops& X, const Gas& G, double& UU) {
     const i64 wR = sqrt_over(mulk<0, 0>(f.PR.m, G.g), f.PR.e + G.ge, f.RR, kR);
     const int kmax = imax(kL, kR);
     f.kmin = imin(kL, kR);
-    const int32_t hL = hi32(q.uL), hR = hi32(q.uR);
-    const int lz = clz32((uint32_t)((hL ^ (hL >> 31)) | (hR ^ (hR >> 31))));
-    f.E = imax(kmax + 2, X.v + imax(4 - lz, 0));
+    f.E = imax(kmax + 2, scale_of(q.uL, q.uR, X.n));
     f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 8;
     if (!f.ok) return f;
     i64 cL = wL >> (f.E - 1 - kL), cR = wR >> (f.E - 1 - kR);
@@ -291,7 +432,7 @@ GD_HD Fan fan_of(const States& q, const Tops& X, const Gas& G, double& UU) {
         cL = cL > cR ? cL : cR;
         cR = cL;
     }
-    const int sh = imin(f.E - X.v, 63);
+    const int sh = imin(f.E - X.n, 63);
     f.uL = q.uL >> sh;
     f.uR = q.uR >> sh;
     const i64 aL = f.uL - cL, aR = f.uR - cR, bL = f.uL + cL, bR = f.uR + cR;
@@ -328,7 +469,7 @@ GD_HD bool hllc(const Fan& f, const States& s, const Tops& X, const Gas& G, doub
     const Pos Pk{takeL ? f.PL.m : f.PR.m, takeL ? f.PL.e : f.PR.e};
     const i64 un = takeL ? f.uL : f.uR, S = takeL ? f.SL : f.SR;
     const i64 o = takeL ? oL : oR;
-    const Pos T = signed_of(takeL ? s.vL : s.vR, X.v);
+    const Pos T = signed_of(takeL ? s.vL : s.vR, X.t);
 
     i64 qs = un;  // outside the fan the physical flux: S_M -> u, q (S - u) -> u
     if (star) {
@@ -395,7 +536,7 @@ GD_HD bool hll(const Fan& f, const States& s, const Tops& X, const Gas& G, doubl
     const i64 pR = mulk<2, 2>(b, f.PR.m >> imin(sp + 2 - f.PR.e, 63));
     Fn = to_double(mulk<2, 2>(A, f.uL) + mulk<2, 2>(B, f.uR) + pL + pR, ER + 2 * E - 60);
     const i64 TL = mulk<2, 1>(A, s.vL), TR = mulk<2, 1>(B, s.vR);
-    Ft = to_double(TL + TR, ER + E + X.v - 59);
+    Ft = to_double(TL + TR, ER + E + X.t - 59);
     // energy: p (u - D) / (gamma - 1) + p u + rho (u - D) (u^2 + v^2) / 2, units
     // 2^(ER + 3E - 62 + room)
     const i64 qL = mulk<2, 2>(a, sra(mulk<0, 0>(f.PL.m, G.gi), sp - f.PL.e - G.gie + G.room));
@@ -403,7 +544,7 @@ GD_HD bool hll(const Fan& f, const States& s, const Tops& X, const Gas& G, doubl
     const int z = clz32((uint32_t)(hi32(qL) | hi32(qR))) - 1;
     const i64 h = mulk<0, 1>(qL << z, gL) + mulk<0, 1>(qR << z, gR);
     const i64 t = mulk<1, 1>(TL, s.vL) + mulk<1, 1>(TR, s.vR);
-    const int st = 2 * (E - X.v) - 3;
+    const int st = 2 * (E - X.t) - 3;
     if (!(fits(iabs(h), z - 4) && fits(iabs(t), st))) return false;
     const i64 k = mulk<2, 2>(A, mulk<2, 2>(f.uL, f.uL)) + mulk<2, 2>(B, mulk<2, 2>(f.uR, f.uR)) +
                   mulk<3, 2>(pL, f.uL) + mulk<3, 2>(pR, f.uR) + shift(t, st);
@@ -411,52 +552,29 @@ GD_HD bool hll(const Fan& f, const States& s, const Tops& X, const Gas& G, doubl
     return true;
 }
 
-// Exponent field of x (0x7ff for infinities and NaN, 1 for subnormal numbers), and with its sign
-// bit above it.
-GD_HD uint32_t exp_field(double x) {
-    uint32_t hi, lo;
-    swfp::halves(x, hi, lo);
-    const uint32_t e = (hi >> 20) & 0x7ffu;
-    return e == 0 && ((hi << 1) | lo) != 0 ? 1u : e;
+// The flux (HLL or HLLC) and the larger wave speed of one face given by its two states, {rho, p,
+// normal, tangential velocity}; false where the integer solver does not take it.
+template <bool HLL>
+GD_HD bool euler_flux(const i64* a, const i64* b, const int* top, const Gas& G, double* F,
+                      double& UU, bool& speed, bool speed_only) {
+    const Tops X{top[0], top[1], top[2], top[3]};
+    const States s{a[0], b[0], a[1], b[1], a[2], b[2], a[3], b[3]};
+    const Fan f = fan_of<HLL>(s, X, G, UU);
+    speed = f.ok;
+    if (!f.ok) return false;
+    if (speed_only) return true;
+    return HLL ? hll(f, s, X, G, F[0], F[1], F[2], F[3]) : hllc(f, s, X, G, F[0], F[1], F[2], F[3]);
 }
-GD_HD uint32_t signed_exp_field(double x) {
-    uint32_t hi, lo;
-    swfp::halves(x, hi, lo);
-    return hi >> 20;
-}
-// Whether the largest velocity or field, of exponent field e, gives a unit: 0, or not so small
-// that a product with it could fall below the normal numbers (to_double).
-GD_HD bool unit_of(uint32_t e) { return e == 0 || (e >= 1023 - kLow && e <= 1023 + kRange); }
-// Whether cells whose densities have exponent fields (sign bit included) in [r0, r1], pressures
-// in [p0, p1] and velocities up to v1 can be held in the units of Tops.
-GD_HD bool tops_of(uint32_t r0, uint32_t r1, uint32_t p0, uint32_t p1, uint32_t v1, const Gas& G,
-                   Tops& X) {
-    const uint32_t low = 1023 - kRange, high = 1023 + kRange;
-    X.r = (int)r1 - 1023;
-    X.p = (int)p1 - 1023;
-    X.v = imax((int)v1 - 1023, -kLow);
-    return G.room >= 0 && r0 >= low && r1 <= high && r1 - r0 <= kSpan && p0 >= low &&
-           p1 <= high && p1 - p0 <= kSpan && unit_of(v1);
-}
-// The flux (HLL or HLLC) and the larger wave speed of one face given by its two states; false
-// where the integer solver does not take it.
 template <bool HLL>
 GD_HD bool euler_face(const double* L, const double* R, const Gas& G, double* F, double& UU) {
-    const uint32_t rL = signed_exp_field(L[0]), rR = signed_exp_field(R[0]);
-    const uint32_t pL = signed_exp_field(L[1]), pR = signed_exp_field(R[1]);
-    const uint32_t v0 = imax(exp_field(L[2]), exp_field(L[3]));
-    const uint32_t v1 = imax(exp_field(R[2]), exp_field(R[3]));
-    Tops X;
-    if (!tops_of(rL < rR ? rL : rR, rL < rR ? rR : rL, pL < pR ? pL : pR, pL < pR ? pR : pL,
-                 v0 < v1 ? v1 : v0, G, X))
-        return false;
-    const States s{2 * to_units(L[0], X.r), 2 * to_units(R[0], X.r), 2 * to_units(L[1], X.p),
-                   2 * to_units(R[1], X.p), 2 * to_units(L[2], X.v), 2 * to_units(R[2], X.v),
-                   2 * to_units(L[3], X.v), 2 * to_units(R[3], X.v)};
-    const Fan f = fan_of<HLL>(s, X, G, UU);
-    if (!f.ok) return false;
-    if (!HLL) return hllc(f, s, X, G, F[0], F[1], F[2], F[3]);
-    return hll(f, s, X, G, F[0], F[1], F[2], F[3]);
+    i64 q[8], a[4], b[4];
+    Keys<4> k[2];
+    int top[4];
+    bool speed;
+    cell_units<4>(L, q, 1, k[0]);
+    cell_units<4>(R, q + 4, 1, k[1]);
+    return G.room >= 0 && face_states<4, 1>(q + 4, 4, 1, k + 1, 1, true, a, b, top) &&
+           euler_flux<HLL>(a, b, top, G, F, UU, speed, false);
 }
 
 }  // namespace fx

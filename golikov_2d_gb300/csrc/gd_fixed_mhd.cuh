@@ -23,12 +23,11 @@
 namespace gd {
 namespace fx {
 
+// Exponents of a face's units: densities, pressures, normal and tangential velocities are in units
+// of 2^(X - 61), below 2^62; all fields in one of 2^(X.b - 61), below 2^60.
 struct TopsM {
-    int r, p, v, b;
+    int r, p, n, t, b;
 };
-// fields are held with two bits of room above their largest value
-constexpr int kFieldRoom = 2;
-
 struct StatesM {
     i64 r, p, un, ut, bn, bt, bz;
 };
@@ -148,20 +147,16 @@ GD_HD FanM fan_of(const StatesM& a, const StatesM& b, const TopsM& X, const Gas&
     const int kmax = imax(f.A.k, f.B.k);
     f.kmin = imin(f.A.k, f.B.k);
     f.ER = imax(f.A.R.e, f.B.R.e);
-    const int32_t h1 = hi32(a.un), h2 = hi32(b.un), h3 = hi32(a.ut), h4 = hi32(b.ut);
-    const int lz = clz32((uint32_t)((h1 ^ (h1 >> 31)) | (h2 ^ (h2 >> 31)) | (h3 ^ (h3 >> 31)) |
-                                    (h4 ^ (h4 >> 31))));
-    f.E = imax(kmax + 2, X.v + imax(4 - lz, 0));
+    f.E = imax(kmax + 2, imax(scale_of(a.un, b.un, X.n), scale_of(a.ut, b.ut, X.t)));
     const int dr = f.A.R.e - f.B.R.e;
     f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 8 && (uint32_t)(dr + 3) <= 6u;
     if (!f.ok) return f;
     const i64 cA = f.A.w >> (f.E - 1 - f.A.k), cB = f.B.w >> (f.E - 1 - f.B.k);
     const i64 c = cA > cB ? cA : cB;
-    const int sh = imin(f.E - X.v, 63);
-    f.uA = a.un >> sh;
-    f.uB = b.un >> sh;
-    f.vA = a.ut >> sh;
-    f.vB = b.ut >> sh;
+    f.uA = asr(a.un, f.E - X.n);
+    f.uB = asr(b.un, f.E - X.n);
+    f.vA = asr(a.ut, f.E - X.t);
+    f.vB = asr(b.ut, f.E - X.t);
     f.SL = (f.uA < f.uB ? f.uA : f.uB) - c;
     f.SR = (f.uA > f.uB ? f.uA : f.uB) + c;
     UU = to_double(-f.SL > f.SR ? -f.SL : f.SR, f.E - 61);
@@ -348,50 +343,45 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     return true;
 }
 
-// Whether the cells can be held in the units of TopsM (b1: the largest field's exponent field).
-GD_HD bool tops_of(uint32_t r0, uint32_t r1, uint32_t p0, uint32_t p1, uint32_t v1, uint32_t b1,
-                   const Gas& G, TopsM& X) {
-    Tops Y;
-    const bool ok = tops_of(r0, r1, p0, p1, v1, G, Y);
-    X.r = Y.r;
-    X.p = Y.p;
-    X.v = Y.v;
-    X.b = imax((int)b1 - 1023, -kLow) + kFieldRoom;
-    return ok && unit_of(b1);
+// The sides of a face from its states and their exponents (face_states): the fields' units become
+// one.
+GD_HD void sides_of(const i64* a, const i64* b, const int* top, StatesM& A, StatesM& B, TopsM& X) {
+    const int e4 = scale_of(a[4], b[4], top[4]), e5 = scale_of(a[5], b[5], top[5]);
+    const int e6 = scale_of(a[6], b[6], top[6]);
+    X = TopsM{top[0], top[1], top[2], top[3], imax(imax(e4, e5), imax(e6, -kLow))};
+    A = StatesM{a[0], a[1], a[2], a[3], asr(a[4], X.b - top[4]), asr(a[5], X.b - top[5]),
+                asr(a[6], X.b - top[6])};
+    B = StatesM{b[0], b[1], b[2], b[3], asr(b[4], X.b - top[4]), asr(b[5], X.b - top[5]),
+                asr(b[6], X.b - top[6])};
 }
-
+// The flux and the larger wave speed of that face; speed: whether the latter is valid.
+template <bool HLLD>
+GD_HD bool mhd_face_flux(const i64* a, const i64* b, const int* top, const Gas& G, FluxI& F,
+                         double& UU, bool& speed, bool speed_only) {
+    StatesM A, B;
+    TopsM X;
+    sides_of(a, b, top, A, B, X);
+    const FanM f = fan_of(A, B, X, G, UU);
+    speed = f.ok;
+    return f.ok && (speed_only || mhd_flux<HLLD>(f, A, B, X, G, F));
+}
 // The two states {rho, p, un, ut, bn, bt, bz} of a face in units of their own; false where the
 // integer solver does not take them.
-GD_HD bool face_units(const double* L, const double* R, const Gas& G, StatesM& A, StatesM& B,
-                      TopsM& X) {
-    const uint32_t rL = signed_exp_field(L[0]), rR = signed_exp_field(R[0]);
-    const uint32_t pL = signed_exp_field(L[1]), pR = signed_exp_field(R[1]);
-    uint32_t v1 = 0, b1 = 0;
-#pragma unroll
-    for (int f = 2; f < 7; ++f) {
-        const uint32_t x = exp_field(L[f]), y = exp_field(R[f]), m = x > y ? x : y;
-        if (f < 4) v1 = m > v1 ? m : v1;
-        else b1 = m > b1 ? m : b1;
-    }
-    if (!tops_of(rL < rR ? rL : rR, rL < rR ? rR : rL, pL < pR ? pL : pR, pL < pR ? pR : pL, v1,
-                 b1, G, X))
-        return false;
-    A = StatesM{2 * to_units(L[0], X.r), 2 * to_units(L[1], X.p), 2 * to_units(L[2], X.v),
-                2 * to_units(L[3], X.v), 2 * to_units(L[4], X.b), 2 * to_units(L[5], X.b),
-                2 * to_units(L[6], X.b)};
-    B = StatesM{2 * to_units(R[0], X.r), 2 * to_units(R[1], X.p), 2 * to_units(R[2], X.v),
-                2 * to_units(R[3], X.v), 2 * to_units(R[4], X.b), 2 * to_units(R[5], X.b),
-                2 * to_units(R[6], X.b)};
-    return true;
+GD_HD bool face_units(const double* L, const double* R, const Gas& G, i64* a, i64* b, int* top) {
+    i64 q[14];
+    Keys<7> k[2];
+    cell_units<7>(L, q, 1, k[0]);
+    cell_units<7>(R, q + 7, 1, k[1]);
+    return G.room >= 0 && face_states<7, 1>(q + 7, 7, 1, k + 1, 1, true, a, b, top);
 }
 // Flux and larger wave speed of that face.
 template <bool HLLD>
 GD_HD bool mhd_face(const double* L, const double* R, const Gas& G, FluxI& F, double& UU) {
-    StatesM A, B;
-    TopsM X;
-    if (!face_units(L, R, G, A, B, X)) return false;
-    const FanM f = fan_of(A, B, X, G, UU);
-    return f.ok && mhd_flux<HLLD>(f, A, B, X, G, F);
+    i64 a[7], b[7];
+    int top[7];
+    bool speed;
+    return face_units(L, R, G, a, b, top) &&
+           mhd_face_flux<HLLD>(a, b, top, G, F, UU, speed, false);
 }
 
 }  // namespace fx

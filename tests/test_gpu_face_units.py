@@ -1,0 +1,110 @@
+"""A face's arithmetic depends on its own cells alone.  Weak components beside strong ones in the
+same tile keep their digits: the quiet side of a jump to 1e-12 of the quiet values themselves against
+the oracle, a slow flow across a fast one to rounding.  States with faces out of the integers'
+range come out with the same bits whatever tiles, thread counts and bands they are cut into."""
+import numpy as np
+import pytest
+
+import golikov_2d_gb300 as g
+from golikov_2d_gb300 import problems
+from gpu_util import gpu_run, gpu_step_ref, grid_of
+from test_gpu_batch import run_batch
+from test_gpu_hoststep import pinned
+from test_gpu_integer_tiles import METHODS, config
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+@pytest.mark.parametrize("weak", [1e-3, 1e-8, 1e-12])
+@pytest.mark.parametrize("solver", ["hlld", "hllc_mhd"])
+def test_weak_field_beside_a_strong_one(cuda, oracle_lib, solver, weak):
+    """Left half: field of order 1, right half: weak times that; uniform flow through both."""
+    N, M = 100, 40
+    cfg = config(*METHODS[solver], N, M)
+    rng = np.random.default_rng(5)
+    K = N * M
+    s = np.stack([rng.uniform(1, 1.5, K), rng.uniform(3, 4, K)], 1)
+    u = np.tile([0.4, 0.3], (K, 1)) + rng.uniform(-0.05, 0.05, (K, 2))
+    b = rng.uniform(-1, 1, (K, 3))
+    quiet = np.arange(K) % N >= N // 2 + 3
+    b[np.arange(K) % N >= N // 2] *= weak
+    T = 0.2 * cfg.dx / 4
+    so, uo, bo, _ = oracle_lib.step(grid_of(cfg), s, u, b, T)
+    sg, ug, bg, _ = gpu_step_ref(cfg, s, u, b, T)
+    quiet &= np.arange(K) % N < N - 3  # the periodic edge is a jump too
+    for k in range(3):
+        assert np.abs(bg[quiet, k] - bo[quiet, k]).max() <= TOL * weak, k
+        assert np.abs(bg[:, k] - bo[:, k]).max() <= TOL, k
+
+
+@pytest.mark.parametrize("solver", ["hllc", "hll"])
+def test_slow_cross_flow(cuda, solver):
+    """A flow along x of order 1, uniform in y, that carries a velocity along y; in the right half
+    1000 times weaker.  The carried velocity is a passive quantity: scaled by 2^-40 it is the same
+    field to rounding (the kinetic energy that it adds at full strength stays in the pressure)."""
+    N, M = 100, 40
+    cfg = config(*METHODS[solver], N, M)
+    rng = np.random.default_rng(6)
+    s = np.stack([rng.uniform(1, 1.5, N), rng.uniform(3, 4, N)], 1)
+    u = np.stack([rng.uniform(-0.5, 0.5, N), rng.uniform(-1, 1, N)], 1)
+    u[N // 2:, 1] *= 1e-3
+    s, u = np.tile(s, (M, 1)), np.tile(u, (M, 1))
+    T = 0.2 * cfg.dx / 4
+    full = gpu_step_ref(cfg, s, u, None, T)[1][:, 1]
+    slow = gpu_step_ref(cfg, s, u * [1.0, 2.0 ** -40], None, T)[1][:, 1] * 2.0 ** 40
+    col = np.arange(N * M) % N
+    for part, unit in ((col < N // 2 - 3, 1.0), ((col >= N // 2 + 3) & (col < N - 3), 1e-3)):
+        assert np.abs(slow[part] - full[part]).max() <= 4e-16 * unit
+
+
+def jumpy(physics, K, seed):
+    """Densities over 2^16, pressures over 2^12, velocities and fields over 2^40: a part of the
+    faces in integers, a part in floating point."""
+    rng = np.random.default_rng(seed)
+    s = np.stack([2.0 ** rng.uniform(-4, 12, K), 2.0 ** rng.uniform(0, 12, K)], 1)
+    u = rng.uniform(-0.05, 0.05, (K, 2)) * 2.0 ** rng.uniform(-40, 0, (K, 2))
+    b = None
+    if physics == g.MHD:
+        b = rng.uniform(-1, 1, (K, 3)) * 2.0 ** rng.uniform(-40, 0, (K, 3))
+    return s, u, b
+
+
+@pytest.mark.parametrize("N,M", [(200, 140), (321, 177), (640, 400)])
+@pytest.mark.parametrize("solver", METHODS)
+def test_bands_of_the_host_step_change_no_bit(cuda, solver, N, M):
+    """One launch, with the few-tiles kernel or without, and the host step's bands."""
+    physics, method = METHODS[solver]
+    cfg = config(physics, method, N, M)
+    s, u, b = jumpy(physics, N * M, 3)
+    T = 1e-3 * cfg.dx / 256
+    one = gpu_run(cfg, s, u, b, 1, T_do=T)
+    sol = g.Solver(cfg)
+    sol.import_state(s, u, b)
+    sol.set_time(T, 0.0)
+    ins = [pinned(x) for x in (s, u, b)]
+    outs = [None if x is None else pinned(np.zeros_like(x)) for x in (s, u, b)]
+    sol.step_host(*ins, *outs)
+    dt = sol.stats(allow_nonfinite=True).dt
+    sol.close()
+    for x, y in zip(one[:3], outs):
+        assert (x is None and y is None) or np.array_equal(x, np.asarray(y))
+    assert one[3].dt == dt
+
+
+@pytest.mark.parametrize("solver", ["hllc", "hll"])
+def test_tile_shapes_and_threads_change_no_bit(cuda, solver):
+    """A batch in the tuner's shape, in the default one, and each grid by itself."""
+    grids = problems.batch_four_quadrant(8, lo=100, hi=300, seed=12)
+    out = []
+    for cfg, s, u, _ in grids:
+        cfg.method = METHODS[solver][1]
+        s, u, _ = jumpy(g.EULER, cfg.N * cfg.M, cfg.N)
+        out.append((cfg, s, u, None))
+    a, ia = run_batch(out, 3)
+    c, ic = run_batch(out, 3, autotune=True)
+    for (cfg, s, u, _), x, y in zip(out, a, c):
+        one = gpu_run(cfg, s, u, None, 3)
+        assert np.array_equal(one[0], x[0]) and np.array_equal(one[1], x[1])
+        assert np.array_equal(one[0], y[0]) and np.array_equal(one[1], y[1])
+        assert one[3].dt == x[2].dt == y[2].dt
