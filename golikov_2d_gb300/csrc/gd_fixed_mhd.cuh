@@ -23,13 +23,17 @@
 namespace gd {
 namespace fx {
 
-// Exponents of a face's units: densities, pressures, normal and tangential velocities are in units
-// of 2^(X - 61), below 2^62; all fields in one of 2^(X.b - 61), below 2^60.
+// Exponents of a face's units: densities, pressures, velocities and fields are in units of
+// 2^(X - 61), below 2^62; b is the largest field's, with the normal field in units of 2^(X.b - 61),
+// below 2^60.
 struct TopsM {
-    int r, p, n, t, b;
+    int r, p, n, t, b, bt, bz;
 };
 struct StatesM {
     i64 r, p, un, ut, bn, bt, bz;
+};
+struct FluxI {
+    double m, mn, mt, e, bn, bt, bz;
 };
 
 // |x| < 2^61 (and a little beyond on the negative side)
@@ -89,13 +93,13 @@ GD_HD SideM side_of(const StatesM& s, const TopsM& X, const Gas& G) {
 
 // The star state of one side: v - v0, w, b_t, b_z behind the fast wave (Gas_Dinamic.cu:1306-1350).
 // am = |rho (S - u)|, ad = |S - S_M|, as = |S - u|; bn2 the square of the mean normal field in
-// units of 2^(ER + 2E - 59), sh the shift that brings products of two fields to them, thr the
-// guard's 1e-5 in them.  False where a ratio leaves its range.
+// units of 2^(ER + 2E - 59), st and sh the shifts that bring products of two fields to them (to the
+// tangential velocity's where one is tangential), thr the guard's 1e-5 in them.  False where a ratio leaves its range.
 struct StarM {
     i64 dv, dw, bt, bz;
 };
-GD_HD bool star_of(i64 am, i64 ad, i64 as, i64 SMu, i64 bn, i64 bn2, int sh, i64 thr, i64 bt,
-                   i64 bz, StarM& T) {
+GD_HD bool star_of(i64 am, i64 ad, i64 as, i64 SMu, i64 bn, i64 bn2, int st, int sh, i64 thr,
+                   i64 bt, i64 bz, StarM& T) {
     const i64 tt = mulk<2, 1>(am, ad) - bn2;
     const i64 at = iabs(tt);
     if (at < thr) {
@@ -106,7 +110,7 @@ GD_HD bool star_of(i64 am, i64 ad, i64 as, i64 SMu, i64 bn, i64 bn2, int sh, i64
     int lz;
     const i64 it = rcp(at, lz);
     const i64 num = mulk<2, 1>(am, as) - bn2;
-    const i64 x1 = shift(mulk<0, 0>(bn, bt), sh), x2 = shift(mulk<0, 0>(bn, bz), sh);
+    const i64 x1 = shift(mulk<0, 0>(bn, bt), st), x2 = shift(mulk<0, 0>(bn, bz), sh);
     if (!(iabs(num >> 1) < 2 * (at >> 1) && iabs(x1) < at && iabs(x2) < at)) return false;
     const i64 k1 = mulk<0, 2>(x1 << (lz - 2), it), k2 = mulk<0, 2>(x2 << (lz - 2), it);
     const i64 d = mulk<0, 2>((num >> 1) << (lz - 2), it);
@@ -134,20 +138,31 @@ GD_HD i64 root_of(Pos R, int& k, i64& rs) {
 }
 
 // The larger wave speed of the face between A and B, and all speeds.
+//
+// Tangential components may be far below the normal ones and are carried by them, so they have
+// units of their own: tangential velocities 2^(E - 61 - tv), tangential fields 2^(X.b - 61 - tb),
+// and the z field and velocity 2^(X.b - 61 - z) and 2^(E - 61 - z).  Every flux is linear in each
+// pair, or has products of two of it, which shift back.  Where a normal field couples velocity and
+// field, both units follow the larger of v and b / sqrt(rho), 2^(-sh/2) of the speed per unit of the
+// field.  kRoom bits are left above the components, for star states above them.
+constexpr int kRoom = 3;
 struct FanM {
     SideM A, B;
     i64 uA, uB, vA, vB, SL, SR;
-    int E, ER, kmin;
+    int E, ER, kmin, tv, tb, z;
+    int sh;  // what brings products of two fields to units of 2^(ER + 2E - 59)
     bool ok;
 };
-GD_HD FanM fan_of(const StatesM& a, const StatesM& b, const TopsM& X, const Gas& G, double& UU) {
+GD_HD FanM fan_of(StatesM& a, StatesM& b, const TopsM& X, const Gas& G, double& UU) {
     FanM f;
-    f.A = side_of(a, X, G);
-    f.B = side_of(b, X, G);
+    const int bt = X.b - X.bt, bz = X.b - X.bz;
+    f.A = side_of(StatesM{a.r, a.p, a.un, a.ut, a.bn, asr(a.bt, bt), asr(a.bz, bz)}, X, G);
+    f.B = side_of(StatesM{b.r, b.p, b.un, b.ut, b.bn, asr(b.bt, bt), asr(b.bz, bz)}, X, G);
     const int kmax = imax(f.A.k, f.B.k);
     f.kmin = imin(f.A.k, f.B.k);
     f.ER = imax(f.A.R.e, f.B.R.e);
-    f.E = imax(kmax + 2, imax(scale_of(a.un, b.un, X.n), scale_of(a.ut, b.ut, X.t)));
+    const int xv = scale_of(a.ut, b.ut, X.t);
+    f.E = imax(kmax + 2, imax(scale_of(a.un, b.un, X.n), xv));
     const int dr = f.A.R.e - f.B.R.e;
     f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 8 && (uint32_t)(dr + 3) <= 6u;
     if (!f.ok) return f;
@@ -155,17 +170,26 @@ GD_HD FanM fan_of(const StatesM& a, const StatesM& b, const TopsM& X, const Gas&
     const i64 c = cA > cB ? cA : cB;
     f.uA = asr(a.un, f.E - X.n);
     f.uB = asr(b.un, f.E - X.n);
-    f.vA = asr(a.ut, f.E - X.t);
-    f.vB = asr(b.ut, f.E - X.t);
+    f.tv = imax(f.E - xv - kRoom, 0);
+    f.tb = imax(X.b - scale_of(a.bt, b.bt, X.bt) - kRoom, 0);
+    f.z = imax(X.b - scale_of(a.bz, b.bz, X.bz) - kRoom, 0);
+    f.sh = f.ER + 2 * f.E - 1 - 2 * X.b;
+    if ((a.bn | b.bn) != 0) {
+        const int h = imax(f.sh, 0) >> 1, tv = f.tv;
+        f.tv = imin(tv, f.tb + h);
+        f.tb = imin(f.tb, imax(tv - h, 0));
+    }
+    f.vA = asr(a.ut, f.E - X.t - f.tv);
+    f.vB = asr(b.ut, f.E - X.t - f.tv);
+    a.bt = asr(a.bt, bt - f.tb);
+    b.bt = asr(b.bt, bt - f.tb);
+    a.bz = asr(a.bz, bz - f.z);
+    b.bz = asr(b.bz, bz - f.z);
     f.SL = (f.uA < f.uB ? f.uA : f.uB) - c;
     f.SR = (f.uA > f.uB ? f.uA : f.uB) + c;
     UU = to_double(-f.SL > f.SR ? -f.SL : f.SR, f.E - 61);
     return f;
 }
-
-struct FluxI {
-    double m, mn, mt, e, bn, bt, bz;
-};
 
 // m 2^(e - 62) in units of 2^u, at least 1, or the largest integer where it does not fit
 GD_HD i64 threshold(i64 m, int e, int u) {
@@ -184,7 +208,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const i64 mA = mulk<0, 0>(f.A.R.m, suA) >> (ER - f.A.R.e);
     const i64 mB = mulk<0, 0>(f.B.R.m, suB) >> (ER - f.B.R.e);
     // total pressures in units of 2^(ER + 2E - 60)
-    const int sp = ER + 2 * E + 2, sq = ER + 2 * E - 1 - XB;
+    const int sp = ER + 2 * E + 2, sq = f.sh;
     const i64 ptA = (f.A.P.m >> imin(sp - f.A.P.e, 63)) + shift(f.A.bb, sq);
     const i64 ptB = (f.B.P.m >> imin(sp - f.B.P.e, 63)) + shift(f.B.bb, sq);
     const i64 N = mulk<1, 3>(mB, f.uB) - mulk<1, 3>(mA, f.uA) + (ptA - ptB);
@@ -207,8 +231,10 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const i64 m = takeL ? mA : mB, ptK = (takeL ? ptA : ptB) >> 1;
     const i64 S = takeL ? f.SL : f.SR, su = takeL ? suA : suB;
 
-    const int sh = ER + 2 * E - 1 - XB;  // products of fields to units of 2^(ER + 2E - 59)
-    const i64 ub = mulk<2, 1>(un, bnK) + mulk<2, 1>(ut, btK);  // units 2^(E + X.b - 61)
+    const int sh = f.sh, dt = f.tv - f.tb, st = sh - dt;  // st: of a tangential one, to momenta
+    const int vb = f.tv + f.tb;
+    // units 2^(E + X.b - 61)
+    const i64 ub = mulk<2, 1>(un, bnK) + asr(mulk<2, 1>(ut, btK), vb);
     i64 qs = un, qsg = 0, sb = ub, S2 = 0;
     StarM K{0, 0, btK, bzK};
     Pos RK = R;
@@ -228,7 +254,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
             am = iabs(m);
             bn2 = shift(mulk<0, 0>(bn, bn), sh);
             thr = threshold(0x53e2d6238da3c211LL, -17, ER + 2 * E - 59);  // 1e-5
-            if (!star_of(am, ad, iabs(su), SM - un, bn, bn2, sh, thr, btK, bzK, K)) return false;
+            if (!star_of(am, ad, iabs(su), SM - un, bn, bn2, st, sh, thr, btK, bzK, K)) return false;
             RK = star_density(am, iA, lza, ER);
             i64 rs;
             sK = root_of<true>(RK, kK, rs);
@@ -244,10 +270,10 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
             const i64 tA = mulk<0, 0>(a.bn, a.bt), tB = mulk<0, 0>(b.bn, b.bt);
             const i64 zA = mulk<0, 0>(a.bn, a.bz), zB = mulk<0, 0>(b.bn, b.bz);
             const i64 N1 = N + (shift(nB - nA, sq) << 1);
-            const i64 N2 = mulk<1, 3>(mB, f.vB) - mulk<1, 3>(mA, f.vA) + (shift(tB - tA, sq) << 1);
+            const i64 N2 = mulk<1, 3>(mB, f.vB) - mulk<1, 3>(mA, f.vA) + (shift(tB - tA, st) << 1);
             const i64 N3 = shift(zB - zA, sq) << 1;
-            const i64 Tt = mulk<1, 2>(suB, b.bt) + mulk<2, 1>(f.vB, b.bn) -
-                           (mulk<1, 2>(suA, a.bt) + mulk<2, 1>(f.vA, a.bn));
+            const i64 Tt = mulk<1, 2>(suB, b.bt) - mulk<1, 2>(suA, a.bt) +
+                           asr(mulk<2, 1>(f.vB, b.bn) - mulk<2, 1>(f.vA, a.bn), dt);
             const i64 Tz = mulk<1, 2>(suB, b.bz) - mulk<1, 2>(suA, a.bz);
             if (!(scales(iabs(N1) | iabs(N2) | iabs(N3), lz) &&
                   scales(iabs(Tt) | iabs(Tz), lzs)))
@@ -259,7 +285,8 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
             K.dv = vs - ut;
             if (!(below61(u1) && below61(ws) && below61(vs) && below61(K.bt) && below61(K.bz)))
                 return false;
-            sb = mulk<2, 1>(u1, bn) + mulk<2, 1>(vs, K.bt) + mulk<2, 1>(ws, K.bz);
+            sb = mulk<2, 1>(u1, bn) + asr(mulk<2, 1>(vs, K.bt), vb) +
+                 asr(mulk<2, 1>(ws, K.bz), 2 * f.z);
         }
     } else {  // the physical flux of K: no mean of both sides in it
         SM = un;
@@ -267,7 +294,9 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     }
     const i64 SMu = SM - un, vK = ut + K.dv;
     if (!(below61(vK) && below61(K.dw) && below61(K.bt) && below61(K.bz))) return false;
-    if (HLLD && star) sb = mulk<2, 1>(SM, bn) + mulk<2, 1>(vK, K.bt) + mulk<2, 1>(K.dw, K.bz);
+    if (HLLD && star)
+        sb = mulk<2, 1>(SM, bn) + asr(mulk<2, 1>(vK, K.bt), vb) +
+             asr(mulk<2, 1>(K.dw, K.bz), 2 * f.z);
 
     const int32_t qh = hi32(qs);
     const int z = clz32((uint32_t)(qh ^ (qh >> 31))) - 1;
@@ -276,12 +305,12 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const int em = R.e + E - 59 - z;
     F.m = to_double(M, em);
     const int dR = ER - R.e;
-    const i64 n2s = shift(n2K, sh), bnt = shift(mulk<0, 0>(bnK, btK), sh);
+    const i64 n2s = shift(n2K, sh), bnt = shift(mulk<0, 0>(bnK, btK), st);
     const i64 mn = ptK + (mulk<1, 2>(M, SM) >> imin(z + dR, 63)) + mulk<2, 1>(m, SMu) - n2s;
     i64 mt = (mulk<1, 2>(M, vK) >> imin(z + dR, 63)) + mulk<2, 1>(m, K.dv) - bnt;
-    i64 ft = mulk<2, 1>(S, K.bt) - mulk<1, 2>(su, btK) - mulk<2, 1>(ut, bnK);
+    i64 ft = mulk<2, 1>(S, K.bt) - mulk<1, 2>(su, btK) - asr(mulk<2, 1>(ut, bnK), dt);
     i64 fz = mulk<2, 1>(S, K.bz) - mulk<1, 2>(su, bzK);
-    const i64 H = mulk<1, 1>(un, un) + mulk<1, 1>(ut, ut) + mulk<2, 1>(S, SMu);
+    const i64 H = mulk<1, 1>(un, un) + asr(mulk<1, 1>(ut, ut), 2 * f.tv) + mulk<2, 1>(S, SMu);
     const i64 B = sra(mulk<0, 0>(Pk.m, G.gg), ER + 2 * E - Pk.e - G.gge + G.room) +
                   ((mulk<0, 1>(R.m, H) >> dR) + shift(bbK, ER + 2 * E - 2 - XB) >> G.room);
     const i64 y = (mulk<2, 1>(qsg, ub - sb) << 1) - sb;
@@ -300,7 +329,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
         const i64 adO = takeL ? f.SR - SM : SM - f.SL;
         if (hi32(adO) <= 0) return false;
         StarM O;
-        if (!star_of(amO, adO, asO, SM - unO, bn, bn2, sh, thr, btO, bzO, O)) return false;
+        if (!star_of(amO, adO, asO, SM - unO, bn, bn2, st, sh, thr, btO, bzO, O)) return false;
         const i64 vO = utO + O.dv;
         if (!(below61(vO) && below61(O.dw) && below61(O.bt) && below61(O.bz))) return false;
         int lzO, kO, lzt;
@@ -313,7 +342,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
         const i64 w = mulk<0, 2>(aK << (lzt - 2), iT);
         const bool flip = takeL != (bn > 0);  // sign of b times that of O - K in R - L
         const int sv = E + kk + 3 - lzt - X.b;
-        const i64 xt = shift(mulk<1, 2>(O.bt - K.bt, iT), sv);
+        const i64 xt = shift(mulk<1, 2>(O.bt - K.bt, iT), sv - dt);
         const i64 xz = shift(mulk<1, 2>(O.bz - K.bz, iT), sv);
         const i64 v3 = vO + (mulk<2, 1>(w, vK - vO) << 1) + (flip ? -xt : xt);
         const i64 w3 = O.dw + (mulk<2, 1>(w, K.dw - O.dw) << 1) + (flip ? -xz : xz);
@@ -321,13 +350,14 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
         const int sc = X.b - kk - E - 1;
         const i64 ct = mulk<2, 1>(wo, vO - vK), cz = mulk<2, 1>(wo, O.dw - K.dw);
         // root(rho) times the jump of v may be far above a weak field
-        if (!fits(iabs(ct) | iabs(cz), sc)) return false;
-        const i64 yt = shift(ct, sc), yz = shift(cz, sc);
+        if (!(fits(iabs(ct), sc + dt) && fits(iabs(cz), sc))) return false;
+        const i64 yt = shift(ct, sc + dt), yz = shift(cz, sc);
         const i64 bt3 = K.bt + (mulk<2, 1>(w, O.bt - K.bt) << 1) + (flip ? -yt : yt);
         const i64 bz3 = K.bz + (mulk<2, 1>(w, O.bz - K.bz) << 1) + (flip ? -yz : yz);
         if (!(below61(v3) && below61(w3) && below61(bt3) && below61(bz3) && below61(S2)))
             return false;
-        const i64 sb3 = mulk<2, 1>(SM, bn) + mulk<2, 1>(v3, bt3) + mulk<2, 1>(w3, bz3);
+        const i64 sb3 = mulk<2, 1>(SM, bn) + asr(mulk<2, 1>(v3, bt3), vb) +
+                        asr(mulk<2, 1>(w3, bz3), 2 * f.z);
         mt += shift(mulk<2, 1>(mulk<0, 0>(RK.m, S2), v3 - vK), ER - RK.e);
         ft += mulk<2, 1>(S2, bt3 - K.bt);
         fz += mulk<2, 1>(S2, bz3 - K.bz);
@@ -335,35 +365,30 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
         e += flip ? de : -de;
     }
     F.mn = to_double(mn, ER + 2 * E - 59);
-    F.mt = to_double(mt, ER + 2 * E - 59);
+    F.mt = to_double(mt, ER + 2 * E - 59 - f.tv);
     F.e = to_double(e, ER + 3 * E - 61);
-    F.bt = to_double(ft, E + X.b - 61);
-    F.bz = to_double(fz, E + X.b - 61);
-    F.bn = -to_double(mulk<2, 1>(-f.SL > f.SR ? -f.SL : f.SR, b.bn - a.bn), E + X.b - 61);
+    F.bt = to_double(ft, E + X.b - 61 - f.tb);
+    F.bz = to_double(fz, E + X.b - 61 - f.z);
     return true;
 }
 
-// The sides of a face from its states and their exponents (face_states): the fields' units become
-// one.
-GD_HD void sides_of(const i64* a, const i64* b, const int* top, StatesM& A, StatesM& B, TopsM& X) {
-    const int e4 = scale_of(a[4], b[4], top[4]), e5 = scale_of(a[5], b[5], top[5]);
-    const int e6 = scale_of(a[6], b[6], top[6]);
-    X = TopsM{top[0], top[1], top[2], top[3], imax(imax(e4, e5), imax(e6, -kLow))};
-    A = StatesM{a[0], a[1], a[2], a[3], asr(a[4], X.b - top[4]), asr(a[5], X.b - top[5]),
-                asr(a[6], X.b - top[6])};
-    B = StatesM{b[0], b[1], b[2], b[3], asr(b[4], X.b - top[4]), asr(b[5], X.b - top[5]),
-                asr(b[6], X.b - top[6])};
-}
-// The flux and the larger wave speed of that face; speed: whether the latter is valid.
+// The flux and the larger wave speed of a face from its states and their exponents (face_states);
+// speed: whether the latter is valid.
 template <bool HLLD>
-GD_HD bool mhd_face_flux(const i64* a, const i64* b, const int* top, const Gas& G, FluxI& F,
+GD_HD bool mhd_face_flux(const i64* p, const i64* q, const int* top, const Gas& G, FluxI& F,
                          double& UU, bool& speed, bool speed_only) {
-    StatesM A, B;
-    TopsM X;
-    sides_of(a, b, top, A, B, X);
-    const FanM f = fan_of(A, B, X, G, UU);
+    const int e4 = scale_of(p[4], q[4], top[4]), e5 = scale_of(p[5], q[5], top[5]);
+    const int e6 = scale_of(p[6], q[6], top[6]);
+    const TopsM X{top[0], top[1], top[2], top[3], imax(imax(e4, e5), imax(e6, -kLow)), top[5], top[6]};
+    StatesM a{p[0], p[1], p[2], p[3], asr(p[4], X.b - top[4]), p[5], p[6]};
+    StatesM b{q[0], q[1], q[2], q[3], asr(q[4], X.b - top[4]), q[5], q[6]};
+    const FanM f = fan_of(a, b, X, G, UU);
     speed = f.ok;
-    return f.ok && (speed_only || mhd_flux<HLLD>(f, A, B, X, G, F));
+    if (!f.ok) return false;
+    if (speed_only) return true;
+    // the normal field's flux in its own unit
+    F.bn = to_double(mulk<2, 0>(-f.SL > f.SR ? -f.SL : f.SR, p[4] - q[4]), f.E + top[4] - 60);
+    return mhd_flux<HLLD>(f, a, b, X, G, F);
 }
 // The two states {rho, p, un, ut, bn, bt, bz} of a face in units of their own; false where the
 // integer solver does not take them.

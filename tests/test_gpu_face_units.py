@@ -108,3 +108,40 @@ def test_tile_shapes_and_threads_change_no_bit(cuda, solver):
         assert np.array_equal(one[0], x[0]) and np.array_equal(one[1], x[1])
         assert np.array_equal(one[0], y[0]) and np.array_equal(one[1], y[1])
         assert one[3].dt == x[2].dt == y[2].dt
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("solver", ["hlld", "hllc_mhd"])
+def test_weak_out_of_plane_field(cuda, solver, order):
+    """A field along z too weak to act on the flow is carried by it: scaled by 2^-60 it is the same
+    field to rounding."""
+    N, M = 70, 45
+    cfg = config(*METHODS[solver], N, M)
+    cfg.order = order
+    rng = np.random.default_rng(8)
+    K = N * M
+    s = np.stack([rng.uniform(1, 1.5, K), rng.uniform(1, 1.5, K)], 1)
+    u = rng.uniform(-0.5, 0.5, (K, 2))
+    b = rng.uniform(-2, 2, (K, 3))
+    T = 0.2 * cfg.dx / 4
+    out = [gpu_step_ref(cfg, s, u, b * [1.0, 1.0, w], T)[2][:, 2] / w for w in (2.0 ** -40, 2.0 ** -100)]
+    assert np.abs(out[1] - out[0]).max() <= 2e-15
+
+
+@pytest.mark.parametrize("solver", ["hlld", "hllc_mhd"])
+def test_weak_transverse_wave(cuda, solver):
+    """Velocity and field along y, uniform in y, on a strong field along x."""
+    N, M = 90, 23
+    cfg = config(*METHODS[solver], N, M)
+    rng = np.random.default_rng(9)
+    s = np.stack([rng.uniform(1, 1.5, N), rng.uniform(3, 4, N)], 1)
+    u = np.stack([rng.uniform(-0.5, 0.5, N), rng.uniform(-1, 1, N)], 1)
+    b = np.stack([np.full(N, 3.0), rng.uniform(-1, 1, N), rng.uniform(-1, 1, N)], 1)
+    s, u, b = (np.tile(x, (M, 1)) for x in (s, u, b))
+    T = 0.2 * cfg.dx / 6
+    out = []
+    for w in (2.0 ** -40, 2.0 ** -90):
+        _, u2, b2, _ = gpu_step_ref(cfg, s, u * [1.0, w], b * [1.0, w, w], T)
+        out.append((u2[:, 1] / w, b2[:, 1] / w, b2[:, 2] / w))
+    for x, y in zip(*out):
+        assert np.abs(x - y).max() <= 2e-15
