@@ -380,11 +380,14 @@ GD_HD double to_double(i64 x, int ue) {
     swfp::halves((double)x, hi, lo);
     return swfp::from_halves(x == 0 ? 0u : hi + ((uint32_t)ue << 20), lo);
 }
-// The least E >= top for which both x 2^(top - 61) and y 2^(top - 61) are below 2^(E - 1)
-GD_HD int scale_of(i64 x, i64 y, int top) {
+// E for which both x 2^(top - 61) and y 2^(top - 61) are below 2^(E - 1), from their leading words:
+// the least one, and at least top - 28
+GD_HD int top_of(i64 x, i64 y, int top) {
     const int32_t h = hi32(x), k = hi32(y);
-    return top + imax(4 - clz32((uint32_t)((h ^ (h >> 31)) | (k ^ (k >> 31)))), 0);
+    return top + 4 - clz32((uint32_t)((h ^ (h >> 31)) | (k ^ (k >> 31))));
 }
+// at least top
+GD_HD int scale_of(i64 x, i64 y, int top) { return imax(top_of(x, y, top), top); }
 
 // The two sides of a face in its local frame, per component (rho, p, normal and tangential
 // velocity) in units of 2^(X - 61), below 2^62.
@@ -409,8 +412,8 @@ struct Fan {
     bool ok;
 };
 // ok is false where a scale would leave a quantity fewer bits than binary64 does: accepted are
-// sound speeds within a factor of about 4 of each other, and normal velocities to about 64 of
-// them.  UU: the larger wave speed.
+// sound speeds within a factor of about 4 of each other, and normal velocities to about 2^22 of
+// them (the larger velocity is then the scale of every flux).  UU: the larger wave speed.
 // HLL: the fan min(u) - max(c), max(u) + max(c) of kernel.cu:1516-1517 instead of Davis'.
 template <bool HLL = false>
 GD_HD Fan fan_of(const States& q, const Tops& X, const Gas& G, double& UU) {
@@ -425,7 +428,7 @@ GD_HD Fan fan_of(const States& q, const Tops& X, const Gas& G, double& UU) {
     const int kmax = imax(kL, kR);
     f.kmin = imin(kL, kR);
     f.E = imax(kmax + 2, scale_of(q.uL, q.uR, X.n));
-    f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 8;
+    f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 24;
     if (!f.ok) return f;
     i64 cL = wL >> (f.E - 1 - kL), cR = wR >> (f.E - 1 - kR);
     if (HLL) {
@@ -544,11 +547,13 @@ GD_HD bool hll(const Fan& f, const States& s, const Tops& X, const Gas& G, doubl
     const int z = clz32((uint32_t)(hi32(qL) | hi32(qR))) - 1;
     const i64 h = mulk<0, 1>(qL << z, gL) + mulk<0, 1>(qR << z, gR);
     const i64 t = mulk<1, 1>(TL, s.vL) + mulk<1, 1>(TR, s.vR);
-    const int st = 2 * (E - X.t) - 3;
-    if (!(fits(iabs(h), z - 4) && fits(iabs(t), st))) return false;
+    // a faster flow along the face sets the unit, rr bits above
+    const int st = 2 * (E - X.t) - 3, rr = imax(-st, 0);
+    if (!fits(iabs(h), z - 4 + rr)) return false;
     const i64 k = mulk<2, 2>(A, mulk<2, 2>(f.uL, f.uL)) + mulk<2, 2>(B, mulk<2, 2>(f.uR, f.uR)) +
-                  mulk<3, 2>(pL, f.uL) + mulk<3, 2>(pR, f.uR) + shift(t, st);
-    Fe = to_double(shift(h, z - 4) + (k >> G.room), ER + 3 * E - 62 + G.room);
+                  mulk<3, 2>(pL, f.uL) + mulk<3, 2>(pR, f.uR);
+    Fe = to_double(shift(h, z - 4 + rr) + (sra(k, rr) + shift(t, st + rr) >> G.room),
+                   ER + 3 * E - 62 + G.room + rr);
     return true;
 }
 

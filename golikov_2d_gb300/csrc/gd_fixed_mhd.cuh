@@ -145,10 +145,15 @@ GD_HD i64 root_of(Pos R, int& k, i64& rs) {
 // pair, or has products of two of it, which shift back.  Where a normal field couples velocity and
 // field, both units follow the larger of v and b / sqrt(rho), 2^(-sh/2) of the speed per unit of the
 // field.  kRoom bits are left above the components, for star states above them.
+//
+// A flow along the face far faster than its waves would set the unit of all speeds and cost the fan
+// its digits.  The fluxes follow a change of frame exactly, so the face is solved in a frame that
+// moves along it with w, one side's tangential velocity to 52 bits (units 2^(X.t - 61); 0 in all
+// other faces), and mhd_flux adds w's momentum, energy and induction.
 constexpr int kRoom = 3;
 struct FanM {
     SideM A, B;
-    i64 uA, uB, vA, vB, SL, SR;
+    i64 uA, uB, vA, vB, SL, SR, w;
     int E, ER, kmin, tv, tb, z;
     int sh;  // what brings products of two fields to units of 2^(ER + 2E - 59)
     bool ok;
@@ -161,10 +166,18 @@ GD_HD FanM fan_of(StatesM& a, StatesM& b, const TopsM& X, const Gas& G, double& 
     const int kmax = imax(f.A.k, f.B.k);
     f.kmin = imin(f.A.k, f.B.k);
     f.ER = imax(f.A.R.e, f.B.R.e);
-    const int xv = scale_of(a.ut, b.ut, X.t);
-    f.E = imax(kmax + 2, imax(scale_of(a.un, b.un, X.n), xv));
+    f.E = imax(kmax + 2, scale_of(a.un, b.un, X.n));
+    int xv = scale_of(a.ut, b.ut, X.t);
+    f.w = 0;
+    if (xv > f.E + 1) {
+        f.w = a.ut & ~1023LL;
+        a.ut -= f.w;
+        b.ut -= f.w;
+        xv = top_of(a.ut, b.ut, X.t);
+    }
+    f.E = imax(f.E, xv);
     const int dr = f.A.R.e - f.B.R.e;
-    f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 8 && (uint32_t)(dr + 3) <= 6u;
+    f.ok = kmax - f.kmin <= 2 && f.E - kmax <= 24 && (uint32_t)(dr + 3) <= 6u;
     if (!f.ok) return f;
     const i64 cA = f.A.w >> (f.E - 1 - f.A.k), cB = f.B.w >> (f.E - 1 - f.B.k);
     const i64 c = cA > cB ? cA : cB;
@@ -179,8 +192,8 @@ GD_HD FanM fan_of(StatesM& a, StatesM& b, const TopsM& X, const Gas& G, double& 
         f.tv = imin(tv, f.tb + h);
         f.tb = imin(f.tb, imax(tv - h, 0));
     }
-    f.vA = asr(a.ut, f.E - X.t - f.tv);
-    f.vB = asr(b.ut, f.E - X.t - f.tv);
+    f.vA = shift(a.ut, f.E - X.t - f.tv);
+    f.vB = shift(b.ut, f.E - X.t - f.tv);
     a.bt = asr(a.bt, bt - f.tb);
     b.bt = asr(b.bt, bt - f.tb);
     a.bz = asr(a.bz, bz - f.z);
@@ -272,9 +285,15 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
             const i64 N1 = N + (shift(nB - nA, sq) << 1);
             const i64 N2 = mulk<1, 3>(mB, f.vB) - mulk<1, 3>(mA, f.vA) + (shift(tB - tA, st) << 1);
             const i64 N3 = shift(zB - zA, sq) << 1;
-            const i64 Tt = mulk<1, 2>(suB, b.bt) - mulk<1, 2>(suA, a.bt) +
+            i64 Tt = mulk<1, 2>(suB, b.bt) - mulk<1, 2>(suA, a.bt) +
                            asr(mulk<2, 1>(f.vB, b.bn) - mulk<2, 1>(f.vA, a.bn), dt);
             const i64 Tz = mulk<1, 2>(suB, b.bz) - mulk<1, 2>(suA, a.bz);
+            if (f.w != 0) {  // the one term that a jump of the normal field keeps out of the frame
+                const i64 wb = mulk<1, 1>(f.w, b.bn - a.bn);
+                const int sw = E - f.tb - X.t - 1;
+                if (!fits(iabs(wb), sw)) return false;
+                Tt += shift(wb, sw);
+            }
             if (!(scales(iabs(N1) | iabs(N2) | iabs(N3), lz) &&
                   scales(iabs(Tt) | iabs(Tz), lzs)))
                 return false;
@@ -320,6 +339,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     i64 e = shift(e0, z - 2 - G.room) +
             shift(mulk<2, 0>(bn, y) + mulk<2, 0>(bn - bnK, ub), ER + 2 * E - 1 - XB);
 
+    i64 dm = 0;
     if (HLLD && alfven) {
         // the other side's star state and the states between the Alfven waves
         // (Gas_Dinamic.cu:1371-1430); v3 = vO + w (vK - vO) + ..., w = sK / (sK + sO)
@@ -358,7 +378,8 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
             return false;
         const i64 sb3 = mulk<2, 1>(SM, bn) + asr(mulk<2, 1>(v3, bt3), vb) +
                         asr(mulk<2, 1>(w3, bz3), 2 * f.z);
-        mt += shift(mulk<2, 1>(mulk<0, 0>(RK.m, S2), v3 - vK), ER - RK.e);
+        dm = shift(mulk<2, 1>(mulk<0, 0>(RK.m, S2), v3 - vK), ER - RK.e);
+        mt += dm;
         ft += mulk<2, 1>(S2, bt3 - K.bt);
         fz += mulk<2, 1>(S2, bz3 - K.bz);
         const i64 de = shift(mulk<1, 2>(mulk<2, 0>(sK, sb - sb3), S2), ER + E - kK - X.b - 2);
@@ -369,6 +390,16 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     F.e = to_double(e, ER + 3 * E - 61);
     F.bt = to_double(ft, E + X.b - 61 - f.tb);
     F.bz = to_double(fz, E + X.b - 61 - f.z);
+    if (f.w != 0) {
+        // what w multiplies in the energy flux: the momentum flux, but for guarded star states
+        const i64 yt = (mulk<2, 1>(qsg, btK - K.bt) << 1) - K.bt;
+        const i64 et = (mulk<1, 2>(M, ut) >> imin(z + dR, 63)) + dm +
+                       shift(mulk<0, 0>(bn, yt) + mulk<0, 0>(bn - bnK, btK), st);
+        const double w = to_double(f.w, X.t - 61), et_d = to_double(et, ER + 2 * E - 59 - f.tv);
+        F.e = std::fma(w, std::fma(0.5 * w, F.m, et_d), F.e);
+        F.mt = std::fma(w, F.m, F.mt);
+        F.bt = std::fma(-w, to_double(bnK, X.b - 61), F.bt);
+    }
     return true;
 }
 
