@@ -265,7 +265,7 @@ struct TileMemInt {
 // One face of a tile: faces 0 .. NFX-1 have an x normal, the rest a y normal.
 template <int TX, int TY>
 struct Face {
-    static constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
+    static constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1), kAll = NFX + NFY;
     bool isx, used;
     int lx, ly;
     // used: inside the grid, and next to a cell that the step updates
@@ -514,7 +514,7 @@ __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT
 
     // ---- F: faces ---------------------------------------------------------------------------
     Speeds fastest{0.0, 0.0};
-    for (int i = tid; i < Face<TX, TY>::NFX + Face<TX, TY>::NFY; i += NT) {
+    for (int i = tid; i < Face<TX, TY>::kAll; i += NT) {
         const Face<TX, TY> f(P, tx0, ty0, i);
         if (f.used) fastest.take(f.isx, value_of(face_flux<T, ORDER, TX, TY>(P, mem, f)));
     }
@@ -540,19 +540,18 @@ __device__ __noinline__ FluxE<double> float_flux(const Params& P, const double* 
     return flux_of(P, qa, qb, UU);
 }
 
-// The faces of a thread that the integer solver left (bit k: the k-th), in floating point from the
-// cells themselves.  Out of line, and after the loop over the faces: a second solver inside it
-// would take registers from every face for what a few need.  speed: the faces whose wave speed is
-// missing too.
+// The faces that the integer solver left, in floating point from the cells themselves.  Out of
+// line, and after the loop over the faces: a second solver inside it would take registers from
+// every face for what a few need; and as a list for the whole block, so that a few faces of each
+// warp cost what they are (a step of 1024^2 cells with densities and pressures at random over 2^6:
+// 239 us, 489 with each thread redoing its own).
 template <int ORDER, int TX, int TY, int NT>
 __device__ __noinline__ void faces_left(const Params& P, const CPlanes& in, double* smem, int tx0,
-                                        int ty0, unsigned int left, unsigned int speed,
+                                        int ty0, const LeftFaces<Face<TX, TY>::kAll>& left,
                                         Speeds& u) {
     const TileMemInt<ORDER, TX, TY> t(smem);
-    while (left) {
-        const int k = __ffs((int)left) - 1;
-        left &= left - 1;
-        const Face<TX, TY> w(P, tx0, ty0, threadIdx.x + k * NT);
+    for (unsigned int k = threadIdx.x; k < left.n; k += NT) {
+        const Face<TX, TY> w(P, tx0, ty0, left.face(k));
         const int gx = tx0 + w.lx, gy = ty0 + w.ly, sx = w.isx ? 1 : 0, sy = w.isx ? 0 : 1;
         double c[4][NF], qa[NF], qb[NF], UU;
         load_cell(P, in, gx - sx, gy - sy, c[1]);
@@ -575,19 +574,18 @@ __device__ __noinline__ void faces_left(const Params& P, const CPlanes& in, doub
         const double lb[NF] = {qb[0], qb[1], w.isx ? qb[2] : qb[3], w.isx ? qb[3] : qb[2]};
         const FluxE<double> F = float_flux(P, la, lb, UU);
         w.store(t.fx, t.fy, F.m, F.e, F.mn, F.mt);
-        if (speed & (1u << k)) u.take(w.isx, UU);
+        if (left.no_speed(k)) u.take(w.isx, UU);
     }
 }
 
-// Every face of a tile.  dt_only: the wave speeds alone.
+// Every face of a tile, up to those left.  dt_only: the wave speeds alone.
 template <bool HLL, int ORDER, int TX, int TY, int NT>
-__device__ __forceinline__ void faces(const Params& P, const CPlanes& in, double* smem, int tx0,
-                                      int ty0, int dt_only, Speeds& u) {
+__device__ __forceinline__ void faces(const Params& P, double* smem, int tx0, int ty0, int dt_only,
+                                      LeftFaces<Face<TX, TY>::kAll>& left, Speeds& u) {
     using S = Shape<ORDER, TX, TY>;
     using fx::i64;
     const TileMemInt<ORDER, TX, TY> t(smem);
-    unsigned int left = 0, speed = 0, bit = 1;
-    for (int i = threadIdx.x; i < Face<TX, TY>::NFX + Face<TX, TY>::NFY; i += NT, bit <<= 1) {
+    for (int i = threadIdx.x; i < Face<TX, TY>::kAll; i += NT) {
         const Face<TX, TY> w(P, tx0, ty0, i);
         if (!w.used) continue;
         const int c = (w.ly + S::H) * S::SX + w.lx + S::H, st = w.isx ? 1 : S::SX;
@@ -599,11 +597,9 @@ __device__ __forceinline__ void faces(const Params& P, const CPlanes& in, double
                                                           w.isx, a, b, top))
             done = fx::euler_flux<HLL>(a, b, top, P.gas, F, UU, speed_ok, dt_only);
         if (speed_ok) u.take(w.isx, UU);
-        else speed |= bit;
-        if (!done) left |= bit;
+        if (!done) left.add(i, speed_ok);
         else if (!dt_only) w.store(t.fx, t.fy, F[0], F[3], F[1], F[2]);
     }
-    if (left) faces_left<ORDER, TX, TY, NT>(P, in, smem, tx0, ty0, left, speed, u);
 }
 
 // One TX x TY tile of the step whose lower-left cell is (tx0, ty0).  Reads `in`, writes `out`,
@@ -618,6 +614,8 @@ __device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, co
     using S = Shape<ORDER, TX, TY>;
     constexpr int H = S::H, SX = S::SX, SY = S::SY;
     const TileMemInt<ORDER, TX, TY> t(smem);
+    __shared__ LeftFaces<Face<TX, TY>::kAll> left;
+    if (threadIdx.x == 0) left.n = 0;
     const int N = P.N, M = P.M;
     for (int i = threadIdx.x; i < SY * SX; i += NT) {
         const int ly = i / SX, lx = i - ly * SX;
@@ -637,10 +635,14 @@ __device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, co
     __syncthreads();
     Speeds fastest{0.0, 0.0};
     if (METHODS == 2 || (METHODS == 3 && P.method == GD_METHOD_HLL))
-        faces<true, ORDER, TX, TY, NT>(P, in, smem, tx0, ty0, dt_only, fastest);
+        faces<true, ORDER, TX, TY, NT>(P, smem, tx0, ty0, dt_only, left, fastest);
     else
-        faces<false, ORDER, TX, TY, NT>(P, in, smem, tx0, ty0, dt_only, fastest);
+        faces<false, ORDER, TX, TY, NT>(P, smem, tx0, ty0, dt_only, left, fastest);
     __syncthreads();
+    if (left.n != 0) {
+        faces_left<ORDER, TX, TY, NT>(P, in, smem, tx0, ty0, left, fastest);
+        __syncthreads();
+    }
     update_cells<double, ORDER, TX, TY, NT, TX, TX * TY>(P, out, tx0, ty0, T_do, dt_only, t.cell, t.fx,
                                                      t.fy, res, aux);
     res.umax_x = fastest.x;

@@ -153,23 +153,20 @@ struct FaceH {
     }
 };
 
-// The faces of a thread that the integer solver left (bit k: the k-th), in floating point; speed:
-// those whose wave speed is missing too.
+// The faces that the integer solver left, in floating point.
 __device__ __noinline__ void faces_left(const Params& P, double* smem, const unsigned char* flag,
-                                        unsigned int left, unsigned int speed, double& umax_x,
+                                        const LeftFaces<NFX + NFY>& left, double& umax_x,
                                         double& umax_y) {
     const double *pA = smem + kUnion, *pDX = pA + kPred, *pDY = pDX + kPred;
-    while (left) {
-        const int k = __ffs((int)left) - 1;
-        left &= left - 1;
-        const FaceH w(flag, threadIdx.x + k * NT);
+    for (unsigned int k = threadIdx.x; k < left.n; k += NT) {
+        const FaceH w(flag, left.face(k));
         double qa[NF], qb[NF], UU;
         w.states(pA, w.isx ? pDX : pDY, qa, qb);
         Side<double> A, B;
         side(A, qa[0], qa[1], qa[2], qa[3], qa[4], qa[5], qa[6], P);
         side(B, qb[0], qb[1], qb[2], qb[3], qb[4], qb[5], qb[6], P);
         w.store(smem, smem + kFx, hlld_local(A, B, GD_METHOD_HLLD, P, UU));
-        if (speed >> k & 1) {
+        if (left.no_speed(k)) {
             if (w.isx) umax_x = max_nonneg(umax_x, UU);
             else umax_y = max_nonneg(umax_y, UU);
         }
@@ -195,8 +192,10 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
     double* rowiy = rowy + PY;     // its reciprocal
     double* colx = rowiy + PY;     // x of the tile's columns
     unsigned char* flag = reinterpret_cast<unsigned char*>(colx + TX);  // [TY][TX]
+    __shared__ LeftFaces<NFX + NFY> left;
 
     const int tid = threadIdx.x;
+    if (tid == 0) left.n = 0;
     const int N = P.N, M = P.M;
     const int tx0 = 2 + blockIdx.x * TX, ty0 = 2 + (blockIdx.y + P.tile_row0) * TY;
 
@@ -336,8 +335,7 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
     // two states of a face in units of their own; the corrector and the predictor keep the FP64
     // pipe (the flux took 240 of the step's 671 FP64 operations a cell)
     double umax_x = 0.0, umax_y = 0.0;
-    unsigned int left = 0, speed = 0, bit = 1;
-    for (int i = tid; i < NFX + NFY; i += NT, bit <<= 1) {
+    for (int i = tid; i < NFX + NFY; i += NT) {
         const FaceH w(flag, i);
         if (!w.used) continue;
         double qa[NF], qb[NF], UU;
@@ -348,14 +346,18 @@ __global__ void __launch_bounds__(NT, 2) hancock_tile_kernel(const __grid_consta
         bool speed_ok = false, done = false;
         if (fx::face_units(qa, qb, P.gas, a, b, top))
             done = fx::mhd_face_flux<true>(a, b, top, P.gas, F, UU, speed_ok, dt_only);
-        if (!speed_ok) speed |= bit;
-        else if (w.isx) umax_x = max_nonneg(umax_x, UU);
-        else umax_y = max_nonneg(umax_y, UU);
-        if (!done) left |= bit;
+        if (speed_ok) {
+            if (w.isx) umax_x = max_nonneg(umax_x, UU);
+            else umax_y = max_nonneg(umax_y, UU);
+        }
+        if (!done) left.add(i, speed_ok);
         else if (!dt_only) w.store(fx, fy, F);
     }
-    if (left) faces_left(P, smem, flag, left, speed, umax_x, umax_y);
     __syncthreads();
+    if (left.n != 0) {
+        faces_left(P, smem, flag, left, umax_x, umax_y);
+        __syncthreads();
+    }
 
     // ---- U: corrector (kernel.cu:3256-3281, Pdiv = 0) --------------------------------------
     unsigned int nfl_r = 0, nfl_p = 0, nbad = 0;

@@ -154,7 +154,7 @@ struct MhdTileResult {
 // One face of a tile: faces 0 .. NFX-1 have an x normal, the rest a y normal.
 template <int TY>
 struct FaceM {
-    static constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1);
+    static constexpr int NFX = (TX + 1) * TY, NFY = TX * (TY + 1), kAll = NFX + NFY;
     bool isx, used;
     int lx, ly;
     // used: inside the grid, and next to a cell that the step updates
@@ -480,18 +480,17 @@ __device__ __forceinline__ void load_cell(const Params& P, const CPlanes& in, in
     for (int f = 4; f < NF; ++f) v[f] = __dmul_rn(v[f], kInvSpi4);
 }
 
-// The faces of a thread that the integer solver left (bit k: the k-th), in floating point from the
-// cells themselves; speed: those whose wave speed is missing too.  Out of line and after the loop
-// over the faces, so that it takes no registers from it.
+// The faces that the integer solver left, in floating point from the cells themselves.  Out of
+// line and after the loop over the faces, so that it takes no registers from it; a list for the
+// whole block, so that a few faces of each warp cost what they are (an HLLD step of 1024^2 cells with
+// densities and pressures at random over 2^6: 776 us, 1549 with each thread redoing its own).
 template <int ORDER, int TY, int NT>
 __device__ __noinline__ void faces_left(const Params& P, const CPlanes& in, double* smem, int tx0,
-                                        int ty0, unsigned int left, unsigned int speed,
+                                        int ty0, const LeftFaces<FaceM<TY>::kAll>& left,
                                         SpeedsM& u) {
     const MemInt<ORDER, TY> t(smem);
-    while (left) {
-        const int k = __ffs((int)left) - 1;
-        left &= left - 1;
-        const FaceM<TY> w(P, tx0, ty0, threadIdx.x + k * NT);
+    for (unsigned int k = threadIdx.x; k < left.n; k += NT) {
+        const FaceM<TY> w(P, tx0, ty0, left.face(k));
         const int gx = tx0 + w.lx, gy = ty0 + w.ly, sx = w.isx ? 1 : 0, sy = w.isx ? 0 : 1;
         double c[4][NF], qa[NF], qb[NF], UU;
         load_cell(P, in, gx - sx, gy - sy, c[1]);
@@ -511,7 +510,7 @@ __device__ __noinline__ void faces_left(const Params& P, const CPlanes& in, doub
             qb[w.field(f)] = b;
         }
         w.store(t.fx, t.fy, float_flux_of(P, qa, qb, UU));
-        if (speed & (1u << k)) u.take(w.isx, UU);
+        if (left.no_speed(k)) u.take(w.isx, UU);
     }
 }
 
@@ -537,7 +536,9 @@ __device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, co
     using fx::i64;
     constexpr int H = S::H, SX = S::SX, SY = S::SY, FS = SY * SX;
     const MemInt<ORDER, TY> t(smem);
+    __shared__ LeftFaces<FaceM<TY>::kAll> left;
     const int tid = threadIdx.x, N = P.N, M = P.M;
+    if (tid == 0) left.n = 0;
     for (int i = tid; i < FS; i += NT) {
         const int ly = i / SX - H, lx = i % SX - H;
         const bool xh = lx < 0 || lx >= TX, yh = ly < 0 || ly >= TY;
@@ -560,8 +561,7 @@ __device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, co
     __syncthreads();
 
     SpeedsM u{0.0, 0.0};
-    unsigned int left = 0, speed = 0, bit = 1;
-    for (int i = tid; i < FaceM<TY>::NFX + FaceM<TY>::NFY; i += NT, bit <<= 1) {
+    for (int i = tid; i < FaceM<TY>::kAll; i += NT) {
         const FaceM<TY> w(P, tx0, ty0, i);
         if (!w.used) continue;
         const int c = (w.ly + H) * SX + w.lx + H, st = w.isx ? 1 : SX;
@@ -574,13 +574,15 @@ __device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, co
             fx::face_states<NF, ORDER>(t.q + c, st, FS, t.key + c, st, w.isx, a, b, top))
             done = fx::mhd_face_flux<HLLD>(a, b, top, P.gas, F, UU, speed_ok, dt_only);
         if (speed_ok) u.take(w.isx, UU);
-        else speed |= bit;
-        if (!done) left |= bit;
+        if (!done) left.add(i, speed_ok);
         else if (!dt_only)
             w.store(t.fx, t.fy, FluxM<double>{F.m, F.mn, F.mt, F.e, F.bn, F.bt, F.bz});
     }
-    if (left) faces_left<ORDER, TY, NT>(P, in, smem, tx0, ty0, left, speed, u);
     __syncthreads();
+    if (left.n != 0) {
+        faces_left<ORDER, TY, NT>(P, in, smem, tx0, ty0, left, u);
+        __syncthreads();
+    }
 
     update_cells<double, NT, TY, TX, TX * TY>(P, in, out, tx0, ty0, T_do, dt_only, t.cell,
                                           JumpCells<TY>{t.cell, t.edgex, t.edgey}, t.fx, t.fy,

@@ -663,6 +663,21 @@ __device__ __forceinline__ bool dt_above(double krad, unsigned long long u, doub
     return seed_f32(krad) * r > seed_f32(T) * 1.000244140625f;
 }
 
+// The faces of a tile that the integer solver left to floating point, in shared memory; n = 0
+// before the first add.  In any order: each face has its own place among the fluxes.
+template <int MAX>
+struct LeftFaces {
+    unsigned int n;
+    unsigned short list[MAX];
+    static_assert(MAX < 0x8000, "a bit beside the index");
+    __device__ __forceinline__ void add(int i, bool speed) {
+        list[atomicAdd(&n, 1u)] = (unsigned short)(i | (speed ? 0 : 0x8000));
+    }
+    __device__ __forceinline__ int face(unsigned int k) const { return list[k] & 0x7fff; }
+    // its wave speed is missing as well
+    __device__ __forceinline__ bool no_speed(unsigned int k) const { return list[k] >> 15; }
+};
+
 // Reduces the per-thread maximum wave speeds of x and y faces over the block, turns them
 // into the block's dt (min over faces of krit*rad/UU, capped at 1000) and min-combines it
 // into *T_bits.  `any_active` says whether the block contains a non-frozen cell.  Then,
