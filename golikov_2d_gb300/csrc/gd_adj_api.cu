@@ -277,25 +277,33 @@ gd_status gd_tangent(gd_ctx* ctx, const double* vs, const double* vu, const doub
     const long long K = ctx->K;
     const int nf = ctx->nf;
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t state = sizeof(double) * (size_t)nf * K;
     double* t[2] = {a->lam, a->lam + (size_t)nf * K};
-    double* u[2] = {a->seg, a->seg + (size_t)nf * K};
-    a->seg_holds = -1;  // seg is the work space of this sweep
     GD_TRY(gd::launch_aos_to_soa(vs, vu, vb, planes_at(t[0], nf, K), K, nf, st));
-    GD_TRY(cudaMemcpyAsync(u[0], a->ckpt, state, cudaMemcpyDeviceToDevice, st));
+    // The values are the recorded run's: the tangent kernel's own, in FP64 throughout, part from
+    // the step's by rounding, and a run through ties and shocks makes that 3e-4 of the derivative
+    // after 100 steps.  A segment that a buffer holds is read from it (17.3 -> 15.0 ms for 20 MHD steps
+    // at 512^2 in two segments, 5.6 -> 4.7 Euler); any other is stepped again from its checkpoint, in
+    // the scratch planes of the reverse sweep (two states: 14 and 8 planes).
     int c = 0;
+    const double* u = nullptr;  // the input state of step k
     for (int k = 0; k < a->nsteps; ++k) {
-        const CPlanes ui = cplanes_at(u[c], nf, K), ti = cplanes_at(t[c], nf, K);
-        const Planes uo = planes_at(u[c ^ 1], nf, K), to = planes_at(t[c ^ 1], nf, K);
-        GD_TRY(nf == 7 ? gd::launch_mhd_tangent(ctx->P, ui, ti, uo, to, a->dts + k, st)
-                       : gd::launch_euler_tangent(ctx->P, ui, ti, uo, to, a->dts + k, st));
-        // The values are the recorded run's: the tangent kernel's own, in FP64 throughout, part
-        // from the step's by rounding, and a run through ties and shocks makes that 3e-4 of the
-        // derivative after 100 steps.
-        GD_TRY(step_aux(ctx, ctx->P, ui, uo, a->dts + k, (unsigned long long*)a->tbits, nullptr,
-                        nullptr, nullptr, st));
-        ctx->launches += 2;
+        const int sg = k / a->every, j = k - sg * a->every;
+        const double* held = a->seg_holds == sg ? a->seg : (a->seg2_holds == sg ? a->seg2 : nullptr);
+        if (held) u = held + (size_t)j * nf * K;
+        else if (j == 0) u = a->ckpt + (size_t)sg * nf * K;
+        const CPlanes ui = cplanes_at(u, nf, K), ti = cplanes_at(t[c], nf, K);
+        const Planes to = planes_at(t[c ^ 1], nf, K);
+        GD_TRY(nf == 7 ? gd::launch_mhd_tangent(ctx->P, ui, ti, to, a->dts + k, st)
+                       : gd::launch_euler_tangent(ctx->P, ui, ti, to, a->dts + k, st));
+        ctx->launches += 1;
         c ^= 1;
+        if (!held && j + 1 < a->every && k + 1 < a->nsteps) {
+            double* next = a->scratch + (size_t)(j & 1) * nf * K;
+            GD_TRY(step_aux(ctx, ctx->P, ui, planes_at(next, nf, K), a->dts + k,
+                            (unsigned long long*)a->tbits, nullptr, nullptr, nullptr, st));
+            ctx->launches += 1;
+            u = next;
+        }
     }
     GD_TRY(gd::launch_soa_to_aos(cplanes_at(t[c], nf, K), os, ou, ob, K, nf, st));
     return GD_OK;

@@ -198,8 +198,8 @@ struct Shape {
 struct DualIn {
     CPlanes v, d;
 };
-struct DualOut {
-    Planes v, d;
+struct DualOut {  // the tangent alone: the values are the recorded run's
+    Planes d;
 };
 
 __device__ __forceinline__ void load_cell(const Params& P, const CPlanes& in, int gx, int gy,
@@ -230,7 +230,6 @@ __device__ __forceinline__ void store_cell2(const DualOut& out, long long k, int
     store_cell(out, k, f0 + 1, b);
 }
 __device__ __forceinline__ void store_cell(const DualOut& out, long long k, int f, Dual x) {
-    out.v.f[f][k] = x.v;
     out.d.f[f][k] = x.d;
 }
 
@@ -673,19 +672,19 @@ __global__ void __launch_bounds__(NT, NT == kNT ? kCtas<TX, TY> : 1) euler_fast_
     block_dt_and_rotate<NT>(P, r.umax_x, r.umax_y, r.any_active, T_bits, rot, P.tile_nblocks);
 }
 
-// Tangent of one step: (U, dU) -> (U', dU') with the dt read from *T_do_ptr (held fixed):
+// Tangent of one step: (U, dU) -> dU' with the dt read from *T_do_ptr (held fixed):
 // the same tile instantiated with Dual values.  32 x 8 tiles: a Dual tile holds twice the
 // bytes of a double one (101 KB at second order), so two CTAs fit on an SM (at 32 x 16, 186 KB,
 // one).
 constexpr int kTanTX = 32, kTanTY = 8;
 template <int ORDER>
 __global__ void __launch_bounds__(kNTTan) euler_tangent_kernel(Params P, CPlanes in, CPlanes din,
-                                                           Planes out, Planes dout,
+                                                           Planes dout,
                                                            const double* __restrict__ T_do_ptr) {
     extern __shared__ __align__(16) double smem[];
     TileResult r;
     const DualIn I{in, din};
-    const DualOut O{out, dout};
+    const DualOut O{dout};
     euler_tile<Dual, ORDER, kTanTX, kTanTY, kNTTan>(P, I, O, blockIdx.x * kTanTX, blockIdx.y * kTanTY,
                                             *T_do_ptr, 0, reinterpret_cast<Dual*>(smem), r,
                                             nullptr);
@@ -917,15 +916,14 @@ cudaError_t launch_euler_fast(const Params& P, const CPlanes& in, const Planes& 
 }
 
 cudaError_t launch_euler_tangent(const Params& P, const CPlanes& in, const CPlanes& din,
-                                 const Planes& out, const Planes& dout, const double* T_do,
-                                 cudaStream_t st) {
+                                 const Planes& dout, const double* T_do, cudaStream_t st) {
     const dim3 grid((P.N + kTanTX - 1) / kTanTX, (P.M + kTanTY - 1) / kTanTY);
     if (P.order == 1)
         euler_tangent_kernel<1><<<grid, kNTTan, Shape<1, kTanTX, kTanTY>::dual_bytes, st>>>(
-            P, in, din, out, dout, T_do);
+            P, in, din, dout, T_do);
     else
         euler_tangent_kernel<2><<<grid, kNTTan, Shape<2, kTanTX, kTanTY>::dual_bytes, st>>>(
-            P, in, din, out, dout, T_do);
+            P, in, din, dout, T_do);
     return cudaGetLastError();
 }
 

@@ -53,8 +53,8 @@ constexpr int NF = 7;  // rho, p, vx, vy, bx, by, bz
 struct DualCPlanes {
     CPlanes v, d;
 };
-struct DualPlanes {
-    Planes v, d;
+struct DualPlanes {  // the tangent alone: the values are the recorded run's
+    Planes d;
 };
 
 __device__ __forceinline__ void load_state(const Params& P, const CPlanes& in, int gx, int gy,
@@ -100,7 +100,6 @@ __device__ __forceinline__ void store_state2(const DualPlanes& out, long long k,
     store_state(out, k, f0 + 1, b);
 }
 __device__ __forceinline__ void store_state(const DualPlanes& out, long long k, int f, Dual x) {
-    out.v.f[f][k] = x.v;
     out.d.f[f][k] = x.d;
 }
 __device__ __forceinline__ void copy_cell(const CPlanes& in, const Planes& out, long long k) {
@@ -110,10 +109,7 @@ __device__ __forceinline__ void copy_cell(const CPlanes& in, const Planes& out, 
 __device__ __forceinline__ void copy_cell(const DualCPlanes& in, const DualPlanes& out,
                                           long long k) {
 #pragma unroll
-    for (int f = 0; f < NF; ++f) {
-        out.v.f[f][k] = in.v.f[f][k];
-        out.d.f[f][k] = in.d.f[f][k];
-    }
+    for (int f = 0; f < NF; ++f) out.d.f[f][k] = in.d.f[f][k];
 }
 
 // The tangent's tile.
@@ -610,16 +606,16 @@ __global__ void __launch_bounds__(NT, NT == kNT ? 2 : 1) mhd_fast_kernel(const _
     block_dt_and_rotate<NT>(P, r.umax_x, r.umax_y, r.any_active, T_bits, rot, P.tile_nblocks);
 }
 
-// Tangent of one step: (U, dU) -> (U', dU') with the dt read from *T_do_ptr (held fixed).
+// Tangent of one step: (U, dU) -> dU' with the dt read from *T_do_ptr (held fixed).
 template <int ORDER, int TY>
 __global__ void __launch_bounds__(NTDual) mhd_tangent_kernel(const __grid_constant__ Params P,
                                                          CPlanes in, CPlanes din,
-                                                         Planes out, Planes dout,
+                                                         Planes dout,
                                                          const double* __restrict__ T_do_ptr) {
     extern __shared__ __align__(16) double smem[];
     MhdTileResult r;
     const DualCPlanes I{in, din};
-    const DualPlanes O{out, dout};
+    const DualPlanes O{dout};
     mhd_tile<Dual, NTDual, ORDER, TY>(P, I, O, blockIdx.x * TX, blockIdx.y * TY, *T_do_ptr, 0,
                               reinterpret_cast<Dual*>(smem), r, nullptr);
 }
@@ -659,11 +655,10 @@ cudaError_t launch_t(const Params& P, const CPlanes& in, const Planes& out, cons
 
 template <int ORDER>
 cudaError_t launch_tangent_t(const Params& P, const CPlanes& in, const CPlanes& din,
-                             const Planes& out, const Planes& dout, const double* T_do,
-                             cudaStream_t st) {
+                             const Planes& dout, const double* T_do, cudaStream_t st) {
     dim3 grid((P.N + TX - 1) / TX, (P.M + kTYDual - 1) / kTYDual);
     mhd_tangent_kernel<ORDER, kTYDual><<<grid, NTDual, SmemM<Dual, ORDER, kTYDual>::bytes, st>>>(
-        P, in, din, out, dout, T_do);
+        P, in, din, dout, T_do);
     return cudaGetLastError();
 }
 
@@ -712,10 +707,9 @@ cudaError_t launch_mhd_fast_aux(const Params& P, const CPlanes& in, const Planes
 }
 
 cudaError_t launch_mhd_tangent(const Params& P, const CPlanes& in, const CPlanes& din,
-                               const Planes& out, const Planes& dout, const double* T_do,
-                               cudaStream_t st) {
-    if (P.order == 1) return launch_tangent_t<1>(P, in, din, out, dout, T_do, st);
-    return launch_tangent_t<2>(P, in, din, out, dout, T_do, st);
+                               const Planes& dout, const double* T_do, cudaStream_t st) {
+    if (P.order == 1) return launch_tangent_t<1>(P, in, din, dout, T_do, st);
+    return launch_tangent_t<2>(P, in, din, dout, T_do, st);
 }
 
 

@@ -15,10 +15,9 @@ cudaError_t prepare_mhd_fast();
 // Fast face-once step.  `rot` (may be null) receives the fused funk_time rotation by the
 // last block; `ctr` (may be null) receives floor / non-finite counters.  dt_only != 0
 // computes only the dt minimum.
-// Tangent of one Euler step (value and derivative planes), dt read from *T_do.
+// Tangent of one Euler step, (in, din) -> dout, dt read from *T_do.
 cudaError_t launch_euler_tangent(const Params& P, const CPlanes& in, const CPlanes& din,
-                                 const Planes& out, const Planes& dout, const double* T_do,
-                                 cudaStream_t st);
+                                 const Planes& dout, const double* T_do, cudaStream_t st);
 // The Euler step (variant 0, as gd_advance launches it) writing its flux differences d[0..3] per cell to `aux`.
 cudaError_t launch_euler_fast_aux(const Params& P, const CPlanes& in, const Planes& out,
                                   const double* T_do, unsigned long long* T_bits, Scalars* rot,
@@ -66,10 +65,9 @@ cudaError_t launch_euler_batch(int variant, int order, const BatchGrid* grids, c
                                bool hllc_only, cudaStream_t st);
 
 // Tangent (forward-mode JVP) of one fast MHD step with the dt read from *T_do:
-// (in, din) -> (out, dout).
+// (in, din) -> dout.
 cudaError_t launch_mhd_tangent(const Params& P, const CPlanes& in, const CPlanes& din,
-                               const Planes& out, const Planes& dout, const double* T_do,
-                               cudaStream_t st);
+                               const Planes& dout, const double* T_do, cudaStream_t st);
 
 // Fast MHD step that also stores, per cell, the flux differences and the Powell term the
 // update used (8 planes of N*M in `aux`), for the adjoint.  `rot` / `ctr` as in
