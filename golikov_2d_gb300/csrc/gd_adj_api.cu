@@ -206,13 +206,16 @@ gd_status gd_adj_backward(gd_ctx* ctx, const double* gs, const double* gu, const
         *len = k1 - *k0;
     };
     // the input states and update terms of every step of segment sg, into buffer b
+    Params beside = P;  // on the side stream the steps run beside the reversal
+    beside.few_tiles = 0;
     auto recompute = [&](int sg, int b, cudaStream_t s) -> gd_status {
+        const Params& Q = s == st ? P : beside;
         int k0, len;
         seg_range(sg, &k0, &len);
         GD_TRY(cudaMemcpyAsync(segb[b], a->ckpt + (size_t)sg * nf * K, state,
                                cudaMemcpyDeviceToDevice, s));
         for (int j = 0; j < len; ++j) {
-            GD_TRY(step_aux(ctx, P, cplanes_at(segb[b] + (size_t)j * nf * K, nf, K),
+            GD_TRY(step_aux(ctx, Q, cplanes_at(segb[b] + (size_t)j * nf * K, nf, K),
                             planes_at(segb[b] + (size_t)(j + 1) * nf * K, nf, K),
                             a->dts + k0 + j, (unsigned long long*)a->tbits, nullptr, nullptr,
                             auxb[b] + (size_t)j * aux_planes(ctx) * K, s));

@@ -102,8 +102,18 @@ void frozen_bounds(const gd_config& c, Params& P) {
     P.f_out = (float)(R * R + m);
 }
 
+// SMs of the current device (0 where there is none: gd_create reports that itself)
+int sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        cudaGetLastError();
+    return sms;
+}
+
 Params make_params(const gd_config& c) {
     Params P{};
+    P.few_tiles = sm_count();
     P.N = c.N;
     P.M = c.M;
     P.physics = c.physics;

@@ -49,13 +49,12 @@ constexpr int kNT = 256;  // threads of a tile: single-grid step
 // The tangent's 552 faces in two rounds: 20 tangent steps at 512^2 take 5.55 ms, 5.79 with 256
 // threads, 6.17 with 384.
 constexpr int kNTTan = 288;
-// Threads of a tile of the 16x16 shape where every tile has an SM to itself (152 of them): the
+// Threads of a tile of the 16x16 shape where every tile has an SM to itself (Params::few_tiles): the
 // step is then one tile's latency, and 576 threads take its 544 faces in one round instead of
 // three: 11.7 against 13.5 us at 64x48, 12.1 against 13.9 at 192x192 (144 tiles; 288 threads:
 // 12.8).  From two tiles per SM on (156 tiles: 18.9 against 16.4 us) the 256-thread tiles share
 // an SM better.  The threads of a tile change no result: faces and cells are independent.
 constexpr int kNTFew = 576;
-constexpr long long kFewTiles = 152;
 constexpr int NF = 4;
 // CTAs per SM that the shared memory of a tile shape leaves room for
 template <int TX, int TY>
@@ -799,7 +798,7 @@ cudaError_t launch_single(const Params& P, const CPlanes& in, const Planes& out,
                           Scalars* ctr, int dt_only, cudaStream_t st, double* aux = nullptr) {
     const dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + TY - 1) / TY);
     if constexpr (TX == 16 && TY == 16) {
-        if ((long long)grid.x * grid.y <= kFewTiles) {
+        if ((long long)grid.x * grid.y <= P.few_tiles) {
             launch_tiles<ORDER, TX, TY, kNTFew>(P, grid, in, out, T_do, T_bits, rot, ctr, dt_only,
                                                 st, aux);
             return cudaGetLastError();

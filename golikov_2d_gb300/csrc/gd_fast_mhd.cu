@@ -38,11 +38,10 @@ namespace {
 
 constexpr int TX = 32;
 constexpr int kNT = 384;  // threads of the step (see kTY)
-// Threads where every tile has an SM to itself (152 of them): the step is one tile's latency, and
+// Threads where every tile has an SM to itself (Params::few_tiles): the step is one tile's latency, and
 // 768 threads take its 747 faces in one round: 29.1 against 32.4 us at 64x48, 28.4 against 31.9 at
 // 320x165 (150 tiles).  At 160 tiles 50.0 against 47.0: there the 384-thread tiles stay.
 constexpr int kNTFew = 768;
-constexpr long long kFewTiles = 152;
 // The tangent's: one CTA per SM.  20 tangent steps at 512^2 take 18.4 ms with 256 threads, 17.8
 // with 288, 17.3 with 384, 17.9 with 576.
 constexpr int NTDual = 384;
@@ -646,7 +645,7 @@ cudaError_t launch_t(const Params& P, const CPlanes& in, const Planes& out, cons
                      unsigned long long* T_bits, Scalars* rot, Scalars* ctr, int dt_only,
                      cudaStream_t st, double* aux = nullptr) {
     const dim3 grid((P.N + TX - 1) / TX, P.tile_rows ? P.tile_rows : (P.M + kTY - 1) / kTY);
-    if ((long long)grid.x * grid.y <= kFewTiles)
+    if ((long long)grid.x * grid.y <= P.few_tiles)
         launch_tiles<ORDER, kNTFew>(P, grid, in, out, T_do, T_bits, rot, ctr, dt_only, st, aux);
     else
         launch_tiles<ORDER, kNT>(P, grid, in, out, T_do, T_bits, rot, ctr, dt_only, st, aux);

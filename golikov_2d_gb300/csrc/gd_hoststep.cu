@@ -191,6 +191,8 @@ cudaError_t banded_step(gd_ctx* ctx, const double* s, const double* u, const dou
             nblocks += gd::hancock_fast_blocks(P, row_bound(k), row_bound(k + 1), 2);
     }
     P.tile_nblocks = nblocks;
+    // several bands run at once: a band has no SMs to itself unless the whole grid has
+    if ((long long)nx * T > P.few_tiles) P.few_tiles = 0;
     // in: the AoS staging of the upload; out: the next resident plane set and the AoS
     // staging of the download
     CPlanes in{};

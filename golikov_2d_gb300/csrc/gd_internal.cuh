@@ -43,6 +43,9 @@ struct Params {
     // band launches of one step share one rotation ticket, tile_nblocks (0: this grid's).
     int tile_row0, tile_rows;
     unsigned int tile_nblocks;
+    // Up to how many tiles a launch may count on an SM for each: the device's SMs, or 0 where other
+    // launches share them (gd_step_host's bands, steps recomputed beside a reverse sweep).
+    int few_tiles;
     // derived
     double gm1, inv_gm1, hgm1;  // gamma - 1, 1 / (gamma - 1), (gamma - 1) / 2
     double g_gm1;               // gamma / (gamma - 1)
