@@ -18,6 +18,9 @@ funk_time rotation) over the whole grid.  Metric: FP64 cell-updates/s, whole job
 * cpu_baseline  the oracle (the project's C restatement of the reference step, OpenMP over
             all host cores) timed on a bounded sample of the same workload.
 
+The printed line is the headline, under 1400 characters; the whole result, the secondary
+measurements' long objects included, goes to a file (--details).
+
 --impl reference times the reference path on the host cores (the oracle port: the
 reference's own CUDA sources are compiled for the host only where they are present, and
 they are not on the GPU host) for the same workload, metric and unit.
@@ -943,6 +946,28 @@ def workload_config(workload, cfg, ws):
             "steps_per_launch": 1, "dt": "lagged reference protocol, dt-only pre-pass"}
 
 
+# What the printed line carries of the objects that are longer than it has room for.
+SHORT = {"roofline": ("bound", "frac"), "fp64": ("frac", "ops_per_cell"),
+         "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"),
+         "secondary": ("value", "ms_per_step", "unavailable"),
+         "batched": ("value", "ms_per_step", "unavailable"),
+         "cpu_baseline": ("value", "cores", "kind")}
+DETAILS_ONLY = ("sim", "ot_to_t05", "adjoint", "io", "hancock")
+
+
+def headline(line):
+    """The line to print: the measurement and its conditions, in under 1400 characters whatever
+    the secondary measurements add (a reader that keeps the end of the output still has all of it)."""
+    out = {}
+    for k, v in line.items():
+        if k in DETAILS_ONLY:
+            continue
+        if k in SHORT and isinstance(v, dict):
+            v = {f: v[f][:80] if isinstance(v[f], str) else v[f] for f in SHORT[k] if f in v}
+        out[k] = v
+    return out
+
+
 def run_reference(args):
     ws, rank, _ = dist_info()
     if rank != 0:
@@ -1210,7 +1235,10 @@ def run_gb300(args):
             line["hancock"] = {"unavailable": str(e)}
     if not args.no_cpu_baseline and ws == 1:
         line["cpu_baseline"] = cpu_baseline(args.workload, cfg, s, u, b)
-    print(json.dumps(line), flush=True)
+    with open(args.details, "w") as f:
+        json.dump(line, f, indent=1)
+        f.write("\n")
+    print(json.dumps(headline(line)), flush=True)
     if ws > 1:
         torch.distributed.destroy_process_group()
     return 0
@@ -1229,6 +1257,9 @@ def main():
     ap.add_argument("--adjoint", type=int, default=1)
     ap.add_argument("--io", type=int, default=1)
     ap.add_argument("--hancock", type=int, default=1)
+    ap.add_argument("--details", default=os.path.join(ROOT, "bench_details.json"),
+                    help="file for the whole result, the secondary measurements' long objects "
+                         "included; the printed line is the headline")
     ap.add_argument("--case", default="bench",
                     choices=["bench", "adjoint-step", "adjoint-step-euler", "io", "hancock",
                              "batch-step"],
