@@ -106,9 +106,9 @@ class gd_tecplot_opts(ctypes.Structure):
 _lib = None
 
 # PyBytes_FromStringAndSize: with no string, a bytes object whose contents are still to be written
-_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
-_new_bytes.argtypes = [ctypes.c_void_p, ctypes.c_ssize_t]
-_new_bytes.restype = ctypes.py_object
+# (a prototype of its own: attributes of ctypes.pythonapi's function are every importer's)
+_new_bytes = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_void_p, ctypes.c_ssize_t)(
+    ("PyBytes_FromStringAndSize", ctypes.pythonapi))
 
 
 def lib_path() -> str:

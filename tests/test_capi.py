@@ -134,3 +134,13 @@ def test_every_allocation_goes_through_the_counted_helpers():
     allowed = [("gd_api.cu", "cudaMalloc"), ("gd_api.cu", "cudaMallocHost"),
                ("gd_api.cu", "cudaFree"), ("gd_api.cu", "cudaFreeHost")]
     assert sorted(found) == sorted(allowed), found
+
+
+def test_import_leaves_ctypes_pythonapi_alone():
+    """The wrapper's prototypes are its own: functions of ctypes.pythonapi, shared by everything in
+    the process, keep their defaults."""
+    import ctypes
+    import golikov_2d_gb300 as g
+    f = ctypes.pythonapi.PyBytes_FromStringAndSize
+    assert f.argtypes is None and f.restype is ctypes.c_int
+    assert g._new_bytes(b"abc", 3) == b"abc" and len(g._new_bytes(None, 5)) == 5
