@@ -461,7 +461,8 @@ gd_status gd_advance(gd_ctx* ctx, int nsteps, int use_graph, gd_stream stream) {
         }
         if (ce != cudaSuccess) return cuda_fail(ce);
         cudaGraphExec_t ge = nullptr;
-        ce = cudaGraphInstantiate(&ge, g, 0);
+        // the Hancock band keeps its stream's priority over the tiles
+        ce = cudaGraphInstantiate(&ge, g, cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(g);
         if (ce != cudaSuccess) return cuda_fail(ce);
         it = ctx->graphs.emplace(key, ge).first;
