@@ -216,6 +216,8 @@ __device__ __forceinline__ void side_states(int f, T ca, T da, T cb, T db, T& a,
 }
 
 // ---- U: update (kernel.cu:2606-2660 in Heaviside-Lorentz field units) --------------------------
+// Written so that no product stands alone beside a sum: there is nothing for the compiler to contract
+// in one kernel and not in another, and the step's kernels round alike.
 // cell: the tile's own values, rows RS and fields FS apart; jump: b_x across a cell in x and b_y
 // in y, from its neighbours.  `aux` (T = double only; may be null) receives, per cell, the flux
 // differences d[0..6] and the Powell term divb that the update used (planes of N*M), for the adjoint.
@@ -255,7 +257,7 @@ __device__ __forceinline__ void update_cells(const Params& P, const IN& in, cons
         }
         // Powell divergence from cell-centred field: dx dy div b (kernel.cu:2568-2604)
         T divb = fma(hkx, jump.x(lx, ly), mulx<true>(hky, jump.y(lx, ly)));  // T_do * div b
-        const double iy = axi ? rcp_fast(P.y0 + gy * P.dy) : 0.0;
+        const double iy = axi ? rcp_fast(fma((double)gy, P.dy, P.y0)) : 0.0;
         if (axi) divb = fma(T_do * by, iy, divb);                 // kernel.cu:2615
         if constexpr (std::is_same<T, double>::value) {
             if (aux != nullptr) {
