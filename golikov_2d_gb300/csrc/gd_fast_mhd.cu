@@ -124,8 +124,10 @@ struct SmemM {
     static constexpr int kFy = NF * (TY + 1) * TX;
     static constexpr size_t bytes = sizeof(T) * (kPrim + kSlx + kSly + kFx + kFy);
 };
-// The step's tile: the cells' significands and keys (gd_fixed.cuh), the tile's own values, and
-// b_x beside the tile in x and b_y in y.
+// The step's tile: the cells' significands and keys (gd_fixed.cuh), and b_x and b_y of the tile's
+// cells and of those beside them in x and in y.  The update reads the other values again from global
+// memory: with all seven here (102 KB a tile) the rest of the L1 was too small for the face code's
+// spills (vortex of 1024^2, four steps: 1.90 against 1.88 ms).
 template <int ORDER, int TY>
 struct ShapeInt {
     static constexpr int H = ORDER == 2 ? 2 : 1;
@@ -133,7 +135,7 @@ struct ShapeInt {
     static constexpr int SY = TY + 2 * H;
     static constexpr int kKey = 2 * SY * SX;
     static constexpr int kPrim = NF * SY * SX;
-    static constexpr int kCell = NF * TX * TY;
+    static constexpr int kCell = 2 * TX * TY;
     static constexpr int kEdge = 2 * (TX + TY);
     static constexpr int kFx = NF * TY * (TX + 1);
     static constexpr int kFy = NF * (TY + 1) * TX;
@@ -218,12 +220,12 @@ __device__ __forceinline__ void side_states(int f, T ca, T da, T cb, T db, T& a,
 // ---- U: update (kernel.cu:2606-2660 in Heaviside-Lorentz field units) --------------------------
 // Written so that no product stands alone beside a sum: there is nothing for the compiler to contract
 // in one kernel and not in another, and the step's kernels round alike.
-// cell: the tile's own values, rows RS and fields FS apart; jump: b_x across a cell in x and b_y
+// cell: a cell's values; jump: b_x across a cell in x and b_y
 // in y, from its neighbours.  `aux` (T = double only; may be null) receives, per cell, the flux
 // differences d[0..6] and the Powell term divb that the update used (planes of N*M), for the adjoint.
-template <class T, int BT, int TY, int RS, int FS, class IN, class OUT, class JUMP>
+template <class T, int BT, int TY, class IN, class OUT, class CELL, class JUMP>
 __device__ __forceinline__ void update_cells(const Params& P, const IN& in, const OUT& out, int tx0,
-                                             int ty0, double T_do, int dt_only, const T* cell,
+                                             int ty0, double T_do, int dt_only, const CELL& cell,
                                              const JUMP& jump, const T* fx, const T* fy,
                                              MhdTileResult& res, double* aux) {
     const int N = P.N, M = P.M;
@@ -236,9 +238,6 @@ __device__ __forceinline__ void update_cells(const Params& P, const IN& in, cons
         const int ly = i / TX, lx = i - ly * TX;
         const int gx = tx0 + lx, gy = ty0 + ly;
         if (gx >= N || gy >= M) continue;
-        const T* c = cell + ly * RS + lx;
-        const T r = c[0], p = c[FS], u = c[2 * FS], v = c[3 * FS];
-        const T bx = c[4 * FS], by = c[5 * FS], bz = c[6 * FS];
         const long long k = (long long)gy * N + gx;
         if (P.frozen && !cell_active(P, gx, gy)) {  // the faces' own test
             if (!dt_only) copy_cell(in, out, k);
@@ -246,6 +245,9 @@ __device__ __forceinline__ void update_cells(const Params& P, const IN& in, cons
         }
         any_active = true;
         if (dt_only) continue;
+        T c[NF];
+        cell(lx, ly, gx, gy, c);
+        const T r = c[0], p = c[1], u = c[2], v = c[3], bx = c[4], by = c[5], bz = c[6];
         const T* fxc = fx + ly * (TX + 1) + lx;
         const T* fyc = fy + ly * TX + lx;
         T d[NF];
@@ -434,8 +436,12 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
     __syncthreads();
 
     const T* own = prim + H * SX + H;
-    update_cells<T, BT, TY, SX, SY * SX>(P, in, out, tx0, ty0, T_do, dt_only, own,
-                                     JumpFloat<T, SX, SY * SX>{own}, fx, fy, res, aux);
+    const auto cell = [&](int lx, int ly, int, int, T* v) {
+#pragma unroll
+        for (int f = 0; f < NF; ++f) v[f] = own[f * SY * SX + ly * SX + lx];
+    };
+    update_cells<T, BT, TY>(P, in, out, tx0, ty0, T_do, dt_only, cell,
+                            JumpFloat<T, SX, SY * SX>{own}, fx, fy, res, aux);
     res.umax_x = u.x;
     res.umax_y = u.y;
 }
@@ -454,7 +460,7 @@ struct MemInt {
     static_assert(sizeof(Key) == 2 * sizeof(double), "keys take two doubles a cell");
     Key* key;      // [SY][SX]
     fx::i64* q;    // [NF][SY][SX]
-    double* cell;  // [NF][TY][TX]
+    double* cell;  // [2][TY][TX]  b_x, b_y
     double* edgex;  // [2][TY]  b_x of the cells at x = -1 and TX
     double* edgey;  // [2][TX]  b_y of the cells at y = -1 and TY
     double *fx, *fy;
@@ -515,11 +521,11 @@ template <int TY>
 struct JumpCells {
     const double *cell, *edgex, *edgey;
     __device__ __forceinline__ double x(int lx, int ly) const {
-        const double* c = cell + 4 * TX * TY + ly * TX + lx;
+        const double* c = cell + ly * TX + lx;
         return (lx < TX - 1 ? c[1] : edgex[TY + ly]) - (lx > 0 ? c[-1] : edgex[ly]);
     }
     __device__ __forceinline__ double y(int lx, int ly) const {
-        const double* c = cell + 5 * TX * TY + ly * TX + lx;
+        const double* c = cell + TX * TY + ly * TX + lx;
         return (ly < TY - 1 ? c[TX] : edgey[TX + lx]) - (ly > 0 ? c[-TX] : edgey[lx]);
     }
 };
@@ -548,7 +554,7 @@ __device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, co
         fx::cell_units<NF>(v, t.q + i, FS, t.key[i]);
         if (!xh && !yh) {
 #pragma unroll
-            for (int f = 0; f < NF; ++f) t.cell[(f * TY + ly) * TX + lx] = v[f];
+            for (int f = 0; f < 2; ++f) t.cell[(f * TY + ly) * TX + lx] = v[4 + f];
         } else if (lx == -1 || lx == TX) {
             t.edgex[(lx == TX ? TY : 0) + ly] = v[4];
         } else if (ly == -1 || ly == TY) {
@@ -581,9 +587,9 @@ __device__ __forceinline__ void step_tile(const Params& P, const CPlanes& in, co
         __syncthreads();
     }
 
-    update_cells<double, NT, TY, TX, TX * TY>(P, in, out, tx0, ty0, T_do, dt_only, t.cell,
-                                          JumpCells<TY>{t.cell, t.edgex, t.edgey}, t.fx, t.fy,
-                                          res, aux);
+    const auto cell = [&](int, int, int gx, int gy, double* v) { load_cell(P, in, gx, gy, v); };
+    update_cells<double, NT, TY>(P, in, out, tx0, ty0, T_do, dt_only, cell,
+                                 JumpCells<TY>{t.cell, t.edgex, t.edgey}, t.fx, t.fy, res, aux);
     res.umax_x = u.x;
     res.umax_y = u.y;
 }
