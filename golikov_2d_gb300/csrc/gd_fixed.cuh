@@ -236,9 +236,6 @@ GD_HD uint32_t rotate(uint32_t x, int n) {  // by 0 or 16 bits
 // beside large ones, or a quiet cell in a tile with a shock, keeps its digits.
 constexpr int kSpan = 8;     // exponents that the face's densities, and the pressures, may span
 constexpr int kRange = 128;  // exponents of densities, pressures (both signs) and velocities
-// Below 2^-300 a velocity or field that is not 0 goes to the floating-point solver: with densities
-// and fan speeds down to 2^-128 every result stays above 2^-1022.
-constexpr int kLow = 300;
 constexpr uint32_t kNoKey = 0x7ff;  // key of a value that the integers do not take
 
 // {rho, p}, {vx, vy}, {bx, by}, {bz, 0}
@@ -285,7 +282,7 @@ GD_HD uint32_t cell_units(double x, i64& q) {
     const i64 m = (i64)(((u64)((h << 8) | (lo >> 24)) << 32) | (lo << 8));
     q = (int32_t)hi < 0 ? -m : m;
     if (POSITIVE) return (hi >> 20) - 1u < 0x7feu ? e : kNoKey;  // zeros and negatives out
-    return e >= 1023 - kLow || m == 0 ? e : kNoKey;
+    return e != 0 || m == 0 ? e : kNoKey;  // subnormal numbers out
 }
 template <int NF>
 GD_HD void cell_units(const double* v, i64* q, int fs, Keys<NF>& k) {
@@ -373,12 +370,21 @@ GD_HD bool face_states(const i64* q, int st, int fs, const Keys<NF>* key, int ks
     return true;
 }
 
-// x 2^ue as a double, a normal number (or 0): ue is added to the exponent field.  The same bits on
-// the host, so that what is checked there is what the kernels compute.
+// x 2^ue as a double, a normal number or 0: ue is added to the exponent field.  Densities, pressures
+// and fan speeds of the accepted range make normal numbers of every flux but those that a tangential
+// velocity or a field enters alone: for them the sign bit of `bad` is set where the result is no
+// normal number, and the face goes to the floating-point solver.
 GD_HD double to_double(i64 x, int ue) {
     uint32_t hi, lo;
+    swfp::halves((double)x, hi, lo);  // hi is 0 for x = 0 alone
+    return swfp::from_halves(hi + (hi == 0 ? 0u : (uint32_t)ue << 20), lo);
+}
+GD_HD double to_double(i64 x, int ue, uint32_t& bad) {
+    uint32_t hi, lo;
     swfp::halves((double)x, hi, lo);
-    return swfp::from_halves(x == 0 ? 0u : hi + ((uint32_t)ue << 20), lo);
+    const uint32_t r = hi + (hi == 0 ? 0u : (uint32_t)ue << 20);
+    bad |= (r - (hi == 0 ? 0u : 0x100000u)) ^ hi;
+    return swfp::from_halves(r, lo);
 }
 // E for which both x 2^(top - 61) and y 2^(top - 61) are below 2^(E - 1), from their leading words:
 // the least one, and at least top - 28
@@ -452,6 +458,7 @@ GD_HD Fan fan_of(const States& q, const Tops& X, const Gas& G, double& UU) {
 // so |S_M / (S - S_M)| <= 1: no product below overflows.
 GD_HD bool hllc(const Fan& f, const States& s, const Tops& X, const Gas& G, double& Fm,
                 double& Fn, double& Ft, double& Fe) {
+    uint32_t bad = 0;
     const int E = f.E, ER = imax(f.RL.e, f.RR.e);
     const i64 suL = f.SL - f.uL, suR = f.SR - f.uR;
     // r (S - u), each side in units of its own density's, 2^(e + E - 59), and in the larger's
@@ -500,7 +507,7 @@ GD_HD bool hllc(const Fan& f, const States& s, const Tops& X, const Gas& G, doub
     const i64 pt = (Pk.m >> imin(et - Pk.e + 62, 63)) + t;
     Fn = to_double(t == 0 ? Pk.m : pt, t == 0 ? Pk.e - 62 : et);
     const i64 MT = mulk<0, 0>(M, T.m);
-    Ft = to_double(MT, em + T.e + 2);
+    Ft = to_double(MT, em + T.e + 2, bad);
     // energy: q su (p gamma / (gamma - 1) + r (u^2 / 2 + S (S_M - u))) + (mass flux) v^2 / 2
     const i64 H = mulk<1, 1>(un, un) + mulk<2, 1>(S, SMu);
     const i64 B = sra(mulk<0, 0>(Pk.m, G.gg), R.e + 2 * E - Pk.e - G.gge + G.room) +
@@ -510,7 +517,7 @@ GD_HD bool hllc(const Fan& f, const States& s, const Tops& X, const Gas& G, doub
     const int dx = 2 * (E - T.e) + 1 + G.room;
     const int x1 = R.e + 3 * E - 57 - z + G.room;
     Fe = to_double(sra(e1, imax(-dx, 0)) + sra(e2, imax(dx, 0)), dx > 0 ? x1 : x1 - dx);
-    return true;
+    return (int32_t)bad >= 0;
 }
 
 // HLL flux of that face (kernel.cu:1485-1609) with fan_of<true>.  With the fan cut at the face,
@@ -520,6 +527,7 @@ GD_HD bool hllc(const Fan& f, const States& s, const Tops& X, const Gas& G, doub
 // with nothing to use, where the energy would not fit its unit.
 GD_HD bool hll(const Fan& f, const States& s, const Tops& X, const Gas& G, double& Fm, double& Fn,
                double& Ft, double& Fe) {
+    uint32_t bad = 0;
     const int E = f.E, ER = imax(f.RL.e, f.RR.e);
     const i64 DL = f.SL < 0 ? f.SL : 0, DR = f.SR > 0 ? f.SR : 0;
     int lz;
@@ -539,7 +547,7 @@ GD_HD bool hll(const Fan& f, const States& s, const Tops& X, const Gas& G, doubl
     const i64 pR = mulk<2, 2>(b, f.PR.m >> imin(sp + 2 - f.PR.e, 63));
     Fn = to_double(mulk<2, 2>(A, f.uL) + mulk<2, 2>(B, f.uR) + pL + pR, ER + 2 * E - 60);
     const i64 TL = mulk<2, 1>(A, s.vL), TR = mulk<2, 1>(B, s.vR);
-    Ft = to_double(TL + TR, ER + E + X.t - 59);
+    Ft = to_double(TL + TR, ER + E + X.t - 59, bad);
     // energy: p (u - D) / (gamma - 1) + p u + rho (u - D) (u^2 + v^2) / 2, units
     // 2^(ER + 3E - 62 + room)
     const i64 qL = mulk<2, 2>(a, sra(mulk<0, 0>(f.PL.m, G.gi), sp - f.PL.e - G.gie + G.room));
@@ -554,7 +562,7 @@ GD_HD bool hll(const Fan& f, const States& s, const Tops& X, const Gas& G, doubl
                   mulk<3, 2>(pL, f.uL) + mulk<3, 2>(pR, f.uR);
     Fe = to_double(shift(h, z - 4 + rr) + (sra(k, rr) + shift(t, st + rr) >> G.room),
                    ER + 3 * E - 62 + G.room + rr);
-    return true;
+    return (int32_t)bad >= 0;
 }
 
 // The flux (HLL or HLLC) and the larger wave speed of one face given by its two states, {rho, p,

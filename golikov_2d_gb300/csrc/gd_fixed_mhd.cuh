@@ -215,7 +215,7 @@ GD_HD bool scales(i64 x, int lz) { return x >> imin(65 - lz, 63) == 0; }
 
 template <bool HLLD>
 GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const TopsM& X, const Gas& G,
-                FluxI& F) {
+                    FluxI& F) {
     const int E = f.E, ER = f.ER, XB = 2 * X.b;
     const i64 suA = f.SL - f.uA, suB = f.SR - f.uB;
     const i64 mA = mulk<0, 0>(f.A.R.m, suA) >> (ER - f.A.R.e);
@@ -385,22 +385,23 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
         const i64 de = shift(mulk<1, 2>(mulk<2, 0>(sK, sb - sb3), S2), ER + E - kK - X.b - 2);
         e += flip ? de : -de;
     }
+    uint32_t bad = 0;
     F.mn = to_double(mn, ER + 2 * E - 59);
-    F.mt = to_double(mt, ER + 2 * E - 59 - f.tv);
+    F.mt = to_double(mt, ER + 2 * E - 59 - f.tv, bad);
     F.e = to_double(e, ER + 3 * E - 61);
-    F.bt = to_double(ft, E + X.b - 61 - f.tb);
-    F.bz = to_double(fz, E + X.b - 61 - f.z);
+    F.bt = to_double(ft, E + X.b - 61 - f.tb, bad);
+    F.bz = to_double(fz, E + X.b - 61 - f.z, bad);
     if (f.w != 0) {
         // what w multiplies in the energy flux: the momentum flux, but for guarded star states
         const i64 yt = (mulk<2, 1>(qsg, btK - K.bt) << 1) - K.bt;
         const i64 et = (mulk<1, 2>(M, ut) >> imin(z + dR, 63)) + dm +
                        shift(mulk<0, 0>(bn, yt) + mulk<0, 0>(bn - bnK, btK), st);
-        const double w = to_double(f.w, X.t - 61), et_d = to_double(et, ER + 2 * E - 59 - f.tv);
+        const double w = to_double(f.w, X.t - 61), et_d = to_double(et, ER + 2 * E - 59 - f.tv, bad);
         F.e = std::fma(w, std::fma(0.5 * w, F.m, et_d), F.e);
         F.mt = std::fma(w, F.m, F.mt);
-        F.bt = std::fma(-w, to_double(bnK, X.b - 61), F.bt);
+        F.bt = std::fma(-w, to_double(bnK, X.b - 61, bad), F.bt);
     }
-    return true;
+    return (int32_t)bad >= 0;
 }
 
 // The flux and the larger wave speed of a face from its states and their exponents (face_states);
@@ -410,15 +411,17 @@ GD_HD bool mhd_face_flux(const i64* p, const i64* q, const int* top, const Gas& 
                          double& UU, bool& speed, bool speed_only) {
     const int e4 = scale_of(p[4], q[4], top[4]), e5 = scale_of(p[5], q[5], top[5]);
     const int e6 = scale_of(p[6], q[6], top[6]);
-    const TopsM X{top[0], top[1], top[2], top[3], imax(imax(e4, e5), imax(e6, -kLow)), top[5], top[6]};
+    const TopsM X{top[0], top[1], top[2], top[3], imax(imax(e4, e5), e6), top[5], top[6]};
     StatesM a{p[0], p[1], p[2], p[3], asr(p[4], X.b - top[4]), p[5], p[6]};
     StatesM b{q[0], q[1], q[2], q[3], asr(q[4], X.b - top[4]), q[5], q[6]};
     const FanM f = fan_of(a, b, X, G, UU);
     speed = f.ok;
     if (!f.ok) return false;
     if (speed_only) return true;
-    // the normal field's flux in its own unit
-    F.bn = to_double(mulk<2, 0>(-f.SL > f.SR ? -f.SL : f.SR, p[4] - q[4]), f.E + top[4] - 60);
+    // the normal field's flux in its own unit, cut at 2^-1020
+    const int un = f.E + top[4] - 60, low = imax(-1020 - un, 0);
+    const i64 S = -f.SL > f.SR ? -f.SL : f.SR;
+    F.bn = to_double(asr(mulk<2, 0>(S, p[4] - q[4]), low), un + low);
     return mhd_flux<HLLD>(f, a, b, X, G, F);
 }
 // The two states {rho, p, un, ut, bn, bt, bz} of a face in units of their own; false where the

@@ -170,3 +170,26 @@ def test_recomputed_mhd_steps_keep_their_bits(cuda):
         sol.close()
     for x, y in zip(*grads):
         assert np.isfinite(x).all() and np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("solver", ["hlld", "hllc_mhd"])
+def test_tail_down_to_the_smallest_numbers(cuda, oracle_lib, solver):
+    """The front that numerical diffusion sends ahead of a wave: a z field and a transverse velocity
+    falling by 1000 per cell, past the smallest normal number.  Every cell to 1e-12 of the larger of
+    its neighbours."""
+    N, M = 130, 12
+    cfg = config(*METHODS[solver], N, M)
+    rng = np.random.default_rng(11)
+    K = N * M
+    tail = 10.0 ** (-3.0 * (np.arange(K) % N))  # 0 from 1e-324 on
+    s = np.stack([rng.uniform(1, 1.2, K), rng.uniform(1, 1.2, K)], 1)
+    u = np.stack([np.full(K, 0.3), np.zeros(K)], 1)
+    b = np.stack([np.zeros(K), np.zeros(K), tail * rng.uniform(0.5, 1, K)], 1)
+    T = 0.2 * cfg.dx / 4
+    _, _, bo, _ = oracle_lib.step(grid_of(cfg), s, u, b, T)
+    _, _, bg, _ = gpu_step_ref(cfg, s, u, b, T)
+    scale = np.maximum(np.roll(tail.reshape(M, N), 2, 1), tail.reshape(M, N)).ravel()
+    inner = (np.arange(K) % N >= 3) & (np.arange(K) % N < N - 3)
+    d = np.abs(bg[:, 2] - bo[:, 2])
+    assert (d <= 1e-12 * scale + 1e-307)[inner].all()
+    assert np.count_nonzero(bg[inner, 2]) > 0.7 * inner.sum()
