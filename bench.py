@@ -950,7 +950,7 @@ def workload_config(workload, cfg, ws):
 SHORT = {"roofline": ("bound", "frac"), "fp64": ("frac", "ops_per_cell"),
          "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"),
          "secondary": ("value", "ms_per_step", "unavailable"),
-         "batched": ("value", "ms_per_step", "unavailable"),
+         "batched": ("speedup", "speedup_vs_looped_sync", "unavailable"),
          "cpu_baseline": ("value", "cores", "kind")}
 DETAILS_ONLY = ("sim", "ot_to_t05", "adjoint", "io", "hancock")
 

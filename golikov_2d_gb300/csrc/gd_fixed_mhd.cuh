@@ -111,16 +111,21 @@ GD_HD bool star_of(i64 am, i64 ad, i64 as, i64 SMu, i64 bn, i64 bn2, int st, int
     const i64 it = rcp(at, lz);
     const i64 num = mulk<2, 1>(am, as) - bn2;
     const i64 x1 = shift(mulk<0, 0>(bn, bt), st), x2 = shift(mulk<0, 0>(bn, bz), sh);
-    if (!(iabs(num >> 1) < 2 * (at >> 1) && iabs(x1) < at && iabs(x2) < at)) return false;
-    const i64 k1 = mulk<0, 2>(x1 << (lz - 2), it), k2 = mulk<0, 2>(x2 << (lz - 2), it);
-    const i64 d = mulk<0, 2>((num >> 1) << (lz - 2), it);
-    const i64 dv = mulk<2, 1>(k1, SMu) << 1, dw = mulk<2, 1>(k2, SMu) << 1;
-    const i64 ct = mulk<2, 1>(d, bt) << 2, cz = mulk<2, 1>(d, bz) << 2;
+    // The ratios to at, up to 2^r: r > 0 towards the speeds where the Alfven and the fast wave meet.
+    // Beyond 4 the cancellation in at costs the ratios more digits than in binary64.
+    const i64 top = iabs(num >> 1) | iabs(x1) | iabs(x2);
+    const int r = imax(lz - clz32((uint32_t)hi32(top)) + 1, 0);
+    const i64 k1 = mulk<0, 2>((x1 >> r) << (lz - 2), it), k2 = mulk<0, 2>((x2 >> r) << (lz - 2), it);
+    const i64 d = mulk<0, 2>((num >> 1 >> r) << (lz - 2), it);
+    const i64 dv = mulk<2, 1>(k1, SMu), dw = mulk<2, 1>(k2, SMu);
+    const i64 ct = mulk<2, 1>(d, bt), cz = mulk<2, 1>(d, bz);
+    if (r > 2 || (r > 0 && !(fits(iabs(dv) | iabs(dw), -r - 1) && fits(iabs(ct) | iabs(cz), -r - 2))))
+        return false;
     const bool neg = tt < 0;
-    T.dv = neg ? dv : -dv;
-    T.dw = neg ? dw : -dw;
-    T.bt = neg ? -ct : ct;
-    T.bz = neg ? -cz : cz;
+    T.dv = (neg ? dv : -dv) << (1 + r);
+    T.dw = (neg ? dw : -dw) << (1 + r);
+    T.bt = (neg ? -ct : ct) << (2 + r);
+    T.bz = (neg ? -cz : cz) << (2 + r);
     return true;
 }
 
