@@ -46,13 +46,13 @@ namespace gd {
 namespace {
 
 constexpr int kNT = 256;  // threads of a tile: single-grid step
-// The tangent's 552 faces in two rounds: 20 tangent steps at 512^2 take 5.55 ms, 5.79 with 256
-// threads, 6.17 with 384.
+// The tangent's 552 faces in two rounds: 20 tangent steps at 512^2 take 4.73 ms, 4.95 with 256
+// threads, 5.30 with 384.
 constexpr int kNTTan = 288;
 // Threads of a tile of the 16x16 shape where every tile has an SM to itself (Params::few_tiles): the
 // step is then one tile's latency, and 576 threads take its 544 faces in one round instead of
-// three: 11.7 against 13.5 us at 64x48, 12.1 against 13.9 at 192x192 (144 tiles; 288 threads:
-// 12.8).  From two tiles per SM on (156 tiles: 18.9 against 16.4 us) the 256-thread tiles share
+// three: 11.4 against 13.9 us at 64x48, 12.1 against 14.3 at 192x192 (144 tiles).  From two
+// tiles on an SM (156 tiles: 19.0 against 16.1 us) the 256-thread tiles share
 // an SM better.  The threads of a tile change no result: faces and cells are independent.
 constexpr int kNTFew = 576;
 constexpr int NF = 4;
@@ -529,7 +529,9 @@ __device__ __noinline__ void euler_tile(const Params& P, const IN& in, const OUT
 // The cells of the tile and its halo are held as significands and exponents (gd_fixed.cuh); a face
 // shifts its stencil to units of its own.  Slopes, minmod and face states are then plain 64-bit
 // adds and selects, and the HLLC flux is fx::hllc: the FP64 pipe is left with the conversion of
-// the fluxes and the update (about 40 instructions a cell instead of 103).
+// the fluxes and the update (about 44 instructions a cell instead of 103).  Bound by the ALU (69 %),
+// FP64 (63 %) and the chains between (issue 63 %): one step at 4096^2 takes 1.86 ms, 3.86 in FP64, 1.70
+// with one set of units for the tile, which cut small components (see face_states).
 
 // One compiled body for every kernel, so that a face left to floating point has the same bits
 // whichever kernel solves it.
@@ -701,11 +703,11 @@ __device__ __forceinline__ void async_copy4(void* to, const void* from) {
 }
 __device__ __forceinline__ void async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// One pass of 128 grids: 6.54 ms with 192 threads per tile (80 registers, no spills); 6.80 ms with
-// 256 (64 registers: the descriptors and the prefetch on top of the step spill), 6.66 ms with
-// 160.  The single-grid step, which holds less, is the other way round (4.79 against 4.92 ms for
-// two steps at 4096^2).  Tiles of 512 cells, two per SM, have the registers at 256 threads.
-// METHODS 1: every grid's method is HLLC (6.54 against 6.59 ms with both solvers); 3: any.
+// One pass of 128 grids: 6.72 ms with 192 threads per tile (78 registers, no spills); 6.80 ms with
+// 256 (64 registers: the descriptors and the prefetch on top of the step spill), 6.73 ms with
+// 160.  Tiles of 512 cells, two per SM, have the registers at 256 threads.
+// METHODS 1: every grid's method is HLLC (0.8 % faster than with both solvers when the cells were in
+// units of the tile); 3: any.
 template <int METHODS, int ORDER, int TX, int TY>
 __global__ void __launch_bounds__(kNTBatch<TX, TY>, kCtas<TX, TY>) euler_batch_kernel(const BatchGrid* __restrict__ grids,
                                                          const int2* __restrict__ items,

@@ -23,9 +23,9 @@
 // write disjoint cells); the blocks of both share one ticket, and the last block of either to
 // finish performs the funk_time rotation.
 //
-// The tile kernel is bound by the FP64 pipe (73 % active): 307 FP64 operations per cell of the
+// The tile kernel is bound by the FP64 pipe (71 % active): 305 FP64 operations per cell of the
 // grid, most of them the predictor's; 671 with FP64 faces and a predictor in conserved
-// quantities.  One step at 3226 x 1792: 4.49 ms, 8.01 ms before.
+// quantities.  One step at 3226 x 1792: 4.55 ms, 8.01 ms before.
 //
 // Differences from the parity step are rounding only: contraction, reciprocals instead of
 // divisions, slopes minmod(a - b, b - c) instead of h minmod((a - b)/h, (b - c)/h), the

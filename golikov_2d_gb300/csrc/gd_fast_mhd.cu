@@ -3,7 +3,7 @@
 // update), and its forward-mode tangent.
 //
 // The step's slopes and faces run in scaled 64-bit integers (gd_fixed_mhd.cuh), as in
-// gd_fast_euler.cu: 91 FP64 operations per cell against 448.  A face whose states or fan leave the
+// gd_fast_euler.cu: 92 FP64 operations per cell against 448.  A face whose states or fan leave the
 // integers' range is solved in FP64 from the cells themselves.  The tangent's tile is floating
 // point throughout; it and the flux are templates on the scalar type, and `Dual` (gd_dual.cuh)
 // gives the tangent (JVP), with the dt held fixed and derivatives taken along the branches the
@@ -39,11 +39,11 @@ namespace {
 constexpr int TX = 32;
 constexpr int kNT = 384;  // threads of the step (see kTY)
 // Threads where every tile has an SM to itself (Params::few_tiles): the step is one tile's latency, and
-// 768 threads take its 747 faces in one round: 29.1 against 32.4 us at 64x48, 28.4 against 31.9 at
-// 320x165 (150 tiles).  At 160 tiles 50.0 against 47.0: there the 384-thread tiles stay.
+// 768 threads take its 747 faces in one round: 31.5 against 37.1 us at 64x48, 30.5 against 37.1 at
+// 320x165 (150 tiles).  At 160 tiles 53.8 against 51.5: there the 384-thread tiles stay.
 constexpr int kNTFew = 768;
-// The tangent's: one CTA per SM.  20 tangent steps at 512^2 take 18.4 ms with 256 threads, 17.8
-// with 288, 17.3 with 384, 17.9 with 576.
+// The tangent's: one CTA per SM.  20 tangent steps at 512^2 take 16.1 ms with 256 threads, 15.0
+// with 384, 15.3 with 576.
 constexpr int NTDual = 384;
 constexpr int NF = 7;  // rho, p, vx, vy, bx, by, bz
 
@@ -452,7 +452,8 @@ __device__ __noinline__ void mhd_tile(const Params& P, const IN& in, const OUT& 
 // partition each, they held the tile to 35 000 cycles per 32 cells.  Here the cells of the tile
 // and its halo are significands and exponents (gd_fixed.cuh), a face shifts its stencil to units of
 // its own, slopes and face states are adds and selects, and the flux is fx::mhd_flux.  The FP64 pipe
-// keeps the conversion of the fluxes and the update.
+// keeps the conversion of the fluxes and the update.  Bound by the latency of the integer chains (ALU
+// 50 %, issue 47 %, FP64 37 %).
 template <int ORDER, int TY>
 struct MemInt {
     using S = ShapeInt<ORDER, TY>;
@@ -627,11 +628,12 @@ __global__ void __launch_bounds__(NTDual) mhd_tangent_kernel(const __grid_consta
                               reinterpret_cast<Dual*>(smem), r, nullptr);
 }
 
-// 32 x 11 tiles of 384 threads, two CTAs (24 warps) per SM at 80 registers and 93 KB of shared
-// memory: the tile's 747 faces are two rounds of 384 threads (97 % of them busy), and the face code
-// (45 KB) is fetched by 12 warps together.  32 x 8 with 256 threads, three CTAs: 2.25 rounds, 27 %
-// of the instruction fetches missing; 1.82 against 1.66 ms per pass of 1024^2, 3.05 against 3.00
-// for the wind.
+// 32 x 11 tiles of 384 threads, two CTAs (24 warps) per SM at 80 registers (about 500 bytes of spills a
+// thread, which the L1 beside 88 KB of shared memory a tile mostly holds): the tile's 747 faces are
+// two rounds of 384 threads (97 % of them busy).  One pass of 1024^2 / the wind: 1.92 / 3.35 ms; 32 x 8
+// with 256 threads, three CTAs 2.10 / 3.42; 32 x 9 with 320 threads at 96 registers 2.04 / 3.45; 32 x 8
+// with 288 at 112 registers 2.24 / 3.66.  One HLLD step at 1024^2: 0.42 ms, 0.98 in FP64, 0.37 with one
+// set of units for the tile.
 constexpr int kTY = 11;
 constexpr int kTYDual = 8;
 

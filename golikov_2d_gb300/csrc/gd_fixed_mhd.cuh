@@ -13,7 +13,8 @@
 // and v*.b* of the HLL state of the fan, which the two sides' m and iS = 1 / (S_R - S_L) give:
 //   b_t* = [(S_R - u_R) b_t,R + v_R b_R - (L)] iS,  v* = [m_R v_R + b_R b_t,R - (L)] / (m_R - m_L).
 //
-// Units: velocities 2^(E - 61) as for HLLC; fields 2^(X.b - 61), below 2^60; rho v^2 quantities
+// Units: velocities 2^(E - 61) as for HLLC; fields 2^(X.b - 61), below 2^60 (tangential ones in units
+// of their own, see FanM); rho v^2 quantities
 // 2^(ER + 2E - 59) and 2^(ER + 2E - 60), ER the larger density's exponent.  Squares of the field
 // move to those by a shift: |b|^2 / 2 <= rho c_f^2 bounds them there.
 #pragma once

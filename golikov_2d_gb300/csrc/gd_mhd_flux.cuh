@@ -1,7 +1,7 @@
 // gd_mhd_flux.cuh -- the fast path's HLLD / HLLC-MHD flux in a face's local frame, field in
 // Heaviside-Lorentz units (b = B / sqrt(4 pi)), templated on the scalar type (double, or
 // Dual for the tangent).  Used by the fast MHD step (gd_fast_mhd.cu) and the fast
-// MUSCL-Hancock step (gd_fast_hancock.cu) for the tangent and for the faces and tiles that the
+// MUSCL-Hancock step (gd_fast_hancock.cu) for the tangent and for the faces that the
 // integer solvers (gd_fixed_mhd.cuh) leave.
 //
 // Reference semantics kept (Gas_Dinamic.cu:964-1510): wave speeds SL = min(u) - max(cf),

@@ -5,8 +5,8 @@
 // mostly idle in the step kernels.  mul_rn computes the binary64 product rounded to
 // nearest even -- the bits of the hardware multiply -- with 32-bit integer instructions, so
 // a kernel can move part of its multiplications off the FP64 pipe without changing a
-// result bit.  The FP64 tile bodies, the tangents and the adjoints use it; the integer tile
-// bodies (gd_fixed.cuh) have no binary64 products to move in their faces.
+// result bit.  The FP64 faces, the tangents and the adjoints use it; the integer faces
+// (gd_fixed.cuh) have no binary64 products to move.
 //
 //   dmul_fast: normal operands with a normal product (result exponent field in [1, 2045]
 //              before rounding) and zero operands with a finite partner: four 32x32->64
