@@ -1235,9 +1235,12 @@ def run_gb300(args):
             line["hancock"] = {"unavailable": str(e)}
     if not args.no_cpu_baseline and ws == 1:
         line["cpu_baseline"] = cpu_baseline(args.workload, cfg, s, u, b)
-    with open(args.details, "w") as f:
-        json.dump(line, f, indent=1)
-        f.write("\n")
+    try:
+        with open(args.details, "w") as f:
+            json.dump(line, f, indent=1)
+            f.write("\n")
+    except OSError as e:  # the printed line does not depend on it
+        print(f"bench.py: {args.details}: {e}", file=sys.stderr)
     print(json.dumps(headline(line)), flush=True)
     if ws > 1:
         torch.distributed.destroy_process_group()
