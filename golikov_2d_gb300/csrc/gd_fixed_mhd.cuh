@@ -25,10 +25,10 @@ namespace gd {
 namespace fx {
 
 // Exponents of a face's units: densities, pressures, velocities and fields are in units of
-// 2^(X - 61), below 2^62; b is the largest field's, with the normal field in units of 2^(X.b - 61),
-// below 2^60.
+// 2^(X - 61), below 2^62; b is the largest field's, and the normal field is below 2^60 in units of
+// 2^(X.bn - 61).
 struct TopsM {
-    int r, p, n, t, b, bt, bz;
+    int r, p, n, t, b, bn, bt, bz;
 };
 struct StatesM {
     i64 r, p, un, ut, bn, bt, bz;
@@ -148,9 +148,11 @@ GD_HD i64 root_of(Pos R, int& k, i64& rs) {
 // Tangential components may be far below the normal ones and are carried by them, so they have
 // units of their own: tangential velocities 2^(E - 61 - tv), tangential fields 2^(X.b - 61 - tb),
 // and the z field and velocity 2^(X.b - 61 - z) and 2^(E - 61 - z).  Every flux is linear in each
-// pair, or has products of two of it, which shift back.  Where a normal field couples velocity and
-// field, both units follow the larger of v and b / sqrt(rho), 2^(-sh/2) of the speed per unit of the
-// field.  kRoom bits are left above the components, for star states above them.
+// pair, or has products of two of it, which shift back.  A normal field couples velocity and field:
+// both units then follow the larger of v and b / sqrt(rho), 2^(-sh/2) of the speed per unit of the
+// field, up to the bits by which the normal field's own speed is below the fan's (what v adds to the
+// field's flux, and b to the momentum's, is that much less).  kRoom bits are left above the
+// components, for star states above them.
 //
 // A flow along the face far faster than its waves would set the unit of all speeds and cost the fan
 // its digits.  The fluxes follow a change of frame exactly, so the face is solved in a frame that
@@ -160,15 +162,16 @@ constexpr int kRoom = 3;
 struct FanM {
     SideM A, B;
     i64 uA, uB, vA, vB, SL, SR, w;
-    int E, ER, kmin, tv, tb, z;
+    int E, ER, kmin, tv, tb, z, nb;
     int sh;  // what brings products of two fields to units of 2^(ER + 2E - 59)
     bool ok;
 };
 GD_HD FanM fan_of(StatesM& a, StatesM& b, const TopsM& X, const Gas& G, double& UU) {
     FanM f;
     const int bt = X.b - X.bt, bz = X.b - X.bz;
-    f.A = side_of(StatesM{a.r, a.p, a.un, a.ut, a.bn, asr(a.bt, bt), asr(a.bz, bz)}, X, G);
-    f.B = side_of(StatesM{b.r, b.p, b.un, b.ut, b.bn, asr(b.bt, bt), asr(b.bz, bz)}, X, G);
+    f.nb = X.b - X.bn;
+    f.A = side_of(StatesM{a.r, a.p, a.un, a.ut, asr(a.bn, f.nb), asr(a.bt, bt), asr(a.bz, bz)}, X, G);
+    f.B = side_of(StatesM{b.r, b.p, b.un, b.ut, asr(b.bn, f.nb), asr(b.bt, bt), asr(b.bz, bz)}, X, G);
     const int kmax = imax(f.A.k, f.B.k);
     f.kmin = imin(f.A.k, f.B.k);
     f.ER = imax(f.A.R.e, f.B.R.e);
@@ -195,8 +198,9 @@ GD_HD FanM fan_of(StatesM& a, StatesM& b, const TopsM& X, const Gas& G, double& 
     f.sh = f.ER + 2 * f.E - 1 - 2 * X.b;
     if ((a.bn | b.bn) != 0) {
         const int h = imax(f.sh, 0) >> 1, tv = f.tv;
-        f.tv = imin(tv, f.tb + h);
-        f.tb = imin(f.tb, imax(tv - h, 0));
+        const int k = imax(h + f.nb - 2, 0);
+        f.tv = imin(tv, f.tb + h + k);
+        f.tb = imin(imin(f.tb, imax(tv - h, 0) + k), f.tv + f.nb);
     }
     f.vA = shift(a.ut, f.E - X.t - f.tv);
     f.vB = shift(b.ut, f.E - X.t - f.tv);
@@ -250,10 +254,12 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const i64 m = takeL ? mA : mB, ptK = (takeL ? ptA : ptB) >> 1;
     const i64 S = takeL ? f.SL : f.SR, su = takeL ? suA : suB;
 
-    const int sh = f.sh, dt = f.tv - f.tb, st = sh - dt;  // st: of a tangential one, to momenta
+    // of products of the normal field with itself, the z field and a tangential one, to momenta; and
+    // with a tangential velocity, to the tangential field's flux
+    const int nb = f.nb, sn = f.sh + nb, st = sn - (f.tv - f.tb), dn = f.tv - f.tb + nb;
     const int vb = f.tv + f.tb;
     // units 2^(E + X.b - 61)
-    const i64 ub = mulk<2, 1>(un, bnK) + asr(mulk<2, 1>(ut, btK), vb);
+    const i64 ub = asr(mulk<2, 1>(un, bnK), nb) + asr(mulk<2, 1>(ut, btK), vb);
     i64 qs = un, qsg = 0, sb = ub, S2 = 0;
     StarM K{0, 0, btK, bzK};
     Pos RK = R;
@@ -271,16 +277,16 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
         qs = mulk<2, 1>(qsg, su) << 1;
         if constexpr (HLLD) {
             am = iabs(m);
-            bn2 = shift(mulk<0, 0>(bn, bn), sh);
+            bn2 = shift(mulk<0, 0>(bn, bn), sn + nb);
             thr = threshold(0x53e2d6238da3c211LL, -17, ER + 2 * E - 59);  // 1e-5
-            if (!star_of(am, ad, iabs(su), SM - un, bn, bn2, st, sh, thr, btK, bzK, K)) return false;
+            if (!star_of(am, ad, iabs(su), SM - un, bn, bn2, st, sn, thr, btK, bzK, K)) return false;
             RK = star_density(am, iA, lza, ER);
             i64 rs;
             sK = root_of<true>(RK, kK, rs);
             const i64 abn = iabs(bn);
             // |b| / sqrt(rho*), where |b| > 1e-6 (Gas_Dinamic.cu:1352-1369)
-            const i64 va = abn > threshold(0x431bde82d7b634daLL, -20, X.b - 61)
-                               ? shift(mulk<1, 2>(abn, rs), kK + E - 1 - X.b) : 0;
+            const i64 va = abn > threshold(0x431bde82d7b634daLL, -20, X.bn - 61)
+                               ? shift(mulk<1, 2>(abn, rs), kK + E - 1 - X.bn) : 0;
             S2 = takeL ? SM - va : SM + va;
             alfven = takeL ? S2 < 0 : S2 > 0;
         } else {
@@ -290,13 +296,13 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
             const i64 zA = mulk<0, 0>(a.bn, a.bz), zB = mulk<0, 0>(b.bn, b.bz);
             const i64 N1 = N + (shift(nB - nA, sq) << 1);
             const i64 N2 = mulk<1, 3>(mB, f.vB) - mulk<1, 3>(mA, f.vA) + (shift(tB - tA, st) << 1);
-            const i64 N3 = shift(zB - zA, sq) << 1;
+            const i64 N3 = shift(zB - zA, sn) << 1;
             i64 Tt = mulk<1, 2>(suB, b.bt) - mulk<1, 2>(suA, a.bt) +
-                           asr(mulk<2, 1>(f.vB, b.bn) - mulk<2, 1>(f.vA, a.bn), dt);
+                     asr(mulk<2, 1>(f.vB, b.bn) - mulk<2, 1>(f.vA, a.bn), dn);
             const i64 Tz = mulk<1, 2>(suB, b.bz) - mulk<1, 2>(suA, a.bz);
             if (f.w != 0) {  // the one term that a jump of the normal field keeps out of the frame
                 const i64 wb = mulk<1, 1>(f.w, b.bn - a.bn);
-                const int sw = E - f.tb - X.t - 1;
+                const int sw = E - f.tb - X.t - 1 + nb;
                 if (!fits(iabs(wb), sw)) return false;
                 Tt += shift(wb, sw);
             }
@@ -310,7 +316,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
             K.dv = vs - ut;
             if (!(below61(u1) && below61(ws) && below61(vs) && below61(K.bt) && below61(K.bz)))
                 return false;
-            sb = mulk<2, 1>(u1, bn) + asr(mulk<2, 1>(vs, K.bt), vb) +
+            sb = asr(mulk<2, 1>(u1, bn), nb) + asr(mulk<2, 1>(vs, K.bt), vb) +
                  asr(mulk<2, 1>(ws, K.bz), 2 * f.z);
         }
     } else {  // the physical flux of K: no mean of both sides in it
@@ -320,7 +326,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const i64 SMu = SM - un, vK = ut + K.dv;
     if (!(below61(vK) && below61(K.dw) && below61(K.bt) && below61(K.bz))) return false;
     if (HLLD && star)
-        sb = mulk<2, 1>(SM, bn) + asr(mulk<2, 1>(vK, K.bt), vb) +
+        sb = asr(mulk<2, 1>(SM, bn), nb) + asr(mulk<2, 1>(vK, K.bt), vb) +
              asr(mulk<2, 1>(K.dw, K.bz), 2 * f.z);
 
     const int32_t qh = hi32(qs);
@@ -330,10 +336,10 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const int em = R.e + E - 59 - z;
     F.m = to_double(M, em);
     const int dR = ER - R.e;
-    const i64 n2s = shift(n2K, sh), bnt = shift(mulk<0, 0>(bnK, btK), st);
+    const i64 n2s = shift(n2K, sq), bnt = shift(mulk<0, 0>(bnK, btK), st);
     const i64 mn = ptK + (mulk<1, 2>(M, SM) >> imin(z + dR, 63)) + mulk<2, 1>(m, SMu) - n2s;
     i64 mt = (mulk<1, 2>(M, vK) >> imin(z + dR, 63)) + mulk<2, 1>(m, K.dv) - bnt;
-    i64 ft = mulk<2, 1>(S, K.bt) - mulk<1, 2>(su, btK) - asr(mulk<2, 1>(ut, bnK), dt);
+    i64 ft = mulk<2, 1>(S, K.bt) - mulk<1, 2>(su, btK) - asr(mulk<2, 1>(ut, bnK), dn);
     i64 fz = mulk<2, 1>(S, K.bz) - mulk<1, 2>(su, bzK);
     const i64 H = mulk<1, 1>(un, un) + asr(mulk<1, 1>(ut, ut), 2 * f.tv) + mulk<2, 1>(S, SMu);
     const i64 B = sra(mulk<0, 0>(Pk.m, G.gg), ER + 2 * E - Pk.e - G.gge + G.room) +
@@ -343,7 +349,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const i64 e0 = mulk<0, 2>(qn, B);
     if (!(below61(B) && fits(iabs(e0), z - 2 - G.room))) return false;
     i64 e = shift(e0, z - 2 - G.room) +
-            shift(mulk<2, 0>(bn, y) + mulk<2, 0>(bn - bnK, ub), ER + 2 * E - 1 - XB);
+            shift(mulk<2, 0>(bn, y) + mulk<2, 0>(bn - bnK, ub), sn);
 
     i64 dm = 0;
     if (HLLD && alfven) {
@@ -355,7 +361,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
         const i64 adO = takeL ? f.SR - SM : SM - f.SL;
         if (hi32(adO) <= 0) return false;
         StarM O;
-        if (!star_of(amO, adO, asO, SM - unO, bn, bn2, st, sh, thr, btO, bzO, O)) return false;
+        if (!star_of(amO, adO, asO, SM - unO, bn, bn2, st, sn, thr, btO, bzO, O)) return false;
         const i64 vO = utO + O.dv;
         if (!(below61(vO) && below61(O.dw) && below61(O.bt) && below61(O.bz))) return false;
         int lzO, kO, lzt;
@@ -368,21 +374,24 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
         const i64 w = mulk<0, 2>(aK << (lzt - 2), iT);
         const bool flip = takeL != (bn > 0);  // sign of b times that of O - K in R - L
         const int sv = E + kk + 3 - lzt - X.b;
-        const i64 xt = shift(mulk<1, 2>(O.bt - K.bt, iT), sv - dt);
+        const i64 xt0 = mulk<1, 2>(O.bt - K.bt, iT);
+        const int dt = f.tv - f.tb;
         const i64 xz = shift(mulk<1, 2>(O.bz - K.bz, iT), sv);
+        // root(rho) times the jump of v may be far above a weak field, and the other way round
+        if (!fits(iabs(xt0), sv - dt)) return false;
+        const i64 xt = shift(xt0, sv - dt);
         const i64 v3 = vO + (mulk<2, 1>(w, vK - vO) << 1) + (flip ? -xt : xt);
         const i64 w3 = O.dw + (mulk<2, 1>(w, K.dw - O.dw) << 1) + (flip ? -xz : xz);
         const i64 wo = mulk<2, 2>(w, aO);
         const int sc = X.b - kk - E - 1;
         const i64 ct = mulk<2, 1>(wo, vO - vK), cz = mulk<2, 1>(wo, O.dw - K.dw);
-        // root(rho) times the jump of v may be far above a weak field
         if (!(fits(iabs(ct), sc + dt) && fits(iabs(cz), sc))) return false;
         const i64 yt = shift(ct, sc + dt), yz = shift(cz, sc);
         const i64 bt3 = K.bt + (mulk<2, 1>(w, O.bt - K.bt) << 1) + (flip ? -yt : yt);
         const i64 bz3 = K.bz + (mulk<2, 1>(w, O.bz - K.bz) << 1) + (flip ? -yz : yz);
         if (!(below61(v3) && below61(w3) && below61(bt3) && below61(bz3) && below61(S2)))
             return false;
-        const i64 sb3 = mulk<2, 1>(SM, bn) + asr(mulk<2, 1>(v3, bt3), vb) +
+        const i64 sb3 = asr(mulk<2, 1>(SM, bn), nb) + asr(mulk<2, 1>(v3, bt3), vb) +
                         asr(mulk<2, 1>(w3, bz3), 2 * f.z);
         dm = shift(mulk<2, 1>(mulk<0, 0>(RK.m, S2), v3 - vK), ER - RK.e);
         mt += dm;
@@ -405,7 +414,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
         const double w = to_double(f.w, X.t - 61), et_d = to_double(et, ER + 2 * E - 59 - f.tv, bad);
         F.e = std::fma(w, std::fma(0.5 * w, F.m, et_d), F.e);
         F.mt = std::fma(w, F.m, F.mt);
-        F.bt = std::fma(-w, to_double(bnK, X.b - 61, bad), F.bt);
+        F.bt = std::fma(-w, to_double(bnK, X.bn - 61, bad), F.bt);
     }
     return (int32_t)bad >= 0;
 }
@@ -417,9 +426,9 @@ GD_HD bool mhd_face_flux(const i64* p, const i64* q, const int* top, const Gas& 
                          double& UU, bool& speed, bool speed_only) {
     const int e4 = scale_of(p[4], q[4], top[4]), e5 = scale_of(p[5], q[5], top[5]);
     const int e6 = scale_of(p[6], q[6], top[6]);
-    const TopsM X{top[0], top[1], top[2], top[3], imax(imax(e4, e5), e6), top[5], top[6]};
-    StatesM a{p[0], p[1], p[2], p[3], asr(p[4], X.b - top[4]), p[5], p[6]};
-    StatesM b{q[0], q[1], q[2], q[3], asr(q[4], X.b - top[4]), q[5], q[6]};
+    const TopsM X{top[0], top[1], top[2], top[3], imax(imax(e4, e5), e6), e4, top[5], top[6]};
+    StatesM a{p[0], p[1], p[2], p[3], asr(p[4], e4 - top[4]), p[5], p[6]};
+    StatesM b{q[0], q[1], q[2], q[3], asr(q[4], e4 - top[4]), q[5], q[6]};
     const FanM f = fan_of(a, b, X, G, UU);
     speed = f.ok;
     if (!f.ok) return false;

@@ -1,10 +1,11 @@
-// Host check that the integer face solvers keep small transverse components: an out-of-plane field,
-// a transverse velocity and field together, or a transverse velocity alone (fluid solvers, and no
-// normal field), 2^-k times the normal ones.  Usage: fixed_components_check <faces per class>.  One
+// Host check that the integer face solvers keep small components: an out-of-plane field, a
+// transverse velocity and field together, or a transverse velocity alone (fluid solvers, and no
+// normal field), 2^-k times the normal ones; a weak normal field, alone or with the transverse one (the
+// field of the plane beside a strong field out of it).  Usage: fixed_components_check <faces per class>.  One
 // line per solver, class and k: the faces taken and left, and the largest error of the transverse
 // momentum over density x fan speed x the transverse speed v (v plus b / sqrt(density) of the
-// transverse field b where a normal field couples the two), of the transverse field over fan speed
-// x b (or b + sqrt(density) v), of the z field over fan speed x field and of the normal field over
+// transverse field b where a normal field couples the two, times its 2^-k), of the transverse field over
+// fan speed x b (or b + sqrt(density) v, as above), of the z field over fan speed x field and of the normal field over
 // fan speed x normal field.
 #define main ordinary_faces
 #include "fixed_check.cpp"
@@ -16,10 +17,12 @@ int main(int argc, char** argv) {
     auto U = [&](double a, double b) { return a + (b - a) * (double)(R() >> 11) * 0x1p-53; };
     const char* solver[] = {"hllc", "hll", "hlld", "hllc_mhd"};
     // which components are small: transverse velocity, transverse field, z field, normal field
-    struct { const char* name; bool v, t, z, nofield; double mach; } cls[] = {
-        {"z_field", false, false, true, false, 0.5},     {"z_field_fast", false, false, true, false, 3},
-        {"transverse", true, true, false, false, 0.5},   {"transverse_fast", true, true, false, false, 3},
-        {"all", true, true, true, false, 0.5},           {"velocity_across", true, false, false, true, 0.5}};
+    struct { const char* name; bool v, t, z, n, nofield; double mach; } cls[] = {
+        {"z_field", 0, 0, 1, 0, 0, 0.5},    {"z_field_fast", 0, 0, 1, 0, 0, 3},
+        {"transverse", 1, 1, 0, 0, 0, 0.5}, {"transverse_fast", 1, 1, 0, 0, 0, 3},
+        {"all", 1, 1, 1, 0, 0, 0.5},        {"velocity_across", 1, 0, 0, 0, 1, 0.5},
+        {"normal", 0, 0, 0, 1, 0, 0.5},     {"in_plane", 0, 1, 0, 1, 0, 0.5},
+        {"in_plane_fast", 0, 1, 0, 1, 0, 3}};
     for (int m = 0; m < 4; ++m)
         for (const auto& c : cls)
             for (int k : {0, 7, 14, 27, 40, 100}) {
@@ -37,7 +40,7 @@ int main(int argc, char** argv) {
                         x[1] = U(0.5, 0.8);
                         x[2] = u + 0.3 * U(-1, 1);
                         x[3] = (c.v ? w : 1) * U(-1, 1);
-                        x[4] = c.nofield ? 0 : 0.7 * U(-1, 1);
+                        x[4] = c.nofield ? 0 : (c.n ? w : 1) * 0.7 * U(-1, 1);
                         x[5] = (c.t ? w : 1) * U(-1, 1);
                         x[6] = (c.z ? w : 1) * U(-1, 1);
                     }
@@ -64,7 +67,7 @@ int main(int argc, char** argv) {
                     const L bn = mhd ? fmax(fabs(q[4]), fabs(q[11])) : 0;
                     const L bt = mhd ? fmax(fabs(q[5]), fabs(q[12])) : 0;
                     const L bz = mhd ? fmax(fabs(q[6]), fabs(q[13])) : 0;
-                    const L w1 = bn > 0 ? 1 : 0, root = sqrtl(r);
+                    const L w1 = bn > 0 ? (c.n ? w : 1) : 0, root = sqrtl(r);
                     const L sc[8] = {r * S, r * S * S, r * S * (vt + w1 * bt / root), r * S * S * S,
                                      S * bn, S * (bt + w1 * root * vt), S * bz, S};
                     for (int i = 0; i < 8; ++i) {
