@@ -223,6 +223,12 @@ GD_HD i64 threshold(i64 m, int e, int u) {
 // x << (lz - 2) fits, x >= 0
 GD_HD bool scales(i64 x, int lz) { return x >> imin(65 - lz, 63) == 0; }
 
+// At a mirror the contact stands on the face, and the flux may jump from one side's to the other's;
+// binary64 finds S_M = 0 there exactly and takes the side below.  Products here round down, so that
+// S_M's numerator comes out as 0 to some units (2^(ER + 2E - 60)); up to kTie, 2^-54 of rho c^2 and
+// the size of binary64's own roundings, it counts as 0.
+constexpr i64 kTie = 32;
+
 template <bool HLLD>
 GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const TopsM& X, const Gas& G,
                     FluxI& F) {
@@ -234,7 +240,8 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const int sp = ER + 2 * E + 2, sq = f.sh;
     const i64 ptA = (f.A.P.m >> imin(sp - f.A.P.e, 63)) + shift(f.A.bb, sq);
     const i64 ptB = (f.B.P.m >> imin(sp - f.B.P.e, 63)) + shift(f.B.bb, sq);
-    const i64 N = mulk<1, 3>(mB, f.uB) - mulk<1, 3>(mA, f.uA) + (ptA - ptB);
+    const i64 N0 = mulk<1, 3>(mB, f.uB) - mulk<1, 3>(mA, f.uA) + (ptA - ptB);
+    const i64 N = (u64)(N0 + kTie) <= 2 * kTie ? 0 : N0;
     int lz;
     const i64 iD = rcp(mB - mA, lz);
     i64 SM = mulk<0, 2>(N << (lz - 2), iD);
