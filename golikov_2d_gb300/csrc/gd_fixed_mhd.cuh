@@ -225,8 +225,9 @@ GD_HD bool scales(i64 x, int lz) { return x >> imin(65 - lz, 63) == 0; }
 
 // At a mirror the contact stands on the face, and the flux may jump from one side's to the other's;
 // binary64 finds S_M = 0 there exactly and takes the side below.  Products here round down, so that
-// S_M's numerator comes out as 0 to some units (2^(ER + 2E - 60)); up to kTie, 2^-54 of rho c^2 and
-// the size of binary64's own roundings, it counts as 0.
+// S_M's numerator comes out as 0 to some units (2^(ER + 2E - 60)): the side below is taken down to
+// -kTie, 2^-54 of rho c^2 and the size of binary64's own roundings.  (Setting such a numerator to 0
+// says the same and took 1.95 ms for four steps of 1024^2 where this takes 1.89.)
 constexpr i64 kTie = 32;
 
 template <bool HLLD>
@@ -240,8 +241,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const int sp = ER + 2 * E + 2, sq = f.sh;
     const i64 ptA = (f.A.P.m >> imin(sp - f.A.P.e, 63)) + shift(f.A.bb, sq);
     const i64 ptB = (f.B.P.m >> imin(sp - f.B.P.e, 63)) + shift(f.B.bb, sq);
-    const i64 N0 = mulk<1, 3>(mB, f.uB) - mulk<1, 3>(mA, f.uA) + (ptA - ptB);
-    const i64 N = (u64)(N0 + kTie) <= 2 * kTie ? 0 : N0;
+    const i64 N = mulk<1, 3>(mB, f.uB) - mulk<1, 3>(mA, f.uA) + (ptA - ptB);
     int lz;
     const i64 iD = rcp(mB - mA, lz);
     i64 SM = mulk<0, 2>(N << (lz - 2), iD);
@@ -251,7 +251,7 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
     const i64 bs = mulk<2, 1>(f.SR, b.bn) - mulk<2, 1>(f.SL, a.bn);
     i64 bn = mulk<0, 2>(bs << (lzs - 2), iS) << 1;
 
-    const bool takeL = f.SL >= 0 || N >= 0;
+    const bool takeL = f.SL >= 0 || N >= -kTie;
     const bool star = takeL ? f.SL < 0 : f.SR > 0;
     const Pos R{takeL ? f.A.R.m : f.B.R.m, takeL ? f.A.R.e : f.B.R.e};
     const Pos Pk{takeL ? f.A.P.m : f.B.P.m, takeL ? f.A.P.e : f.B.P.e};
@@ -292,10 +292,10 @@ GD_HD bool mhd_flux(const FanM& f, const StatesM& a, const StatesM& b, const Top
             sK = root_of<true>(RK, kK, rs);
             const i64 abn = iabs(bn);
             // |b| / sqrt(rho*), where |b| > 1e-6 (Gas_Dinamic.cu:1352-1369)
-            const i64 va = abn > threshold(0x431bde82d7b634daLL, -20, X.bn - 61)
-                               ? shift(mulk<1, 2>(abn, rs), kK + E - 1 - X.bn) : 0;
+            const bool va0 = abn <= threshold(0x431bde82d7b634daLL, -20, X.bn - 61);
+            const i64 va = va0 ? 0 : shift(mulk<1, 2>(abn, rs), kK + E - 1 - X.bn);
             S2 = takeL ? SM - va : SM + va;
-            alfven = takeL ? S2 < 0 : S2 > 0;
+            alfven = !va0 && (takeL ? S2 < 0 : S2 > 0);
         } else {
             // the fan's HLL state: v*, b*, and v*.b* with its own u and w
             const i64 nA = f.A.n2, nB = f.B.n2;  // b_n^2

@@ -28,6 +28,7 @@ int main(int argc, char** argv) {
                 q[2] = v * U(-1, 1);
                 q[3] = v * U(-1, 1);
                 for (int k = 4; k < 7; ++k) q[k] = v * U(-1, 1);
+                if (it % 5 == 0) q[4 + it / 5 % 3] = 0;
                 const double s[7] = {1, 1, -1, 1, c.n, c.t, c.z};
                 for (int k = 0; k < 7; ++k) q[7 + k] = s[k] * q[k];
                 const fx::Gas G = fx::gas_of(g);
