@@ -630,9 +630,9 @@ __global__ void __launch_bounds__(NTDual) mhd_tangent_kernel(const __grid_consta
 
 // 32 x 11 tiles of 384 threads, two CTAs (24 warps) per SM at 80 registers (about 500 bytes of spills a
 // thread, which the L1 beside 88 KB of shared memory a tile mostly holds): the tile's 747 faces are
-// two rounds of 384 threads (97 % of them busy).  One pass of 1024^2 / the wind: 1.92 / 3.35 ms; 32 x 8
-// with 256 threads, three CTAs 2.10 / 3.42; 32 x 9 with 320 threads at 96 registers 2.04 / 3.45; 32 x 8
-// with 288 at 112 registers 2.24 / 3.66.  One HLLD step at 1024^2: 0.42 ms, 0.98 in FP64, 0.37 with one
+// two rounds of 384 threads (97 % of them busy).  Four steps of 1024^2 / one of the wind: 1.89 / 3.30 ms;
+// 32 x 8 with 256 threads, three CTAs 2.10 / 3.42; 32 x 9 with 320 threads at 96 registers 2.04 / 3.45;
+// 32 x 8 with 288 at 112 registers 2.24 / 3.66 (those where this took 1.92 / 3.35).  One HLLD step at 1024^2: 0.42 ms, 0.98 in FP64, 0.37 with one
 // set of units for the tile.
 constexpr int kTY = 11;
 constexpr int kTYDual = 8;
